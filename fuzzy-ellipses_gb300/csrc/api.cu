@@ -717,8 +717,19 @@ int fe_render_pixels(const fe_pixlist_desc* d_in, const float* means, const floa
   Arena* a = nullptr;
   int rc = arena_for(st, &a);
   if (rc) return rc;
-  rc = a->rec.reserve(std::max<size_t>(pixlist_scratch_bytes(d->n_gaussians, d->n_poses), 256),
-                      st);
+  // Ordering a long list needs scratch by its length. A stream under capture cannot grow the
+  // arena: there a list longer than the arena was warmed up for is rendered in its own order.
+  int64_t ordered = pixlist_ordered_rays(d->n_gaussians, d->n_rays, weights != nullptr);
+  size_t bytes = pixlist_scratch_bytes(d->n_gaussians, d->n_poses, ordered);
+  if (ordered > 0 && bytes > a->rec.cap) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      (void)cudaGetLastError();
+      ordered = 0;
+      bytes = pixlist_scratch_bytes(d->n_gaussians, d->n_poses, 0);
+    }
+  }
+  rc = a->rec.reserve(std::max<size_t>(bytes, 256), st);
   if (rc) return rc;
   PixRayModel rm;
   rm.inv_f = d->inv_f;
@@ -729,7 +740,7 @@ int fe_render_pixels(const fe_pixlist_desc* d_in, const float* means, const floa
   launch_render_pixels(d->n_gaussians, cam ? 1 : d->n_poses, means, prec, logw, poses, d->n_rays,
                        rays, rm, d->beta2, d->beta3, d->cull_mode, d->cull_param, features,
                        d->n_features, depth, alpha, flow_next, flow_prev, out_features, weights,
-                       a->rec.ptr, st);
+                       ordered, a->rec.ptr, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }

@@ -135,7 +135,8 @@ void launch_transform_points_bwd(int64_t n, const float* points, const float* po
 
 // pixlist.cu
 // Pixel-list render (fm_render.py render_func_idx_quattrans[_flow], render_func_quat_cam);
-// scratch: pixlist_scratch_bytes(n, n_poses). feats (n x nf, nf <= 16), flows, out_feats and
+// scratch: pixlist_scratch_bytes(n, n_poses, ordered_rays); ordered_rays > 0 (at most n_rays, from
+// pixlist_ordered_rays) renders the rays bucketed by pose and cell, 0 in the order given. feats (n x nf, nf <= 16), flows, out_feats and
 // weights (n x n_rays) are optional (NULL).
 // Ray model: rows of `stride` floats (x, y, c[, pose]); the camera ray is
 // ((x - shift_x) inv_f, (y - shift_y) aspect inv_f, c) of pose `pose` (stride 4) or pose 0.
@@ -143,14 +144,16 @@ struct PixRayModel {
   float inv_f, aspect, shift_x, shift_y;
   int stride;
 };
-size_t pixlist_scratch_bytes(int n, int n_poses);
+size_t pixlist_scratch_bytes(int n, int n_poses, int64_t ordered_rays);
+// n_rays when bucketing pays (long lists; dense weights are written along the given order), else 0.
+int64_t pixlist_ordered_rays(int n, int64_t n_rays, bool weights);
 void launch_render_pixels(int n, int n_poses, const float* means, const float* prec,
                           const float* logw, const float* poses, int64_t n_rays, const float* rays,
                           const PixRayModel& rm, float beta2, float beta3, int cull_mode,
                           float cull_param,
                           const float* feats, int nf, float* depth, float* alpha,
                           float* flow_next, float* flow_prev, float* out_feats, float* weights,
-                          void* scratch, cudaStream_t st);
+                          int64_t ordered_rays, void* scratch, cudaStream_t st);
 
 // features.cu
 // Softmax-weighted features (nf per Gaussian) of an image render from the forward's statistics.

@@ -443,8 +443,10 @@ int fe_gmm_log_likelihood(const float *d_means, const float *d_prec, const float
  * outputs per ray: d_depth, d_alpha; optional (NULL to skip): d_flow_next / d_flow_prev
  * (n_rays, 2) the flow to poses pose+1 / pose-1 (clamped), d_out_features (n_rays, n_features)
  * the softmax-weighted features, d_weights (n, n_rays) the dense softmax weights (fm_render's w).
- * Gaussians are culled per ray at the renderer's k-sigma screen bound. Uses the per-stream arena
- * (112 B per Gaussian and pose). */
+ * Gaussians are culled per ray at the renderer's k-sigma screen bound. Uses the per-stream arena:
+ * 112 B per Gaussian and pose, 48 B per pose, and for long lists, whose rays are bucketed by pose
+ * and position, up to 1 MB plus 12 B per ray (at most 4 Mi rays at a time). Under stream capture
+ * an arena too small for the bucketing is not grown: the list is rendered in its own order. */
 typedef struct fe_pixlist_desc {
   uint32_t magic;      /* FE_DESC_MAGIC */
   uint32_t version;    /* FE_DESC_VERSION */

@@ -98,3 +98,34 @@ def test_scaled_rays_weights_and_features(cuda_device):
     assert np.max(np.abs(wts - rw)[:, mask]) <= 1e-4
     assert np.allclose(wts.sum(0)[mask], 1.0, atol=1e-5)
     assert np.max(np.abs(of - (rw.T @ feats.astype(np.float64)))[mask]) <= 1e-3
+
+
+@pytest.mark.parametrize("n,n_rays,n_poses", [(41, 20011, 3), (130, 12345, 70), (1100, 9729, 1)])
+def test_long_lists_match_their_pieces(cuda_device, n, n_rays, n_poses):
+    """A ray's result does not depend on the list around it: a long shuffled list (bucketed by
+    pose and cell, 64 rays per warp or fewer) equals, bit for bit, the same rays rendered in short
+    pieces (a few rays per warp, in the order given); a sample agrees with the oracle."""
+    rng = np.random.default_rng(n)
+    scene = S.random_gaussians(n, 0.15, rng)
+    cams = [S.Camera(96, 160, 120.0, 120.0, 80.0, 48.0, *S.look_at(0.6 * d))
+            for d in S.random_unit_vectors(n_poses, rng)]
+    poses, inv_f = pose_list(cams), 1.0 / 120.0
+    rays = np.stack([rng.uniform(-90, 90, n_rays), rng.uniform(-60, 60, n_rays), np.ones(n_rays),
+                     rng.integers(0, n_poses, n_rays)], 1).astype(np.float32)
+    m, p, w = scene_to_dev(scene, cuda_device)
+    feats = torch.from_numpy(rng.normal(size=(n, 5)).astype(np.float32))
+    rd, pd = torch.from_numpy(rays), torch.from_numpy(poses)
+    whole = fe.render_pixels(m, p, w, rd, inv_f, pd, flow=True, features=feats)
+    for lo, hi in ((0, 1), (1, 63), (63, 127), (127, 5000), (5000, n_rays - 7001),
+                   (n_rays - 33, n_rays)):
+        part = fe.render_pixels(m, p, w, rd[lo:hi], inv_f, pd, flow=True, features=feats)
+        for x, y in zip(whole, part):
+            if x is not None:
+                torch.testing.assert_close(x[lo:hi], y, rtol=0, atol=0, equal_nan=True)
+    pick = rng.choice(n_rays, 200, replace=False)
+    ref_d, ref_a, _, _ = O.render_func_idx_quattrans(scene.means, scene.prec, scene.logw,
+                                                     rays[pick], inv_f, poses, 21.4, 2.66)
+    d, a = (x.cpu().numpy().astype(np.float64)[pick] for x in whole[:2])
+    seen = ref_a > DEPTH_MASK_ALPHA
+    assert np.max(np.abs(a - ref_a)) <= TOL_ALPHA
+    assert np.max(np.abs(d - ref_d)[seen] / ref_d[seen]) <= TOL_DEPTH_REL
