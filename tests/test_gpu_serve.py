@@ -201,3 +201,35 @@ def test_fused_silhouette_bce_matches_float64(cuda_device):
         err = (galpha[lo:hi].double() - d[lo:hi] / (hi - lo)).abs()
         assert bool((err <= 1e-6 * scale + 1e-30).all())
         lo = hi
+
+
+@pytest.mark.parametrize("offset,soft", [(0, False), (0, True), (1, False), (3, True)])
+def test_silhouette_bce_ragged_renders(cuda_device, offset, soft):
+    """Renders of 1 to 70001 pixels back to back, on buffers at 16-byte boundaries and off them,
+    binary and soft targets, saturated alphas; against the formulas in float64. Tolerances: a
+    term's float32 logarithm and 1 - alpha are each within 1.2e-7 (absolute below alpha = 1/2); a
+    derivative takes a subtraction, a division, the scaling and, with soft targets, a sum."""
+    sizes = [1, 3, 127, 128, 129, 5, 640, 1, 70001, 2, 4096, 33]
+    n = sum(sizes)
+    g = torch.Generator(device=cuda_device).manual_seed(offset + soft)
+    pool = torch.rand((2, n + offset), device=cuda_device, generator=g)
+    alpha, target = pool[0][offset:], pool[1][offset:]
+    target.copy_(target if soft else (target > 0.5).float())
+    alpha[::7], alpha[1::7], alpha[2::7] = 0.0, 1.0, alpha[2::7] * 1e-6
+    ends = torch.tensor(np.cumsum(sizes), dtype=torch.int64, device=cuda_device)
+    out = torch.empty(n + offset, device=cuda_device)[offset:]
+    loss, galpha = fe.silhouette_bce(alpha, target, ends, galpha=out)
+    a, t, clip = alpha.double(), target.double(), 3e-8
+    one, zero = a.clamp(min=clip), (1 - a).clamp(min=clip)
+    terms = -(t * one.log() + (1 - t) * zero.log())
+    inside = ((a > clip) & (1 - a > clip)).double()
+    count = torch.tensor(sizes, device=cuda_device).repeat_interleave(
+        torch.tensor(sizes, device=cuda_device)).double()
+    want = inside * (-t / one + (1 - t) / zero) / count
+    size = inside * (t / one + (1 - t) / zero) / count
+    assert torch.all((galpha.double() - want).abs() <= 6e-7 * size)
+    start = 0
+    for s, k in enumerate(sizes):
+        ref = terms[start:start + k].mean()
+        assert abs(loss[s] - ref) <= 2.4e-7 + 2.4e-7 * ref
+        start += k
