@@ -527,7 +527,7 @@ int fe_render_features(const fe_render_desc* d, const float* means, const float*
                    sorted);
   if (rc) return rc;
   launch_features(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, stats, npix,
-                  p.beta2, p.beta3, features, n_features, out, rs.ctrl, st);
+                  p.beta2, p.beta3, features, n_features, out, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }

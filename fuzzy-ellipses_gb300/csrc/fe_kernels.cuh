@@ -160,7 +160,7 @@ void launch_render_pixels(int n, int n_poses, const float* means, const float* p
 void launch_features(const ViewsArg& va, int tile_w, int tile_h, int64_t n_tiles,
                      const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
                      const float* stats, int64_t stats_stride, float beta2, float beta3,
-                     const float* feats, int nf, float* out, Control* ctrl, cudaStream_t st);
+                     const float* feats, int nf, float* out, cudaStream_t st);
 
 // profiling.cu
 void launch_wait_selftest(unsigned long long limit_ns, uint32_t* status,

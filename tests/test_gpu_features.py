@@ -54,3 +54,24 @@ def test_features_equal_the_pixel_list_path(cuda_device):
                            torch.from_numpy(pose), features=feats)
     ok = (a > DEPTH_MASK_ALPHA).reshape(-1)
     assert torch.allclose(out.reshape(-1, 3)[ok], res[4][ok], rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (8, 8), (32, 8)])
+@pytest.mark.parametrize("nf", [1, 4, 5, 8, 17, 33, 64])
+def test_feature_widths_agree(cuda_device, tile, nf):
+    """Every width's kernel and its last, partial pass: column j of a wide table equals the same
+    column rendered alone (the weights are the same bits; a sum over at most 70 keys is reassociated
+    only where the table's padding differs, so to 70 ulp), and a constant column gives the constant
+    times the weights' sum. More than one stage of keys per tile, odd image sides."""
+    rng = np.random.default_rng(nf)
+    scene = S.random_gaussians(150, 0.08, rng)
+    H, W, f = 43, 61, 60.0
+    quat, trans = S.look_at(0.5 * S.random_unit_vectors(1, rng)[0])
+    m, p, w = scene_to_dev(scene, cuda_device)
+    feats = torch.from_numpy(rng.normal(size=(scene.n, nf)).astype(np.float32)).to(cuda_device)
+    cam = (f, f, W / 2, H / 2, quat, trans, H, W)
+    wide = fe.render_features(m, p, w, feats, *cam, tile=tile)[2]
+    for j in {0, nf // 2, nf - 1}:
+        one = fe.render_features(m, p, w, feats[:, j:j + 1].contiguous(), *cam, tile=tile)[2]
+        torch.testing.assert_close(wide[..., j], one[..., 0], rtol=0,
+                                   atol=70 * 6e-8 * float(feats.abs().max()))
