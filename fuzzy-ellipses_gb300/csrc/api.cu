@@ -295,7 +295,7 @@ int run_binning(const Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf
   // non-empty ones.
   FE_CUDA(zero_ctrl_rows(rs, rp.ok ? rp.max_gy + 1 : 0, st));
   if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
-  launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, nullptr, p.trans, p.cull_mode,
+  launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
                     rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
   if (exact) {
@@ -379,7 +379,55 @@ Pipeline single_view_pipeline(const fe_render_desc* d, const float* means, const
   p.beta2 = d->beta2;
   p.beta3 = d->beta3;
   p.means = means; p.prec = prec; p.logw = logw; p.quat = quat; p.trans = trans;
+  if (d->flags & FE_FLAG_HOST_POSE) {
+    std::memcpy(p.va.pose, quat, 4 * sizeof(float));
+    std::memcpy(p.va.pose + 4, trans, 3 * sizeof(float));
+    p.va.has_pose = 1;
+    p.quat = p.trans = nullptr;
+  }
   return p;
+}
+
+// Features of an image render over one binning; with `depth` (and `alpha`) the forward that writes
+// the statistics runs over the same binning first, else `stats` holds them.
+int render_features(const fe_render_desc* d, const float* means, const float* prec,
+                    const float* logw, const float* quat, const float* trans, float* depth,
+                    float* alpha, float* stats, const float* features, int32_t n_features,
+                    float* out, cudaStream_t st) {
+  int rc = check_desc(d);
+  if (rc) return rc;
+  if (n_features < 1) return fail(FE_ERR_INVALID_ARGUMENT, "n_features must be >= 1");
+  if (!stats || !features || !out || !quat || !trans)
+    return fail(FE_ERR_INVALID_ARGUMENT, "NULL pointer");
+  const int64_t npix = (int64_t)d->height * d->width;
+  if (d->n_gaussians == 0) {
+    if (depth) {
+      FE_CUDA(cudaMemsetAsync(depth, 0, sizeof(float) * npix, st));
+      FE_CUDA(cudaMemsetAsync(alpha, 0, sizeof(float) * npix, st));
+      FE_CUDA(cudaMemsetAsync(stats, 0, sizeof(float) * 3 * npix, st));
+    }
+    FE_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * npix * n_features, st));
+    return FE_OK;
+  }
+  if (!means || !prec || !logw) return fail(FE_ERR_INVALID_ARGUMENT, "NULL Gaussian pointer");
+  Arena* a = nullptr;
+  rc = arena_for(st, &a);
+  if (rc) return rc;
+  Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
+  RecSpace rs;
+  KeySpace ks;
+  int64_t cap = 0;
+  uint64_t* sorted = nullptr;
+  rc = run_binning(p, p.n_rec * p.n_tiles, a->rec, a->keys, a->h_pinned, false, st, rs, ks, cap,
+                   sorted);
+  if (rc) return rc;
+  if (depth)
+    launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, sorted, rs.recs,
+                     rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+  launch_features(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, stats, npix,
+                  p.beta2, p.beta3, features, n_features, out, st);
+  FE_CUDA(cudaGetLastError());
+  return FE_OK;
 }
 
 }  // namespace
@@ -493,7 +541,7 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
   FE_CUDA(cudaMemsetAsync(rs.rgrad, 0, sizeof(RecGrad) * (size_t)p.n_rec, st));
   launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, depth,
                    stats, p.n_pix, gdepth, galpha, p.beta2, p.beta3, rs.rgrad, rs.ctrl, st);
-  launch_record_vjp(p.va, p.n_rec, means, prec, quat, trans, rs.recs, rs.rgrad, gmeans, gprec,
+  launch_record_vjp(p.va, p.n_rec, means, prec, p.quat, p.trans, rs.recs, rs.rgrad, gmeans, gprec,
                     glogw, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
@@ -502,34 +550,19 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
 int fe_render_features(const fe_render_desc* d, const float* means, const float* prec,
                        const float* logw, const float* quat, const float* trans,
                        const float* stats, const float* features, int32_t n_features,
-                       float* out, fe_stream_t stream_) {
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_);
-  int rc = check_desc(d);
-  if (rc) return rc;
-  if (n_features < 1) return fail(FE_ERR_INVALID_ARGUMENT, "n_features must be >= 1");
-  if (!stats || !features || !out || !quat || !trans)
-    return fail(FE_ERR_INVALID_ARGUMENT, "NULL pointer");
-  const int64_t npix = (int64_t)d->height * d->width;
-  if (d->n_gaussians == 0) {
-    FE_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * npix * n_features, st));
-    return FE_OK;
-  }
-  if (!means || !prec || !logw) return fail(FE_ERR_INVALID_ARGUMENT, "NULL Gaussian pointer");
-  Arena* a = nullptr;
-  rc = arena_for(st, &a);
-  if (rc) return rc;
-  Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
-  RecSpace rs;
-  KeySpace ks;
-  int64_t cap = 0;
-  uint64_t* sorted = nullptr;
-  rc = run_binning(p, p.n_rec * p.n_tiles, a->rec, a->keys, a->h_pinned, false, st, rs, ks, cap,
-                   sorted);
-  if (rc) return rc;
-  launch_features(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, stats, npix,
-                  p.beta2, p.beta3, features, n_features, out, st);
-  FE_CUDA(cudaGetLastError());
-  return FE_OK;
+                       float* out, fe_stream_t stream) {
+  return render_features(d, means, prec, logw, quat, trans, nullptr, nullptr,
+                         const_cast<float*>(stats), features, n_features, out,
+                         reinterpret_cast<cudaStream_t>(stream));
+}
+
+int fe_render_fwd_features(const fe_render_desc* d, const float* means, const float* prec,
+                           const float* logw, const float* quat, const float* trans, float* depth,
+                           float* alpha, float* stats, const float* features, int32_t n_features,
+                           float* out, fe_stream_t stream) {
+  if (!depth || !alpha) return fail(FE_ERR_INVALID_ARGUMENT, "NULL output pointer");
+  return render_features(d, means, prec, logw, quat, trans, depth, alpha, stats, features,
+                         n_features, out, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int fe_render_binning(const fe_render_desc* d, const float* means, const float* prec,
@@ -814,8 +847,9 @@ int fe_reference_binning(int32_t P, int32_t height, int32_t width, float n_std,
   if (rc) return rc;
   carve_rec(a->rec.ptr, P, T, 0, false, [&](const RecSpace& s_) { rs = s_; });
   FE_CUDA(cudaMemsetAsync(rs.ctrl, 0, sizeof(Control), st));
-  launch_preprocess_reference(P, n_std, means, scales, rots, view, proj, width, height, tan_fovx,
-                              tan_fovy, gx, gy, radii, means2d, rs.rects, rs.touched, st);
+  launch_preprocess_reference(P, n_std, means, scales, rots, LegacyMatrices{view, proj, {}, {}},
+                              width, height, tan_fovx, tan_fovy, gx, gy, radii, means2d, rs.rects,
+                              rs.touched, st);
   launch_scan(rs.touched, tiles_touched, P, key_capacity, rs.scan_tmp, rs.ctrl, st);
   FE_CUDA(cudaMemcpyAsync(a->h_pinned, &rs.ctrl->want_keys, sizeof(unsigned long long),
                           cudaMemcpyDeviceToHost, st));
@@ -849,11 +883,10 @@ static float reference_num_stds(int n) {
   return 0.10f;
 }
 
-int fe_rasterize_legacy(const fe_legacy_desc* d, const float* means, const float* weights,
-                        const float* scales, const float* rots, const float* rays,
-                        const float* rot, const float* trans, const float* view,
-                        const float* proj, float* out_z, float* out_alpha, fe_stream_t stream_) {
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_);
+static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const float* weights,
+                            const float* scales, const float* rots, const float* rays,
+                            const float* rot, const float* trans, const LegacyMatrices& mats,
+                            float* out_z, float* out_alpha, cudaStream_t st) {
   if (!d || d->P < 0 || d->image_height < 1 || d->image_width < 1)
     return fail(FE_ERR_INVALID_ARGUMENT, "bad legacy descriptor");
   const int P = d->P, H = d->image_height, W = d->image_width;
@@ -865,7 +898,7 @@ int fe_rasterize_legacy(const fe_legacy_desc* d, const float* means, const float
     FE_CUDA(cudaMemsetAsync(out_alpha, 0, sizeof(float) * npix, st));
     return FE_OK;
   }
-  if (!means || !weights || !scales || !rots || !rays || !rot || !trans || !view || !proj)
+  if (!means || !weights || !scales || !rots || !rays || !rot || !trans)
     return fail(FE_ERR_INVALID_ARGUMENT, "NULL input");
   Arena* a = nullptr;
   int rc = arena_for(st, &a);
@@ -891,7 +924,7 @@ int fe_rasterize_legacy(const fe_legacy_desc* d, const float* means, const float
   va.one.fx = 1.f; va.one.fy = 1.f;
   FE_CUDA(cudaMemsetAsync(rs.ctrl, 0, sizeof(Control), st));
   FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)T, st));
-  launch_preprocess_reference(P, reference_num_stds(P), means, scales, rots, view, proj, W, H,
+  launch_preprocess_reference(P, reference_num_stds(P), means, scales, rots, mats, W, H,
                               d->tan_fovx, d->tan_fovy, gx, gy, radii, means2d, rs.rects,
                               rs.touched, st);
   launch_legacy_records(va, P, means, scales, rots, weights, rot, trans, rays, rs.recs, st);
@@ -922,6 +955,29 @@ int fe_rasterize_legacy(const fe_legacy_desc* d, const float* means, const float
   return FE_OK;
 }
 
+int fe_rasterize_legacy(const fe_legacy_desc* d, const float* means, const float* weights,
+                        const float* scales, const float* rots, const float* rays,
+                        const float* rot, const float* trans, const float* view,
+                        const float* proj, float* out_z, float* out_alpha, fe_stream_t stream) {
+  if (d && d->P > 0 && (!view || !proj)) return fail(FE_ERR_INVALID_ARGUMENT, "NULL input");
+  return rasterize_legacy(d, means, weights, scales, rots, rays, rot, trans,
+                          LegacyMatrices{view, proj, {}, {}}, out_z, out_alpha,
+                          reinterpret_cast<cudaStream_t>(stream));
+}
+
+int fe_rasterize_legacy_host(const fe_legacy_desc* d, const float* means, const float* weights,
+                             const float* scales, const float* rots, const float* rays,
+                             const float* rot, const float* trans, const float* h_view,
+                             const float* h_proj, float* out_z, float* out_alpha,
+                             fe_stream_t stream) {
+  if (!h_view || !h_proj) return fail(FE_ERR_INVALID_ARGUMENT, "NULL input");
+  LegacyMatrices m{};
+  std::memcpy(m.view, h_view, sizeof(m.view));
+  std::memcpy(m.proj, h_proj, sizeof(m.proj));
+  return rasterize_legacy(d, means, weights, scales, rots, rays, rot, trans, m, out_z, out_alpha,
+                          reinterpret_cast<cudaStream_t>(stream));
+}
+
 // ---------------------------------------------------------------------------------------------
 // XLA custom-call targets (api_version 2)
 // ---------------------------------------------------------------------------------------------
@@ -943,6 +999,7 @@ void fe_render_fwd_xla(fe_stream_t stream, void** buffers, const char* opaque, s
     return;
   }
   std::memcpy(&d, opaque, sizeof d);
+  d.flags &= ~FE_FLAG_HOST_POSE;  // the buffers are device memory
   float** b = reinterpret_cast<float**>(buffers);
   xla_report(status, fe_render_fwd(&d, b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7], stream));
 }
@@ -955,6 +1012,7 @@ void fe_render_bwd_xla(fe_stream_t stream, void** buffers, const char* opaque, s
     return;
   }
   std::memcpy(&d, opaque, sizeof d);
+  d.flags &= ~FE_FLAG_HOST_POSE;  // the buffers are device memory
   float** b = reinterpret_cast<float**>(buffers);
   xla_report(status, fe_render_bwd(&d, b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7], b[8], b[9],
                                    b[10], b[11], b[12], stream));
@@ -1228,7 +1286,7 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
   FE_CUDA(zero_ctrl_rows(rs, rp.ok ? (int64_t)rp.n_views * (rp.max_gy + 1) : 0, st));
   if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   if (ev) FE_CUDA(cudaEventRecord(ev[0], st));
-  launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, nullptr, p.trans, p.cull_mode,
+  launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
                     rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
   if (ev) FE_CUDA(cudaEventRecord(ev[1], st));
@@ -1684,7 +1742,7 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
   const RowPlan rp = p.radix ? RowPlan{} : row_plan(&p.va.one, 1);
   FE_CUDA(zero_ctrl_rows(rs, rp.ok ? rp.max_gy + 1 : 0, st));
   if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
-  launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, nullptr, p.trans, p.cull_mode,
+  launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
                     rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
   uint64_t* sorted = ks.keys_a;

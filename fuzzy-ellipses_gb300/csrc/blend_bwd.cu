@@ -341,9 +341,11 @@ __global__ void record_vjp_kernel(ViewsArg va, int64_t n_rec, const float* __res
 
     T U[9], R[9];
     for (int k = 0; k < 9; ++k) U[k] = (k == 3 || k == 6 || k == 7) ? T(0) : (T)prec[9 * gi + k];
-    quat_to_rot<T>(quat + 4 * V.pose, R);
-    const T t[3] = {trans[3 * V.pose], trans[3 * V.pose + 1], trans[3 * V.pose + 2]};
-    const V3<T> p = v3<T>(means[3 * gi] - t[0], means[3 * gi + 1] - t[1], means[3 * gi + 2] - t[2]);
+    float q[4], t[3];
+    load_pose(va, quat, trans, V.pose, q, t);
+    quat_to_rot<T>(q, R);
+    const V3<T> p = v3<T>((T)means[3 * gi] - (T)t[0], (T)means[3 * gi + 1] - (T)t[1],
+                          (T)means[3 * gi + 2] - (T)t[2]);
     const V3<T> pc = matvec(R, p);
     T M[9], Y[9];
     for (int a = 0; a < 3; ++a)

@@ -181,7 +181,28 @@ struct ViewsArg {
   // so that kernels working per tile look it up with one load instead of a binary search over
   // the views (11 dependent loads for a thousand views). NULL otherwise.
   const uint32_t* tile_view;
+  // The one view's pose by value (quaternion, translation), used in place of the pose arrays when
+  // has_pose is set.
+  float pose[7];
+  int32_t has_pose;
 };
+
+// Pose `i`'s quaternion and translation: the one passed by value, or from the arrays.
+__device__ __forceinline__ void load_pose(const ViewsArg& va, const float* __restrict__ quat,
+                                          const float* __restrict__ trans, int i, float (&q)[4],
+                                          float (&t)[3]) {
+  if (va.has_pose) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q[k] = va.pose[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] = va.pose[4 + k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q[k] = quat[4 * i + k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] = trans[3 * i + k];
+  }
+}
 
 __device__ __forceinline__ const ViewDev& view_at(const ViewsArg& va, int i) {
   return va.table ? va.table[i] : va.one;

@@ -7,15 +7,18 @@ namespace fe {
 
 // preprocess.cu
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
-                       const float* logw, const float* quat, const float* rotm,
-                       const float* trans, int cull_mode, float cull_param, int tile_w,
+                       const float* logw, const float* quat, const float* trans, int cull_mode, float cull_param, int tile_w,
                        int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
                        uint32_t* touched, unsigned long long* row_tot, int max_gy, Control* ctrl,
                        cudaStream_t st);
+// The legacy interface's view and projection matrices: device arrays, or NULL and by value.
+struct LegacyMatrices {
+  const float *d_view, *d_proj;
+  float view[16], proj[16];
+};
 void launch_preprocess_reference(int P, float n_std, const float* means, const float* scales,
-                                 const float* rots, const float* viewmatrix,
-                                 const float* projmatrix, int W, int H, float tan_fovx,
-                                 float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
+                                 const float* rots, const LegacyMatrices& mats, int W, int H,
+                                 float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
                                  TileRect* rects, uint32_t* touched, cudaStream_t st);
 void launch_legacy_records(const ViewsArg& va, int P, const float* means, const float* scales,
                            const float* rots, const float* logw, const float* rotm,

@@ -82,16 +82,6 @@ __device__ void write_record(const RecordInputs& in, const double M[9], const do
   *out = r;
 }
 
-__device__ __forceinline__ void load_pose(const float* quat, const float* rotm, const float* trans,
-                                          int pose, double R[9], double t[3]) {
-  if (rotm) {
-    for (int k = 0; k < 9; ++k) R[k] = rotm[9 * pose + k];
-  } else {
-    quat_to_rot<double>(quat + 4 * pose, R);
-  }
-  t[0] = trans[3 * pose]; t[1] = trans[3 * pose + 1]; t[2] = trans[3 * pose + 2];
-}
-
 // Clamp a floating tile coordinate into [lo, hi] before converting to int.
 __device__ __forceinline__ int clamp_tile(float x, int lo, int hi) {
   if (!(x > (float)lo)) return lo;   // also catches NaN
@@ -193,7 +183,7 @@ __device__ __forceinline__ void footprint_and_record(
 
 __global__ void __launch_bounds__(64) preprocess_kernel(
     ViewsArg va, int64_t n_rec, const float* __restrict__ means, const float* __restrict__ prec,
-    const float* __restrict__ logw, const float* __restrict__ quat, const float* __restrict__ rotm,
+    const float* __restrict__ logw, const float* __restrict__ quat,
     const float* __restrict__ trans, int cull_mode, float cull_param, int tile_w, int tile_h,
     GaussRec* __restrict__ recs, TileRect* __restrict__ rects, FootRows* __restrict__ foot,
     uint32_t* __restrict__ touched, unsigned long long* __restrict__ row_tot, int max_gy,
@@ -204,18 +194,11 @@ __global__ void __launch_bounds__(64) preprocess_kernel(
     const int vi = find_view<&ViewDev::rec_base>(va, i);
     const ViewDev& V = view_at(va, vi);
     const int64_t gi = V.gauss_base + (i - V.rec_base);
-    float R[9], t[3], m[3], pr[9];
-    if (rotm) {
+    float R[9], q[4], t[3], m[3], pr[9];
+    load_pose(va, quat, trans, V.pose, q, t);
+    quat_to_rot<float>(q, R);
 #pragma unroll
-      for (int k = 0; k < 9; ++k) R[k] = rotm[9 * V.pose + k];
-    } else {
-      quat_to_rot<float>(quat + 4 * V.pose, R);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      t[k] = trans[3 * V.pose + k];
-      m[k] = means[3 * gi + k];
-    }
+    for (int k = 0; k < 3; ++k) m[k] = means[3 * gi + k];
 #pragma unroll
     for (int k = 0; k < 9; ++k) pr[k] = prec[9 * gi + k];
     GaussRec rec;
@@ -324,12 +307,17 @@ __device__ __forceinline__ void ref_get_rect(float px, float py, int r, int gx, 
 
 __global__ void preprocess_reference_kernel(
     int P, float n_std, const float* __restrict__ means, const float* __restrict__ scales,
-    const float* __restrict__ rots, const float* __restrict__ viewmatrix,
-    const float* __restrict__ projmatrix, int W, int H, float tan_fovx, float tan_fovy,
-    float focal_x, float focal_y, int gx, int gy, int32_t* __restrict__ radii,
+    const float* __restrict__ rots, LegacyMatrices mats, int W, int H, float tan_fovx,
+    float tan_fovy, float focal_x, float focal_y, int gx, int gy, int32_t* __restrict__ radii,
     float* __restrict__ means2d, TileRect* __restrict__ rects, uint32_t* __restrict__ touched) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= P) return;
+  float viewmatrix[16], projmatrix[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    viewmatrix[k] = mats.d_view ? mats.d_view[k] : mats.view[k];
+    projmatrix[k] = mats.d_proj ? mats.d_proj[k] : mats.proj[k];
+  }
   radii[idx] = 0;
   touched[idx] = 0;
   rects[idx] = TileRect{0, 0, 0, 0};
@@ -450,7 +438,8 @@ __global__ void legacy_records_kernel(ViewsArg va, int P, const float* __restric
   const double i20 = -(l20 * i00 + l21 * i10) / l22;
   const double U[9] = {i00, i10, i20, 0.0, i11, i21, 0.0, 0.0, i22};
   for (int k = 0; k < 9; ++k) in.U[k] = U[k];
-  load_pose(nullptr, rotm, trans, 0, in.R, in.t);
+  for (int k = 0; k < 9; ++k) in.R[k] = rotm[k];
+  for (int k = 0; k < 3; ++k) in.t[k] = trans[k];
   double M[9], Y[9];
   V3<double> pc;
   build_camera_terms(in, M, Y, pc);
@@ -462,8 +451,7 @@ __global__ void legacy_records_kernel(ViewsArg va, int P, const float* __restric
 // ------------------------------------------------------------------------------------------
 
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
-                       const float* logw, const float* quat, const float* rotm,
-                       const float* trans, int cull_mode, float cull_param, int tile_w,
+                       const float* logw, const float* quat, const float* trans, int cull_mode, float cull_param, int tile_w,
                        int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
                        uint32_t* touched, unsigned long long* row_tot, int max_gy, Control* ctrl,
                        cudaStream_t st) {
@@ -471,22 +459,21 @@ void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, co
   const int threads = 64;
   const int64_t want = (n_rec + threads - 1) / threads;
   const int blocks = (int)(want < 65535 ? want : 65535);
-  preprocess_kernel<<<blocks, threads, 0, st>>>(va, n_rec, means, prec, logw, quat, rotm, trans,
+  preprocess_kernel<<<blocks, threads, 0, st>>>(va, n_rec, means, prec, logw, quat, trans,
                                                 cull_mode, cull_param, tile_w, tile_h, recs,
                                                 rects, foot, touched, row_tot, max_gy, ctrl);
 }
 
 void launch_preprocess_reference(int P, float n_std, const float* means, const float* scales,
-                                 const float* rots, const float* viewmatrix,
-                                 const float* projmatrix, int W, int H, float tan_fovx,
-                                 float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
+                                 const float* rots, const LegacyMatrices& mats, int W, int H,
+                                 float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
                                  TileRect* rects, uint32_t* touched, cudaStream_t st) {
   if (P <= 0) return;
   // rasterizer_impl.cu:205-206 (float arithmetic on the host).
   const float fx = (float)W / (2.0f * tan_fovx);
   const float fy = (float)H / (2.0f * tan_fovy);
   preprocess_reference_kernel<<<(P + 255) / 256, 256, 0, st>>>(
-      P, n_std, means, scales, rots, viewmatrix, projmatrix, W, H, tan_fovx, tan_fovy, fx, fy, gx,
+      P, n_std, means, scales, rots, mats, W, H, tan_fovx, tan_fovy, fx, fy, gx,
       gy, radii, means2d, rects, touched);
 }
 

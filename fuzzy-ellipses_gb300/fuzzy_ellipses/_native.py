@@ -29,6 +29,7 @@ FE_FLAG_KEEP_BINNING = 4
 FE_FLAG_RADIX_BINNING = 8
 FE_FLAG_HEAVY_TILES_FIRST = 0x10000
 FE_FLAG_RECT_BINNING = 0x20000
+FE_FLAG_HOST_POSE = 0x40000
 FE_VIEW_NO_GRAD = 1
 FE_ERR_OUT_OF_MEMORY = 4
 
@@ -150,6 +151,7 @@ PROTOTYPES = {
     "fe_render_fwd": (ctypes.c_int, [ctypes.POINTER(RenderDesc)] + [P] * 8 + [P]),
     "fe_render_fwd_noalloc": (ctypes.c_int, [ctypes.POINTER(RenderDesc)] + [P] * 9 + [P]),
     "fe_render_features": (ctypes.c_int, [ctypes.POINTER(RenderDesc)] + [P] * 7 + [I32, P, P]),
+    "fe_render_fwd_features": (ctypes.c_int, [ctypes.POINTER(RenderDesc)] + [P] * 9 + [I32, P, P]),
     "fe_silhouette_bce": (ctypes.c_int, [P, P, P, I32, I64, P, P, P]),
     "fe_gmm_log_likelihood": (ctypes.c_int, [P, P, P, I32, P, I64, P, P, P, P]),
     "fe_pixlist_desc_init": (None, [ctypes.POINTER(PixlistDesc), I32, I32, I64, F32]),
@@ -165,6 +167,7 @@ PROTOTYPES = {
     "fe_render_bwd_xla": (None, [P, P, P, ctypes.c_size_t, P]),
     "fe_rasterize_legacy_xla": (None, [P, P, P, ctypes.c_size_t, P]),
     "fe_rasterize_legacy": (ctypes.c_int, [ctypes.POINTER(LegacyDesc)] + [P] * 11 + [P]),
+    "fe_rasterize_legacy_host": (ctypes.c_int, [ctypes.POINTER(LegacyDesc)] + [P] * 11 + [P]),
     "fe_reference_binning": (ctypes.c_int, [I32, I32, I32, F32, P, P, P, P, P, F32, F32,
                                             P, P, P, P, I64, P, ctypes.POINTER(I64), P]),
     "fe_batch_create": (ctypes.c_int, [ctypes.POINTER(RenderDesc), ctypes.POINTER(SceneEntry), I32,

@@ -45,6 +45,40 @@ def _as_dev(x, device, shape=None, name="tensor"):
     return x
 
 
+def _host_vec(x, n):
+    """x as n host float32 values, or None when it lives on a device or has another size."""
+    if torch.is_tensor(x):
+        if x.device.type != "cpu":
+            return None
+        x = x.detach().to(torch.float32).numpy()
+    x = np.asarray(x, dtype=np.float32)
+    return x.reshape(n) if x.size == n else None
+
+
+class _Pose:
+    """A camera pose for the native single-view entries: the pointers to pass and the descriptor
+    flag that says where they point. A pose given in host memory (arrays, lists, CPU tensors) is
+    copied here and goes to the kernels by value, with no upload (an upload from pageable memory
+    holds the caller until the stream has drained: two of them took 45 of the 88 us of a 200x200
+    call of 40 Gaussians); one given on the device stays there. Under stream capture the upload,
+    which a capture refuses, stays: a graph would replay the captured values."""
+
+    __slots__ = ("flag", "q", "t", "tensors", "_host")
+
+    def __init__(self, quat, t, dev):
+        q, tt = _host_vec(quat, 4), _host_vec(t, 3)
+        if q is None or tt is None or torch.cuda.is_current_stream_capturing():
+            self.tensors = (_as_dev(quat, dev, (4,)), _as_dev(t, dev, (3,)))
+            self.q, self.t = (x.data_ptr() for x in self.tensors)
+            self.flag = 0
+        else:
+            self.tensors = (None, None)
+            self._host = np.concatenate((q, tt))
+            self.q = self._host.ctypes.data
+            self.t = self.q + 16
+            self.flag = N.FE_FLAG_HOST_POSE
+
+
 def _check_inputs(means, prec, logw):
     if not (torch.is_tensor(means) and means.is_cuda):
         raise TypeError("means must be a CUDA tensor (the renderer has no CPU path)")
@@ -57,7 +91,7 @@ def _check_inputs(means, prec, logw):
 
 class _RenderFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, means, prec, logw, quat, trans, desc):
+    def forward(ctx, means, prec, logw, quat, trans, pose, desc):
         lib = N.load()
         dev = means.device
         means = means.detach().contiguous().float()
@@ -69,10 +103,11 @@ class _RenderFn(torch.autograd.Function):
         need = any(ctx.needs_input_grad[:3])
         stats = torch.empty((3, H, W), device=dev, dtype=torch.float32) if need else None
         N.check(lib.fe_render_fwd(ctypes.byref(desc), _ptr(means), _ptr(prec), _ptr(logw),
-                                  _ptr(quat), _ptr(trans), _ptr(depth), _ptr(alpha), _ptr(stats),
+                                  pose.q, pose.t, _ptr(depth), _ptr(alpha), _ptr(stats),
                                   _stream()))
         ctx.desc = desc
-        if need:
+        ctx.pose = pose
+        if need:  # (quat, trans: a pose on the device, else None)
             ctx.save_for_backward(means, prec, logw, quat, trans, depth, alpha, stats)
         return depth, alpha
 
@@ -80,15 +115,17 @@ class _RenderFn(torch.autograd.Function):
     def backward(ctx, gdepth, galpha):
         lib = N.load()
         means, prec, logw, quat, trans, depth, alpha, stats = ctx.saved_tensors
+        q = ctx.pose.q if quat is None else _ptr(quat)
+        t = ctx.pose.t if trans is None else _ptr(trans)
         gm = torch.empty_like(means)
         gp = torch.empty_like(prec)
         gw = torch.empty_like(logw)
         gd = gdepth.contiguous().float() if gdepth is not None else None
         ga = galpha.contiguous().float() if galpha is not None else None
         N.check(lib.fe_render_bwd(ctypes.byref(ctx.desc), _ptr(means), _ptr(prec), _ptr(logw),
-                                  _ptr(quat), _ptr(trans), _ptr(depth), _ptr(alpha), _ptr(stats),
-                                  _ptr(gd), _ptr(ga), _ptr(gm), _ptr(gp), _ptr(gw), _stream()))
-        return gm, gp, gw, None, None, None
+                                  q, t, _ptr(depth), _ptr(alpha), _ptr(stats), _ptr(gd), _ptr(ga),
+                                  _ptr(gm), _ptr(gp), _ptr(gw), _stream()))
+        return gm, gp, gw, None, None, None, None
 
 
 def render(means, prec, logw, fx, fy, cx, cy, quat, t, height, width, beta2=21.4, beta3=2.66, *,
@@ -102,10 +139,10 @@ def render(means, prec, logw, fx, fy, cx, cy, quat, t, height, width, beta2=21.4
     """
     n = _check_inputs(means, prec, logw)
     dev = means.device
-    q = _as_dev(quat, dev, (4,))
-    tt = _as_dev(t, dev, (3,))
-    desc = N.make_desc(n, height, width, fx, fy, cx, cy, beta2, beta3, cull, cull_param, tile)
-    return _RenderFn.apply(means, prec, logw, q, tt, desc)
+    pose = _Pose(quat, t, dev)
+    desc = N.make_desc(n, height, width, fx, fy, cx, cy, beta2, beta3, cull, cull_param, tile,
+                       flags=pose.flag)
+    return _RenderFn.apply(means, prec, logw, *pose.tensors, pose, desc)
 
 
 def render_forward(means, prec, logw, fx, fy, cx, cy, quat, t, height, width, beta2=21.4,
@@ -115,14 +152,13 @@ def render_forward(means, prec, logw, fx, fy, cx, cy, quat, t, height, width, be
     lib = N.load()
     n = _check_inputs(means, prec, logw)
     dev = means.device
-    q = _as_dev(quat, dev, (4,))
-    tt = _as_dev(t, dev, (3,))
+    pose = _Pose(quat, t, dev)
     desc = N.make_desc(n, height, width, fx, fy, cx, cy, beta2, beta3, cull, cull_param, tile,
-                       flags=_binning_flag(binning))
+                       flags=_binning_flag(binning) | pose.flag)
     if out is None:
         out = (torch.empty((height, width), device=dev), torch.empty((height, width), device=dev))
-    N.check(lib.fe_render_fwd(ctypes.byref(desc), _ptr(means), _ptr(prec), _ptr(logw), _ptr(q),
-                              _ptr(tt), _ptr(out[0]), _ptr(out[1]), _ptr(stats), _stream()))
+    N.check(lib.fe_render_fwd(ctypes.byref(desc), _ptr(means), _ptr(prec), _ptr(logw), pose.q,
+                              pose.t, _ptr(out[0]), _ptr(out[1]), _ptr(stats), _stream()))
     return out
 
 
@@ -137,18 +173,16 @@ def render_features(means, prec, logw, features, fx, fy, cx, cy, quat, t, height
     feats = features.to(device=dev, dtype=torch.float32).contiguous()
     if feats.dim() != 2 or feats.shape[0] != n or feats.shape[1] < 1:
         raise ValueError("features must be (N, F) with F >= 1")
-    q = _as_dev(quat, dev, (4,))
-    tt = _as_dev(t, dev, (3,))
-    desc = N.make_desc(n, height, width, fx, fy, cx, cy, beta2, beta3, cull, cull_param, tile)
+    pose = _Pose(quat, t, dev)
+    desc = N.make_desc(n, height, width, fx, fy, cx, cy, beta2, beta3, cull, cull_param, tile,
+                       flags=pose.flag)
     depth = torch.empty((height, width), device=dev)
     alpha = torch.empty((height, width), device=dev)
     stats = torch.empty((3, height, width), device=dev)
     out = torch.empty((height, width, feats.shape[1]), device=dev)
-    N.check(lib.fe_render_fwd(ctypes.byref(desc), _ptr(means), _ptr(prec), _ptr(logw), _ptr(q),
-                              _ptr(tt), _ptr(depth), _ptr(alpha), _ptr(stats), _stream()))
-    N.check(lib.fe_render_features(ctypes.byref(desc), _ptr(means), _ptr(prec), _ptr(logw),
-                                   _ptr(q), _ptr(tt), _ptr(stats), _ptr(feats), feats.shape[1],
-                                   _ptr(out), _stream()))
+    N.check(lib.fe_render_fwd_features(ctypes.byref(desc), _ptr(means), _ptr(prec), _ptr(logw),
+                                       pose.q, pose.t, _ptr(depth), _ptr(alpha), _ptr(stats),
+                                       _ptr(feats), feats.shape[1], _ptr(out), _stream()))
     return depth, alpha, out
 
 
@@ -405,12 +439,17 @@ def rasterize(means3D, scales, rotations, weights, camera_rays, camera_rot, came
     tfx, tfy, view, proj = _legacy_scalars(H, W, fx, fy, cx, cy, near, far)
     d = N.LegacyDesc(H, W, P, float(tfx), float(tfy))
     bufs = [means, _as_dev(weights, dev), _as_dev(scales, dev), _as_dev(rotations, dev),
-            _as_dev(camera_rays, dev), _as_dev(camera_rot, dev), _as_dev(camera_trans, dev),
-            _as_dev(view, dev), _as_dev(proj, dev)]
+            _as_dev(camera_rays, dev), _as_dev(camera_rot, dev), _as_dev(camera_trans, dev)]
     z = torch.empty((H, W), device=dev)
     alpha = torch.empty((H, W), device=dev)
-    N.check(lib.fe_rasterize_legacy(ctypes.byref(d), *[_ptr(b) for b in bufs], _ptr(z), _ptr(alpha),
-                                    _stream()))
+    if torch.cuda.is_current_stream_capturing():  # (refuses the matrices' upload: see _Pose)
+        bufs += [_as_dev(view, dev), _as_dev(proj, dev)]
+        N.check(lib.fe_rasterize_legacy(ctypes.byref(d), *[_ptr(b) for b in bufs], _ptr(z),
+                                        _ptr(alpha), _stream()))
+    else:
+        N.check(lib.fe_rasterize_legacy_host(ctypes.byref(d), *[_ptr(b) for b in bufs],
+                                             view.ctypes.data, proj.ctypes.data, _ptr(z),
+                                             _ptr(alpha), _stream()))
     z = torch.nan_to_num(z, posinf=10.0, neginf=0.0)        # __init__.py:233
     alpha = torch.nan_to_num(alpha, posinf=1.0, neginf=0.0)  # __init__.py:234
     return z, alpha

@@ -86,6 +86,10 @@ typedef enum fe_cull_mode {
  * the mean, so the tiles dropped by default hold only pixels where the Gaussian's density is
  * below the cut-off; on 16 views of 640x480 they are a quarter of the rectangle's keys. */
 #define FE_FLAG_RECT_BINNING 0x20000u
+/* Single-view entries (fe_render_fwd, _fwd_noalloc, _bwd, _binning, _features, _fwd_features): the
+ * pose pointers d_quat and d_trans are host memory, read during the call and passed to the kernels
+ * by value, so a pose that lives on the host needs no upload. Batches and XLA targets ignore it. */
+#define FE_FLAG_HOST_POSE 0x40000u
 
 /* Render descriptor: everything a render needs besides the Gaussian and pose buffers. It is also
  * the opaque payload of the XLA custom call targets (bit-copied; the size and magic are checked).
@@ -156,6 +160,14 @@ int fe_render_features(const fe_render_desc *desc, const float *d_means, const f
                        const float *d_stats, const float *d_features, int32_t n_features,
                        float *d_out, fe_stream_t stream);
 
+/* fe_render_fwd with statistics and fe_render_features in one call, over one binning: writes
+ * d_depth, d_alpha, d_stats (all required) and d_out. */
+int fe_render_fwd_features(const fe_render_desc *desc, const float *d_means, const float *d_prec,
+                           const float *d_logw, const float *d_quat, const float *d_trans,
+                           float *d_depth, float *d_alpha, float *d_stats,
+                           const float *d_features, int32_t n_features, float *d_out,
+                           fe_stream_t stream);
+
 /* XLA custom-call targets (api_version 2: status-returning), registered under the names
  * "fe_render_fwd" and "fe_render_bwd". opaque = an fe_render_desc.
  * fwd buffers: [means, prec, logw, quat, trans, depth, alpha, stats]
@@ -212,6 +224,14 @@ int fe_rasterize_legacy(const fe_legacy_desc *desc, const float *d_means, const 
                         const float *d_camera_rot, const float *d_camera_trans,
                         const float *d_viewmatrix, const float *d_projmatrix, float *d_out_z,
                         float *d_out_alpha, fe_stream_t stream);
+/* fe_rasterize_legacy with the view and projection matrices in host memory, read during the call
+ * and passed to the kernels by value. */
+int fe_rasterize_legacy_host(const fe_legacy_desc *desc, const float *d_means,
+                             const float *d_weights, const float *d_scales,
+                             const float *d_rotations, const float *d_camera_rays,
+                             const float *d_camera_rot, const float *d_camera_trans,
+                             const float *h_viewmatrix, const float *h_projmatrix, float *d_out_z,
+                             float *d_out_alpha, fe_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Batched renders: many scenes and cameras in one launch sequence.

@@ -8,7 +8,7 @@ import fuzzy_ellipses as fe
 from fuzzy_ellipses import synthetic as S
 from oracle import fm_render_np as O
 from tests.helpers import (TOL_ALPHA, TOL_DEPTH_REL, floor_dominated, oracle_pixels, parity_errors,
-                           scene_to_dev, tile_lists_from_keys)
+                           scene_to_dev, tile_lists_from_keys, to_dev)
 
 pytestmark = pytest.mark.gpu
 TILES = [(8, 8), (16, 16), (32, 8)]
@@ -242,3 +242,38 @@ def test_large_scene_beyond_the_key_budget(cuda_device):
     a2.sum().backward()
     for g in (mr.grad, pr.grad, wr.grad):
         assert torch.isfinite(g).all() and float(g.abs().sum()) > 0
+
+
+@pytest.mark.parametrize("kind", ["array", "list", "cpu tensor", "double"])
+def test_host_pose_equals_device_pose(cuda_device, kind):
+    """A pose in host memory goes to the kernels by value: the same bits as the same pose in device
+    tensors, in the forward, the features and the gradients, also when the caller overwrites its
+    array between the forward and the backward."""
+    scene, cams = S.config0(seed=2)
+    c = cams[0]
+    m, p, w = scene_to_dev(scene, cuda_device)
+    q, t = c.quat.copy(), c.trans.copy()
+    if kind == "list":
+        q, t = [float(x) for x in q], [float(x) for x in t]
+    elif kind == "cpu tensor":
+        q, t = torch.from_numpy(q), torch.from_numpy(t)
+    elif kind == "double":
+        q, t = q.astype(np.float64), t.astype(np.float64)
+    dq, dt = to_dev(c.quat, cuda_device), to_dev(c.trans, cuda_device)
+    size = (c.height, c.width)
+    feats = torch.rand(scene.n, 3, device=cuda_device)
+    a = fe.render_features(m, p, w, feats, c.fx, c.fy, c.cx, c.cy, q, t, *size)
+    b = fe.render_features(m, p, w, feats, c.fx, c.fy, c.cx, c.cy, dq, dt, *size)
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+    fwd = fe.render_forward(m, p, w, c.fx, c.fy, c.cx, c.cy, q, t, *size)
+    assert torch.equal(fwd[0], b[0]) and torch.equal(fwd[1], b[1])
+    grads = []
+    for quat, trans in ((q, t), (dq, dt)):
+        mm = m.clone().requires_grad_()
+        depth, alpha = fe.render(mm, p, w, c.fx, c.fy, c.cx, c.cy, quat, trans, *size)
+        if quat is q and not isinstance(q, list):
+            q[0], t[0] = 9.0, 9.0
+        (alpha.sum() + depth.sum()).backward()
+        grads.append(mm.grad)
+    # (the backward's atomics leave the order of a Gaussian's tile sums open)
+    torch.testing.assert_close(grads[0], grads[1], rtol=1e-5, atol=1e-5 * float(grads[1].abs().max()))
