@@ -883,10 +883,14 @@ static float reference_num_stds(int n) {
   return 0.10f;
 }
 
+// The legacy render: the reference's footprints on 8x8 tiles, binned tile-major where that applies
+// (a 640x480 call of 1000 Gaussians: one launch of 8 us in place of the eight of the scan,
+// emission, sort and ranges, 35 us) and by emission + sort otherwise; both give the reference's
+// keys. `clean`: outputs through nan_to_num.
 static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const float* weights,
                             const float* scales, const float* rots, const float* rays,
                             const float* rot, const float* trans, const LegacyMatrices& mats,
-                            float* out_z, float* out_alpha, cudaStream_t st) {
+                            float* out_z, float* out_alpha, bool clean, cudaStream_t st) {
   if (!d || d->P < 0 || d->image_height < 1 || d->image_width < 1)
     return fail(FE_ERR_INVALID_ARGUMENT, "bad legacy descriptor");
   const int P = d->P, H = d->image_height, W = d->image_width;
@@ -903,54 +907,52 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   Arena* a = nullptr;
   int rc = arena_for(st, &a);
   if (rc) return rc;
-  // Per-record space plus the reference's radii/means2d outputs.
   RecSpace rs;
-  Carver extra{nullptr};
-  const size_t rb = carve_rec(nullptr, P, T, 0, false, [](const RecSpace&) {});
-  extra.off = rb;
-  extra.take<int32_t>(P);
-  extra.take<float>(2 * (int64_t)P);
-  rc = a->rec.reserve(extra.off, st);
+  rc = a->rec.reserve(carve_rec(nullptr, P, T, 0, false, [](const RecSpace&) {}), st);
   if (rc) return rc;
   carve_rec(a->rec.ptr, P, T, 0, false, [&](const RecSpace& s_) { rs = s_; });
-  Carver ex2{a->rec.ptr};
-  ex2.off = rb;
-  int32_t* radii = ex2.take<int32_t>(P);
-  float* means2d = ex2.take<float>(2 * (int64_t)P);
 
   ViewsArg va{};
   va.count = 1;
   va.one.H = H; va.one.W = W; va.one.gx = gx; va.one.gy = gy; va.one.n = P;
   va.one.fx = 1.f; va.one.fy = 1.f;
-  FE_CUDA(cudaMemsetAsync(rs.ctrl, 0, sizeof(Control), st));
-  FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)T, st));
-  launch_preprocess_reference(P, reference_num_stds(P), means, scales, rots, mats, W, H,
-                              d->tan_fovx, d->tan_fovy, gx, gy, radii, means2d, rs.rects,
-                              rs.touched, st);
-  launch_legacy_records(va, P, means, scales, rots, weights, rot, trans, rays, rs.recs, st);
+  const RowPlan rp = row_plan(&va.one, 1);
+  FE_CUDA(zero_ctrl_rows(rs, rp.ok ? rp.max_gy + 1 : 0, st));
+  if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)T, st));
+  launch_legacy_preprocess(P, reference_num_stds(P), means, scales, rots, weights, rot, trans, rays,
+                           mats, W, H, d->tan_fovx, d->tan_fovy, gx, gy, rs.recs, rs.rects,
+                           rs.touched, rp.ok ? rs.row_tot : nullptr, rs.ctrl, st);
   const int64_t worst = (int64_t)P * T;
-  int64_t cap;
-  if ((size_t)worst * kBytesPerKey <= key_budget_bytes()) {
-    cap = worst;
-    launch_scan(rs.touched, rs.incl, P, cap, rs.scan_tmp, rs.ctrl, st);
-  } else {
-    launch_scan(rs.touched, rs.incl, P, INT64_C(0xffffffff), rs.scan_tmp, rs.ctrl, st);
+  const bool exact = (size_t)worst * kBytesPerKey <= key_budget_bytes();
+  int64_t cap = worst;
+  if (!exact) {
+    if (!rp.ok) launch_scan(rs.touched, rs.incl, P, INT64_C(0xffffffff), rs.scan_tmp, rs.ctrl, st);
     FE_CUDA(cudaMemcpyAsync(a->h_pinned, &rs.ctrl->want_keys, sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, st));
     FE_CUDA(cudaStreamSynchronize(st));
-    cap = (int64_t)*a->h_pinned;
-    if (cap < 1) cap = 1;
+    cap = std::max<int64_t>(1, (int64_t)*a->h_pinned);
   }
   KeySpace ks;
   const size_t kb = carve_keys(nullptr, cap, [](const KeySpace&) {});
   rc = a->keys.reserve(kb, st);
   if (rc) return rc;
   carve_keys(a->keys.ptr, cap, [&](const KeySpace& s_) { ks = s_; });
-  launch_emit_keys(va, rs.incl, rs.rects, nullptr, 8, 8, P, rs.ctrl, ks.keys_a, cap, st);
-  uint64_t* sorted = launch_sort(ks.keys_a, ks.keys_b, bits_for(T), rs.ctrl, cap, ks.hist, st);
-  launch_ranges(sorted, rs.ctrl, cap, rs.ranges, st);
-  launch_blend_fwd(va, 8, 8, 0, 0, T, nullptr, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z,
-                   out_alpha, nullptr, 0, rs.ctrl, st);
+  uint64_t* sorted = ks.keys_a;
+  if (rp.ok) {
+    launch_tile_binning_emit(va, 1, rp.max_gy, rp.max_gx, rs.rects, nullptr, 8, 8, rs.row_tot, cap,
+                             rs.ctrl, rs.ranges, nullptr, ks.keys_a, nullptr, T, st);
+  } else {
+    if (exact) launch_scan(rs.touched, rs.incl, P, cap, rs.scan_tmp, rs.ctrl, st);
+    launch_emit_keys(va, rs.incl, rs.rects, nullptr, 8, 8, P, rs.ctrl, ks.keys_a, cap, st);
+    sorted = launch_sort(ks.keys_a, ks.keys_b, bits_for(T), rs.ctrl, cap, ks.hist, st);
+    launch_ranges(sorted, rs.ctrl, cap, rs.ranges, st);
+  }
+  if (clean)
+    launch_blend_fwd_clean(va, T, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z, out_alpha,
+                           rs.ctrl, st);
+  else
+    launch_blend_fwd(va, 8, 8, 0, 0, T, nullptr, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z,
+                     out_alpha, nullptr, 0, rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }
@@ -961,21 +963,21 @@ int fe_rasterize_legacy(const fe_legacy_desc* d, const float* means, const float
                         const float* proj, float* out_z, float* out_alpha, fe_stream_t stream) {
   if (d && d->P > 0 && (!view || !proj)) return fail(FE_ERR_INVALID_ARGUMENT, "NULL input");
   return rasterize_legacy(d, means, weights, scales, rots, rays, rot, trans,
-                          LegacyMatrices{view, proj, {}, {}}, out_z, out_alpha,
+                          LegacyMatrices{view, proj, {}, {}}, out_z, out_alpha, false,
                           reinterpret_cast<cudaStream_t>(stream));
 }
 
 int fe_rasterize_legacy_host(const fe_legacy_desc* d, const float* means, const float* weights,
                              const float* scales, const float* rots, const float* rays,
                              const float* rot, const float* trans, const float* h_view,
-                             const float* h_proj, float* out_z, float* out_alpha,
+                             const float* h_proj, int32_t clean, float* out_z, float* out_alpha,
                              fe_stream_t stream) {
   if (!h_view || !h_proj) return fail(FE_ERR_INVALID_ARGUMENT, "NULL input");
   LegacyMatrices m{};
   std::memcpy(m.view, h_view, sizeof(m.view));
   std::memcpy(m.proj, h_proj, sizeof(m.proj));
   return rasterize_legacy(d, means, weights, scales, rots, rays, rot, trans, m, out_z, out_alpha,
-                          reinterpret_cast<cudaStream_t>(stream));
+                          clean != 0, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------------

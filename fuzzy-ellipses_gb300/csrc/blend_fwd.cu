@@ -168,7 +168,14 @@ __device__ __forceinline__ void blend_group(const TilePair* grp, const f2_t (&DU
   }
 }
 
-template <int TW, int TH, int PX, int CH>
+// nan_to_num with the limits of the reference's wrapper (fuzzy_ellipses/__init__.py:233-234): NaN
+// and -inf become 0, +inf becomes `top`.
+__device__ __forceinline__ float clean_value(float x, float top) {
+  return x != x || x == -INFINITY ? 0.f : x == INFINITY ? top : x;
+}
+
+// CLEAN: the outputs go through clean_value.
+template <int TW, int TH, int PX, int CH, bool CLEAN>
 __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
                                   BlendShape<TW, TH, PX, CH>::MIN_CTAS) blend_fwd_kernel(
     ViewsArg va, uint32_t tile_begin, uint32_t tile_end, uint32_t* __restrict__ counter,
@@ -414,6 +421,10 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
                                : 1.f - ex2_approx(-A * kLog2e);
         wsum[k] = W;
         asum[k] = A;
+        if (CLEAN) {
+          dep[k] = clean_value(dep[k], 10.f);
+          alp[k] = clean_value(alp[k], 1.f);
+        }
       }
       const int64_t pix = V.pix_base + (int64_t)v * V.W + u0;
       store_pixels<PX>(depth + pix, dep, V.W - u0);
@@ -428,13 +439,13 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
   }
 }
 
-template <int TW, int TH, int PX, int CH>
+template <int TW, int TH, int PX, int CH, bool CLEAN = false>
 void launch_tiles(const ViewsArg& va, int64_t tile_begin, int64_t tile_end, uint32_t* counter,
                   const uint32_t* order, const uint64_t* keys, const GaussRec* recs,
                   const uint2* ranges, float nb2, float beta3, float* depth, float* alpha,
                   float* stats, int64_t stats_stride, Control* ctrl, cudaStream_t st) {
   constexpr int NT = BlendShape<TW, TH, PX, CH>::NT;
-  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH>;
+  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, CLEAN>;
   const int64_t grid = std::min<int64_t>(tile_end - tile_begin, resident_ctas<kern>(NT));
   kern<<<(unsigned)grid, NT, 0, st>>>(va, (uint32_t)tile_begin, (uint32_t)tile_end, counter,
                                       order, keys, recs, ranges, nb2, beta3, depth, alpha, stats,
@@ -502,6 +513,14 @@ void launch_blend_fwd(const ViewsArg& va, int tile_w, int tile_h, int px, int ch
                       Control* ctrl, cudaStream_t st) {
   blend_dispatch(va, tile_w, tile_h, px, chunk, 0, n_tiles, &ctrl->next_tile, order, keys, recs,
                  ranges, beta2, beta3, depth, alpha, stats, stats_stride, ctrl, st);
+}
+
+void launch_blend_fwd_clean(const ViewsArg& va, int64_t n_tiles, const uint64_t* keys,
+                            const GaussRec* recs, const uint2* ranges, float beta2, float beta3,
+                            float* depth, float* alpha, Control* ctrl, cudaStream_t st) {
+  if (n_tiles <= 0) return;
+  launch_tiles<8, 8, 2, 32, true>(va, 0, n_tiles, &ctrl->next_tile, nullptr, keys, recs, ranges,
+                                  -beta2 * kLog2e, beta3, depth, alpha, nullptr, 0, ctrl, st);
 }
 
 }  // namespace fe

@@ -20,10 +20,14 @@ void launch_preprocess_reference(int P, float n_std, const float* means, const f
                                  const float* rots, const LegacyMatrices& mats, int W, int H,
                                  float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
                                  TileRect* rects, uint32_t* touched, cudaStream_t st);
-void launch_legacy_records(const ViewsArg& va, int P, const float* means, const float* scales,
-                           const float* rots, const float* logw, const float* rotm,
-                           const float* trans, const float* rays, GaussRec* recs,
-                           cudaStream_t st);
+// Footprints (the reference's) and records of the legacy interface; with row_tot (gy + 1 zeroed
+// entries) also the key counts launch_tile_binning_emit takes, for rectangles without `foot`.
+void launch_legacy_preprocess(int P, float n_std, const float* means, const float* scales,
+                              const float* rots, const float* logw, const float* rotm,
+                              const float* trans, const float* rays, const LegacyMatrices& mats,
+                              int W, int H, float tan_fovx, float tan_fovy, int gx, int gy,
+                              GaussRec* recs, TileRect* rects, uint32_t* touched,
+                              unsigned long long* row_tot, Control* ctrl, cudaStream_t st);
 
 // binning.cu
 // Blocks used by the fixed-grid scan / sort kernels.
@@ -79,6 +83,11 @@ void launch_blend_fwd(const ViewsArg& va, int tile_w, int tile_h, int px, int ch
                       const uint2* ranges, float beta2,
                       float beta3, float* depth, float* alpha, float* stats, int64_t stats_stride,
                       Control* ctrl, cudaStream_t st);
+// launch_blend_fwd on 8x8 tiles with the outputs through nan_to_num (NaN and -inf to 0, +inf depth
+// to 10 and +inf alpha to 1), as the legacy interface's wrapper returns them.
+void launch_blend_fwd_clean(const ViewsArg& va, int64_t n_tiles, const uint64_t* keys,
+                            const GaussRec* recs, const uint2* ranges, float beta2, float beta3,
+                            float* depth, float* alpha, Control* ctrl, cudaStream_t st);
 // The blend over global tiles [tile_begin, tile_end) only, taking tiles from `counter` (zero at
 // launch); bands with their own counters may run concurrently on different streams.
 void launch_blend_fwd_band(const ViewsArg& va, int tile_w, int tile_h, int px, int chunk,

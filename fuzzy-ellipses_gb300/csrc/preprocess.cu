@@ -15,73 +15,6 @@
 
 namespace fe {
 
-// ------------------------------------------------------------------------------------------
-// Record builder, double precision (the legacy-interface records).
-// ------------------------------------------------------------------------------------------
-
-// U: upper-triangular precision factor (row-major 3x3, lower entries ignored), precision U U^T.
-// R: row-major camera rotation (rays_world = rays_cam @ R). t: camera centre.
-struct RecordInputs {
-  double m[3];
-  double U[9];
-  double w;
-  double R[9];
-  double t[3];
-};
-
-__device__ void build_camera_terms(const RecordInputs& in, double M[9], double Y[9],
-                                   V3<double>& pc) {
-  V3<double> p = v3(in.m[0] - in.t[0], in.m[1] - in.t[1], in.m[2] - in.t[2]);
-  pc = matvec(in.R, p);  // camera-frame mean
-  // M = U^T R^T:  a = M rays_cam = U^T (rays_cam @ R)
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      double s = 0.0;
-      for (int k = 0; k <= i; ++k) s += in.U[k * 3 + i] * in.R[j * 3 + k];
-      M[i * 3 + j] = s;
-    }
-  cofactor3(M, Y);
-}
-
-__device__ void write_record(const RecordInputs& in, const double M[9], const double Y[9],
-                             const V3<double>& pc, float fx, float fy, float cx, float cy,
-                             int H, int W, GaussRec* out) {
-  // Expansion centre: the projected mean when it is finite and near the image, else the image
-  // centre. Any centre is exact in real arithmetic; a nearby one keeps the float32 terms small.
-  double uc = 0.5 * W, vc = 0.5 * H;
-  const double pn = sqrt(dot(pc, pc));
-  if (fabs(pc.z) > 1e-6 * pn) {
-    double u0 = fx * pc.x / pc.z + cx;
-    double v0 = fy * pc.y / pc.z + cy;
-    if (isfinite(u0) && isfinite(v0)) {
-      uc = fmin(fmax(u0, -1.0 * W), 2.0 * W);
-      vc = fmin(fmax(v0, -1.0 * H), 2.0 * H);
-    }
-  }
-  const float ucf = (float)uc, vcf = (float)vc;
-  V3<double> r0 = v3(((double)ucf - cx) / fx, ((double)vcf - cy) / fy, 1.0);
-  V3<double> a0 = matvec(M, r0);
-  V3<double> a1 = v3(M[0] / fx, M[3] / fx, M[6] / fx);
-  V3<double> a2 = v3(M[1] / fy, M[4] / fy, M[7] / fy);
-  V3<double> b = matvec(M, pc);
-  V3<double> c0 = cross(r0, pc);
-  V3<double> cxv = v3(0.0, -pc.z / fx, pc.y / fx);
-  V3<double> cyv = v3(pc.z / fy, 0.0, -pc.x / fy);
-  V3<double> y0 = matvec(Y, c0), y1 = matvec(Y, cxv), y2 = matvec(Y, cyv);
-  GaussRec r;
-  r.a0[0] = a0.x; r.a0[1] = a0.y; r.a0[2] = a0.z;
-  r.a1[0] = a1.x; r.a1[1] = a1.y; r.a1[2] = a1.z;
-  r.a2[0] = a2.x; r.a2[1] = a2.y; r.a2[2] = a2.z;
-  r.b[0] = b.x; r.b[1] = b.y; r.b[2] = b.z;
-  r.y0[0] = y0.x; r.y0[1] = y0.y; r.y0[2] = y0.z;
-  r.y1[0] = y1.x; r.y1[1] = y1.y; r.y1[2] = y1.z;
-  r.y2[0] = y2.x; r.y2[1] = y2.y; r.y2[2] = y2.z;
-  r.uc = ucf;
-  r.vc = vcf;
-  r.c2 = (float)(in.w * kLog2eD);
-  *out = r;
-}
-
 // Clamp a floating tile coordinate into [lo, hi] before converting to int.
 __device__ __forceinline__ int clamp_tile(float x, int lo, int hi) {
   if (!(x > (float)lo)) return lo;   // also catches NaN
@@ -305,29 +238,30 @@ __device__ __forceinline__ void ref_get_rect(float px, float py, int r, int gx, 
   y1 = min(gy, max(0, f2i_trunc(__fdiv_rn(fs(fa(fa(py, rf), 8.f), 1.f), 8.f))));
 }
 
-__global__ void preprocess_reference_kernel(
-    int P, float n_std, const float* __restrict__ means, const float* __restrict__ scales,
-    const float* __restrict__ rots, LegacyMatrices mats, int W, int H, float tan_fovx,
-    float tan_fovy, float focal_x, float focal_y, int gx, int gy, int32_t* __restrict__ radii,
-    float* __restrict__ means2d, TileRect* __restrict__ rects, uint32_t* __restrict__ touched) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= P) return;
+struct RefFootprint {
+  int radius = 0;
+  float x = 0.f, y = 0.f;
+  TileRect rect{0, 0, 0, 0};
+  uint32_t area = 0;  // tiles of the rectangle; 0: culled
+};
+
+// The reference's projected centre, radius and 8x8-tile rectangle of one Gaussian.
+__device__ __forceinline__ RefFootprint reference_footprint(
+    int idx, float n_std, const float* __restrict__ means, const float* __restrict__ scales,
+    const float* __restrict__ rots, const LegacyMatrices& mats, int W, int H, float tan_fovx,
+    float tan_fovy, float focal_x, float focal_y, int gx, int gy) {
+  RefFootprint f;
   float viewmatrix[16], projmatrix[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
     viewmatrix[k] = mats.d_view ? mats.d_view[k] : mats.view[k];
     projmatrix[k] = mats.d_proj ? mats.d_proj[k] : mats.proj[k];
   }
-  radii[idx] = 0;
-  touched[idx] = 0;
-  rects[idx] = TileRect{0, 0, 0, 0};
-  means2d[2 * idx] = 0.f;
-  means2d[2 * idx + 1] = 0.f;
   const float px = means[3 * idx], py = means[3 * idx + 1], pz = means[3 * idx + 2];
 
   // in_frustum (auxiliary.h:144-169): near cull on the view-space depth.
   const float vz = tp_row(viewmatrix, 2, px, py, pz);
-  if (vz <= 0.2f) return;
+  if (vz <= 0.2f) return f;
   const float hx = tp_row(projmatrix, 0, px, py, pz);
   const float hy = tp_row(projmatrix, 1, px, py, pz);
   const float hw = tp_row(projmatrix, 3, px, py, pz);
@@ -371,7 +305,7 @@ __global__ void preprocess_reference_kernel(
   const float ca = fa(cov.c[0][0], 0.3f), cb = cov.c[0][1], cc = fa(cov.c[1][1], 0.3f);
 
   const float det = fs(fm(ca, cc), fm(cb, cb));
-  if (det == 0.0f) return;
+  if (det == 0.0f) return f;
   const float mid = fm(0.5f, fa(ca, cc));
   const float disc = __fsqrt_rn(fmaxf(0.1f, fs(fm(mid, mid), det)));
   const float l1 = fa(mid, disc), l2 = fs(mid, disc);
@@ -381,69 +315,172 @@ __global__ void preprocess_reference_kernel(
   int x0, y0, x1, y1;
   ref_get_rect(pix_x, pix_y, ir, gx, gy, x0, y0, x1, y1);
   const uint32_t area = (uint32_t)(x1 - x0) * (uint32_t)(y1 - y0);
-  if (area == 0) return;
-  radii[idx] = ir;
-  means2d[2 * idx] = pix_x;
-  means2d[2 * idx + 1] = pix_y;
-  rects[idx] = TileRect{(uint16_t)x0, (uint16_t)y0, (uint16_t)x1, (uint16_t)y1};
-  touched[idx] = area;
+  if (area == 0) return f;
+  f.radius = ir;
+  f.x = pix_x;
+  f.y = pix_y;
+  f.rect = TileRect{(uint16_t)x0, (uint16_t)y0, (uint16_t)x1, (uint16_t)y1};
+  f.area = area;
+  return f;
 }
 
-// Records for the legacy interface: precision from (scale, rotation) as the reference's
-// computeCov3D defines the covariance (Sigma = R diag(s^2) R^T with R from the unnormalised
-// quaternion formula), factorised as U = inv(chol(Sigma))^T; pose given as a rotation matrix.
-__global__ void legacy_records_kernel(ViewsArg va, int P, const float* __restrict__ means,
-                                      const float* __restrict__ scales,
-                                      const float* __restrict__ rots,
-                                      const float* __restrict__ logw,
-                                      const float* __restrict__ rotm,
-                                      const float* __restrict__ trans,
-                                      const float* __restrict__ rays,
-                                      GaussRec* __restrict__ recs) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P) return;
-  const ViewDev& V = view_at(va, 0);
-  // Pinhole intrinsics recovered from the ray buffer ((u-cx)/fx, (v-cy)/fy, 1): the slope between
-  // the first and last pixel of the first row and column, then the offset at pixel (0,0).
-  const int H = V.H, W = V.W;
-  const double sx = W > 1 ? ((double)rays[3 * (W - 1)] - rays[0]) / (W - 1) : 1.0 / V.fx;
-  const double sy = H > 1 ? ((double)rays[3 * (int64_t)(H - 1) * W + 1] - rays[1]) / (H - 1)
-                          : 1.0 / V.fy;
-  const float fx = (float)(1.0 / sx), fy = (float)(1.0 / sy);
-  const float cx = (float)(-(double)rays[0] / sx), cy = (float)(-(double)rays[1] / sy);
-  RecordInputs in;
-  for (int k = 0; k < 3; ++k) in.m[k] = means[3 * i + k];
-  in.w = logw[i];
+__global__ void preprocess_reference_kernel(
+    int P, float n_std, const float* __restrict__ means, const float* __restrict__ scales,
+    const float* __restrict__ rots, LegacyMatrices mats, int W, int H, float tan_fovx,
+    float tan_fovy, float focal_x, float focal_y, int gx, int gy, int32_t* __restrict__ radii,
+    float* __restrict__ means2d, TileRect* __restrict__ rects, uint32_t* __restrict__ touched) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= P) return;
+  const RefFootprint f = reference_footprint(idx, n_std, means, scales, rots, mats, W, H, tan_fovx,
+                                             tan_fovy, focal_x, focal_y, gx, gy);
+  radii[idx] = f.radius;
+  touched[idx] = f.area;
+  rects[idx] = f.rect;
+  means2d[2 * idx] = f.x;
+  means2d[2 * idx + 1] = f.y;
+}
+
+// Pinhole intrinsics recovered from the ray buffer ((u-cx)/fx, (v-cy)/fy, 1): the slope between
+// the first and last pixel of the first row and column, then the offset at pixel (0,0); float32
+// values as doubles, with the focal lengths' reciprocals. Even lanes take the x axis and odd lanes
+// the y axis (all 32 lanes call this).
+struct Intrinsics {
+  double fx, fy, cx, cy, ifx, ify;
+};
+
+__device__ __forceinline__ Intrinsics legacy_intrinsics(const float* __restrict__ rays, int W,
+                                                        int H, int lane) {
+  const int axis = lane & 1, n = axis ? H : W;
+  const int64_t last = axis ? 3 * (int64_t)(H - 1) * W + 1 : 3 * (int64_t)(W - 1);
+  const double r0 = rays[axis];
+  const double s = n > 1 ? ((double)rays[last] - r0) / (n - 1) : 1.0;
+  const double is = 1.0 / s;
+  const double f = (float)is, c = (float)(-r0 * is);
+  const double rf = 1.0 / f;
+  auto from = [&](double x, int src) { return __shfl_sync(0xffffffffu, x, src); };
+  return Intrinsics{from(f, 0), from(f, 1), from(c, 0), from(c, 1), from(rf, 0), from(rf, 1)};
+}
+
+// Record of the legacy interface: precision from (scale, rotation) as the reference's computeCov3D
+// defines the covariance (Sigma = R diag(s^2) R^T with R from the unnormalised quaternion formula),
+// factorised as U = inv(chol(Sigma))^T; pose given as a rotation matrix; float64.
+__device__ __forceinline__ void legacy_record(int i, const float* __restrict__ means,
+                                              const float* __restrict__ scales,
+                                              const float* __restrict__ rots,
+                                              const float* __restrict__ logw,
+                                              const float* __restrict__ rotm,
+                                              const float* __restrict__ trans, const Intrinsics& in,
+                                              int W, int H, GaussRec* out) {
   const double r = rots[4 * i], x = rots[4 * i + 1], y = rots[4 * i + 2], z = rots[4 * i + 3];
   const double Rq[9] = {1 - 2 * (y * y + z * z), 2 * (x * y - r * z), 2 * (x * z + r * y),
                         2 * (x * y + r * z), 1 - 2 * (x * x + z * z), 2 * (y * z - r * x),
                         2 * (x * z - r * y), 2 * (y * z + r * x), 1 - 2 * (x * x + y * y)};
-  const double s[3] = {scales[3 * i], scales[3 * i + 1], scales[3 * i + 2]};
-  double S[9];
-  for (int a = 0; a < 3; ++a)
-    for (int c = 0; c < 3; ++c) {
-      double acc = 0.0;
-      for (int k = 0; k < 3; ++k) acc += Rq[a * 3 + k] * s[k] * s[k] * Rq[c * 3 + k];
-      S[a * 3 + c] = acc;
-    }
-  // Cholesky S = L L^T, then U = (L^-1)^T.
-  const double l00 = sqrt(S[0]);
-  const double l10 = S[3] / l00, l20 = S[6] / l00;
-  const double l11 = sqrt(S[4] - l10 * l10);
-  const double l21 = (S[7] - l20 * l10) / l11;
-  const double l22 = sqrt(S[8] - l20 * l20 - l21 * l21);
-  const double i00 = 1.0 / l00, i11 = 1.0 / l11, i22 = 1.0 / l22;
-  const double i10 = -l10 * i00 / l11;
-  const double i21 = -l21 * i11 / l22;
-  const double i20 = -(l20 * i00 + l21 * i10) / l22;
-  const double U[9] = {i00, i10, i20, 0.0, i11, i21, 0.0, 0.0, i22};
-  for (int k = 0; k < 9; ++k) in.U[k] = U[k];
-  for (int k = 0; k < 9; ++k) in.R[k] = rotm[k];
-  for (int k = 0; k < 3; ++k) in.t[k] = trans[k];
+  double Rs[9];  // Rq diag(s^2)
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double s = scales[3 * i + k];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) Rs[3 * a + k] = Rq[3 * a + k] * (s * s);
+  }
+  auto cov = [&](int a, int c) {
+    return Rs[3 * a] * Rq[3 * c] + Rs[3 * a + 1] * Rq[3 * c + 1] + Rs[3 * a + 2] * Rq[3 * c + 2];
+  };
+  // Cholesky S = L L^T with the reciprocals i_kk of L's diagonal, then U = (L^-1)^T.
+  const double i00 = rsqrt(cov(0, 0));
+  const double l10 = cov(1, 0) * i00, l20 = cov(2, 0) * i00;
+  const double i11 = rsqrt(cov(1, 1) - l10 * l10);
+  const double l21 = (cov(2, 1) - l20 * l10) * i11;
+  const double i22 = rsqrt(cov(2, 2) - l20 * l20 - l21 * l21);
+  const double i10 = -l10 * i00 * i11;
+  const double i21 = -l21 * i11 * i22;
+  const double i20 = -(l20 * i00 + l21 * i10) * i22;
+  double R[9], t[3];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) R[k] = rotm[k];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) t[k] = trans[k];
+  const V3<double> pc =
+      matvec(R, v3((double)means[3 * i] - t[0], (double)means[3 * i + 1] - t[1],
+                   (double)means[3 * i + 2] - t[2]));  // camera-frame mean
+  // M = U^T R^T:  a = M rays_cam = U^T (rays_cam @ R)
   double M[9], Y[9];
-  V3<double> pc;
-  build_camera_terms(in, M, Y, pc);
-  write_record(in, M, Y, pc, fx, fy, cx, cy, H, W, &recs[i]);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    M[j] = i00 * R[3 * j];
+    M[3 + j] = i10 * R[3 * j] + i11 * R[3 * j + 1];
+    M[6 + j] = i20 * R[3 * j] + i21 * R[3 * j + 1] + i22 * R[3 * j + 2];
+  }
+  cofactor3(M, Y);
+  // Expansion centre: the projected mean when it is finite and near the image, else the image
+  // centre. Any centre is exact in real arithmetic; a nearby one keeps the float32 terms small.
+  double uc = 0.5 * W, vc = 0.5 * H;
+  if (pc.z * pc.z > 1e-12 * dot(pc, pc)) {
+    const double iz = 1.0 / pc.z;
+    const double u0 = in.fx * pc.x * iz + in.cx, v0 = in.fy * pc.y * iz + in.cy;
+    if (isfinite(u0) && isfinite(v0)) {
+      uc = fmin(fmax(u0, -1.0 * W), 2.0 * W);
+      vc = fmin(fmax(v0, -1.0 * H), 2.0 * H);
+    }
+  }
+  const float ucf = (float)uc, vcf = (float)vc;
+  const V3<double> r0 = v3(((double)ucf - in.cx) * in.ifx, ((double)vcf - in.cy) * in.ify, 1.0);
+  const V3<double> a0 = matvec(M, r0), b = matvec(M, pc), c0 = cross(r0, pc);
+  const V3<double> y0 = matvec(Y, c0);
+  const V3<double> y1 = matvec(Y, v3(0.0, -pc.z * in.ifx, pc.y * in.ifx));
+  const V3<double> y2 = matvec(Y, v3(pc.z * in.ify, 0.0, -pc.x * in.ify));
+  GaussRec g;
+  g.a0[0] = a0.x; g.a0[1] = a0.y; g.a0[2] = a0.z;
+  g.a1[0] = M[0] * in.ifx; g.a1[1] = M[3] * in.ifx; g.a1[2] = M[6] * in.ifx;
+  g.a2[0] = M[1] * in.ify; g.a2[1] = M[4] * in.ify; g.a2[2] = M[7] * in.ify;
+  g.b[0] = b.x; g.b[1] = b.y; g.b[2] = b.z;
+  g.y0[0] = y0.x; g.y0[1] = y0.y; g.y0[2] = y0.z;
+  g.y1[0] = y1.x; g.y1[1] = y1.y; g.y1[2] = y1.z;
+  g.y2[0] = y2.x; g.y2[1] = y2.y; g.y2[2] = y2.z;
+  g.uc = ucf;
+  g.vc = vcf;
+  g.c2 = (float)(logw[i] * kLog2eD);
+  *out = g;
+}
+
+// Footprints and records of the legacy interface, 32 Gaussians per block: one warp takes their
+// reference footprints (float32) while the other builds their records (float64). GB300 issues a
+// float64 warp instruction every 16 cycles of an SM, so the records want many SMs and few
+// instructions: in blocks of 128 on 8 SMs, with a division wherever the formula has one, 1000
+// records took 22 us after 5 us of footprints; spread over 32 SMs, with shared reciprocals, both
+// take 12.6 us together.
+// With row_tot (zeroed) the keys of every tile row and the total are counted as
+// launch_tile_binning_emit expects them.
+__global__ void __launch_bounds__(64) legacy_preprocess_kernel(
+    int P, float n_std, const float* __restrict__ means, const float* __restrict__ scales,
+    const float* __restrict__ rots, const float* __restrict__ logw, const float* __restrict__ rotm,
+    const float* __restrict__ trans, const float* __restrict__ rays, LegacyMatrices mats, int W,
+    int H, float tan_fovx, float tan_fovy, float focal_x, float focal_y, int gx, int gy,
+    GaussRec* __restrict__ recs, TileRect* __restrict__ rects, uint32_t* __restrict__ touched,
+    unsigned long long* __restrict__ row_tot, Control* __restrict__ ctrl) {
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 32 + lane;
+  if (threadIdx.x < 32) {
+    uint32_t keys = 0;
+    if (i < P) {
+      const RefFootprint f = reference_footprint(i, n_std, means, scales, rots, mats, W, H, tan_fovx,
+                                                 tan_fovy, focal_x, focal_y, gx, gy);
+      rects[i] = f.rect;
+      touched[i] = keys = f.area;
+      if (row_tot && f.area)
+        for (int y = f.rect.y0; y < f.rect.y1; ++y)
+          atomicAdd(&row_tot[y], (unsigned long long)(f.rect.x1 - f.rect.x0));
+    }
+    if (row_tot) {
+      unsigned long long sum = keys;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0 && sum) atomicAdd(&ctrl->want_keys, sum);
+    }
+  } else {
+    // (the divisions of the intrinsics, one axis per lane)
+    const Intrinsics in = legacy_intrinsics(rays, W, H, lane);
+    if (i < P) legacy_record(i, means, scales, rots, logw, rotm, trans, in, W, H, &recs[i]);
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -477,13 +514,19 @@ void launch_preprocess_reference(int P, float n_std, const float* means, const f
       gy, radii, means2d, rects, touched);
 }
 
-void launch_legacy_records(const ViewsArg& va, int P, const float* means, const float* scales,
-                           const float* rots, const float* logw, const float* rotm,
-                           const float* trans, const float* rays, GaussRec* recs,
-                           cudaStream_t st) {
+void launch_legacy_preprocess(int P, float n_std, const float* means, const float* scales,
+                              const float* rots, const float* logw, const float* rotm,
+                              const float* trans, const float* rays, const LegacyMatrices& mats,
+                              int W, int H, float tan_fovx, float tan_fovy, int gx, int gy,
+                              GaussRec* recs, TileRect* rects, uint32_t* touched,
+                              unsigned long long* row_tot, Control* ctrl, cudaStream_t st) {
   if (P <= 0) return;
-  legacy_records_kernel<<<(P + 127) / 128, 128, 0, st>>>(va, P, means, scales, rots, logw, rotm,
-                                                         trans, rays, recs);
+  // rasterizer_impl.cu:205-206 (float arithmetic on the host).
+  const float fx = (float)W / (2.0f * tan_fovx);
+  const float fy = (float)H / (2.0f * tan_fovy);
+  legacy_preprocess_kernel<<<(P + 31) / 32, 64, 0, st>>>(
+      P, n_std, means, scales, rots, logw, rotm, trans, rays, mats, W, H, tan_fovx, tan_fovy, fx,
+      fy, gx, gy, recs, rects, touched, row_tot, ctrl);
 }
 
 }  // namespace fe

@@ -167,7 +167,7 @@ PROTOTYPES = {
     "fe_render_bwd_xla": (None, [P, P, P, ctypes.c_size_t, P]),
     "fe_rasterize_legacy_xla": (None, [P, P, P, ctypes.c_size_t, P]),
     "fe_rasterize_legacy": (ctypes.c_int, [ctypes.POINTER(LegacyDesc)] + [P] * 11 + [P]),
-    "fe_rasterize_legacy_host": (ctypes.c_int, [ctypes.POINTER(LegacyDesc)] + [P] * 11 + [P]),
+    "fe_rasterize_legacy_host": (ctypes.c_int, [ctypes.POINTER(LegacyDesc)] + [P] * 9 + [I32, P, P, P]),
     "fe_reference_binning": (ctypes.c_int, [I32, I32, I32, F32, P, P, P, P, P, F32, F32,
                                             P, P, P, P, I64, P, ctypes.POINTER(I64), P]),
     "fe_batch_create": (ctypes.c_int, [ctypes.POINTER(RenderDesc), ctypes.POINTER(SceneEntry), I32,

@@ -446,12 +446,12 @@ def rasterize(means3D, scales, rotations, weights, camera_rays, camera_rot, came
         bufs += [_as_dev(view, dev), _as_dev(proj, dev)]
         N.check(lib.fe_rasterize_legacy(ctypes.byref(d), *[_ptr(b) for b in bufs], _ptr(z),
                                         _ptr(alpha), _stream()))
+        z = torch.nan_to_num(z, posinf=10.0, neginf=0.0)        # __init__.py:233
+        alpha = torch.nan_to_num(alpha, posinf=1.0, neginf=0.0)  # __init__.py:234
     else:
         N.check(lib.fe_rasterize_legacy_host(ctypes.byref(d), *[_ptr(b) for b in bufs],
-                                             view.ctypes.data, proj.ctypes.data, _ptr(z),
+                                             view.ctypes.data, proj.ctypes.data, 1, _ptr(z),
                                              _ptr(alpha), _stream()))
-    z = torch.nan_to_num(z, posinf=10.0, neginf=0.0)        # __init__.py:233
-    alpha = torch.nan_to_num(alpha, posinf=1.0, neginf=0.0)  # __init__.py:234
     return z, alpha
 
 

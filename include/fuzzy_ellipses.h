@@ -225,13 +225,14 @@ int fe_rasterize_legacy(const fe_legacy_desc *desc, const float *d_means, const 
                         const float *d_viewmatrix, const float *d_projmatrix, float *d_out_z,
                         float *d_out_alpha, fe_stream_t stream);
 /* fe_rasterize_legacy with the view and projection matrices in host memory, read during the call
- * and passed to the kernels by value. */
+ * and passed to the kernels by value. clean != 0: the outputs as the reference's wrapper returns
+ * them (fuzzy_ellipses/__init__.py:233-234): NaN and -inf become 0, +inf depth 10 and +inf alpha 1. */
 int fe_rasterize_legacy_host(const fe_legacy_desc *desc, const float *d_means,
                              const float *d_weights, const float *d_scales,
                              const float *d_rotations, const float *d_camera_rays,
                              const float *d_camera_rot, const float *d_camera_trans,
-                             const float *h_viewmatrix, const float *h_projmatrix, float *d_out_z,
-                             float *d_out_alpha, fe_stream_t stream);
+                             const float *h_viewmatrix, const float *h_projmatrix, int32_t clean,
+                             float *d_out_z, float *d_out_alpha, fe_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Batched renders: many scenes and cameras in one launch sequence.

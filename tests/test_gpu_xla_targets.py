@@ -85,3 +85,35 @@ def test_legacy_target_matches_rasterize(cuda_device):
     z = torch.nan_to_num(z, posinf=10.0, neginf=0.0)
     a = torch.nan_to_num(a, posinf=1.0, neginf=0.0)
     assert torch.equal(z, z0.reshape(H, W)) and torch.equal(a, a0.reshape(H, W))
+
+
+@pytest.mark.parametrize("n,H,W", [(33, 40, 50), (1000, 37, 129), (4200, 64, 64)])
+def test_rasterize_cleans_its_outputs(cuda_device, n, H, W):
+    """rasterize() returns nan_to_num of the raw legacy entry's outputs, with degenerate and
+    non-finite Gaussians among the inputs, on both binning paths (4200 Gaussians over 8 tile rows
+    take emission + sort)."""
+    rng = np.random.default_rng(n)
+    f = 60.0
+    z = rng.uniform(0.5, 1.5, n)
+    means = np.stack([rng.uniform(-0.3, 0.3, n) * z, rng.uniform(-0.3, 0.3, n) * z, z], 1)
+    scales = np.exp(rng.uniform(np.log(0.005), np.log(0.03), (n, 3)))
+    quats = rng.standard_normal((n, 4))
+    quats /= np.linalg.norm(quats, axis=1, keepdims=True)
+    logw = rng.normal(0, 0.5, n)
+    logw[::17], logw[1::29], logw[2::31] = np.nan, np.inf, -np.inf
+    scales[3::23, 1] = 0.0
+    rays = np.stack(list(np.meshgrid((np.arange(W) - W / 2) / f, (np.arange(H) - H / 2) / f)) +
+                    [np.ones((H, W))], -1).reshape(-1, 3)
+    ins = [to_dev(x.astype(np.float32), cuda_device)
+           for x in (means, logw, scales, quats, rays, np.eye(3), np.zeros(3))]
+    m, w, s, q, r, rot, trans = ins
+    zc, ac = fe.rasterize(m, s, q, w, r, rot, trans, H, W, f, f, W / 2, H / 2, 0.01, 4.5)
+    tx, ty, view, proj = fe.api._legacy_scalars(H, W, f, f, W / 2, H / 2, 0.01, 4.5)
+    d = N.LegacyDesc(H, W, n, float(tx), float(ty))
+    zr, ar = torch.empty_like(zc), torch.empty_like(ac)
+    bufs = ins + [to_dev(view, cuda_device), to_dev(proj, cuda_device), zr, ar]
+    N.check(N.load().fe_rasterize_legacy(ctypes.byref(d), *[b.data_ptr() for b in bufs],
+                                         torch.cuda.current_stream().cuda_stream))
+    assert not (torch.isfinite(zr).all() and torch.isfinite(ar).all())
+    assert torch.equal(zc, torch.nan_to_num(zr, posinf=10.0, neginf=0.0))
+    assert torch.equal(ac, torch.nan_to_num(ar, posinf=1.0, neginf=0.0))
