@@ -230,6 +230,7 @@ struct Pipeline {
   bool radix;  // FE_FLAG_RADIX_BINNING: emit + sort even where tile-major binning applies
   bool rect_binning;  // FE_FLAG_RECT_BINNING: every tile of each footprint's rectangle
   bool heavy_first;  // FE_FLAG_HEAVY_TILES_FIRST: work-class tile lists for the blend
+  bool tile_lists;   // the binning writes the lists: for the blend, or for a backward
   int cull_mode;
   float cull_param;
   float beta2, beta3;
@@ -524,9 +525,6 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
   if (!means || !prec || !logw || !quat || !trans || !depth || !stats || !gmeans || !gprec ||
       !glogw)
     return fail(FE_ERR_INVALID_ARGUMENT, "NULL pointer");
-  FE_CUDA(cudaMemsetAsync(gmeans, 0, sizeof(float) * 3 * n, st));
-  FE_CUDA(cudaMemsetAsync(gprec, 0, sizeof(float) * 9 * n, st));
-  FE_CUDA(cudaMemsetAsync(glogw, 0, sizeof(float) * n, st));
   Arena* a = nullptr;
   rc = arena_for(st, &a);
   if (rc) return rc;
@@ -538,8 +536,8 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
   rc = run_binning(p, p.n_rec * p.n_tiles, a->rec, a->keys, a->h_pinned, true, st, rs, ks, cap,
                    sorted);
   if (rc) return rc;
-  FE_CUDA(cudaMemsetAsync(rs.rgrad, 0, sizeof(RecGrad) * (size_t)p.n_rec, st));
-  launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, depth,
+  launch_bwd_zero(gmeans, gprec, glogw, n, rs.rgrad, p.n_rec, rs.ctrl, st);
+  launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, rs.order, sorted, rs.ranges, rs.recs, depth,
                    stats, p.n_pix, gdepth, galpha, p.beta2, p.beta3, rs.rgrad, rs.ctrl, st);
   launch_record_vjp(p.va, p.n_rec, means, prec, p.quat, p.trans, rs.recs, rs.rgrad, gmeans, gprec,
                     glogw, st);
@@ -1267,6 +1265,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   p.radix = (b->desc.flags & FE_FLAG_RADIX_BINNING) != 0;
   p.rect_binning = (b->desc.flags & FE_FLAG_RECT_BINNING) != 0;
   p.heavy_first = (b->desc.flags & FE_FLAG_HEAVY_TILES_FIRST) != 0;
+  p.tile_lists = p.heavy_first || b->keep_binning;
   p.cull_mode = b->desc.cull_mode;
   p.cull_param = b->desc.cull_param;
   p.beta2 = b->desc.beta2;
@@ -1278,6 +1277,13 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
 // The work-class tile lists of the last binning, when it was tile-major (else NULL).
 static const uint32_t* batch_order(const fe_batch* b, const Pipeline& p) {
   return (p.heavy_first && !p.radix && b->rows.ok) ? b->rs.order : nullptr;
+}
+
+// The same for the backward, which always takes the heaviest tiles first where the binning lists
+// them: its warps are each on a tile for 30 us at the median of the 16-view workload and 100 us at
+// the heaviest, so index order leaves a long tail (16-view step 503 -> 477 us, lists included).
+static const uint32_t* bwd_order(const fe_batch* b, const Pipeline& p) {
+  return (!p.radix && b->rows.ok) ? b->rs.order : nullptr;
 }
 
 // Binning of a batch. With exact key sizing the key count is read back after the scan (one
@@ -1314,7 +1320,7 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
   if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
                              p.tile_w, p.tile_h, rs.row_tot, b->cap, rs.ctrl, rs.ranges,
-                             rs.tile_view, ks.keys_a, p.heavy_first ? rs.order : nullptr,
+                             rs.tile_view, ks.keys_a, p.tile_lists ? rs.order : nullptr,
                              p.n_tiles, st);
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
     b->sorted = ks.keys_a;
@@ -1553,21 +1559,17 @@ int fe_batch_bwd(fe_batch* b, const float* means, const float* prec, const float
     return fail(FE_ERR_INVALID_ARGUMENT, "NULL argument");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_);
   Pipeline p = batch_pipeline(b, means, prec, logw);
-  FE_CUDA(cudaMemsetAsync(gmeans, 0, sizeof(float) * 3 * (size_t)b->n_gauss, st));
-  FE_CUDA(cudaMemsetAsync(gprec, 0, sizeof(float) * 9 * (size_t)b->n_gauss, st));
-  FE_CUDA(cudaMemsetAsync(glogw, 0, sizeof(float) * (size_t)b->n_gauss, st));
-  if (b->keep_binning && b->binned && b->binned_for[0] == means && b->binned_for[1] == prec &&
-      b->binned_for[2] == logw) {
-    // Reuse the forward's binning; only the blend's tile counter must start again at zero.
-    FE_CUDA(cudaMemsetAsync(&b->rs.ctrl->next_tile, 0, sizeof(uint32_t), st));
-  } else {
+  p.tile_lists = true;
+  // (the forward's binning is reused when it was kept for these arrays)
+  if (!(b->keep_binning && b->binned && b->binned_for[0] == means && b->binned_for[1] == prec &&
+        b->binned_for[2] == logw)) {
     b->binned = false;
     int rc = batch_binning(b, p, st, nullptr);
     if (rc) return rc;
     note_binning(b, means, prec, logw);
   }
-  FE_CUDA(cudaMemsetAsync(b->rs.rgrad, 0, sizeof(RecGrad) * (size_t)p.n_rec, st));
-  launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, b->sorted, b->rs.ranges, b->rs.recs,
+  launch_bwd_zero(gmeans, gprec, glogw, b->n_gauss, b->rs.rgrad, p.n_rec, b->rs.ctrl, st);
+  launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, bwd_order(b, p), b->sorted, b->rs.ranges, b->rs.recs,
                    depth, stats, p.n_pix, gdepth, galpha, p.beta2, p.beta3, b->rs.rgrad,
                    b->rs.ctrl, st);
   launch_record_vjp(p.va, p.n_rec, means, prec, p.quat, p.trans, b->rs.recs, b->rs.rgrad, gmeans,

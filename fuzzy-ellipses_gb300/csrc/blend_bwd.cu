@@ -46,16 +46,37 @@ struct alignas(16) BwdSlice {
   float plane[4][TH * ROW];
 };
 
-// Persistent warps: each warp takes a tile from the device counter, stages the tile's pixel data
-// in its shared-memory slice and processes the tile's keys in groups of up to 32. A group of n
+// Zeroes what the backward accumulates into, and its work counter, in one launch (a memset each
+// took five, about 1.5 us apiece).
+__global__ void __launch_bounds__(256) bwd_zero_kernel(float* __restrict__ gmeans,
+                                                       float* __restrict__ gprec,
+                                                       float* __restrict__ glogw, int64_t n_gauss,
+                                                       RecGrad* __restrict__ rgrad, int64_t n_rec,
+                                                       Control* __restrict__ ctrl) {
+  const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  if (first == 0) ctrl->next_tile = 0u;
+  float4* r = reinterpret_cast<float4*>(rgrad);
+  for (int64_t i = first; i < n_rec * (int64_t)(sizeof(RecGrad) / sizeof(float4)); i += step)
+    r[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int64_t i = first; i < 9 * n_gauss; i += step) {  // (callers' buffers: float alignment)
+    gprec[i] = 0.f;
+    if (i < 3 * n_gauss) gmeans[i] = 0.f;
+    if (i < n_gauss) glogw[i] = 0.f;
+  }
+}
+
+// Persistent warps: each warp takes an item from the device counter -- a tile, or one of the
+// 2^seg_bits parts of it, which take its groups of 32 keys in turn --, stages the tile's pixel data
+// in its shared-memory slice and processes the item's keys in groups of up to 32. A group of n
 // keys gets s = 32 / n lanes per key (s a power of two), which split the tile's rows; their
 // partial sums are combined with shuffles. Pixels are evaluated in adjacent pairs with packed
 // f32x2 arithmetic (one instruction for both pixels; rcp and ex2 per pixel).
 template <int TW, int TH>
 __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
-    ViewsArg va, uint32_t n_tiles, const uint64_t* __restrict__ keys,
-    const uint2* __restrict__ ranges, const GaussRec* __restrict__ recs,
-    const float* __restrict__ depth, const float* __restrict__ stats, int64_t stride,
+    ViewsArg va, uint32_t n_tiles, int seg_bits, const uint32_t* __restrict__ order,
+    const uint64_t* __restrict__ keys, const uint2* __restrict__ ranges,
+    const GaussRec* __restrict__ recs, const float* __restrict__ depth, const float* __restrict__ stats, int64_t stride,
     const float* __restrict__ gdepth, const float* __restrict__ galpha, float nb2, float beta3,
     float beta2, RecGrad* __restrict__ rgrad, Control* ctrl) {
   using Slice = BwdSlice<TW, TH>;
@@ -66,14 +87,42 @@ __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
   const f2_t B3 = f2_pack(beta3, beta3), NB2 = f2_pack(nb2, nb2);
   const f2_t NEGB2 = f2_pack(-beta2, -beta2), TWO = f2_pack(2.f, 2.f);
   const f2_t B3L = f2_pack(beta3 * kLn2, beta3 * kLn2), FOUR = f2_pack(4.f, 4.f);
+  // With the work-class lists (see blend_fwd_kernel) tiles are taken heaviest class first: lane c
+  // holds the work index of class c's first tile.
+  uint32_t cls_first = 0;
+  bool listed = false;
+  if (order) {
+    const uint32_t in_class = lane < kTileClasses ? ctrl->tile_class[lane] : 0u;
+    uint32_t incl = in_class;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(full, incl, o);
+      if (lane >= o) incl += y;
+    }
+    cls_first = incl - in_class;
+    listed = __shfl_sync(full, incl, 31) == n_tiles;
+  }
   for (;;) {
-    uint32_t tile = 0;
-    if (lane == 0) tile = atomicAdd(&ctrl->next_tile, 1u);
-    tile = __shfl_sync(full, tile, 0);
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(&ctrl->next_tile, 1u);
+    item = __shfl_sync(full, item, 0);
+    uint32_t tile = item >> seg_bits;
     if (tile >= n_tiles) break;
-    const uint2 range = ranges[tile];
-    if (range.y <= range.x) continue;
-    const int vi = view_of_tile(va, tile);
+    uint2 range;
+    int vi;
+    if (listed) {
+      const int c = 31 - __clz(__ballot_sync(full, lane < kTileClasses && cls_first <= tile));
+      const uint4 e = reinterpret_cast<const uint4*>(order)[(int64_t)c * n_tiles + tile -
+                                                            __shfl_sync(full, cls_first, c)];
+      tile = e.x;
+      range = make_uint2(e.y, e.z);
+      vi = (int)e.w;
+    } else {
+      range = ranges[tile];
+      vi = view_of_tile(va, tile);
+    }
+    const uint32_t seg = item & ((1u << seg_bits) - 1u);
+    if (range.y <= range.x + 32u * seg) continue;
     const ViewDev& V = view_at(va, vi);
     if (V.flags & FE_VIEW_NO_GRAD) continue;
     const int lt = (int)(tile - V.tile_base);
@@ -99,7 +148,14 @@ __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
     }
     __syncwarp();
 
-    for (uint32_t base = range.x, step = 0; base < range.y; base += step) {
+    for (uint32_t base = range.x + 32u * seg, group = base, step = 0; base < range.y;
+         base += step) {
+      // (the item's next group of 32 keys)
+      if (base == group + 32u) {
+        base += 32u * ((1u << seg_bits) - 1u);
+        group = base;
+        if (base >= range.y) break;
+      }
       // Groups of 32 keys, then the rest; a rest of p + a keys (p a power of two of at least 8,
       // a <= p / 2) runs as p keys and then a, which gives each group more lanes per key: 20
       // keys take 8 + 2 row steps per lane as 16 + 4 instead of 16 as one group (one lane per
@@ -425,31 +481,40 @@ __global__ void record_vjp_kernel(ViewsArg va, int64_t n_rec, const float* __res
 }
 
 template <int TW, int TH>
-void launch_bwd_tiles(const ViewsArg& va, int64_t n_tiles, const uint64_t* keys,
-                      const uint2* ranges, const GaussRec* recs, const float* depth,
+void launch_bwd_tiles(const ViewsArg& va, int64_t n_tiles, const uint32_t* order,
+                      const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
+                      const float* depth,
                       const float* stats, int64_t stride, const float* gdepth,
                       const float* galpha, float beta2, float beta3, RecGrad* rgrad,
                       Control* ctrl, cudaStream_t st) {
   constexpr auto kern = blend_bwd_kernel<TW, TH>;
   const int resident = resident_ctas<kern>(32 * kBwdWarps);
+  // Key groups of a tile shared over 2^bits items while the tiles give each resident warp fewer
+  // than three: a launch of few tiles is as long as its heaviest one (20 views of 128x128, 1280
+  // tiles: 60 us whole, 45 at two items per warp, 28 at three or more), while a launch of many
+  // would only take more empty items (8 views of 640x480 of 40 Gaussians, 9600 tiles: step 128.5
+  // us whole, 131 halved).
+  int bits = 0;
+  while (bits < 3 && (n_tiles << bits) < 3 * (int64_t)resident * kBwdWarps) ++bits;
+  const int64_t items = n_tiles << bits;
   const int64_t grid =
-      std::max<int64_t>(1, std::min<int64_t>((n_tiles + kBwdWarps - 1) / kBwdWarps, resident));
-  kern<<<(unsigned)grid, 32 * kBwdWarps, 0, st>>>(va, (uint32_t)n_tiles, keys, ranges, recs, depth,
-                                                  stats, stride, gdepth, galpha, -beta2 * kLog2e,
-                                                  beta3, beta2, rgrad, ctrl);
+      std::max<int64_t>(1, std::min<int64_t>((items + kBwdWarps - 1) / kBwdWarps, resident));
+  kern<<<(unsigned)grid, 32 * kBwdWarps, 0, st>>>(va, (uint32_t)n_tiles, bits, order, keys, ranges,
+                                                  recs, depth, stats, stride, gdepth, galpha,
+                                                  -beta2 * kLog2e, beta3, beta2, rgrad, ctrl);
 }
 
 }  // namespace
 
 
 void launch_blend_bwd(const ViewsArg& va, int tile_w, int tile_h, int64_t n_tiles,
-                      const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
+                      const uint32_t* order, const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
                       const float* depth, const float* stats, int64_t stats_stride,
                       const float* grad_depth, const float* grad_alpha, float beta2, float beta3,
                       RecGrad* rgrad, Control* ctrl, cudaStream_t st) {
   if (n_tiles <= 0) return;
 #define FE_BWD(TW_, TH_)                                                                       \
-  launch_bwd_tiles<TW_, TH_>(va, n_tiles, keys, ranges, recs, depth, stats, stats_stride,     \
+  launch_bwd_tiles<TW_, TH_>(va, n_tiles, order, keys, ranges, recs, depth, stats, stats_stride,     \
                              grad_depth, grad_alpha, beta2, beta3, rgrad, ctrl, st)
   if (tile_w == 8 && tile_h == 8)
     FE_BWD(8, 8);
@@ -458,6 +523,14 @@ void launch_blend_bwd(const ViewsArg& va, int tile_w, int tile_h, int64_t n_tile
   else
     FE_BWD(16, 16);
 #undef FE_BWD
+}
+
+void launch_bwd_zero(float* gmeans, float* gprec, float* glogw, int64_t n_gauss, RecGrad* rgrad,
+                     int64_t n_rec, Control* ctrl, cudaStream_t st) {
+  const int64_t work = std::max(9 * n_gauss, 6 * n_rec);
+  const int64_t blocks = std::min<int64_t>(std::max<int64_t>((work + 255) / 256, 1), 152 * 8);
+  bwd_zero_kernel<<<(unsigned)blocks, 256, 0, st>>>(gmeans, gprec, glogw, n_gauss, rgrad, n_rec,
+                                                    ctrl);
 }
 
 void launch_record_vjp(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,

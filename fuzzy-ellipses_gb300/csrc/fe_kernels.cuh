@@ -100,11 +100,15 @@ void launch_blend_fwd_band(const ViewsArg& va, int tile_w, int tile_h, int px, i
 // Tile records are built per key from the Gaussian records (fe_tilerec.cuh), as in the forward;
 // each tile's per-pixel terms are formed from depth, the forward's statistics (stats, stride) and
 // the cotangents (NULL = zero) when the tile is staged.
+// `order`: as launch_blend_fwd.
 void launch_blend_bwd(const ViewsArg& va, int tile_w, int tile_h, int64_t n_tiles,
-                      const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
+                      const uint32_t* order, const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
                       const float* depth, const float* stats, int64_t stats_stride,
                       const float* grad_depth, const float* grad_alpha, float beta2, float beta3,
                       RecGrad* rgrad, Control* ctrl, cudaStream_t st);
+// Zeroes the gradients (n_gauss Gaussians), the record gradients and the blend's work counter.
+void launch_bwd_zero(float* gmeans, float* gprec, float* glogw, int64_t n_gauss, RecGrad* rgrad,
+                     int64_t n_rec, Control* ctrl, cudaStream_t st);
 // Gradients are accumulated (atomically) into gmeans/gprec/glogw, which must be zeroed first.
 void launch_record_vjp(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
                        const float* quat, const float* trans, const GaussRec* recs,
