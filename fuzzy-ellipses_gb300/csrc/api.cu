@@ -246,11 +246,24 @@ constexpr int kRowPlanSmallN = 4096;
 constexpr int kRowPlanLargeN = 16384;
 constexpr int kRowPlanBlocks = 152;  // row blocks that fill a GB300 (its SM count)
 
+// Above kSegMinN Gaussians (of the largest view) the records are taken in segments, a block per
+// tile row and segment (launch_seg_binning): per call, one view of 640x480, segments against a
+// block per row, 1100 Gaussians 60 / 53 us, 2000 73 / 68, 2600 85 / 86, 4000 102 / 119; against
+// emit + sort 8000 157 / 188, 24000 at 1280x720 323 / 357, 50000 167 / 188. Its two passes test every
+// record against every row, where emit + sort works per key: at 1280x720 the two meet near 150000
+// Gaussians, hence the limit on rows x records. Up to 32 views (beyond, each block's sum over the
+// rows before it would be quadratic).
+constexpr int64_t kSegTests = INT64_C(1) << 23;
+constexpr int kSegMinN = 2500;
+
 struct RowPlan {
-  bool ok = false;
+  bool ok = false;     // a block per tile row is the plan
   int max_gy = 0;
   int max_gx = 0;
   int n_views = 0;
+  bool plain = false;  // a block per tile row applies
+  int segs = 0;        // > 0: in segments of the records instead (launch_seg_binning)
+  bool tiled() const { return ok || segs > 0; }
 };
 
 RowPlan row_plan(const ViewDev* views, int n_views) {
@@ -271,7 +284,19 @@ RowPlan row_plan(const ViewDev* views, int n_views) {
   }
   if (max_n > kRowPlanLargeN || (max_n > kRowPlanSmallN && rows < kRowPlanBlocks)) r.ok = false;
   if (tests > std::max<int64_t>(INT64_C(1) << 24, 64 * n_rec)) r.ok = false;
+  r.plain = r.ok;
+  if (max_n > kSegMinN && n_views >= 1 && n_views <= kRowBaseViews && r.max_gx <= kMaxRowTiles &&
+      r.max_gy <= 65535 && tests <= kSegTests) {
+    r.segs = row_segments(max_n);
+    r.ok = false;
+  }
   return r;
+}
+
+// The segment counts of a segmented plan live in the sort's second key buffer (`cap` keys), which
+// the tile-major binning does not use; a plan they do not fit gives way to emit + sort.
+inline void fit_segments(RowPlan& r, int64_t n_tiles, int64_t cap) {
+  if (r.segs > 0 && seg_count_words(n_tiles, r.segs) > 2 * cap) r.segs = 0;
 }
 
 // Footprint rows of the records, or NULL when each footprint's whole rectangle is binned.
@@ -291,11 +316,12 @@ int run_binning(const Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf
   const bool exact = worst > 0 && (size_t)worst * kBytesPerKey <= key_budget_bytes();
 
   // The single-view pipelines describe their view on the host (va.one).
-  const RowPlan rp = (p.va.table || p.radix) ? RowPlan{} : row_plan(&p.va.one, 1);
+  RowPlan rp = (p.va.table || p.radix) ? RowPlan{} : row_plan(&p.va.one, 1);
+  fit_segments(rp, p.n_tiles, exact ? worst : 0);
   // The tile-major emission writes every tile's range; the emit + sort path writes only the
   // non-empty ones.
-  FE_CUDA(zero_ctrl_rows(rs, rp.ok ? rp.max_gy + 1 : 0, st));
-  if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
+  FE_CUDA(zero_ctrl_rows(rs, rp.tiled() ? rp.max_gy + 1 : 0, st));
+  if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
                     rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
@@ -315,12 +341,18 @@ int run_binning(const Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf
   rc = keybuf.reserve(key_bytes, st);
   if (rc) return rc;
   carve_keys(keybuf.ptr, cap, [&](const KeySpace& s) { ks = s; });
-  if (exact && !rp.ok) launch_scan(rs.touched, rs.incl, p.n_rec, cap, rs.scan_tmp, rs.ctrl, st);
-  if (!rp.ok || !p.heavy_first) rs.order = nullptr;  // the blend takes tiles in index order
+  if (exact && !rp.tiled())
+    launch_scan(rs.touched, rs.incl, p.n_rec, cap, rs.scan_tmp, rs.ctrl, st);
+  if (!rp.tiled() || !p.heavy_first) rs.order = nullptr;  // the blend takes tiles in index order
   if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
                              p.tile_w, p.tile_h, rs.row_tot, cap, rs.ctrl, rs.ranges, nullptr,
                              ks.keys_a, rs.order, p.n_tiles, st);
+    sorted = ks.keys_a;
+  } else if (rp.segs) {
+    launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h,
+                       rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), cap, rs.ctrl, rs.ranges,
+                       nullptr, ks.keys_a, rs.order, p.n_tiles, st);
     sorted = ks.keys_a;
   } else {
     launch_emit_keys(p.va, rs.incl, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h, p.n_rec, rs.ctrl,
@@ -914,14 +946,15 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   va.count = 1;
   va.one.H = H; va.one.W = W; va.one.gx = gx; va.one.gy = gy; va.one.n = P;
   va.one.fx = 1.f; va.one.fy = 1.f;
-  const RowPlan rp = row_plan(&va.one, 1);
-  FE_CUDA(zero_ctrl_rows(rs, rp.ok ? rp.max_gy + 1 : 0, st));
-  if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)T, st));
+  const int64_t worst = (int64_t)P * T;
+  const bool exact = (size_t)worst * kBytesPerKey <= key_budget_bytes();
+  RowPlan rp = row_plan(&va.one, 1);
+  fit_segments(rp, T, exact && !rp.plain ? worst : 0);  // (a few tiles each: one launch if it can)
+  FE_CUDA(zero_ctrl_rows(rs, rp.tiled() ? rp.max_gy + 1 : 0, st));
+  if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)T, st));
   launch_legacy_preprocess(P, reference_num_stds(P), means, scales, rots, weights, rot, trans, rays,
                            mats, W, H, d->tan_fovx, d->tan_fovy, gx, gy, rs.recs, rs.rects,
                            rs.touched, rp.ok ? rs.row_tot : nullptr, rs.ctrl, st);
-  const int64_t worst = (int64_t)P * T;
-  const bool exact = (size_t)worst * kBytesPerKey <= key_budget_bytes();
   int64_t cap = worst;
   if (!exact) {
     if (!rp.ok) launch_scan(rs.touched, rs.incl, P, INT64_C(0xffffffff), rs.scan_tmp, rs.ctrl, st);
@@ -939,6 +972,10 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   if (rp.ok) {
     launch_tile_binning_emit(va, 1, rp.max_gy, rp.max_gx, rs.rects, nullptr, 8, 8, rs.row_tot, cap,
                              rs.ctrl, rs.ranges, nullptr, ks.keys_a, nullptr, T, st);
+  } else if (rp.segs) {
+    launch_seg_binning(va, 1, rp.max_gy, rp.segs, rs.rects, nullptr, 8, 8, rs.row_tot,
+                       reinterpret_cast<uint32_t*>(ks.keys_b), cap, rs.ctrl, rs.ranges, nullptr,
+                       ks.keys_a, nullptr, T, st);
   } else {
     if (exact) launch_scan(rs.touched, rs.incl, P, cap, rs.scan_tmp, rs.ctrl, st);
     launch_emit_keys(va, rs.incl, rs.rects, nullptr, 8, 8, P, rs.ctrl, ks.keys_a, cap, st);
@@ -1122,6 +1159,8 @@ int plan_batch(fe_batch* b, const fe_scene* scenes, int32_t n_scenes, const fe_v
   b->n_pix = pix_end;
   b->worst = worst;
   b->rows = row_plan(b->views_h.data(), n_views);
+  fit_segments(b->rows, tiles,
+               b->exact ? 0 : std::min(worst, (int64_t)(key_budget_bytes() / kBytesPerKey)));
   return FE_OK;
 }
 
@@ -1253,7 +1292,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   p.va.table = b->views_d;
   p.va.count = b->n_views;
   // (written by the tile-major emission, read from the blend on)
-  p.va.tile_view = (b->rows.ok && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_view
+  p.va.tile_view = (b->rows.tiled() && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_view
                                                                              : nullptr;
   p.n_rec = b->n_rec;
   p.n_tiles = b->n_tiles;
@@ -1276,14 +1315,14 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
 
 // The work-class tile lists of the last binning, when it was tile-major (else NULL).
 static const uint32_t* batch_order(const fe_batch* b, const Pipeline& p) {
-  return (p.heavy_first && !p.radix && b->rows.ok) ? b->rs.order : nullptr;
+  return (p.heavy_first && !p.radix && b->rows.tiled()) ? b->rs.order : nullptr;
 }
 
 // The same for the backward, which always takes the heaviest tiles first where the binning lists
 // them: its warps are each on a tile for 30 us at the median of the 16-view workload and 100 us at
 // the heaviest, so index order leaves a long tail (16-view step 503 -> 477 us, lists included).
 static const uint32_t* bwd_order(const fe_batch* b, const Pipeline& p) {
-  return (!p.radix && b->rows.ok) ? b->rs.order : nullptr;
+  return (!p.radix && b->rows.tiled()) ? b->rs.order : nullptr;
 }
 
 // Binning of a batch. With exact key sizing the key count is read back after the scan (one
@@ -1291,8 +1330,8 @@ static const uint32_t* bwd_order(const fe_batch* b, const Pipeline& p) {
 static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEvent_t* ev) {
   const RecSpace& rs = b->rs;
   const RowPlan rp = p.radix ? RowPlan{} : b->rows;
-  FE_CUDA(zero_ctrl_rows(rs, rp.ok ? (int64_t)rp.n_views * (rp.max_gy + 1) : 0, st));
-  if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
+  FE_CUDA(zero_ctrl_rows(rs, rp.tiled() ? (int64_t)rp.n_views * (rp.max_gy + 1) : 0, st));
+  if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   if (ev) FE_CUDA(cudaEventRecord(ev[0], st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
@@ -1312,7 +1351,7 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
       b->cap = K + K / 4;
       carve_keys(b->keys.ptr, b->cap, [&](const KeySpace& s_) { b->ks = s_; });
     }
-  } else if (!rp.ok) {
+  } else if (!rp.tiled()) {
     launch_scan(rs.touched, rs.incl, p.n_rec, b->cap, rs.scan_tmp, rs.ctrl, st);
   }
   if (ev) FE_CUDA(cudaEventRecord(ev[2], st));
@@ -1324,6 +1363,14 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
                              p.n_tiles, st);
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
     b->sorted = ks.keys_a;
+    if (ev) FE_CUDA(cudaEventRecord(ev[4], st));
+  } else if (rp.segs) {
+    launch_seg_binning(p.va, rp.n_views, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w,
+                       p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), b->cap, rs.ctrl,
+                       rs.ranges, rs.tile_view, ks.keys_a, p.tile_lists ? rs.order : nullptr,
+                       p.n_tiles, st);
+    b->sorted = ks.keys_a;
+    if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
     if (ev) FE_CUDA(cudaEventRecord(ev[4], st));
   } else {
     launch_emit_keys(p.va, rs.incl, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h, p.n_rec, rs.ctrl,
@@ -1632,6 +1679,7 @@ int fe_batch_launch_count(const fe_batch* b) {
   const bool radix = (b->desc.flags & FE_FLAG_RADIX_BINNING) != 0;
   // Tile-major binning: preprocess, (row offsets and view bases for many views,) emission, blend.
   if (b->rows.ok && !radix) return b->rows.n_views > kRowBaseViews ? 5 : 3;
+  if (b->rows.segs && !radix) return 5;  // preprocess, counts, bases, keys, blend
   // Emit + sort: preprocess, scan, emission, three kernels per radix pass, ranges, blend.
   const int passes = (bits_for(b->n_tiles) + 7) / 8;
   const int scan = b->n_rec <= 65536 ? 1 : 3;
@@ -1743,15 +1791,20 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
   // blend's tile counter and work-class counts), the row totals of the tile-major binning, and on
   // the emit + sort path the tile ranges (tiles without keys keep an empty range; the tile-major
   // emission writes every tile's range itself).
-  const RowPlan rp = p.radix ? RowPlan{} : row_plan(&p.va.one, 1);
-  FE_CUDA(zero_ctrl_rows(rs, rp.ok ? rp.max_gy + 1 : 0, st));
-  if (!rp.ok) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
+  RowPlan rp = p.radix ? RowPlan{} : row_plan(&p.va.one, 1);
+  fit_segments(rp, p.n_tiles, worst);
+  FE_CUDA(zero_ctrl_rows(rs, rp.tiled() ? rp.max_gy + 1 : 0, st));
+  if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
                     rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
   uint64_t* sorted = ks.keys_a;
-  if (!rp.ok || !p.heavy_first) rs.order = nullptr;
-  if (rp.ok) {
+  if (!rp.tiled() || !p.heavy_first) rs.order = nullptr;
+  if (rp.segs) {
+    launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h,
+                       rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), worst, rs.ctrl, rs.ranges,
+                       nullptr, ks.keys_a, rs.order, p.n_tiles, st);
+  } else if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
                              p.tile_w, p.tile_h, rs.row_tot, worst, rs.ctrl, rs.ranges, nullptr,
                              ks.keys_a, rs.order, p.n_tiles, st);

@@ -68,6 +68,16 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
                               unsigned long long* row_tot, int64_t capacity, Control* ctrl,
                               uint2* ranges, uint32_t* tile_view, uint64_t* keys, uint32_t* order,
                               int64_t n_tiles, cudaStream_t st);
+// The same keys, ranges, views and lists for many Gaussians, the records taken in segments
+// (row_segments of the largest view's count) by a block each. launch_preprocess runs without row_tot;
+// row_tot (n_views * (max_gy + 1)) and ctrl are zeroed beforehand; counts: seg_count_words words.
+int row_segments(int n);
+int64_t seg_count_words(int64_t n_tiles, int segs);
+void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, const TileRect* rects,
+                        const FootRows* foot, int tile_w, int tile_h, unsigned long long* row_tot,
+                        uint32_t* counts, int64_t capacity, Control* ctrl, uint2* ranges,
+                        uint32_t* tile_view, uint64_t* keys, uint32_t* order, int64_t n_tiles,
+                        cudaStream_t st);
 // Tile ranges of the sorted keys (ranges zeroed beforehand; empty tiles keep {0,0}).
 void launch_ranges(const uint64_t* keys, const Control* ctrl, int64_t capacity, uint2* ranges,
                    cudaStream_t st);

@@ -356,3 +356,52 @@ def test_footprint_rows_and_rectangles_render_alike(cuda_device):
     assert float(((d0 - d1).abs()[mask] / d1[mask]).max()) <= 1e-5
     for x, y in zip(g0, g1):
         assert float((x - y).norm() / y.norm()) <= 1e-4
+
+
+@pytest.mark.parametrize("footprint", ["ellipse", "rect"])
+@pytest.mark.parametrize("n,H,W,tile", [(2501, 40, 61, (8, 8)), (3072, 130, 500, (16, 16)),
+                                        (5001, 96, 2050, (32, 8)), (20001, 33, 47, (16, 16))])
+def test_segmented_binning_equals_radix_sort(cuda_device, n, H, W, tile, footprint):
+    """More than 2500 Gaussians are binned in segments of 1024 records per tile row: the same keys
+    and ranges as emission + stable sort, at sizes around whole segments and ragged images."""
+    rng = np.random.default_rng(n)
+    scene = S.random_gaussians(n, 0.3, rng)
+    cam = S.Camera(H, W, 60.0, 60.0, W / 2, H / 2, *S.look_at(S.random_unit_vectors(1, rng)[0]))
+    m, p, w = [torch.from_numpy(x).to(cuda_device) for x in (scene.means, scene.prec, scene.logw)]
+    got = {b: fe.render_binning(m, p, w, cam.fx, cam.fy, cam.cx, cam.cy, cam.quat, cam.trans, H, W,
+                                tile=tile, binning=b, footprint=footprint) for b in ("tiles", "radix")}
+    assert got["tiles"][0].numel() > n
+    assert torch.equal(got["tiles"][0], got["radix"][0])
+    assert torch.equal(got["tiles"][1], got["radix"][1])
+
+
+def test_segmented_batch_equals_single_views(cuda_device):
+    """A batch whose views differ in size and Gaussian count (one above 2500), heaviest tiles first
+    and in index order, renders as its views do alone; its key count is the views' sum."""
+    rng = np.random.default_rng(5)
+    sizes = [(3000, 50, 70), (40, 130, 33), (2600, 64, 64)]
+    scenes, views, parts, off = [], [], [], 0
+    for si, (n, h, w) in enumerate(sizes):
+        sc = S.random_gaussians(n, 0.2, rng)
+        parts.append((sc.means, sc.prec, sc.logw))
+        scenes.append((off, n))
+        off += n
+        q, t = S.look_at(0.8 * S.random_unit_vectors(1, rng)[0])
+        views.append(dict(scene=si, height=h, width=w, fx=60.0, fy=60.0, cx=w / 2, cy=h / 2, quat=q,
+                          trans=t))
+    arrays = [torch.from_numpy(np.concatenate(x)).to(cuda_device) for x in zip(*parts)]
+    for heavy in (False, True):
+        b = fe.Batch(scenes, views, heavy_first=heavy)
+        assert b.launches_per_forward == 5
+        depth, alpha = b.forward(*arrays)
+        st, keys = b.status(), 0
+        assert st["device_error"] == 0 and st["num_keys"] == st["want_keys"]
+        for i, (v, (o, n)) in enumerate(zip(views, scenes)):
+            args = [x[o:o + n].contiguous() for x in arrays]
+            cam = (v["fx"], v["fy"], v["cx"], v["cy"], v["quat"], v["trans"], v["height"], v["width"])
+            d, a = fe.render_forward(*args, *cam)
+            torch.testing.assert_close(b.view_image(depth, i), d, rtol=1e-6, atol=1e-7)
+            torch.testing.assert_close(b.view_image(alpha, i), a, rtol=0, atol=1e-6)
+            keys += fe.render_binning(*args, *cam)[0].numel()
+        assert keys == st["num_keys"]
+        b.close()
