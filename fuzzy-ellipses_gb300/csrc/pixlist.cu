@@ -25,8 +25,8 @@
 //    each), queue the ones that reach it and evaluate them in pairs from shared memory with
 //    packed f32x2 arithmetic, each ray still counting only the Gaussians whose own bound holds it,
 //    in index order: results do not depend on how rays are grouped;
-//  * with few Gaussians, or when the dense weights are wanted, pixlist_direct_kernel tests every
-//    Gaussian for every ray.
+//  * with few Gaussians or few tests in all, or when the dense weights are wanted,
+//    pixlist_direct_kernel tests every Gaussian for every ray.
 // Testing every Gaussian for every ray bounded this path: 1.2 M rays of 16 poses (every other
 // pixel of 640x480) and 1000 Gaussians took 782 us in image order and 4447 us shuffled; bucketed
 // 192 and 218 us, 156 us of it pixlist_kernel, bound by the issue slots of its evaluations (99 M
@@ -77,11 +77,13 @@ __global__ void pixlist_prep_kernel(int n, int n_poses, const float* __restrict_
                                     const float* __restrict__ logw,
                                     const float* __restrict__ poses, float fx, float fy,
                                     int cull_mode, float cull_param, Table tab,
-                                    float* __restrict__ rot) {
+                                    float* __restrict__ rot, uint32_t* __restrict__ count,
+                                    int64_t n_count) {
   const int64_t total = (int64_t)n * n_poses;
   const float L = 4.f * fmaxf(fabsf(fx), fabsf(fy));  // expansion centres within four focal lengths
   const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t k = first; k < n_count; k += step) count[k] = 0u;  // (the first slice's buckets)
   for (int64_t k = first; k < n_poses; k += step) {
     float R[9];
     quat_to_rot<float>(poses + 7 * k, R);
@@ -641,15 +643,21 @@ int pose_bits_for(int n_poses) {
   return b;
 }
 
-// Up to this many Gaussians every ray tests them all: bucketing the rays costs more than it saves
-// (1.2 M rays of 16 poses in image order, with flow: 20 Gaussians 56 us directly, 75 bucketed; 48
-// 92 and 87; 100 154 and 106; 1000 782 and 192).
-constexpr int kDirectN = 40;
 // Warps that fill the GPU.
 constexpr int64_t kFillWarps = 152 * 16;
 // Lists shorter than this are rendered in the order given: their warps hold a few rays each, and
 // the bucketing launches would cost more than their wider boxes.
 constexpr int64_t kOrderRays = 4 * kFillWarps;
+
+// Few Gaussians, or a long list with few tests in all: every ray tests every Gaussian, since
+// bucketing costs more than it saves. Per call, with flow, directly / bucketed: 1.2 M rays in image
+// order, 20 Gaussians 56 / 75 us, 48 92 / 87, 100 154 / 106, 1000 782 / 192; 9 poses, in image order
+// (shuffled), 112 K rays of 100 Gaussians 40 / 43 (44 / 43), 42 K of 300 45 / 52 (65 / 55), 112 K of
+// 300 57 / 52 (105 / 57), 10 K of 1000 122 / 106 (164 / 105).
+bool direct_list(int n, int64_t n_rays, bool weights) {
+  if (n <= 40 || weights) return true;
+  return n_rays >= kOrderRays && n <= 450 && n_rays <= INT64_C(16000000) / n;
+}
 
 // Rays per warp: 64 for long lists; short ones spread over the SMs, down to a ray per warp (which
 // makes their order irrelevant).
@@ -690,7 +698,7 @@ size_t pixlist_scratch_bytes(int n, int n_poses, int64_t ordered_rays) {
 }
 
 int64_t pixlist_ordered_rays(int n, int64_t n_rays, bool weights) {
-  return n > kDirectN && n_rays >= kOrderRays && !weights ? n_rays : 0;
+  return n_rays >= kOrderRays && !direct_list(n, n_rays, weights) ? n_rays : 0;
 }
 
 void launch_render_pixels(int n, int n_poses, const float* means, const float* prec,
@@ -703,7 +711,9 @@ void launch_render_pixels(int n, int n_poses, const float* means, const float* p
   const int64_t slice = std::min(n_rays, ordered_rays > 0 ? kSliceRays : n_rays);
   PixScratch s;
   carve(static_cast<char*>(scratch), n, n_poses, ordered_rays > 0 ? slice : 0, s);
-  const bool direct = n <= kDirectN || weights;
+  const bool direct = direct_list(n, n_rays, weights != nullptr);
+  const int bits = pose_bits_for(n_poses);
+  const int64_t buckets = INT64_C(1) << (2 * kCellBits + bits);
   const InterleavedTable mixed{s.table, s.table + sizeof(float4)};
   const SplitTable split{s.table, s.table + sizeof(float4) * (size_t)n * n_poses};
   {
@@ -712,19 +722,18 @@ void launch_render_pixels(int n, int n_poses, const float* means, const float* p
     const float fx = 1.f / rm.inv_f, fy = 1.f / (rm.aspect * rm.inv_f);
     if (direct)
       pixlist_prep_kernel<<<grid, 128, 0, st>>>(n, n_poses, means, prec, logw, poses, fx, fy,
-                                                cull_mode, cull_param, mixed, s.rot);
+                                                cull_mode, cull_param, mixed, s.rot, nullptr, 0);
     else
       pixlist_prep_kernel<<<grid, 128, 0, st>>>(n, n_poses, means, prec, logw, poses, fx, fy,
-                                                cull_mode, cull_param, split, s.rot);
+                                                cull_mode, cull_param, split, s.rot, s.count,
+                                                s.count ? buckets + 1 : 0);
   }
-  const int bits = pose_bits_for(n_poses);
-  const int64_t buckets = INT64_C(1) << (2 * kCellBits + bits);
   for (int64_t r0 = 0; r0 < n_rays; r0 += slice) {
     const int64_t m = std::min(slice, n_rays - r0);
     const float* rows = rays + rm.stride * r0;
     if (ordered_rays > 0) {
       const unsigned grid = (unsigned)((m + kBucketThreads - 1) / kBucketThreads);
-      cudaMemsetAsync(s.count, 0, sizeof(uint32_t) * (size_t)(buckets + 1), st);
+      if (r0 > 0) cudaMemsetAsync(s.count, 0, sizeof(uint32_t) * (size_t)(buckets + 1), st);
       pixlist_count_kernel<<<grid, kBucketThreads, 0, st>>>(m, rows, rm, n_poses, bits, s.count,
                                                             s.place);
       pixlist_bases_kernel<<<(unsigned)(buckets / (kBucketThreads * kBucketPer)), kBucketThreads, 0,

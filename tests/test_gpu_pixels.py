@@ -100,7 +100,8 @@ def test_scaled_rays_weights_and_features(cuda_device):
     assert np.max(np.abs(of - (rw.T @ feats.astype(np.float64)))[mask]) <= 1e-3
 
 
-@pytest.mark.parametrize("n,n_rays,n_poses", [(41, 20011, 3), (130, 12345, 70), (1100, 9729, 1)])
+@pytest.mark.parametrize("n,n_rays,n_poses", [(41, 20011, 3), (130, 12345, 70), (1100, 9729, 1),
+                                             (500, 40001, 70)])
 def test_long_lists_match_their_pieces(cuda_device, n, n_rays, n_poses):
     """A ray's result does not depend on the list around it: a long shuffled list (bucketed by
     pose and cell, 64 rays per warp or fewer) equals, bit for bit, the same rays rendered in short
