@@ -116,6 +116,7 @@ struct RecSpace {
   uint32_t* order;  // tile-major binning: per work class (kTileClasses lists of n_tiles) the
                     // tiles as uint4 entries (tile id, first key, end key, view)
   RecGrad* rgrad;  // backward only
+  float4* part;    // blend in pieces: the pieces' sums
 };
 
 // Key-proportional scratch.
@@ -134,7 +135,7 @@ inline cudaError_t zero_ctrl_rows(const RecSpace& rs, int64_t rows, cudaStream_t
 }
 
 template <class F>
-size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t n_pix, bool bwd, F&& out) {
+size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, bool bwd, F&& out) {
   Carver c{base};
   RecSpace s;
   s.ctrl = c.take<Control>(1);
@@ -150,6 +151,7 @@ size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t n_pix, bool
   s.tile_view = c.take<uint32_t>(n_tiles);
   s.order = c.take<uint32_t>((int64_t)kTileClasses * n_tiles * 4);  // uint4 entries
   s.rgrad = bwd ? c.take<RecGrad>(n_rec) : nullptr;
+  s.part = part_px > 0 ? c.take<float4>(part_px) : nullptr;
   out(s);
   return c.off;
 }
@@ -227,6 +229,7 @@ struct Pipeline {
   int tile_w, tile_h;
   int px;     // pixels per thread in the blend (0 = default)
   int chunk;  // record pairs per shared-memory stage in the blend (0 = default)
+  int pieces;  // most pieces of a tile's keys in the blend (1: whole tiles)
   bool radix;  // FE_FLAG_RADIX_BINNING: emit + sort even where tile-major binning applies
   bool rect_binning;  // FE_FLAG_RECT_BINNING: every tile of each footprint's rectangle
   bool heavy_first;  // FE_FLAG_HEAVY_TILES_FIRST: work-class tile lists for the blend
@@ -304,13 +307,33 @@ inline FootRows* foot_of(const Pipeline& p, const RecSpace& rs) {
   return p.rect_binning ? nullptr : rs.foot;
 }
 
-int run_binning(const Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
+// Pixels of the blend's piece sums.
+inline int64_t part_pixels(const Pipeline& p) {
+  return p.pieces > 1 ? (int64_t)p.pieces * p.n_tiles * p.tile_w * p.tile_h : 0;
+}
+
+// Whether `buf` holds `bytes` or may be grown to them: a stream under capture cannot.
+bool can_grow(const DevBuf& buf, size_t bytes, cudaStream_t st) {
+  if (bytes <= buf.cap) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return status == cudaStreamCaptureStatusNone;
+}
+
+int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
                 unsigned long long* h_pinned, bool bwd, cudaStream_t st, RecSpace& rs,
                 KeySpace& ks, int64_t& cap, uint64_t*& sorted) {
-  size_t rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, p.n_pix, bwd, [](const RecSpace&) {});
-  int rc = recbuf.reserve(rec_bytes, st);
+  auto rec_bytes = [&] {
+    return carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), bwd, [](const RecSpace&) {});
+  };
+  // (an arena warmed up for whole tiles stays as it is under capture)
+  if (part_pixels(p) > 0 && !can_grow(recbuf, rec_bytes(), st)) p.pieces = 1;
+  int rc = recbuf.reserve(rec_bytes(), st);
   if (rc) return rc;
-  carve_rec(recbuf.ptr, p.n_rec, p.n_tiles, p.n_pix, bwd, [&](const RecSpace& s) { rs = s; });
+  carve_rec(recbuf.ptr, p.n_rec, p.n_tiles, part_pixels(p), bwd, [&](const RecSpace& s) { rs = s; });
 
   // `worst`: every record touching every tile of its view.
   const bool exact = worst > 0 && (size_t)worst * kBytesPerKey <= key_budget_bytes();
@@ -404,6 +427,7 @@ Pipeline single_view_pipeline(const fe_render_desc* d, const float* means, const
   // one round but not the two-pixel blend's.)
   p.px = default_px((int)d->px_per_thread, tw, th, p.n_tiles);
   p.chunk = (int)(d->flags >> 8) & 0xff;
+  p.pieces = blend_pieces(tw, th, p.px, p.chunk, p.n_tiles, p.n_rec);
   p.radix = (d->flags & FE_FLAG_RADIX_BINNING) != 0;
   p.rect_binning = (d->flags & FE_FLAG_RECT_BINNING) != 0;
   p.heavy_first = (d->flags & FE_FLAG_HEAVY_TILES_FIRST) != 0;
@@ -447,6 +471,7 @@ int render_features(const fe_render_desc* d, const float* means, const float* pr
   rc = arena_for(st, &a);
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
+  if (!depth) p.pieces = 1;  // (nothing is blended forward)
   RecSpace rs;
   KeySpace ks;
   int64_t cap = 0;
@@ -455,8 +480,8 @@ int render_features(const fe_render_desc* d, const float* means, const float* pr
                    sorted);
   if (rc) return rc;
   if (depth)
-    launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, sorted, rs.recs,
-                     rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+    launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces, rs.part,
+                     sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
   launch_features(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, stats, npix,
                   p.beta2, p.beta3, features, n_features, out, st);
   FE_CUDA(cudaGetLastError());
@@ -537,8 +562,8 @@ int fe_render_fwd(const fe_render_desc* d, const float* means, const float* prec
   rc = run_binning(p, p.n_rec * p.n_tiles, a->rec, a->keys, a->h_pinned, false, st, rs, ks, cap,
                    sorted);
   if (rc) return rc;
-  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, sorted, rs.recs,
-                   rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces, rs.part,
+                   sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }
@@ -561,6 +586,7 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
   rc = arena_for(st, &a);
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
+  p.pieces = 1;  // (nothing is blended forward)
   RecSpace rs;
   KeySpace ks;
   int64_t cap = 0;
@@ -606,6 +632,7 @@ int fe_render_binning(const fe_render_desc* d, const float* means, const float* 
     return fail(FE_ERR_INVALID_ARGUMENT, "NULL pointer or negative capacity");
   *h_num_keys = 0;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
+  p.pieces = 1;  // (nothing is blended)
   FE_CUDA(cudaMemsetAsync(ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   if (p.n_rec == 0) return FE_OK;
   if (!means || !prec || !logw) return fail(FE_ERR_INVALID_ARGUMENT, "NULL Gaussian pointer");
@@ -784,13 +811,9 @@ int fe_render_pixels(const fe_pixlist_desc* d_in, const float* means, const floa
   // arena: there a list longer than the arena was warmed up for is rendered in its own order.
   int64_t ordered = pixlist_ordered_rays(d->n_gaussians, d->n_rays, weights != nullptr);
   size_t bytes = pixlist_scratch_bytes(d->n_gaussians, d->n_poses, ordered);
-  if (ordered > 0 && bytes > a->rec.cap) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-      (void)cudaGetLastError();
-      ordered = 0;
-      bytes = pixlist_scratch_bytes(d->n_gaussians, d->n_poses, 0);
-    }
+  if (ordered > 0 && !can_grow(a->rec, bytes, st)) {
+    ordered = 0;
+    bytes = pixlist_scratch_bytes(d->n_gaussians, d->n_poses, 0);
   }
   rc = a->rec.reserve(std::max<size_t>(bytes, 256), st);
   if (rc) return rc;
@@ -986,7 +1009,7 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
     launch_blend_fwd_clean(va, T, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z, out_alpha,
                            rs.ctrl, st);
   else
-    launch_blend_fwd(va, 8, 8, 0, 0, T, nullptr, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z,
+    launch_blend_fwd(va, 8, 8, 0, 0, T, nullptr, 1, nullptr, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z,
                      out_alpha, nullptr, 0, rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
@@ -1108,6 +1131,7 @@ struct fe_batch {
   cudaEvent_t ev_bin = nullptr, ev_copy = nullptr;
   std::vector<cudaEvent_t> band_ev;
   RowPlan rows;  // tile-major binning plan (rows.ok) or the emit + sort path
+  int pieces = 1;  // most pieces of a tile's keys in the blend
 };
 
 namespace {
@@ -1159,6 +1183,10 @@ int plan_batch(fe_batch* b, const fe_scene* scenes, int32_t n_scenes, const fe_v
   b->n_pix = pix_end;
   b->worst = worst;
   b->rows = row_plan(b->views_h.data(), n_views);
+  int max_n = 0;
+  for (const ViewDev& d : b->views_h) max_n = std::max(max_n, (int)d.n);
+  const int px = default_px((int)b->desc.px_per_thread, b->tile_w, b->tile_h, tiles);
+  b->pieces = blend_pieces(b->tile_w, b->tile_h, px, (int)(b->desc.flags >> 8) & 0xff, tiles, max_n);
   fit_segments(b->rows, tiles,
                b->exact ? 0 : std::min(worst, (int64_t)(key_budget_bytes() / kBytesPerKey)));
   return FE_OK;
@@ -1185,10 +1213,12 @@ int commit_batch(fe_batch* b, cudaStream_t st) {
   // (ranges and row totals: sized for the tiles and for the tile-major binning's row slots)
   const int64_t tile_slots =
       std::max<int64_t>(b->n_tiles, (int64_t)b->rows.n_views * (b->rows.max_gy + 1));
-  const size_t rb = carve_rec(nullptr, b->n_rec, tile_slots, b->n_pix, true, [](const RecSpace&) {});
+  const int64_t part_px =
+      b->pieces > 1 ? (int64_t)b->pieces * b->n_tiles * b->tile_w * b->tile_h : 0;
+  const size_t rb = carve_rec(nullptr, b->n_rec, tile_slots, part_px, true, [](const RecSpace&) {});
   rc = b->rec.reserve(rb, st);
   if (rc) return rc;
-  carve_rec(b->rec.ptr, b->n_rec, tile_slots, b->n_pix, true, [&](const RecSpace& s_) { b->rs = s_; });
+  carve_rec(b->rec.ptr, b->n_rec, tile_slots, part_px, true, [&](const RecSpace& s_) { b->rs = s_; });
   if (!b->exact) {
     const int64_t budget_keys = (int64_t)(key_budget_bytes() / kBytesPerKey);
     b->cap = std::max<int64_t>(1, std::min<int64_t>({b->worst, budget_keys, INT64_C(0xffffffff)}));
@@ -1301,6 +1331,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   p.tile_h = b->tile_h;
   p.px = default_px((int)b->desc.px_per_thread, b->tile_w, b->tile_h, p.n_tiles);
   p.chunk = (int)(b->desc.flags >> 8) & 0xff;
+  p.pieces = b->pieces;
   p.radix = (b->desc.flags & FE_FLAG_RADIX_BINNING) != 0;
   p.rect_binning = (b->desc.flags & FE_FLAG_RECT_BINNING) != 0;
   p.heavy_first = (b->desc.flags & FE_FLAG_HEAVY_TILES_FIRST) != 0;
@@ -1478,7 +1509,7 @@ static int batch_forward(fe_batch* b, const float* means, const float* prec, con
   if (rc) return rc;
   note_binning(b, means, prec, logw);
   launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles,
-                   heavy_order ? batch_order(b, p) : nullptr, b->sorted, b->rs.recs,
+                   heavy_order ? batch_order(b, p) : nullptr, p.pieces, b->rs.part, b->sorted, b->rs.recs,
                    b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats, p.n_pix, b->rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
@@ -1576,10 +1607,16 @@ int fe_batch_fwd_host(fe_batch* b, const float* h_means, const float* h_prec,
   // the calling thread) cannot delay the renders.
   for (int j = 0; j < nb; ++j) {
     const fe_batch::HostBand& hb = b->bands[j];
-    cudaStream_t sj = (host_band_streams() == 2 && (j & 1)) ? b->s_comp : st;
-    launch_blend_fwd_band(p.va, p.tile_w, p.tile_h, p.px, p.chunk, hb.t0, hb.t1, ctr + j,
-                          b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, dep_d, alp_d,
-                          nullptr, p.n_pix, b->rs.ctrl, sj);
+    const bool second = host_band_streams() == 2 && (j & 1) && p.pieces == 1;
+    cudaStream_t sj = second ? b->s_comp : st;
+    if (p.pieces == 1)
+      launch_blend_fwd_band(p.va, p.tile_w, p.tile_h, p.px, p.chunk, hb.t0, hb.t1, ctr + j,
+                            b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, dep_d, alp_d,
+                            nullptr, p.n_pix, b->rs.ctrl, sj);
+    else if (j == 0)  // few tiles: all of them in one launch, as in the other forwards
+      launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, nullptr, p.pieces,
+                       b->rs.part, b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, dep_d,
+                       alp_d, nullptr, p.n_pix, b->rs.ctrl, sj);
     FE_CUDA(cudaGetLastError());
     FE_CUDA(cudaEventRecord(b->band_ev[j], sj));
   }
@@ -1663,8 +1700,8 @@ int fe_batch_fwd_timed(fe_batch* b, const float* means, const float* prec, const
     return rc;
   }
   note_binning(b, means, prec, logw);
-  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, batch_order(b, p),
-                   b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats,
+  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, batch_order(b, p), p.pieces,
+                   b->rs.part, b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats,
                    p.n_pix, b->rs.ctrl, st);
   FE_CUDA(cudaEventRecord(ev[6], st));
   FE_CUDA(cudaEventSynchronize(ev[6]));
@@ -1768,9 +1805,13 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
 
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
   const int64_t worst = p.n_rec * p.n_tiles;
-  const size_t rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, p.n_pix, false,
-                                     [](const RecSpace&) {});
+  size_t rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), false,
+                               [](const RecSpace&) {});
   const size_t key_bytes = carve_keys(nullptr, worst, [](const KeySpace&) {});
+  if (p.pieces > 1 && rec_bytes + key_bytes > (size_t)FE_NOALLOC_SCRATCH_BYTES) {
+    p.pieces = 1;  // (what fits with whole tiles is accepted)
+    rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, 0, false, [](const RecSpace&) {});
+  }
   if (worst > INT64_C(0xffffffff) || rec_bytes + key_bytes > (size_t)FE_NOALLOC_SCRATCH_BYTES)
     return fail(FE_ERR_SCRATCH_LIMIT,
                 "fe_render_fwd_noalloc: " + std::to_string(p.n_rec) + " Gaussians x " +
@@ -1784,7 +1825,7 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
   if (rc) return rc;
   RecSpace rs;
   KeySpace ks;
-  carve_rec(base, p.n_rec, p.n_tiles, p.n_pix, false, [&](const RecSpace& s) { rs = s; });
+  carve_rec(base, p.n_rec, p.n_tiles, part_pixels(p), false, [&](const RecSpace& s) { rs = s; });
   carve_keys(base + rec_bytes, worst, [&](const KeySpace& s) { ks = s; });
 
   // Must start at zero on every call: the control block (key counters, device error word, the
@@ -1815,8 +1856,8 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
     sorted = launch_sort(ks.keys_a, ks.keys_b, bits_for(p.n_tiles), rs.ctrl, worst, ks.hist, st);
     launch_ranges(sorted, rs.ctrl, worst, rs.ranges, st);
   }
-  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, sorted, rs.recs,
-                   rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces, rs.part,
+                   sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
   if (device_error)
     FE_CUDA(cudaMemcpyAsync(device_error, &rs.ctrl->error, sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, st));

@@ -72,6 +72,8 @@ struct BlendShape {
   static_assert(NT >= GP, "enough threads to pad a chunk");
 };
 
+constexpr int kSplitPx = 2;  // pixels per thread of the split launches
+
 // Initial running max: finite, far below any logit, so logit - max is never inf - inf.
 constexpr float kNoLogit = -1e30f;
 
@@ -174,15 +176,37 @@ __device__ __forceinline__ float clean_value(float x, float top) {
   return x != x || x == -INFINITY ? 0.f : x == INFINITY ? top : x;
 }
 
-// CLEAN: the outputs go through clean_value.
-template <int TW, int TH, int PX, int CH, bool CLEAN>
+__device__ __forceinline__ float pixel_depth(float W, float Z) {
+  return W > 0.f ? Z * rcp_approx(W) : 0.f;
+}
+
+// alpha = 1 - exp(-A): a Taylor polynomial below A = 1/64 (relative error under 1e-9), else from
+// the hardware exp2 (absolute error under 3e-7).
+__device__ __forceinline__ float pixel_alpha(float A) {
+  return A < 0.015625f ? A * fmaf(A, fmaf(A, fmaf(A, -1.f / 24.f, 1.f / 6.f), -0.5f), 1.f)
+                       : 1.f - ex2_approx(-A * kLog2e);
+}
+
+// Pieces of a tile of nk keys when a launch may cut tiles into up to `most`: consecutive keys, at
+// least kMinPiece each; `per` receives a piece's keys (a multiple of 8, the last one fewer).
+constexpr int kMinPiece = 64;
+__device__ __forceinline__ int tile_pieces(int nk, int most, int& per) {
+  const int p = max(1, min(most, nk / kMinPiece));
+  per = p == 1 ? max(nk, 1) : ((nk + p - 1) / p + 7) & ~7;
+  return (nk + per - 1) / per;
+}
+
+// CLEAN: the outputs go through clean_value. SPLIT: work index w is piece w / n_tiles of tile
+// w % n_tiles (tile_end = n_tiles x the most pieces); a tile of several pieces leaves each one's
+// sums (max logit, W, Z, A) per pixel in `part` for blend_merge_kernel.
+template <int TW, int TH, int PX, int CH, bool CLEAN, bool SPLIT>
 __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
                                   BlendShape<TW, TH, PX, CH>::MIN_CTAS) blend_fwd_kernel(
     ViewsArg va, uint32_t tile_begin, uint32_t tile_end, uint32_t* __restrict__ counter,
     const uint32_t* __restrict__ order, const uint64_t* __restrict__ keys,
     const GaussRec* __restrict__ recs, const uint2* __restrict__ ranges, float nb2, float beta3,
     float* __restrict__ depth, float* __restrict__ alpha, float* __restrict__ stats,
-    int64_t stats_stride, Control* __restrict__ ctrl) {
+    int64_t stats_stride, uint32_t n_tiles, float4* __restrict__ part, Control* __restrict__ ctrl) {
   using Sh = BlendShape<TW, TH, PX, CH>;
   constexpr int GP = Sh::GP;
   __shared__ __align__(128) BlendSmem<CH> sm;
@@ -249,8 +273,10 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
     }
     first = false;
     __syncthreads();
-    const uint32_t tile = sm.tile;
-    if (tile >= tile_end) break;
+    const uint32_t item = sm.tile;
+    if (item >= tile_end) break;
+    const uint32_t piece = SPLIT ? item / n_tiles : 0u;
+    const uint32_t tile = SPLIT ? item - piece * n_tiles : item;
     // With the work-class lists the entry carries the tile's range and view.
     const bool listed = order && tile_begin == 0 && use_order_all;
     const int vi = listed ? (int)sm.entry.w : view_of_tile(va, tile);
@@ -260,7 +286,19 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
     const GaussRec* vrec = recs + view_at(va, vi).rec_base;
     const float tcu = tx * TW + hw, tcv = ty * TH + hh;  // tile centre (pixels)
 
-    const uint2 rg = listed ? make_uint2(sm.entry.y, sm.entry.z) : ranges[tile];
+    uint2 rg = listed ? make_uint2(sm.entry.y, sm.entry.z) : ranges[tile];
+    bool whole = true;
+    if (SPLIT) {
+      int per;
+      const uint32_t pieces = (uint32_t)tile_pieces((int)(rg.y - rg.x), (int)(tile_end / n_tiles), per);
+      if (piece > 0 && piece >= pieces) {
+        __syncthreads();  // sm.tile is rewritten next iteration
+        continue;
+      }
+      whole = pieces <= 1;
+      rg.x += piece * (uint32_t)per;
+      rg.y = min(rg.y, rg.x + (uint32_t)per);
+    }
     // m starts finite (kNoLogit) so that logit - m is never (-inf) - (-inf); masked logits are
     // -inf and give weight 0.
     f2_t A2[PX], W2[PX], Z2[PX];
@@ -405,7 +443,17 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
     const ViewDev& V = view_at(va, vi);
     const int v = ty * TH + ly;
     const int u0 = tx * TW + cx * PX;
-    if (v < V.H) {
+    if (SPLIT && !whole) {
+      float4* dst = part + (int64_t)item * (TW * TH) + ly * TW + cx * PX;
+#pragma unroll
+      for (int k = 0; k < PX; ++k) {
+        float a0, a1, w0, w1, z0, z1;
+        f2_unpack(A2[k], a0, a1);
+        f2_unpack(W2[k], w0, w1);
+        f2_unpack(Z2[k], z0, z1);
+        dst[k] = make_float4(m[k], w0 + w1, z0 + z1, a0 + a1);
+      }
+    } else if (v < V.H) {
       float dep[PX], alp[PX], wsum[PX], asum[PX];
 #pragma unroll
       for (int k = 0; k < PX; ++k) {
@@ -414,11 +462,8 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
         f2_unpack(W2[k], w0, w1);
         f2_unpack(Z2[k], z0, z1);
         const float A = a0 + a1, W = w0 + w1, Z = z0 + z1;
-        dep[k] = W > 0.f ? Z * rcp_approx(W) : 0.f;
-        // alpha = 1 - exp(-A): a Taylor polynomial below A = 1/64 (relative error under 1e-9),
-        // else from the hardware exp2 (absolute error under 3e-7).
-        alp[k] = A < 0.015625f ? A * fmaf(A, fmaf(A, fmaf(A, -1.f / 24.f, 1.f / 6.f), -0.5f), 1.f)
-                               : 1.f - ex2_approx(-A * kLog2e);
+        dep[k] = pixel_depth(W, Z);
+        alp[k] = pixel_alpha(A);
         wsum[k] = W;
         asum[k] = A;
         if (CLEAN) {
@@ -439,17 +484,69 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
   }
 }
 
+// The pixels of the tiles that were blended in pieces: a thread per pixel merges the pieces' sums in
+// piece order. One block per tile; the tiles of a single piece are already written.
+template <int TW, int TH>
+__global__ void __launch_bounds__(TW * TH) blend_merge_kernel(
+    ViewsArg va, uint32_t n_tiles, int most, const uint2* __restrict__ ranges,
+    const float4* __restrict__ part, float* __restrict__ depth, float* __restrict__ alpha,
+    float* __restrict__ stats, int64_t stats_stride) {
+  const uint32_t tile = blockIdx.x;
+  const uint2 rg = ranges[tile];
+  int per;
+  const int pieces = tile_pieces((int)(rg.y - rg.x), most, per);
+  if (pieces <= 1) return;
+  const ViewDev& V = view_at(va, view_of_tile(va, tile));
+  const int lt = (int)(tile - V.tile_base);
+  const int u = (lt % V.gx) * TW + (int)threadIdx.x % TW, v = (lt / V.gx) * TH + (int)threadIdx.x / TW;
+  if (u >= V.W || v >= V.H) return;
+  float m = kNoLogit, W = 0.f, Z = 0.f, A = 0.f;
+#pragma unroll 4
+  for (int p = 0; p < pieces; ++p) {
+    const float4 x = part[((int64_t)p * n_tiles + tile) * (TW * TH) + threadIdx.x];
+    const float top = fmaxf(m, x.x), a = ex2_approx(m - top), b = ex2_approx(x.x - top);
+    W = fmaf(W, a, x.y * b);
+    Z = fmaf(Z, a, x.z * b);
+    A += x.w;
+    m = top;
+  }
+  const int64_t pix = V.pix_base + (int64_t)v * V.W + u;
+  depth[pix] = pixel_depth(W, Z);
+  alpha[pix] = pixel_alpha(A);
+  if (stats) {
+    stats[pix] = m;
+    stats[stats_stride + pix] = W;
+    stats[2 * stats_stride + pix] = A;
+  }
+}
+
 template <int TW, int TH, int PX, int CH, bool CLEAN = false>
 void launch_tiles(const ViewsArg& va, int64_t tile_begin, int64_t tile_end, uint32_t* counter,
                   const uint32_t* order, const uint64_t* keys, const GaussRec* recs,
                   const uint2* ranges, float nb2, float beta3, float* depth, float* alpha,
                   float* stats, int64_t stats_stride, Control* ctrl, cudaStream_t st) {
   constexpr int NT = BlendShape<TW, TH, PX, CH>::NT;
-  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, CLEAN>;
+  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, CLEAN, false>;
   const int64_t grid = std::min<int64_t>(tile_end - tile_begin, resident_ctas<kern>(NT));
   kern<<<(unsigned)grid, NT, 0, st>>>(va, (uint32_t)tile_begin, (uint32_t)tile_end, counter,
                                       order, keys, recs, ranges, nb2, beta3, depth, alpha, stats,
-                                      stats_stride, ctrl);
+                                      stats_stride, 0u, nullptr, ctrl);
+}
+
+template <int TW, int TH>
+void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_t* keys,
+                  const GaussRec* recs, const uint2* ranges, float nb2, float beta3, float* depth,
+                  float* alpha, float* stats, int64_t stats_stride, float4* part, Control* ctrl,
+                  cudaStream_t st) {
+  constexpr int PX = kSplitPx, CH = 32, NT = BlendShape<TW, TH, PX, CH>::NT;
+  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, false, true>;
+  const int64_t items = n_tiles * pieces;
+  const int64_t grid = std::min<int64_t>(items, resident_ctas<kern>(NT));
+  kern<<<(unsigned)grid, NT, 0, st>>>(va, 0u, (uint32_t)items, &ctrl->next_tile, nullptr, keys, recs,
+                                      ranges, nb2, beta3, depth, alpha, stats, stats_stride,
+                                      (uint32_t)n_tiles, part, ctrl);
+  blend_merge_kernel<TW, TH><<<(unsigned)n_tiles, TW * TH, 0, st>>>(
+      va, (uint32_t)n_tiles, pieces, ranges, part, depth, alpha, stats, stats_stride);
 }
 
 template <int TW, int TH, int PX>
@@ -506,11 +603,41 @@ void launch_blend_fwd_band(const ViewsArg& va, int tile_w, int tile_h, int px, i
                  ranges, beta2, beta3, depth, alpha, stats, stats_stride, ctrl, st);
 }
 
+int blend_pieces(int tile_w, int tile_h, int px, int chunk, int64_t n_tiles, int64_t max_n) {
+  if ((px != 0 && px != kSplitPx) || (px == 0 && !(tile_w == 8 && tile_h == 8)) ||
+      (chunk != 0 && chunk != 32) || n_tiles <= 0)
+    return 1;
+  // A launch of few tiles leaves SMs idle and lasts as long as its heaviest tile (the keys of a tile
+  // are blended one after the other). Tiles are cut until the pieces could fill the GPU (CTAs as
+  // BlendShape sizes them) twice over, more often the more keys per tile the view can hold; a piece
+  // has at least 128 keys in the densest tile there can be (64 in fact: tile_pieces). Per call,
+  // whole / cut: 2600 Gaussians at 64x64 158 / 57 us, 4378 at 73x419 202 / 96, 1422 at 293x157 96 /
+  // 64, 931 at 347x170 67 / 52, 20000 at 300x400 260 / 168, 8273 at 621x573 172 / 153; with more
+  // pieces where they hold fewer keys, 1100 at 640x480 53 / 58, 1000 at 637x479 75 / 80.
+  const int64_t cta = 152 * std::min(16, 640 / (tile_w * tile_h / kSplitPx));
+  const int64_t most = cta * (max_n < 2 * n_tiles || max_n <= 1024 ? 2 : max_n <= 4096 ? 4 : 8);
+  int pieces = 1;
+  while (pieces < 32 && 2 * pieces * n_tiles <= most && 2 * pieces * 128 <= max_n) pieces *= 2;
+  return pieces;
+}
+
 void launch_blend_fwd(const ViewsArg& va, int tile_w, int tile_h, int px, int chunk,
-                      int64_t n_tiles, const uint32_t* order, const uint64_t* keys,
+                      int64_t n_tiles, const uint32_t* order, int pieces, float4* part,
+                      const uint64_t* keys,
                       const GaussRec* recs, const uint2* ranges, float beta2, float beta3,
                       float* depth, float* alpha, float* stats, int64_t stats_stride,
                       Control* ctrl, cudaStream_t st) {
+  if (pieces > 1 && part) {
+    const float nb2 = -beta2 * kLog2e;
+    auto go = [&](auto launch) {
+      launch(va, n_tiles, pieces, keys, recs, ranges, nb2, beta3, depth, alpha, stats, stats_stride,
+             part, ctrl, st);
+    };
+    if (tile_w == 8 && tile_h == 8) go(launch_split<8, 8>);
+    else if (tile_w == 32 && tile_h == 8) go(launch_split<32, 8>);
+    else go(launch_split<16, 16>);
+    return;
+  }
   blend_dispatch(va, tile_w, tile_h, px, chunk, 0, n_tiles, &ctrl->next_tile, order, keys, recs,
                  ranges, beta2, beta3, depth, alpha, stats, stats_stride, ctrl, st);
 }

@@ -88,9 +88,12 @@ void launch_ranges(const uint64_t* keys, const Control* ctrl, int64_t capacity, 
 // the sorted keys and the Gaussian records (no gathered record stream). Persistent:
 // ctrl->next_tile must be zero. `order`: the tile-major binning's per-class tile lists (heaviest
 // tiles are then taken first) or NULL (tiles in index order).
+// pieces (blend_pieces; 1: whole tiles): the most pieces a tile's keys are cut into, with `part`
+// (pieces x n_tiles x the tile's pixels) for their sums; tiles are then taken in index order.
+int blend_pieces(int tile_w, int tile_h, int px, int chunk, int64_t n_tiles, int64_t max_n);
 void launch_blend_fwd(const ViewsArg& va, int tile_w, int tile_h, int px, int chunk, int64_t n_tiles,
-                      const uint32_t* order, const uint64_t* keys, const GaussRec* recs,
-                      const uint2* ranges, float beta2,
+                      const uint32_t* order, int pieces, float4* part, const uint64_t* keys,
+                      const GaussRec* recs, const uint2* ranges, float beta2,
                       float beta3, float* depth, float* alpha, float* stats, int64_t stats_stride,
                       Control* ctrl, cudaStream_t st);
 // launch_blend_fwd on 8x8 tiles with the outputs through nan_to_num (NaN and -inf to 0, +inf depth

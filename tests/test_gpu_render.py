@@ -277,3 +277,36 @@ def test_host_pose_equals_device_pose(cuda_device, kind):
         grads.append(mm.grad)
     # (the backward's atomics leave the order of a Gaussian's tile sums open)
     torch.testing.assert_close(grads[0], grads[1], rtol=1e-5, atol=1e-5 * float(grads[1].abs().max()))
+
+
+@pytest.mark.parametrize("tile", TILES)
+@pytest.mark.parametrize("n,H,W", [(256, 16, 16), (1000, 33, 50), (2600, 64, 64), (5000, 37, 129)])
+def test_few_tiles_of_many_gaussians(cuda_device, tile, n, H, W):
+    """Launches of few tiles cut each tile's keys into pieces and merge their sums: depth and alpha
+    within the stated tolerance of the float64 oracle, and the statistics they leave give the
+    gradients of the same view blended whole (a batch with 16-pair stages; both backwards
+    accumulate in float32 with open order, so to 1e-4 of the largest entry)."""
+    rng = np.random.default_rng(n)
+    scene = S.random_gaussians(n, 0.12, rng)
+    cam = S.Camera(H, W, float(max(H, W)), float(max(H, W)), W / 2, H / 2,
+                   *S.look_at(0.5 * S.random_unit_vectors(1, rng)[0]))
+    m, p, w = [x.requires_grad_() for x in scene_to_dev(scene, cuda_device)]
+    depth, alpha = fe.render(m, p, w, cam.fx, cam.fy, cam.cx, cam.cy, cam.quat, cam.trans, H, W,
+                             tile=tile)
+    assert fe.device_status() == 0
+    d, a = depth.detach().cpu().numpy().ravel(), alpha.detach().cpu().numpy().ravel()
+    pix = rng.choice(H * W, min(400, H * W), replace=False)
+    ea, ed = parity_errors(d[pix], a[pix], *oracle_pixels(scene, cam, pix))
+    assert ea <= TOL_ALPHA and ed <= TOL_DEPTH_REL, (ea, ed)
+    gd, ga = torch.rand(H, W, device=cuda_device), torch.rand(H, W, device=cuda_device)
+    got = torch.autograd.grad((depth, alpha), (m, p, w), (gd, ga))
+    view = dict(scene=0, height=H, width=W, fx=cam.fx, fy=cam.fy, cx=cam.cx, cy=cam.cy,
+                quat=cam.quat, trans=cam.trans)
+    b = fe.Batch([(0, n)], [view], tile=tile, px=2, chunk=16)
+    args = [x.detach() for x in (m, p, w)]
+    stats = torch.empty(3 * b.n_pixels, device=cuda_device)
+    bd, ba = b.forward(*args, stats=stats)
+    want = b.backward(*args, bd, ba, stats, gd.ravel(), ga.ravel())
+    for x, y in zip(got, want):
+        assert float((x - y).abs().max()) <= 1e-4 * float(y.abs().max())
+    b.close()
