@@ -149,15 +149,25 @@ __device__ __forceinline__ void blend_group(const TilePair* grp, const f2_t (&DU
       cmax[k] = max3f(cmax[k], l0, l1);
     }
   }
+  // One branch for the thread's pixels (a branch each costs more than the rescaling by one of the
+  // pixels whose maximum stays: 16 views 186.7 -> 184.0 us per pass, a 1280x720 view of 24000
+  // Gaussians 323 -> 311).
+  bool up = false;
 #pragma unroll
-  for (int k = 0; k < PX; ++k) {
-    if (cmax[k] > m[k]) {
-      const float sc = ex2_approx(m[k] - cmax[k]);
+  for (int k = 0; k < PX; ++k) up |= cmax[k] > m[k];
+  if (up) {
+#pragma unroll
+    for (int k = 0; k < PX; ++k) {
+      const float top = fmaxf(m[k], cmax[k]);
+      const float sc = ex2_approx(m[k] - top);
       const f2_t S = f2_pack(sc, sc);
       W2[k] = mul2(W2[k], S);
       Z2[k] = mul2(Z2[k], S);
-      m[k] = cmax[k];
+      m[k] = top;
     }
+  }
+#pragma unroll
+  for (int k = 0; k < PX; ++k) {
     const f2_t M = f2_pack(m[k], m[k]);
 #pragma unroll
     for (int q = 0; q < GP; ++q) {
