@@ -114,7 +114,7 @@ struct RecSpace {
   uint32_t* tile_view;  // tile-major binning of a batch: the view of every tile
   unsigned long long* row_tot;  // tile-major binning: key counts of the tile rows, per view
   uint32_t* order;  // tile-major binning: per work class (kTileClasses lists of n_tiles) the
-                    // tiles as uint4 entries (tile id, first key, end key, view)
+                    // tiles as uint4 entries (x | y << 16 in the view, first key, end key, view)
   RecGrad* rgrad;  // backward only
   float4* part;    // blend in pieces: the pieces' sums
 };

@@ -531,7 +531,7 @@ __device__ __forceinline__ unsigned long long keys_before(const ViewsArg& va,
 // within the row (pos; slots from lim on are dropped), and for the tiles [x_lo, x_hi) their ranges,
 // their view and their entries in the work-class lists.
 __device__ __forceinline__ void row_tiles(const int (&cnt)[kTilesPer], unsigned long long csum,
-                                          int x_lo, int x_hi, int64_t tile0,
+                                          int x_lo, int x_hi, int row, int64_t tile0,
                                           unsigned long long row_base, unsigned long long K,
                                           uint32_t lim, Control* __restrict__ ctrl,
                                           uint2* __restrict__ ranges,
@@ -595,7 +595,7 @@ __device__ __forceinline__ void row_tiles(const int (&cnt)[kTilesPer], unsigned 
       const int x = kTilesPer * tid + q;
       if (x >= x_lo && x < x_hi)
         reinterpret_cast<uint4*>(order)[(int64_t)cl[q] * n_tiles + cls_base[cl[q]] + rank[q]] =
-            make_uint4((uint32_t)(tile0 + x), rgq[q].x, rgq[q].y, blockIdx.y);
+            make_uint4((uint32_t)x | (uint32_t)row << 16, rgq[q].x, rgq[q].y, blockIdx.y);
     }
   }
   __syncthreads();
@@ -731,7 +731,7 @@ __device__ __forceinline__ void tile_emit_body(
       csum += (unsigned)run;
     }
   }
-  row_tiles(cnt, csum, x_lo, x_hi, tile0, row_base, K, lim, ctrl, ranges, tile_view, order, n_tiles,
+  row_tiles(cnt, csum, x_lo, x_hi, row, tile0, row_base, K, lim, ctrl, ranges, tile_view, order, n_tiles,
             pos, wsu);
   for (int s0 = 0; s0 < n; s0 += kRowSeg) {
     // (with a single segment the list is still in shared memory)
@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(kRowThreads) seg_bases_kernel(
     cnt[q] = x < gx ? (int)pos[x] : 0;
     csum += (unsigned)cnt[q];
   }
-  row_tiles(cnt, csum, 0, gx, tile0, row_base, K, lim, ctrl, ranges, tile_view, order, n_tiles, pos,
+  row_tiles(cnt, csum, 0, gx, row, tile0, row_base, K, lim, ctrl, ranges, tile_view, order, n_tiles, pos,
             wsu);
 }
 
@@ -1001,7 +1001,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     if (lane < gx) {
       const uint32_t rank = (uint32_t)__popc(same & lt_mask);
       reinterpret_cast<uint4*>(order)[(int64_t)cl * n_tiles + base + rank] =
-          make_uint4((uint32_t)(tile0 + lane), rg.x, rg.y, (uint32_t)v);
+          make_uint4((uint32_t)lane | (uint32_t)row << 16, rg.x, rg.y, (uint32_t)v);
     }
   }
   // Keys: tile x's next slot is lane x's p; a record's rank among the chunk's records covering x

@@ -106,27 +106,29 @@ __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(&ctrl->next_tile, 1u);
     item = __shfl_sync(full, item, 0);
-    uint32_t tile = item >> seg_bits;
+    const uint32_t tile = item >> seg_bits;
     if (tile >= n_tiles) break;
     uint2 range;
-    int vi;
+    int vi, tx, ty;
     if (listed) {
       const int c = 31 - __clz(__ballot_sync(full, lane < kTileClasses && cls_first <= tile));
       const uint4 e = reinterpret_cast<const uint4*>(order)[(int64_t)c * n_tiles + tile -
                                                             __shfl_sync(full, cls_first, c)];
-      tile = e.x;
+      tx = (int)(e.x & 0xffffu);
+      ty = (int)(e.x >> 16);
       range = make_uint2(e.y, e.z);
       vi = (int)e.w;
     } else {
       range = ranges[tile];
       vi = view_of_tile(va, tile);
+      const int lt = (int)(tile - view_at(va, vi).tile_base);
+      ty = lt / view_at(va, vi).gx;
+      tx = lt - ty * view_at(va, vi).gx;
     }
     const uint32_t seg = item & ((1u << seg_bits) - 1u);
     if (range.y <= range.x + 32u * seg) continue;
     const ViewDev& V = view_at(va, vi);
     if (V.flags & FE_VIEW_NO_GRAD) continue;
-    const int lt = (int)(tile - V.tile_base);
-    const int tx = lt % V.gx, ty = lt / V.gx;
     const int xs = min(TW, V.W - tx * TW), ys = min(TH, V.H - ty * TH);
 
     __syncwarp();  // the previous tile's readers are done with the slice

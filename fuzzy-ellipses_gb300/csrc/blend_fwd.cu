@@ -38,7 +38,7 @@ struct BlendSmem {
   GaussRec src[2 * CH];     // source records of the next chunk (TMA bulk copies), record r at src[r]
   uint64_t bar;             // completion of the source-record copies, one phase per chunk
   uint32_t tile;
-  uint4 entry;              // the work-class list entry of the tile: id, range, view
+  uint4 entry;              // the work-class list entry of the tile: x | y << 16, range, view
   uint32_t cls_base[kTileClasses + 1];  // first work index of each tile class (with `order`)
 };
 
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
   constexpr int RPT = (RC + Sh::NT - 1) / Sh::NT;  // records each thread stages and builds
   const float hw = 0.5f * (TW - 1), hh = 0.5f * (TH - 1);
   // Heaviest tiles first: with `order` (the tile-major binning's per-class tile lists over all
-  // tiles [0, tile_end), uint4 entries: tile id, first key, end key, view) work index w of class
+  // tiles [0, tile_end), uint4 entries: place in the view, first key, end key, view) work index w of class
   // c maps to entry c tile_end + w - cls_base[c], so the tiles taken last, which set the
   // kernel's tail, are the lightest, and a tile's range and view come with its id. The lists are
   // used only when they hold every tile exactly once (their counts sum to tile_end); else tiles
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
     }
   }
   __syncthreads();
-  const bool use_order_all = order && tile_begin == 0 && sm.cls_base[kTileClasses] == tile_end;
+  const bool listed = order && tile_begin == 0 && sm.cls_base[kTileClasses] == tile_end;
   uint32_t phase = 0;  // parity of the next completion of sm.bar
 
   // Work index of the CTA's first tile: its own index (the grid never exceeds the tiles), so the
@@ -269,15 +269,13 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
   bool first = true;
   while (true) {
     if (tid == 0) {
-      uint32_t w = first ? tile_begin + blockIdx.x
-                         : tile_begin + gridDim.x + atomicAdd(counter, 1u);
+      const uint32_t w = first ? tile_begin + blockIdx.x
+                               : tile_begin + gridDim.x + atomicAdd(counter, 1u);
       if (use_order && w < tile_end) {
         int c = 0;
         while (c + 1 < kTileClasses && w >= sm.cls_base[c + 1]) ++c;
-        const uint4 e = reinterpret_cast<const uint4*>(order)[(int64_t)c * tile_end +
-                                                              (w - sm.cls_base[c])];
-        sm.entry = e;
-        w = e.x;
+        sm.entry = reinterpret_cast<const uint4*>(order)[(int64_t)c * tile_end +
+                                                         (w - sm.cls_base[c])];
       }
       sm.tile = w;
     }
@@ -287,16 +285,25 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
     if (item >= tile_end) break;
     const uint32_t piece = SPLIT ? item / n_tiles : 0u;
     const uint32_t tile = SPLIT ? item - piece * n_tiles : item;
-    // With the work-class lists the entry carries the tile's range and view.
-    const bool listed = order && tile_begin == 0 && use_order_all;
-    const int vi = listed ? (int)sm.entry.w : view_of_tile(va, tile);
-    const int gx = view_at(va, vi).gx;
-    const int lt = (int)(tile - view_at(va, vi).tile_base);
-    const int tx = lt % gx, ty = lt / gx;
+    // With the work-class lists the entry carries the tile's place, range and view.
+    int vi, tx, ty;
+    uint2 rg;
+    if (listed) {
+      vi = (int)sm.entry.w;
+      tx = (int)(sm.entry.x & 0xffffu);
+      ty = (int)(sm.entry.x >> 16);
+      rg = make_uint2(sm.entry.y, sm.entry.z);
+    } else {
+      rg = ranges[tile];
+      vi = view_of_tile(va, tile);
+      const int gx = view_at(va, vi).gx;
+      const int lt = (int)(tile - view_at(va, vi).tile_base);
+      ty = lt / gx;
+      tx = lt - ty * gx;
+    }
     const GaussRec* vrec = recs + view_at(va, vi).rec_base;
     const float tcu = tx * TW + hw, tcv = ty * TH + hh;  // tile centre (pixels)
 
-    uint2 rg = listed ? make_uint2(sm.entry.y, sm.entry.z) : ranges[tile];
     bool whole = true;
     if (SPLIT) {
       int per;
