@@ -111,7 +111,7 @@ struct RecSpace {
   uint32_t* incl;
   unsigned long long* scan_tmp;
   uint2* ranges;
-  uint32_t* tile_view;  // tile-major binning of a batch: the view of every tile
+  uint4* tile_ent;  // tile-major binning of a batch: every tile's place, keys and view
   unsigned long long* row_tot;  // tile-major binning: key counts of the tile rows, per view
   uint32_t* order;  // tile-major binning: per work class (kTileClasses lists of n_tiles) the
                     // tiles as uint4 entries (x | y << 16 in the view, first key, end key, view)
@@ -135,7 +135,8 @@ inline cudaError_t zero_ctrl_rows(const RecSpace& rs, int64_t rows, cudaStream_t
 }
 
 template <class F>
-size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, bool bwd, F&& out) {
+size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, bool bwd, F&& out,
+                 bool batch = false) {
   Carver c{base};
   RecSpace s;
   s.ctrl = c.take<Control>(1);
@@ -148,7 +149,9 @@ size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, bo
   s.incl = c.take<uint32_t>(n_rec);
   s.scan_tmp = c.take<unsigned long long>(scan_grid(std::max(n_rec, n_tiles)));
   s.ranges = c.take<uint2>(n_tiles);
-  s.tile_view = c.take<uint32_t>(n_tiles);
+  s.tile_ent = nullptr;
+  if (batch) s.tile_ent = c.take<uint4>(n_tiles);
+  else c.take<uint32_t>(n_tiles);  // (keeps the single-view layout's size)
   s.order = c.take<uint32_t>((int64_t)kTileClasses * n_tiles * 4);  // uint4 entries
   s.rgrad = bwd ? c.take<RecGrad>(n_rec) : nullptr;
   s.part = part_px > 0 ? c.take<float4>(part_px) : nullptr;
@@ -1215,10 +1218,10 @@ int commit_batch(fe_batch* b, cudaStream_t st) {
       std::max<int64_t>(b->n_tiles, (int64_t)b->rows.n_views * (b->rows.max_gy + 1));
   const int64_t part_px =
       b->pieces > 1 ? (int64_t)b->pieces * b->n_tiles * b->tile_w * b->tile_h : 0;
-  const size_t rb = carve_rec(nullptr, b->n_rec, tile_slots, part_px, true, [](const RecSpace&) {});
+  const size_t rb = carve_rec(nullptr, b->n_rec, tile_slots, part_px, true, [](const RecSpace&) {}, true);
   rc = b->rec.reserve(rb, st);
   if (rc) return rc;
-  carve_rec(b->rec.ptr, b->n_rec, tile_slots, part_px, true, [&](const RecSpace& s_) { b->rs = s_; });
+  carve_rec(b->rec.ptr, b->n_rec, tile_slots, part_px, true, [&](const RecSpace& s_) { b->rs = s_; }, true);
   if (!b->exact) {
     const int64_t budget_keys = (int64_t)(key_budget_bytes() / kBytesPerKey);
     b->cap = std::max<int64_t>(1, std::min<int64_t>({b->worst, budget_keys, INT64_C(0xffffffff)}));
@@ -1322,7 +1325,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   p.va.table = b->views_d;
   p.va.count = b->n_views;
   // (written by the tile-major emission, read from the blend on)
-  p.va.tile_view = (b->rows.tiled() && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_view
+  p.va.tile_ent = (b->rows.tiled() && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_ent
                                                                              : nullptr;
   p.n_rec = b->n_rec;
   p.n_tiles = b->n_tiles;
@@ -1390,7 +1393,7 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
   if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
                              p.tile_w, p.tile_h, rs.row_tot, b->cap, rs.ctrl, rs.ranges,
-                             rs.tile_view, ks.keys_a, p.tile_lists ? rs.order : nullptr,
+                             rs.tile_ent, ks.keys_a, p.tile_lists ? rs.order : nullptr,
                              p.n_tiles, st);
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
     b->sorted = ks.keys_a;
@@ -1398,7 +1401,7 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
   } else if (rp.segs) {
     launch_seg_binning(p.va, rp.n_views, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w,
                        p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), b->cap, rs.ctrl,
-                       rs.ranges, rs.tile_view, ks.keys_a, p.tile_lists ? rs.order : nullptr,
+                       rs.ranges, rs.tile_ent, ks.keys_a, p.tile_lists ? rs.order : nullptr,
                        p.n_tiles, st);
     b->sorted = ks.keys_a;
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));

@@ -535,7 +535,7 @@ __device__ __forceinline__ void row_tiles(const int (&cnt)[kTilesPer], unsigned 
                                           unsigned long long row_base, unsigned long long K,
                                           uint32_t lim, Control* __restrict__ ctrl,
                                           uint2* __restrict__ ranges,
-                                          uint32_t* __restrict__ tile_view,
+                                          uint4* __restrict__ tile_ent,
                                           uint32_t* __restrict__ order, int64_t n_tiles,
                                           uint32_t* pos, unsigned long long* wsu) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -568,7 +568,8 @@ __device__ __forceinline__ void row_tiles(const int (&cnt)[kTilesPer], unsigned 
       // every tile of the slice: empty tiles (or tiles whose keys were all dropped) get {0,0}
       rgq[q] = hi > lo ? make_uint2((uint32_t)lo, (uint32_t)hi) : make_uint2(0u, 0u);
       ranges[tile0 + x] = rgq[q];
-      if (tile_view) tile_view[tile0 + x] = blockIdx.y;
+      if (tile_ent) tile_ent[tile0 + x] =
+            make_uint4((uint32_t)x | (uint32_t)row << 16, rgq[q].x, rgq[q].y, blockIdx.y);
     }
     cex += (unsigned)cnt[q];
   }
@@ -651,7 +652,7 @@ __device__ __forceinline__ void tile_emit_body(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
     int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, bool bases,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
-    uint32_t* __restrict__ tile_view,
+    uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
   __shared__ RowRect list[kRowSeg];
   __shared__ int diff[kMaxRowTiles + 1];         // +1 at x0, -1 at x1 of every covering rectangle
@@ -731,7 +732,7 @@ __device__ __forceinline__ void tile_emit_body(
       csum += (unsigned)run;
     }
   }
-  row_tiles(cnt, csum, x_lo, x_hi, row, tile0, row_base, K, lim, ctrl, ranges, tile_view, order, n_tiles,
+  row_tiles(cnt, csum, x_lo, x_hi, row, tile0, row_base, K, lim, ctrl, ranges, tile_ent, order, n_tiles,
             pos, wsu);
   for (int s0 = 0; s0 < n; s0 += kRowSeg) {
     // (with a single segment the list is still in shared memory)
@@ -805,7 +806,7 @@ __global__ void __launch_bounds__(kRowThreads) seg_count_kernel(
 __global__ void __launch_bounds__(kRowThreads) seg_bases_kernel(
     ViewsArg va, int segs, int stride, const unsigned long long* __restrict__ row_tot,
     int64_t capacity, uint32_t* __restrict__ counts, Control* __restrict__ ctrl,
-    uint2* __restrict__ ranges, uint32_t* __restrict__ tile_view, uint32_t* __restrict__ order,
+    uint2* __restrict__ ranges, uint4* __restrict__ tile_ent, uint32_t* __restrict__ order,
     int64_t n_tiles) {
   __shared__ uint32_t pos[kMaxRowTiles];
   __shared__ unsigned long long wsu[kRowWarps];
@@ -847,7 +848,7 @@ __global__ void __launch_bounds__(kRowThreads) seg_bases_kernel(
     cnt[q] = x < gx ? (int)pos[x] : 0;
     csum += (unsigned)cnt[q];
   }
-  row_tiles(cnt, csum, 0, gx, row, tile0, row_base, K, lim, ctrl, ranges, tile_view, order, n_tiles, pos,
+  row_tiles(cnt, csum, 0, gx, row, tile0, row_base, K, lim, ctrl, ranges, tile_ent, order, n_tiles, pos,
             wsu);
 }
 
@@ -887,19 +888,19 @@ __global__ void __launch_bounds__(kRowThreads) tile_emit_kernel(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
     int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, bool bases,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
-    uint32_t* __restrict__ tile_view,
+    uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
   tile_emit_body(va, rects, foot, tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges,
-                 tile_view, keys, order, n_tiles, nseg);
+                 tile_ent, keys, order, n_tiles, nseg);
 }
 __global__ void __launch_bounds__(kRowThreads, 8) tile_emit_kernel_waves(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
     int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, bool bases,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
-    uint32_t* __restrict__ tile_view,
+    uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
   tile_emit_body(va, rects, foot, tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges,
-                 tile_view, keys, order, n_tiles, nseg);
+                 tile_ent, keys, order, n_tiles, nseg);
 }
 
 // Tile-major emission for batches of narrow views (at most 32 tiles per row) once the row bases
@@ -930,7 +931,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
     int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, int stride,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
-    uint32_t* __restrict__ tile_view, uint64_t* __restrict__ keys, uint32_t* __restrict__ order,
+    uint4* __restrict__ tile_ent, uint64_t* __restrict__ keys, uint32_t* __restrict__ order,
     int64_t n_tiles) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned full = 0xffffffffu;
@@ -987,7 +988,8 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     // every tile of the row: empty tiles (or tiles whose keys were all dropped) get {0,0}
     rg = hi > lo ? make_uint2((uint32_t)lo, (uint32_t)hi) : make_uint2(0u, 0u);
     ranges[tile0 + lane] = rg;
-    if (tile_view) tile_view[tile0 + lane] = (uint32_t)v;
+    if (tile_ent) tile_ent[tile0 + lane] =
+          make_uint4((uint32_t)lane | (uint32_t)row << 16, rg.x, rg.y, (uint32_t)v);
   }
   if (order) {
     // Work classes: the lanes of one class share one global atomic for their slots.
@@ -1075,7 +1077,7 @@ uint64_t* launch_sort(uint64_t* a, uint64_t* b, int key_bits, const Control* ctr
 void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int max_gx,
                               const TileRect* rects, const FootRows* foot, int tile_w, int tile_h,
                               unsigned long long* row_tot, int64_t capacity, Control* ctrl,
-                              uint2* ranges, uint32_t* tile_view, uint64_t* keys, uint32_t* order,
+                              uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order,
                               int64_t n_tiles, cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0) return;
   // Beyond a few dozen views the per-block sums over earlier views cost more than two extra
@@ -1089,7 +1091,7 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
       // Narrow views: a warp per tile row instead of a block sized for 1024-tile rows.
       const dim3 grid((unsigned)((max_gy + kWarpRowWarps - 1) / kWarpRowWarps), (unsigned)n_views);
       tile_emit_warp_kernel<<<grid, kWarpRowWarps * 32, 0, st>>>(
-          va, rects, foot, tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges, tile_view,
+          va, rects, foot, tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges, tile_ent,
           keys, order, n_tiles);
       return;
     }
@@ -1105,11 +1107,11 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
   // against 26.5).
   if ((int64_t)grid.x * grid.y > 2 * 5 * 152)
     tile_emit_kernel_waves<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, row_tot,
-                                                         bases, capacity, ctrl, ranges, tile_view,
+                                                         bases, capacity, ctrl, ranges, tile_ent,
                                                          keys, order, n_tiles, nseg);
   else
     tile_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, row_tot, bases,
-                                                   capacity, ctrl, ranges, tile_view, keys, order,
+                                                   capacity, ctrl, ranges, tile_ent, keys, order,
                                                    n_tiles, nseg);
 }
 
@@ -1119,14 +1121,14 @@ int row_segments(int n) { return (n + kRowSeg - 1) / kRowSeg; }
 void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, const TileRect* rects,
                         const FootRows* foot, int tile_w, int tile_h, unsigned long long* row_tot,
                         uint32_t* counts, int64_t capacity, Control* ctrl, uint2* ranges,
-                        uint32_t* tile_view, uint64_t* keys, uint32_t* order, int64_t n_tiles,
+                        uint4* tile_ent, uint64_t* keys, uint32_t* order, int64_t n_tiles,
                         cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0 || segs <= 0) return;
   const dim3 grid((unsigned)max_gy, (unsigned)n_views, (unsigned)segs);
   seg_count_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, max_gy + 1, counts,
                                                  row_tot, ctrl);
   seg_bases_kernel<<<dim3(grid.x, grid.y), kRowThreads, 0, st>>>(
-      va, segs, max_gy + 1, row_tot, capacity, counts, ctrl, ranges, tile_view, order, n_tiles);
+      va, segs, max_gy + 1, row_tot, capacity, counts, ctrl, ranges, tile_ent, order, n_tiles);
   seg_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, max_gy + 1, row_tot,
                                                 counts, ctrl, ranges, keys);
 }

@@ -293,6 +293,12 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
       tx = (int)(sm.entry.x & 0xffffu);
       ty = (int)(sm.entry.x >> 16);
       rg = make_uint2(sm.entry.y, sm.entry.z);
+    } else if (va.tile_ent) {
+      const uint4 e = va.tile_ent[tile];
+      vi = (int)e.w;
+      tx = (int)(e.x & 0xffffu);
+      ty = (int)(e.x >> 16);
+      rg = make_uint2(e.y, e.z);
     } else {
       rg = ranges[tile];
       vi = view_of_tile(va, tile);

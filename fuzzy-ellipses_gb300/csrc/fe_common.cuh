@@ -177,10 +177,11 @@ struct ViewsArg {
   const ViewDev* table;
   int32_t count;
   ViewDev one;
-  // With a table and the tile-major binning: the view of every tile, written by the emission,
-  // so that kernels working per tile look it up with one load instead of a binary search over
-  // the views (11 dependent loads for a thousand views). NULL otherwise.
-  const uint32_t* tile_view;
+  // With a table and the tile-major binning: every tile's place in its view (x | y << 16), first
+  // and end key and view, written by the emission, so that kernels working per tile need one load
+  // instead of a binary search over the views (11 dependent loads for a thousand views) and a
+  // division per thread (256 scenes: 690 -> 676 us per pass). NULL otherwise.
+  const uint4* tile_ent;
   // The one view's pose by value (quaternion, translation), used in place of the pose arrays when
   // has_pose is set.
   float pose[7];
@@ -222,7 +223,7 @@ __device__ __forceinline__ int find_view(const ViewsArg& va, int64_t key) {
 
 // View of a global tile id.
 __device__ __forceinline__ int view_of_tile(const ViewsArg& va, int64_t tile) {
-  if (va.table && va.tile_view) return (int)va.tile_view[tile];
+  if (va.table && va.tile_ent) return (int)va.tile_ent[tile].w;
   return find_view<&ViewDev::tile_base>(va, tile);
 }
 

@@ -59,14 +59,14 @@ uint64_t* launch_sort(uint64_t* a, uint64_t* b, int key_bits, const Control* ctr
 // (kTileClasses lists of n_tiles uint4 entries, 16-byte aligned; ctrl's class counts zeroed)
 // every tile is also appended to the list of its work class (tile_class of its key count) as
 // (x | y << 16 in its view, first key, end key, view), which launch_blend_fwd then serves heaviest class first
-// without reading the tile's range or view again. With `tile_view` (n_tiles entries) every tile's view index is
-// written beside its range (ViewsArg::tile_view).
+// without reading the tile's range or view again. With `tile_ent` (n_tiles entries) every tile's
+// entry of the same form is written at the tile's index (ViewsArg::tile_ent).
 constexpr int kMaxRowTiles = 1024;
 constexpr int kRowBaseViews = 32;  // above this many views the row bases are formed first
 void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int max_gx,
                               const TileRect* rects, const FootRows* foot, int tile_w, int tile_h,
                               unsigned long long* row_tot, int64_t capacity, Control* ctrl,
-                              uint2* ranges, uint32_t* tile_view, uint64_t* keys, uint32_t* order,
+                              uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order,
                               int64_t n_tiles, cudaStream_t st);
 // The same keys, ranges, views and lists for many Gaussians, the records taken in segments
 // (row_segments of the largest view's count) by a block each. launch_preprocess runs without row_tot;
@@ -76,7 +76,7 @@ int64_t seg_count_words(int64_t n_tiles, int segs);
 void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, const TileRect* rects,
                         const FootRows* foot, int tile_w, int tile_h, unsigned long long* row_tot,
                         uint32_t* counts, int64_t capacity, Control* ctrl, uint2* ranges,
-                        uint32_t* tile_view, uint64_t* keys, uint32_t* order, int64_t n_tiles,
+                        uint4* tile_ent, uint64_t* keys, uint32_t* order, int64_t n_tiles,
                         cudaStream_t st);
 // Tile ranges of the sorted keys (ranges zeroed beforehand; empty tiles keep {0,0}).
 void launch_ranges(const uint64_t* keys, const Control* ctrl, int64_t capacity, uint2* ranges,
