@@ -107,6 +107,7 @@ struct RecSpace {
   GaussRec* recs;
   TileRect* rects;
   FootRows* foot;  // footprint rows (unless FE_FLAG_RECT_BINNING)
+  uint32_t* spans;  // each record's tiles per tile row (NULL: formed from foot where needed)
   uint32_t* touched;
   uint32_t* incl;
   unsigned long long* scan_tmp;
@@ -135,8 +136,8 @@ inline cudaError_t zero_ctrl_rows(const RecSpace& rs, int64_t rows, cudaStream_t
 }
 
 template <class F>
-size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, bool bwd, F&& out,
-                 bool batch = false) {
+size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, int64_t n_spans,
+                 bool bwd, F&& out, bool batch = false) {
   Carver c{base};
   RecSpace s;
   s.ctrl = c.take<Control>(1);
@@ -155,6 +156,7 @@ size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, bo
   s.order = c.take<uint32_t>((int64_t)kTileClasses * n_tiles * 4);  // uint4 entries
   s.rgrad = bwd ? c.take<RecGrad>(n_rec) : nullptr;
   s.part = part_px > 0 ? c.take<float4>(part_px) : nullptr;
+  s.spans = n_spans > 0 ? c.take<uint32_t>(n_spans) : nullptr;
   out(s);
   return c.off;
 }
@@ -310,6 +312,19 @@ inline FootRows* foot_of(const Pipeline& p, const RecSpace& rs) {
   return p.rect_binning ? nullptr : rs.foot;
 }
 
+// Entries of the views' row spans (their ViewDev::span_base set in order), or 0 when there are too
+// many to keep (or `off`): the binning then forms the spans from the footprints again.
+constexpr int64_t kMaxSpans = INT64_C(1) << 24;  // 64 MB
+int64_t span_words(ViewDev& first, int64_t n_views, bool off) {
+  ViewDev* v = &first;
+  int64_t n = 0;
+  for (int64_t i = 0; i < n_views; ++i) {
+    v[i].span_base = n;
+    n += (int64_t)v[i].gy * v[i].n;
+  }
+  return off || n > kMaxSpans ? 0 : n;
+}
+
 // Pixels of the blend's piece sums.
 inline int64_t part_pixels(const Pipeline& p) {
   return p.pieces > 1 ? (int64_t)p.pieces * p.n_tiles * p.tile_w * p.tile_h : 0;
@@ -329,14 +344,20 @@ bool can_grow(const DevBuf& buf, size_t bytes, cudaStream_t st) {
 int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
                 unsigned long long* h_pinned, bool bwd, cudaStream_t st, RecSpace& rs,
                 KeySpace& ks, int64_t& cap, uint64_t*& sorted) {
+  int64_t n_spans = span_words(p.va.one, 1, p.rect_binning || p.radix);
   auto rec_bytes = [&] {
-    return carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), bwd, [](const RecSpace&) {});
+    return carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), n_spans, bwd,
+                     [](const RecSpace&) {});
   };
-  // (an arena warmed up for whole tiles stays as it is under capture)
-  if (part_pixels(p) > 0 && !can_grow(recbuf, rec_bytes(), st)) p.pieces = 1;
+  // (under capture an arena stays as large as it was warmed up, without the optional parts)
+  if (!can_grow(recbuf, rec_bytes(), st)) {
+    n_spans = 0;
+    if (!can_grow(recbuf, rec_bytes(), st)) p.pieces = 1;
+  }
   int rc = recbuf.reserve(rec_bytes(), st);
   if (rc) return rc;
-  carve_rec(recbuf.ptr, p.n_rec, p.n_tiles, part_pixels(p), bwd, [&](const RecSpace& s) { rs = s; });
+  carve_rec(recbuf.ptr, p.n_rec, p.n_tiles, part_pixels(p), n_spans, bwd,
+            [&](const RecSpace& s) { rs = s; });
 
   // `worst`: every record touching every tile of its view.
   const bool exact = worst > 0 && (size_t)worst * kBytesPerKey <= key_budget_bytes();
@@ -350,7 +371,8 @@ int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
   if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
-                    rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
+                    rp.tiled() ? rs.spans : nullptr, rs.touched, rp.ok ? rs.row_tot : nullptr,
+                    rp.max_gy, rs.ctrl, st);
   if (exact) {
     cap = worst;
   } else {
@@ -372,13 +394,13 @@ int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
   if (!rp.tiled() || !p.heavy_first) rs.order = nullptr;  // the blend takes tiles in index order
   if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
-                             p.tile_w, p.tile_h, rs.row_tot, cap, rs.ctrl, rs.ranges, nullptr,
-                             ks.keys_a, rs.order, p.n_tiles, st);
+                             rs.spans, p.tile_w, p.tile_h, rs.row_tot, cap, rs.ctrl, rs.ranges,
+                             nullptr, ks.keys_a, rs.order, p.n_tiles, st);
     sorted = ks.keys_a;
   } else if (rp.segs) {
-    launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h,
-                       rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), cap, rs.ctrl, rs.ranges,
-                       nullptr, ks.keys_a, rs.order, p.n_tiles, st);
+    launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), rs.spans, p.tile_w,
+                       p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), cap, rs.ctrl,
+                       rs.ranges, nullptr, ks.keys_a, rs.order, p.n_tiles, st);
     sorted = ks.keys_a;
   } else {
     launch_emit_keys(p.va, rs.incl, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h, p.n_rec, rs.ctrl,
@@ -898,10 +920,10 @@ int fe_reference_binning(int32_t P, int32_t height, int32_t width, float n_std,
   int rc = arena_for(st, &a);
   if (rc) return rc;
   RecSpace rs;
-  const size_t rb = carve_rec(nullptr, P, T, 0, false, [](const RecSpace&) {});
+  const size_t rb = carve_rec(nullptr, P, T, 0, 0, false, [](const RecSpace&) {});
   rc = a->rec.reserve(rb, st);
   if (rc) return rc;
-  carve_rec(a->rec.ptr, P, T, 0, false, [&](const RecSpace& s_) { rs = s_; });
+  carve_rec(a->rec.ptr, P, T, 0, 0, false, [&](const RecSpace& s_) { rs = s_; });
   FE_CUDA(cudaMemsetAsync(rs.ctrl, 0, sizeof(Control), st));
   launch_preprocess_reference(P, n_std, means, scales, rots, LegacyMatrices{view, proj, {}, {}},
                               width, height, tan_fovx, tan_fovy, gx, gy, radii, means2d, rs.rects,
@@ -964,9 +986,9 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   int rc = arena_for(st, &a);
   if (rc) return rc;
   RecSpace rs;
-  rc = a->rec.reserve(carve_rec(nullptr, P, T, 0, false, [](const RecSpace&) {}), st);
+  rc = a->rec.reserve(carve_rec(nullptr, P, T, 0, 0, false, [](const RecSpace&) {}), st);
   if (rc) return rc;
-  carve_rec(a->rec.ptr, P, T, 0, false, [&](const RecSpace& s_) { rs = s_; });
+  carve_rec(a->rec.ptr, P, T, 0, 0, false, [&](const RecSpace& s_) { rs = s_; });
 
   ViewsArg va{};
   va.count = 1;
@@ -996,10 +1018,10 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   carve_keys(a->keys.ptr, cap, [&](const KeySpace& s_) { ks = s_; });
   uint64_t* sorted = ks.keys_a;
   if (rp.ok) {
-    launch_tile_binning_emit(va, 1, rp.max_gy, rp.max_gx, rs.rects, nullptr, 8, 8, rs.row_tot, cap,
-                             rs.ctrl, rs.ranges, nullptr, ks.keys_a, nullptr, T, st);
+    launch_tile_binning_emit(va, 1, rp.max_gy, rp.max_gx, rs.rects, nullptr, nullptr, 8, 8, rs.row_tot,
+                             cap,                              rs.ctrl, rs.ranges, nullptr, ks.keys_a, nullptr, T, st);
   } else if (rp.segs) {
-    launch_seg_binning(va, 1, rp.max_gy, rp.segs, rs.rects, nullptr, 8, 8, rs.row_tot,
+    launch_seg_binning(va, 1, rp.max_gy, rp.segs, rs.rects, nullptr, nullptr, 8, 8, rs.row_tot,
                        reinterpret_cast<uint32_t*>(ks.keys_b), cap, rs.ctrl, rs.ranges, nullptr,
                        ks.keys_a, nullptr, T, st);
   } else {
@@ -1135,6 +1157,7 @@ struct fe_batch {
   std::vector<cudaEvent_t> band_ev;
   RowPlan rows;  // tile-major binning plan (rows.ok) or the emit + sort path
   int pieces = 1;  // most pieces of a tile's keys in the blend
+  int64_t n_spans = 0;
 };
 
 namespace {
@@ -1190,6 +1213,8 @@ int plan_batch(fe_batch* b, const fe_scene* scenes, int32_t n_scenes, const fe_v
   for (const ViewDev& d : b->views_h) max_n = std::max(max_n, (int)d.n);
   const int px = default_px((int)b->desc.px_per_thread, b->tile_w, b->tile_h, tiles);
   b->pieces = blend_pieces(b->tile_w, b->tile_h, px, (int)(b->desc.flags >> 8) & 0xff, tiles, max_n);
+  b->n_spans = span_words(b->views_h[0], n_views,
+                          (b->desc.flags & (FE_FLAG_RECT_BINNING | FE_FLAG_RADIX_BINNING)) != 0);
   fit_segments(b->rows, tiles,
                b->exact ? 0 : std::min(worst, (int64_t)(key_budget_bytes() / kBytesPerKey)));
   return FE_OK;
@@ -1218,10 +1243,14 @@ int commit_batch(fe_batch* b, cudaStream_t st) {
       std::max<int64_t>(b->n_tiles, (int64_t)b->rows.n_views * (b->rows.max_gy + 1));
   const int64_t part_px =
       b->pieces > 1 ? (int64_t)b->pieces * b->n_tiles * b->tile_w * b->tile_h : 0;
-  const size_t rb = carve_rec(nullptr, b->n_rec, tile_slots, part_px, true, [](const RecSpace&) {}, true);
-  rc = b->rec.reserve(rb, st);
+  auto carve = [&](char* base, RecSpace& out) {
+    return carve_rec(base, b->n_rec, tile_slots, part_px, b->n_spans, true,
+                     [&](const RecSpace& s_) { out = s_; }, true);
+  };
+  RecSpace sizes;
+  rc = b->rec.reserve(carve(nullptr, sizes), st);
   if (rc) return rc;
-  carve_rec(b->rec.ptr, b->n_rec, tile_slots, part_px, true, [&](const RecSpace& s_) { b->rs = s_; }, true);
+  carve(b->rec.ptr, b->rs);
   if (!b->exact) {
     const int64_t budget_keys = (int64_t)(key_budget_bytes() / kBytesPerKey);
     b->cap = std::max<int64_t>(1, std::min<int64_t>({b->worst, budget_keys, INT64_C(0xffffffff)}));
@@ -1369,7 +1398,8 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
   if (ev) FE_CUDA(cudaEventRecord(ev[0], st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
-                    rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
+                    rp.tiled() ? rs.spans : nullptr, rs.touched, rp.ok ? rs.row_tot : nullptr,
+                    rp.max_gy, rs.ctrl, st);
   if (ev) FE_CUDA(cudaEventRecord(ev[1], st));
   if (b->exact) {
     if (!rp.ok)
@@ -1392,16 +1422,16 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
   const KeySpace& ks = b->ks;
   if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
-                             p.tile_w, p.tile_h, rs.row_tot, b->cap, rs.ctrl, rs.ranges,
+                             rs.spans, p.tile_w, p.tile_h, rs.row_tot, b->cap, rs.ctrl, rs.ranges,
                              rs.tile_ent, ks.keys_a, p.tile_lists ? rs.order : nullptr,
                              p.n_tiles, st);
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
     b->sorted = ks.keys_a;
     if (ev) FE_CUDA(cudaEventRecord(ev[4], st));
   } else if (rp.segs) {
-    launch_seg_binning(p.va, rp.n_views, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w,
-                       p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), b->cap, rs.ctrl,
-                       rs.ranges, rs.tile_ent, ks.keys_a, p.tile_lists ? rs.order : nullptr,
+    launch_seg_binning(p.va, rp.n_views, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), rs.spans,
+                       p.tile_w, p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), b->cap,
+                       rs.ctrl, rs.ranges, rs.tile_ent, ks.keys_a, p.tile_lists ? rs.order : nullptr,
                        p.n_tiles, st);
     b->sorted = ks.keys_a;
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
@@ -1808,12 +1838,12 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
 
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
   const int64_t worst = p.n_rec * p.n_tiles;
-  size_t rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), false,
+  size_t rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), 0, false,
                                [](const RecSpace&) {});
   const size_t key_bytes = carve_keys(nullptr, worst, [](const KeySpace&) {});
   if (p.pieces > 1 && rec_bytes + key_bytes > (size_t)FE_NOALLOC_SCRATCH_BYTES) {
     p.pieces = 1;  // (what fits with whole tiles is accepted)
-    rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, 0, false, [](const RecSpace&) {});
+    rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, 0, 0, false, [](const RecSpace&) {});
   }
   if (worst > INT64_C(0xffffffff) || rec_bytes + key_bytes > (size_t)FE_NOALLOC_SCRATCH_BYTES)
     return fail(FE_ERR_SCRATCH_LIMIT,
@@ -1828,7 +1858,7 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
   if (rc) return rc;
   RecSpace rs;
   KeySpace ks;
-  carve_rec(base, p.n_rec, p.n_tiles, part_pixels(p), false, [&](const RecSpace& s) { rs = s; });
+  carve_rec(base, p.n_rec, p.n_tiles, part_pixels(p), 0, false, [&](const RecSpace& s) { rs = s; });
   carve_keys(base + rec_bytes, worst, [&](const KeySpace& s) { ks = s; });
 
   // Must start at zero on every call: the control block (key counters, device error word, the
@@ -1841,17 +1871,18 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
   if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
                     p.cull_param, p.tile_w, p.tile_h, rs.recs, rs.rects, foot_of(p, rs),
-                    rs.touched, rp.ok ? rs.row_tot : nullptr, rp.max_gy, rs.ctrl, st);
+                    rp.tiled() ? rs.spans : nullptr, rs.touched, rp.ok ? rs.row_tot : nullptr,
+                    rp.max_gy, rs.ctrl, st);
   uint64_t* sorted = ks.keys_a;
   if (!rp.tiled() || !p.heavy_first) rs.order = nullptr;
   if (rp.segs) {
-    launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h,
-                       rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), worst, rs.ctrl, rs.ranges,
-                       nullptr, ks.keys_a, rs.order, p.n_tiles, st);
+    launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), rs.spans, p.tile_w,
+                       p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), worst, rs.ctrl,
+                       rs.ranges, nullptr, ks.keys_a, rs.order, p.n_tiles, st);
   } else if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
-                             p.tile_w, p.tile_h, rs.row_tot, worst, rs.ctrl, rs.ranges, nullptr,
-                             ks.keys_a, rs.order, p.n_tiles, st);
+                             rs.spans, p.tile_w, p.tile_h, rs.row_tot, worst, rs.ctrl, rs.ranges,
+                             nullptr, ks.keys_a, rs.order, p.n_tiles, st);
   } else {
     launch_scan(rs.touched, rs.incl, p.n_rec, worst, rs.scan_tmp, rs.ctrl, st);
     launch_emit_keys(p.va, rs.incl, rs.rects, foot_of(p, rs), p.tile_w, p.tile_h, p.n_rec, rs.ctrl,

@@ -409,6 +409,40 @@ __device__ __forceinline__ bool covers_row(const TileRect& r, int row) {
   return r.y0 <= row && row < r.y1 && r.x0 < r.x1;
 }
 
+// The records of one view in one tile row: their rectangles, and how their spans are found -- read
+// from `spans` (the row's, written by the preprocess), formed from the footprints, or the whole
+// rectangle.
+struct RowView {
+  const TileRect* rects;
+  const FootRows* foot;
+  const uint32_t* spans;
+  int tile_w, tile_h;
+  // Record i's tiles [x0, x1) in `row`; false when it has none there.
+  __device__ __forceinline__ bool span(int i, int row, int& x0, int& x1) const {
+    const TileRect r = rects[i];
+    if (!covers_row(r, row)) return false;
+    x0 = r.x0;
+    x1 = r.x1;
+    if (spans) {
+      const uint32_t s = spans[i];
+      x0 = (int)(s & 0xffffu);
+      x1 = (int)(s >> 16);
+    } else if (foot) {
+      foot_row_tiles(foot[i], r, row, tile_w, tile_h, x0, x1);
+    }
+    return x1 > x0;
+  }
+};
+
+__device__ __forceinline__ RowView row_view(const ViewDev& V, int row,
+                                            const TileRect* __restrict__ rects,
+                                            const FootRows* __restrict__ foot,
+                                            const uint32_t* __restrict__ spans, int tile_w,
+                                            int tile_h) {
+  return RowView{rects + V.rec_base, foot ? foot + V.rec_base : nullptr,
+                 spans ? spans + V.span_base + (int64_t)row * V.n : nullptr, tile_w, tile_h};
+}
+
 // Sum over the block (kRowThreads threads); every thread gets the result.
 __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v,
                                                             unsigned long long* ws) {
@@ -429,27 +463,18 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v
 // number. Without `foot` a record's span is its rectangle's; with it, the tiles its footprint
 // reaches in the row (records whose footprint misses the row are left out). Ends with a barrier
 // after the list is written.
-__device__ __forceinline__ uint32_t filter_row(const TileRect* __restrict__ vr,
-                                               const FootRows* __restrict__ vf, int tile_w,
-                                               int tile_h, int n, int s0, int row, RowRect* list,
-                                               uint32_t* ws) {
+__device__ __forceinline__ uint32_t filter_row(const RowView& rv, int n, int s0, int row,
+                                               RowRect* list, uint32_t* ws) {
   const int tid = threadIdx.x;
   uint16_t x0[kRowPer], x1[kRowPer];
   uint32_t hits = 0, c = 0;
 #pragma unroll
   for (int q = 0; q < kRowPer; ++q) {
     const int i = s0 + kRowPer * tid + q;
-    const TileRect r = i < n ? vr[i] : TileRect{0, 0, 0, 0};
-    bool h = covers_row(r, row);
-    x0[q] = r.x0;
-    x1[q] = r.x1;
-    if (h && vf) {
-      int a, b;
-      foot_row_tiles(vf[i], r, row, tile_w, tile_h, a, b);
-      x0[q] = (uint16_t)a;
-      x1[q] = (uint16_t)b;
-      h = b > a;
-    }
+    int a = 0, b = 0;
+    const bool h = i < n && rv.span(i, row, a, b);
+    x0[q] = (uint16_t)a;
+    x1[q] = (uint16_t)b;
     hits |= (uint32_t)h << q;
     c += h;
   }
@@ -650,7 +675,8 @@ __device__ __forceinline__ void write_row_keys(const RowRect* list, uint32_t tot
 
 __device__ __forceinline__ void tile_emit_body(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
-    int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, bool bases,
+    const uint32_t* __restrict__ spans, int tile_w, int tile_h,
+    const unsigned long long* __restrict__ row_tot, bool bases,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
     uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
@@ -681,8 +707,7 @@ __device__ __forceinline__ void tile_emit_body(
   const int x_lo = seg * seg_w, x_hi = min(gx, x_lo + seg_w);
   if (x_lo >= x_hi) return;  // (uniform over the block)
   const int64_t tile0 = V.tile_base + (int64_t)row * gx;
-  const TileRect* vr = rects + V.rec_base;
-  const FootRows* vf = foot ? foot + V.rec_base : nullptr;
+  const RowView rv = row_view(V, row, rects, foot, spans, tile_w, tile_h);
 
   // row_tot holds, per view, the key counts of its rows (stride max_gy + 1). With `bases` set,
   // row_offsets_kernel and view_bases_kernel have already turned them into row offsets within
@@ -703,7 +728,7 @@ __device__ __forceinline__ void tile_emit_body(
   __syncthreads();
   uint32_t total = 0;
   for (int s0 = 0; s0 < n; s0 += kRowSeg) {
-    total = filter_row(vr, vf, tile_w, tile_h, n, s0, row, list, ws);
+    total = filter_row(rv, n, s0, row, list, ws);
     for (uint32_t j = tid; j < total; j += kRowThreads) {
       atomicAdd(&diff[list[j].x0], 1);
       atomicAdd(&diff[list[j].x1], -1);
@@ -736,7 +761,7 @@ __device__ __forceinline__ void tile_emit_body(
             pos, wsu);
   for (int s0 = 0; s0 < n; s0 += kRowSeg) {
     // (with a single segment the list is still in shared memory)
-    if (n > kRowSeg) total = filter_row(vr, vf, tile_w, tile_h, n, s0, row, list, ws);
+    if (n > kRowSeg) total = filter_row(rv, n, s0, row, list, ws);
     write_row_keys(list, total, pos, x_lo, x_hi, lim, tile0, row_keys);
     __syncthreads();  // the list is rewritten by the next segment
   }
@@ -751,8 +776,9 @@ __device__ __forceinline__ void tile_emit_body(
 // its 1080 blocks spills and takes 2 us longer.)
 // counts: per tile row of gx tiles, `segs` rows of gx counts (offset: the row's first tile x segs).
 __global__ void __launch_bounds__(kRowThreads) seg_count_kernel(
-    ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot, int tile_w,
-    int tile_h, int stride, uint32_t* __restrict__ counts, unsigned long long* __restrict__ row_tot,
+    ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
+    const uint32_t* __restrict__ spans, int tile_w, int tile_h, int stride,
+    uint32_t* __restrict__ counts, unsigned long long* __restrict__ row_tot,
     Control* __restrict__ ctrl) {
   __shared__ int diff[kMaxRowTiles + 1];  // +1 at x0, -1 at x1 of every covering span
   __shared__ unsigned long long wsu[kRowWarps];
@@ -764,16 +790,14 @@ __global__ void __launch_bounds__(kRowThreads) seg_count_kernel(
   uint32_t* out = counts + (V.tile_base + (int64_t)row * gx) * gridDim.z + (int64_t)blockIdx.z * gx;
   for (int x = tid; x <= gx; x += kRowThreads) diff[x] = 0;
   __syncthreads();
+  const RowView rv = row_view(V, row, rects, foot, spans, tile_w, tile_h);
   unsigned long long sum = 0;
 #pragma unroll
   for (int q = 0; q < kRowPer; ++q) {
     const int i = s0 + q * kRowThreads + tid;
     if (i >= n) continue;
-    const TileRect r = rects[V.rec_base + i];
-    if (!covers_row(r, row)) continue;
-    int x0 = r.x0, x1 = r.x1;
-    if (foot) foot_row_tiles(foot[V.rec_base + i], r, row, tile_w, tile_h, x0, x1);
-    if (x1 <= x0) continue;
+    int x0, x1;
+    if (!rv.span(i, row, x0, x1)) continue;
     atomicAdd(&diff[x0], 1);
     atomicAdd(&diff[x1], -1);
     sum += (unsigned)(x1 - x0);
@@ -855,8 +879,9 @@ __global__ void __launch_bounds__(kRowThreads) seg_bases_kernel(
 // A block per (row, segment): the segment's records reaching the row, in id order, written behind
 // the tiles' keys of the segments before.
 __global__ void __launch_bounds__(kRowThreads) seg_emit_kernel(
-    ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot, int tile_w,
-    int tile_h, int stride, const unsigned long long* __restrict__ row_tot,
+    ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
+    const uint32_t* __restrict__ spans, int tile_w, int tile_h, int stride,
+    const unsigned long long* __restrict__ row_tot,
     const uint32_t* __restrict__ counts, const Control* __restrict__ ctrl,
     const uint2* __restrict__ ranges, uint64_t* __restrict__ keys) {
   __shared__ RowRect list[kRowSeg];
@@ -876,9 +901,8 @@ __global__ void __launch_bounds__(kRowThreads) seg_emit_kernel(
     // (a tile without a range has no keys, or none within the capacity)
     pos[x] = rg.y > rg.x ? (uint32_t)(rg.x - row_base) + c[x] : lim;
   }
-  const uint32_t total =
-      filter_row(rects + V.rec_base, foot ? foot + V.rec_base : nullptr, tile_w, tile_h, n, s0, row,
-                 list, ws);  // (its barriers also publish pos)
+  const RowView rv = row_view(V, row, rects, foot, spans, tile_w, tile_h);
+  const uint32_t total = filter_row(rv, n, s0, row, list, ws);  // (its barriers also publish pos)
   write_row_keys(list, total, pos, 0, gx, lim, tile0, keys + row_base);
 }
 
@@ -886,20 +910,22 @@ __global__ void __launch_bounds__(kRowThreads) seg_emit_kernel(
 // sized for 8 resident blocks per SM (32 registers, a few spills) for launches of many waves.
 __global__ void __launch_bounds__(kRowThreads) tile_emit_kernel(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
-    int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, bool bases,
+    const uint32_t* __restrict__ spans, int tile_w, int tile_h,
+    const unsigned long long* __restrict__ row_tot, bool bases,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
     uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
-  tile_emit_body(va, rects, foot, tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges,
+  tile_emit_body(va, rects, foot, spans, tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges,
                  tile_ent, keys, order, n_tiles, nseg);
 }
 __global__ void __launch_bounds__(kRowThreads, 8) tile_emit_kernel_waves(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
-    int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, bool bases,
+    const uint32_t* __restrict__ spans, int tile_w, int tile_h,
+    const unsigned long long* __restrict__ row_tot, bool bases,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
     uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
-  tile_emit_body(va, rects, foot, tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges,
+  tile_emit_body(va, rects, foot, spans, tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges,
                  tile_ent, keys, order, n_tiles, nseg);
 }
 
@@ -914,22 +940,17 @@ constexpr int kWarpRowCache = 512;  // records whose span masks the key pass reu
 
 // Bit x set when record i of the view reaches tile x of `row` (its footprint's span in the row,
 // or its rectangle's without footprint rows).
-__device__ __forceinline__ uint32_t row_span_mask(const TileRect* __restrict__ vr,
-                                                  const FootRows* __restrict__ vf, int tile_w,
-                                                  int tile_h, int n, int i, int row) {
-  if (i >= n) return 0u;
-  const TileRect r = vr[i];
-  if (!covers_row(r, row)) return 0u;
-  int a = r.x0, b = r.x1;
-  if (vf) foot_row_tiles(vf[i], r, row, tile_w, tile_h, a, b);
-  if (b <= a) return 0u;
+__device__ __forceinline__ uint32_t row_span_mask(const RowView& rv, int n, int i, int row) {
+  int a, b;
+  if (i >= n || !rv.span(i, row, a, b)) return 0u;
   const uint32_t below_b = b >= 32 ? 0xffffffffu : ((1u << b) - 1u);
   return below_b & ~((1u << a) - 1u);
 }
 
 __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     ViewsArg va, const TileRect* __restrict__ rects, const FootRows* __restrict__ foot,
-    int tile_w, int tile_h, const unsigned long long* __restrict__ row_tot, int stride,
+    const uint32_t* __restrict__ spans, int tile_w, int tile_h,
+    const unsigned long long* __restrict__ row_tot, int stride,
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
     uint4* __restrict__ tile_ent, uint64_t* __restrict__ keys, uint32_t* __restrict__ order,
     int64_t n_tiles) {
@@ -952,8 +973,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     return;
   }
   const int64_t tile0 = V.tile_base + (int64_t)row * gx;
-  const TileRect* vr = rects + V.rec_base;
-  const FootRows* vf = foot ? foot + V.rec_base : nullptr;
+  const RowView rv = row_view(V, row, rects, foot, spans, tile_w, tile_h);
   // View base (entry stride - 1) + the row's offset within the view.
   const unsigned long long row_base =
       row_tot[(int64_t)v * stride + stride - 1] + row_tot[(int64_t)v * stride + row];
@@ -967,7 +987,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
   __shared__ uint32_t s_mask[kWarpRowWarps][kWarpRowCache];
   uint32_t cnt = 0;
   for (int s0 = 0; s0 < n; s0 += 32) {
-    const uint32_t m = row_span_mask(vr, vf, tile_w, tile_h, n, s0 + lane, row);
+    const uint32_t m = row_span_mask(rv, n, s0 + lane, row);
     if (s0 < kWarpRowCache) s_mask[warp][s0 + lane] = m;
     for (uint32_t u = __reduce_or_sync(full, m); u; u &= u - 1u) {
       const int x = __ffs(u) - 1;
@@ -1012,7 +1032,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
   for (int s0 = 0; s0 < n; s0 += 32) {
     const int i = s0 + lane;
     const uint32_t m = s0 < kWarpRowCache ? s_mask[warp][i]
-                                          : row_span_mask(vr, vf, tile_w, tile_h, n, i, row);
+                                          : row_span_mask(rv, n, i, row);
     for (uint32_t u = __reduce_or_sync(full, m); u; u &= u - 1u) {
       const int x = __ffs(u) - 1;
       const uint32_t bal = __ballot_sync(full, (m >> x) & 1u);
@@ -1075,9 +1095,9 @@ uint64_t* launch_sort(uint64_t* a, uint64_t* b, int key_bits, const Control* ctr
 
 
 void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int max_gx,
-                              const TileRect* rects, const FootRows* foot, int tile_w, int tile_h,
-                              unsigned long long* row_tot, int64_t capacity, Control* ctrl,
-                              uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order,
+                              const TileRect* rects, const FootRows* foot, const uint32_t* spans,
+                              int tile_w, int tile_h, unsigned long long* row_tot,
+                              int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order,
                               int64_t n_tiles, cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0) return;
   // Beyond a few dozen views the per-block sums over earlier views cost more than two extra
@@ -1091,8 +1111,8 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
       // Narrow views: a warp per tile row instead of a block sized for 1024-tile rows.
       const dim3 grid((unsigned)((max_gy + kWarpRowWarps - 1) / kWarpRowWarps), (unsigned)n_views);
       tile_emit_warp_kernel<<<grid, kWarpRowWarps * 32, 0, st>>>(
-          va, rects, foot, tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges, tile_ent,
-          keys, order, n_tiles);
+          va, rects, foot, spans, tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges,
+          tile_ent, keys, order, n_tiles);
       return;
     }
   }
@@ -1106,12 +1126,12 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
   // (16 views of 640x480: 480 blocks) goes faster with the 48 registers it needs (22.5 us
   // against 26.5).
   if ((int64_t)grid.x * grid.y > 2 * 5 * 152)
-    tile_emit_kernel_waves<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, row_tot,
-                                                         bases, capacity, ctrl, ranges, tile_ent,
+    tile_emit_kernel_waves<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h,
+                                                         row_tot, bases, capacity, ctrl, ranges, tile_ent,
                                                          keys, order, n_tiles, nseg);
   else
-    tile_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, row_tot, bases,
-                                                   capacity, ctrl, ranges, tile_ent, keys, order,
+    tile_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h, row_tot,
+                                                   bases, capacity, ctrl, ranges, tile_ent, keys, order,
                                                    n_tiles, nseg);
 }
 
@@ -1119,18 +1139,18 @@ int64_t seg_count_words(int64_t n_tiles, int segs) { return n_tiles * segs; }
 int row_segments(int n) { return (n + kRowSeg - 1) / kRowSeg; }
 
 void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, const TileRect* rects,
-                        const FootRows* foot, int tile_w, int tile_h, unsigned long long* row_tot,
-                        uint32_t* counts, int64_t capacity, Control* ctrl, uint2* ranges,
-                        uint4* tile_ent, uint64_t* keys, uint32_t* order, int64_t n_tiles,
+                        const FootRows* foot, const uint32_t* spans, int tile_w, int tile_h,
+                        unsigned long long* row_tot, uint32_t* counts, int64_t capacity,
+                        Control* ctrl, uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order, int64_t n_tiles,
                         cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0 || segs <= 0) return;
   const dim3 grid((unsigned)max_gy, (unsigned)n_views, (unsigned)segs);
-  seg_count_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, max_gy + 1, counts,
-                                                 row_tot, ctrl);
+  seg_count_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h, max_gy + 1,
+                                                 counts, row_tot, ctrl);
   seg_bases_kernel<<<dim3(grid.x, grid.y), kRowThreads, 0, st>>>(
       va, segs, max_gy + 1, row_tot, capacity, counts, ctrl, ranges, tile_ent, order, n_tiles);
-  seg_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, tile_w, tile_h, max_gy + 1, row_tot,
-                                                counts, ctrl, ranges, keys);
+  seg_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h, max_gy + 1,
+                                                row_tot, counts, ctrl, ranges, keys);
 }
 
 void launch_ranges(const uint64_t* keys, const Control* ctrl, int64_t capacity, uint2* ranges,

@@ -40,6 +40,7 @@ struct ViewDev {
   int64_t rec_base;       // first record of this view
   int64_t tile_base;      // first global tile id of this view
   int64_t pix_base;       // first output pixel of this view
+  int64_t span_base;      // first entry of this view's row spans: row r of record i at r n + i
 };
 
 // Ray-invariant terms of one (Gaussian, view) pair, in pixel coordinates around an expansion

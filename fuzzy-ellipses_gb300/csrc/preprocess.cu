@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(64) preprocess_kernel(
     const float* __restrict__ logw, const float* __restrict__ quat,
     const float* __restrict__ trans, int cull_mode, float cull_param, int tile_w, int tile_h,
     GaussRec* __restrict__ recs, TileRect* __restrict__ rects, FootRows* __restrict__ foot,
-    uint32_t* __restrict__ touched, unsigned long long* __restrict__ row_tot, int max_gy,
-    Control* __restrict__ ctrl) {
+    uint32_t* __restrict__ spans, uint32_t* __restrict__ touched,
+    unsigned long long* __restrict__ row_tot, int max_gy, Control* __restrict__ ctrl) {
   unsigned long long keys = 0;  // this thread's keys (row_tot != NULL)
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rec;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(64) preprocess_kernel(
     rects[i] = tr;
     uint32_t n_keys;
     if (foot) {
-      foot[i] = f;
+      if (!spans) foot[i] = f;  // (the spans are all that is read of it)
       // Keys of every tile row the footprint reaches (its rows' spans differ).
       unsigned long long* rc = row_tot ? row_tot + (int64_t)vi * (max_gy + 1) : nullptr;
       n_keys = 0;
@@ -152,6 +152,9 @@ __global__ void __launch_bounds__(64) preprocess_kernel(
         int x0, x1;
         foot_row_tiles(f, tr, y, tile_w, tile_h, x0, x1);
         const uint32_t w = (uint32_t)(x1 - x0);
+        if (spans)
+          spans[V.span_base + (int64_t)y * V.n + (i - V.rec_base)] =
+              (uint32_t)x0 | (uint32_t)x1 << 16;
         if (rc && w) atomicAdd(&rc[y], (unsigned long long)w);
         n_keys += w;
       }
@@ -490,15 +493,15 @@ __global__ void __launch_bounds__(64) legacy_preprocess_kernel(
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
                        const float* logw, const float* quat, const float* trans, int cull_mode, float cull_param, int tile_w,
                        int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
-                       uint32_t* touched, unsigned long long* row_tot, int max_gy, Control* ctrl,
-                       cudaStream_t st) {
+                       uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
+                       Control* ctrl, cudaStream_t st) {
   if (n_rec <= 0) return;
   const int threads = 64;
   const int64_t want = (n_rec + threads - 1) / threads;
   const int blocks = (int)(want < 65535 ? want : 65535);
   preprocess_kernel<<<blocks, threads, 0, st>>>(va, n_rec, means, prec, logw, quat, trans,
                                                 cull_mode, cull_param, tile_w, tile_h, recs,
-                                                rects, foot, touched, row_tot, max_gy, ctrl);
+                                                rects, foot, spans, touched, row_tot, max_gy, ctrl);
 }
 
 void launch_preprocess_reference(int P, float n_std, const float* means, const float* scales,

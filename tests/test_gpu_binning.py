@@ -271,6 +271,31 @@ def test_many_view_batch_row_bases_equal_radix_batch(cuda_device, tile):
         assert torch.equal(o[0], out[0][0]) and torch.equal(o[1], out[0][1])
 
 
+def test_tile_major_batch_past_the_row_spans_equals_radix_batch(cuda_device):
+    """More records x tile rows than the 2^24 row spans that are kept: the tile-major binning forms
+    each row's tiles from the footprint rows, for the same keys and images."""
+    rng = np.random.default_rng(31)
+    n, n_views, h, w = 16384, 17, 1024, 48
+    assert n * n_views * (h // 16) > 2 ** 24
+    sc = S.random_gaussians(n, 0.3, rng, scale_lo=0.001, scale_hi=0.003)
+    arrays = [torch.from_numpy(x).to(cuda_device) for x in (sc.means, sc.prec, sc.logw)]
+    views = []
+    for d in S.random_unit_vectors(n_views, rng):
+        q, t = S.look_at(0.9 * d)
+        views.append(dict(scene=0, height=h, width=w, fx=900.0, fy=900.0, cx=w / 2, cy=h / 2, quat=q,
+                          trans=t))
+    out = []
+    for binning in ("radix", "tiles"):
+        b = fe.Batch([(0, n)], views, binning=binning)
+        d, a = b.forward(*arrays)
+        st = b.status()
+        assert st["device_error"] == 0 and st["num_keys"] == st["want_keys"] > n
+        out.append((d, a, st["num_keys"]))
+        b.close()
+    assert out[0][2] == out[1][2]
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
 def _footprint_scenes():
     rng = np.random.default_rng(21)
     out = {}
