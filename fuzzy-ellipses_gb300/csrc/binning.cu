@@ -932,19 +932,50 @@ __global__ void __launch_bounds__(kRowThreads, 8) tile_emit_kernel_waves(
 // Tile-major emission for batches of narrow views (at most 32 tiles per row) once the row bases
 // are formed: one warp per (view, tile row), lane x owning tile x of the row, no block barriers.
 // Same outputs as tile_emit_body: each tile's keys in Gaussian-id order from the row's base,
-// every tile's range and view, and the work-class list entries. Lanes take the view's records
-// 32 at a time; a ballot per tile gives the chunk's records covering it and each one's rank.
+// every tile's range and view, and the work-class list entries. Bound by its instructions: a row is
+// reached by a fraction of its view's records, so those are listed first, and a bit transpose of 32
+// listed spans gives each tile its records (and each record its rank in a tile) at once.
+// 1089 views of 8 to 512 Gaussians: 65 -> 34 us against a ballot per tile for every 32 records.
 constexpr int kWarpRowWarps = 8;
 constexpr int kWarpRowTiles = 32;
-constexpr int kWarpRowCache = 512;  // records whose span masks the key pass reuses
+constexpr int kWarpRowList = 512;  // listed records at a time
+static_assert(kWarpRowTiles == 32, "list entries: x0 | (x1 - 1) << 5 | id << 10");
 
-// Bit x set when record i of the view reaches tile x of `row` (its footprint's span in the row,
-// or its rectangle's without footprint rows).
-__device__ __forceinline__ uint32_t row_span_mask(const RowView& rv, int n, int i, int row) {
-  int a, b;
-  if (i >= n || !rv.span(i, row, a, b)) return 0u;
-  const uint32_t below_b = b >= 32 ? 0xffffffffu : ((1u << b) - 1u);
-  return below_b & ~((1u << a) - 1u);
+// Bit i of lane x's result: bit x of lane i's m.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t m, int lane) {
+  uint32_t lo = 0x0000ffffu;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, m, s);
+    m = (lane & s) ? (m & ~lo) | ((y >> s) & lo) : (m & lo) | ((y & lo) << s);
+    lo ^= lo << (s >> 1);
+  }
+  return m;
+}
+
+// Tiles [x0, x1) of a list entry as bits.
+__device__ __forceinline__ uint32_t entry_tiles(uint32_t e) {
+  return (0xffffffffu >> (31 - ((e >> 5) & 31u))) & (0xffffffffu << (e & 31u));
+}
+
+// Lists the view's records from s on that reach `row`, in id order, until the list may be full or
+// the records end; returns their number.
+__device__ __forceinline__ int list_row(const RowView& rv, int n, int row, int& s, int lane,
+                                        uint32_t* list) {
+  int len = 0;
+  while (s < n && len <= kWarpRowList - 32) {
+    int x0 = 0, x1 = 0;
+    const int i = s + lane;
+    const bool hit = i < n && rv.span(i, row, x0, x1);
+    const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+    if (hit)
+      list[len + __popc(bal & ((1u << lane) - 1u))] =
+          (uint32_t)x0 | (uint32_t)(x1 - 1) << 5 | (uint32_t)i << 10;
+    len += __popc(bal);
+    s += 32;
+  }
+  __syncwarp();
+  return len;
 }
 
 __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
@@ -981,20 +1012,21 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
   const unsigned long long left = K > row_base ? K - row_base : 0ull;
   const uint32_t lim = left < 0xffffffffull ? (uint32_t)left : 0xffffffffu;
 
-  // Keys of each tile (lane x: tile x), then their exclusive prefix along the row. The span
-  // masks of the first kWarpRowCache records are kept for the key pass; only tiles that some
-  // record of a chunk reaches are visited.
-  __shared__ uint32_t s_mask[kWarpRowWarps][kWarpRowCache];
+  // Keys of each tile (lane x: tile x), then their exclusive prefix along the row.
+  __shared__ uint32_t s_list[kWarpRowWarps][kWarpRowList];
+  uint32_t* list = s_list[warp];
   uint32_t cnt = 0;
-  for (int s0 = 0; s0 < n; s0 += 32) {
-    const uint32_t m = row_span_mask(rv, n, s0 + lane, row);
-    if (s0 < kWarpRowCache) s_mask[warp][s0 + lane] = m;
-    for (uint32_t u = __reduce_or_sync(full, m); u; u &= u - 1u) {
-      const int x = __ffs(u) - 1;
-      const uint32_t c = (uint32_t)__popc(__ballot_sync(full, (m >> x) & 1u));
-      if (lane == x) cnt += c;
+  int s0 = 0, len;
+  bool whole;  // the list holds all of the row's records
+  do {
+    whole = s0 == 0;
+    len = list_row(rv, n, row, s0, lane, list);
+    for (int j0 = 0; j0 < len; j0 += 32) {
+      const uint32_t m = j0 + lane < len ? entry_tiles(list[j0 + lane]) : 0u;
+      cnt += (uint32_t)__popc(transpose_bits(m, lane));
     }
-  }
+    __syncwarp();
+  } while (s0 < n);
   uint32_t incl = cnt;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -1026,24 +1058,28 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
           make_uint4((uint32_t)lane | (uint32_t)row << 16, rg.x, rg.y, (uint32_t)v);
     }
   }
-  // Keys: tile x's next slot is lane x's p; a record's rank among the chunk's records covering x
-  // is the ballot's bits below its lane.
+  // Keys: tile x's next slot is lane x's p; lane i writes the keys of its record tile by tile, its
+  // rank in a tile being the tile's records of the 32 before it.
   uint32_t p = ex;
-  for (int s0 = 0; s0 < n; s0 += 32) {
-    const int i = s0 + lane;
-    const uint32_t m = s0 < kWarpRowCache ? s_mask[warp][i]
-                                          : row_span_mask(rv, n, i, row);
-    for (uint32_t u = __reduce_or_sync(full, m); u; u &= u - 1u) {
-      const int x = __ffs(u) - 1;
-      const uint32_t bal = __ballot_sync(full, (m >> x) & 1u);
-      const uint32_t px = __shfl_sync(full, p, x);
-      if ((m >> x) & 1u) {
-        const uint32_t k = px + (uint32_t)__popc(bal & lt_mask);
-        if (k < lim) row_keys[k] = ((uint64_t)(tile0 + x) << 32) | (uint32_t)i;
+  if (!whole) s0 = 0;
+  do {
+    if (!whole) len = list_row(rv, n, row, s0, lane, list);
+    for (int j0 = 0; j0 < len; j0 += 32) {
+      const bool on = j0 + lane < len;
+      const uint32_t e = on ? list[j0 + lane] : 0u;
+      const uint32_t t = transpose_bits(on ? entry_tiles(e) : 0u, lane);
+      const int x0 = (int)(e & 31u), w = on ? (int)((e >> 5) & 31u) + 1 - x0 : 0;
+      const int w_max = __reduce_max_sync(full, w);
+      for (int q = 0; q < w_max; ++q) {
+        const int x = x0 + q;  // (shuffles take the lane modulo 32)
+        const uint32_t tx = __shfl_sync(full, t, x), px = __shfl_sync(full, p, x);
+        const uint32_t k = px + (uint32_t)__popc(tx & lt_mask);
+        if (q < w && k < lim) row_keys[k] = ((uint64_t)(tile0 + x) << 32) | (e >> 10);
       }
-      if (lane == x) p += (uint32_t)__popc(bal);
+      p += (uint32_t)__popc(t);
     }
-  }
+    __syncwarp();
+  } while (!whole && s0 < n);
 }
 
 inline int grid_for(int64_t work, int threads, int cap) {
@@ -1097,7 +1133,8 @@ uint64_t* launch_sort(uint64_t* a, uint64_t* b, int key_bits, const Control* ctr
 void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int max_gx,
                               const TileRect* rects, const FootRows* foot, const uint32_t* spans,
                               int tile_w, int tile_h, unsigned long long* row_tot,
-                              int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order,
+                              int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent,
+                              uint64_t* keys, uint32_t* order,
                               int64_t n_tiles, cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0) return;
   // Beyond a few dozen views the per-block sums over earlier views cost more than two extra

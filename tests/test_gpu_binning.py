@@ -271,6 +271,41 @@ def test_many_view_batch_row_bases_equal_radix_batch(cuda_device, tile):
         assert torch.equal(o[0], out[0][0]) and torch.equal(o[1], out[0][1])
 
 
+@pytest.mark.parametrize("tile,footprint", [((16, 16), "ellipse"), ((8, 8), "ellipse"),
+                                            ((32, 8), "rect")])
+def test_narrow_rows_of_many_records_equal_radix_batch(cuda_device, tile, footprint):
+    """The warp-per-row emission lists a row's records 512 at a time: scenes of none, one, 31 to 33,
+    and around and above 512 listed records, in 40 views 1 to 32 tiles wide."""
+    rng = np.random.default_rng(41)
+    counts = [0, 1, 31, 33, 511, 513, 1700]
+    parts, scenes, off = [], [], 0
+    for n in counts:
+        sc = S.random_gaussians(max(n, 1), 0.05, rng)
+        parts.append((sc.means[:n], sc.prec[:n], sc.logw[:n]))
+        scenes.append((off, n))
+        off += n
+    arrays = [torch.from_numpy(np.concatenate(x)).to(cuda_device) for x in zip(*parts)]
+    views = []
+    for i, d in enumerate(S.random_unit_vectors(40, rng)):
+        q, t = S.look_at(0.5 * d)
+        w = tile[0] * [1, 2, 5, 31, 32][i % 5] - i % 3
+        views.append(dict(scene=i % len(counts), height=17 + 13 * (i % 4), width=w, fx=60.0, fy=60.0,
+                          cx=w / 2, cy=24.0, quat=q, trans=t))
+    out = []
+    for binning, heavy in (("radix", False), ("tiles", False), ("tiles", True)):
+        b = fe.Batch(scenes, views, tile=tile, binning=binning, heavy_first=heavy,
+                     footprint=footprint)
+        assert binning != "tiles" or b.launches_per_forward == 5
+        d, a = b.forward(*arrays)
+        st = b.status()
+        assert st["device_error"] == 0 and st["num_keys"] == st["want_keys"]
+        out.append((d, a, st["num_keys"]))
+        b.close()
+    for o in out[1:]:
+        assert o[2] == out[0][2]
+        assert torch.equal(o[0], out[0][0]) and torch.equal(o[1], out[0][1])
+
+
 def test_tile_major_batch_past_the_row_spans_equals_radix_batch(cuda_device):
     """More records x tile rows than the 2^24 row spans that are kept: the tile-major binning forms
     each row's tiles from the footprint rows, for the same keys and images."""
