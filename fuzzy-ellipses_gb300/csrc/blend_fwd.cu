@@ -245,7 +245,6 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
   // kernel's tail, are the lightest, and a tile's range and view come with its id. The lists are
   // used only when they hold every tile exactly once (their counts sum to tile_end); else tiles
   // go in index order.
-  bool use_order = false;
   if (tid == 0) {
     mbar_init(&sm.bar, 1);
     fence_mbar_init();
@@ -256,7 +255,6 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
         b += ctrl->tile_class[c];
       }
       sm.cls_base[kTileClasses] = b;
-      use_order = b == tile_end;
     }
   }
   __syncthreads();
@@ -268,16 +266,19 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
   // counter, offset by the grid.
   bool first = true;
   while (true) {
-    if (tid == 0) {
-      const uint32_t w = first ? tile_begin + blockIdx.x
-                               : tile_begin + gridDim.x + atomicAdd(counter, 1u);
-      if (use_order && w < tile_end) {
-        int c = 0;
-        while (c + 1 < kTileClasses && w >= sm.cls_base[c + 1]) ++c;
-        sm.entry = reinterpret_cast<const uint4*>(order)[(int64_t)c * tile_end +
-                                                         (w - sm.cls_base[c])];
+    if (tid < 32) {
+      uint32_t w = tile_begin + blockIdx.x;
+      if (!first) {
+        if (tid == 0) w = atomicAdd(counter, 1u);
+        w = tile_begin + gridDim.x + __shfl_sync(0xffffffffu, w, 0);
       }
-      sm.tile = w;
+      if (listed) {  // lane c looks at class c
+        const uint32_t b = tid < kTileClasses ? sm.cls_base[tid] : 0u;
+        const int c = 31 - __clz(__ballot_sync(0xffffffffu, tid < kTileClasses && b <= w));
+        if (tid == c && w < tile_end)
+          sm.entry = reinterpret_cast<const uint4*>(order)[(int64_t)c * tile_end + (w - b)];
+      }
+      if (tid == 0) sm.tile = w;
     }
     first = false;
     __syncthreads();

@@ -293,3 +293,37 @@ def test_heavy_tiles_first_renders_identically(cuda_device, tile):
         out.append(b.forward(ms, ps, ws))
         assert b.status()["device_error"] == 0
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n,h,w,views,tile", [
+    (244, 480, 640, 1, (16, 16)),    # 1200 tiles: under and over a Gaussian per five tiles
+    (245, 480, 640, 1, (16, 16)),
+    (900, 304, 960, 1, (16, 16)),    # 1140 tiles: one and a half per CTA, and just below
+    (900, 303, 944, 1, (16, 16)),
+    (3000, 720, 1111, 1, (16, 16)),  # over 3000 tiles
+    (70, 97, 131, 24, (16, 16)),
+    (1700, 200, 260, 6, (8, 8)),
+    (500, 131, 300, 40, (32, 8)),
+])
+def test_tile_order_the_plan_chooses_renders_identically(cuda_device, n, h, w, views, tile):
+    """Heaviest tiles first, where the launch's tiles and Gaussians choose it, or index order: the
+    same bits as the radix-sorted path, which has no work-class lists."""
+    rng = np.random.default_rng(n)
+    sc = S.random_gaussians(n, 0.1, rng)
+    ms, ps, ws = scene_to_dev(sc, cuda_device)
+    vs = []
+    for d in S.random_unit_vectors(views, rng):
+        q, t = S.look_at(0.5 * d)
+        vs.append(dict(scene=0, height=h, width=w, fx=float(w), fy=float(w), cx=w / 2, cy=h / 2,
+                       quat=q, trans=t))
+    out = []
+    for binning in ("radix", "tiles"):
+        if views == 1:
+            v = vs[0]
+            out.append(fe.render_forward(ms, ps, ws, v["fx"], v["fy"], v["cx"], v["cy"], v["quat"],
+                                         v["trans"], h, w, tile=tile, binning=binning))
+        else:
+            b = fe.Batch([(0, n)], vs, tile=tile, binning=binning)
+            out.append(b.forward(ms, ps, ws))
+            assert b.status()["device_error"] == 0
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
