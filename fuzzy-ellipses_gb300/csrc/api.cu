@@ -432,7 +432,7 @@ int default_px(int px, int tw, int th, int64_t n_tiles) {
 bool heavy_tiles_pay(int tw, int th, int px, int pieces, int64_t n_tiles, int64_t n_rec) {
   if (pieces > 1) return false;
   const int threads = tw * th / (px > 0 ? px : tw * th == 64 ? 2 : 4);
-  const int64_t ctas = 152 * std::min(16, 640 / threads);
+  const int64_t ctas = 152 * (threads == 32 ? 24 : 640 / threads);
   return 2 * n_tiles >= 3 * ctas && 256 * n_tiles <= 5 * n_rec * tw * th;
 }
 

@@ -60,13 +60,15 @@ __device__ __forceinline__ void null_slot(TilePair& p, int sl) {
 template <int TW, int TH, int PX, int CH>
 struct BlendShape {
   static constexpr int NT = TW * TH / PX;
-  // Resident CTAs per SM the register budget is sized for: 20 warps (640 threads) per SM, at
-  // most 16 CTAs (one-warp CTAs would otherwise be squeezed into spilling). 20 warps leave the
+  // Resident CTAs per SM the register budget is sized for: 20 warps (640 threads) per SM leave the
   // 16x16 kernel 94 registers and no spills; at 24 warps it is held to 80 registers, spills a
-  // little and runs about 1.3% slower.
-  static constexpr int MIN_CTAS = (640 / NT) < 16 ? (640 / NT) : 16;
+  // little and runs about 1.3% slower. One-warp CTAs take 24 with groups of two pairs (80
+  // registers), which the 8 KB of a 16-pair chunk allow and the 16 KB of a 32-pair one (13 CTAs)
+  // do not. 8x8 tiles, 13 / 24 CTAs per SM: 16 views of 1000 Gaussians at 640x480 287 / 247 us per
+  // forward, of 200 147 / 119, 1089 uneven views 1068 / 812.
+  static constexpr int MIN_CTAS = NT == 32 ? (CH <= 16 ? 24 : 13) : 640 / NT;
   static constexpr int CW = TW / PX;
-  static constexpr int GP = PX >= 4 ? 2 : 4;
+  static constexpr int GP = PX >= 4 || NT == 32 ? 2 : 4;
   static_assert(TW % PX == 0, "PX must divide the tile width");
   static_assert(CH % GP == 0, "groups must tile a chunk");
   static_assert(NT >= GP, "enough threads to pad a chunk");
@@ -562,7 +564,7 @@ void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_
                   const GaussRec* recs, const uint2* ranges, float nb2, float beta3, float* depth,
                   float* alpha, float* stats, int64_t stats_stride, float4* part, Control* ctrl,
                   cudaStream_t st) {
-  constexpr int PX = kSplitPx, CH = 32, NT = BlendShape<TW, TH, PX, CH>::NT;
+  constexpr int PX = kSplitPx, CH = TW * TH / PX == 32 ? 16 : 32, NT = BlendShape<TW, TH, PX, CH>::NT;
   constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, false, true>;
   const int64_t items = n_tiles * pieces;
   const int64_t grid = std::min<int64_t>(items, resident_ctas<kern>(NT));
@@ -582,7 +584,7 @@ void launch_chunk(int chunk, const ViewsArg& va, int64_t tile_begin, int64_t til
   if (chunk == 8)
     launch_tiles<TW, TH, PX, 8>(va, tile_begin, tile_end, counter, order, keys, recs, ranges, nb2,
                                 beta3, depth, alpha, stats, stats_stride, ctrl, st);
-  else if (chunk == 16)
+  else if (chunk == 16 || (chunk != 32 && TW * TH / PX == 32))
     launch_tiles<TW, TH, PX, 16>(va, tile_begin, tile_end, counter, order, keys, recs, ranges,
                                  nb2, beta3, depth, alpha, stats, stats_stride, ctrl, st);
   else
@@ -617,7 +619,7 @@ void blend_dispatch(const ViewsArg& va, int tile_w, int tile_h, int px, int chun
 }  // namespace
 
 // Pixels per thread: px in {1, 2, 4} (8x8 tiles: 1, 2); 0 selects the default for the tile.
-// Chunk: record pairs per shared-memory stage, 8, 16 or 32; 0 selects 32.
+// Chunk: record pairs per shared-memory stage, 8, 16 or 32; 0 selects 32 (one-warp CTAs: 16).
 void launch_blend_fwd_band(const ViewsArg& va, int tile_w, int tile_h, int px, int chunk,
                            int64_t tile_begin, int64_t tile_end, uint32_t* counter,
                            const uint64_t* keys, const GaussRec* recs, const uint2* ranges,
@@ -670,7 +672,7 @@ void launch_blend_fwd_clean(const ViewsArg& va, int64_t n_tiles, const uint64_t*
                             const GaussRec* recs, const uint2* ranges, float beta2, float beta3,
                             float* depth, float* alpha, Control* ctrl, cudaStream_t st) {
   if (n_tiles <= 0) return;
-  launch_tiles<8, 8, 2, 32, true>(va, 0, n_tiles, &ctrl->next_tile, nullptr, keys, recs, ranges,
+  launch_tiles<8, 8, 2, 16, true>(va, 0, n_tiles, &ctrl->next_tile, nullptr, keys, recs, ranges,
                                   -beta2 * kLog2e, beta3, depth, alpha, nullptr, 0, ctrl, st);
 }
 
