@@ -1560,7 +1560,9 @@ static int batch_forward(fe_batch* b, const float* means, const float* prec, con
   int rc = batch_binning(b, p, st, nullptr);
   if (rc) return rc;
   note_binning(b, means, prec, logw);
-  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles,
+  // (see kManyTiles)
+  const int chunk = !heavy_order && p.chunk == 0 && p.tile_w * p.tile_h > 64 ? 32 : p.chunk;
+  launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, chunk, p.n_tiles,
                    heavy_order ? batch_order(b, p) : nullptr, p.pieces, b->rs.part, b->sorted, b->rs.recs,
                    b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats, p.n_pix, b->rs.ctrl, st);
   FE_CUDA(cudaGetLastError());

@@ -57,7 +57,7 @@ __device__ __forceinline__ void null_slot(TilePair& p, int sl) {
 // Threads per CTA for a tile of TW x TH pixels with PX pixels per thread (PX consecutive pixels
 // of one row, CW = TW/PX threads per row); GP record pairs per online-softmax group (one max
 // update per group).
-template <int TW, int TH, int PX, int CH>
+template <int TW, int TH, int PX, int CH, bool MANY>
 struct BlendShape {
   static constexpr int NT = TW * TH / PX;
   // Resident CTAs per SM the register budget is sized for: 20 warps (640 threads) per SM leave the
@@ -66,7 +66,9 @@ struct BlendShape {
   // registers), which the 8 KB of a 16-pair chunk allow and the 16 KB of a 32-pair one (13 CTAs)
   // do not. 8x8 tiles, 13 / 24 CTAs per SM: 16 views of 1000 Gaussians at 640x480 287 / 247 us per
   // forward, of 200 147 / 119, 1089 uneven views 1068 / 812.
-  static constexpr int MIN_CTAS = NT == 32 ? (CH <= 16 ? 24 : 13) : 640 / NT;
+  // MANY: 22 warps (88 registers, 12 bytes spilled). Each is a little slower, the SM faster, so it is
+  // for launches whose last tiles matter little (see kManyTiles).
+  static constexpr int MIN_CTAS = NT == 32 ? (CH <= 16 ? 24 : 13) : (MANY ? 704 : 640) / NT;
   static constexpr int CW = TW / PX;
   static constexpr int GP = PX >= 4 || NT == 32 ? 2 : 4;
   static_assert(TW % PX == 0, "PX must divide the tile width");
@@ -211,15 +213,15 @@ __device__ __forceinline__ int tile_pieces(int nk, int most, int& per) {
 // CLEAN: the outputs go through clean_value. SPLIT: work index w is piece w / n_tiles of tile
 // w % n_tiles (tile_end = n_tiles x the most pieces); a tile of several pieces leaves each one's
 // sums (max logit, W, Z, A) per pixel in `part` for blend_merge_kernel.
-template <int TW, int TH, int PX, int CH, bool CLEAN, bool SPLIT>
-__global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH>::NT,
-                                  BlendShape<TW, TH, PX, CH>::MIN_CTAS) blend_fwd_kernel(
+template <int TW, int TH, int PX, int CH, bool CLEAN, bool SPLIT, bool MANY>
+__global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
+                                  BlendShape<TW, TH, PX, CH, MANY>::MIN_CTAS) blend_fwd_kernel(
     ViewsArg va, uint32_t tile_begin, uint32_t tile_end, uint32_t* __restrict__ counter,
     const uint32_t* __restrict__ order, const uint64_t* __restrict__ keys,
     const GaussRec* __restrict__ recs, const uint2* __restrict__ ranges, float nb2, float beta3,
     float* __restrict__ depth, float* __restrict__ alpha, float* __restrict__ stats,
     int64_t stats_stride, uint32_t n_tiles, float4* __restrict__ part, Control* __restrict__ ctrl) {
-  using Sh = BlendShape<TW, TH, PX, CH>;
+  using Sh = BlendShape<TW, TH, PX, CH, MANY>;
   constexpr int GP = Sh::GP;
   __shared__ __align__(128) BlendSmem<CH> sm;
 
@@ -546,13 +548,13 @@ __global__ void __launch_bounds__(TW * TH) blend_merge_kernel(
   }
 }
 
-template <int TW, int TH, int PX, int CH, bool CLEAN = false>
+template <int TW, int TH, int PX, int CH, bool CLEAN = false, bool MANY = false>
 void launch_tiles(const ViewsArg& va, int64_t tile_begin, int64_t tile_end, uint32_t* counter,
                   const uint32_t* order, const uint64_t* keys, const GaussRec* recs,
                   const uint2* ranges, float nb2, float beta3, float* depth, float* alpha,
                   float* stats, int64_t stats_stride, Control* ctrl, cudaStream_t st) {
-  constexpr int NT = BlendShape<TW, TH, PX, CH>::NT;
-  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, CLEAN, false>;
+  constexpr int NT = BlendShape<TW, TH, PX, CH, MANY>::NT;
+  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, CLEAN, false, MANY>;
   const int64_t grid = std::min<int64_t>(tile_end - tile_begin, resident_ctas<kern>(NT));
   kern<<<(unsigned)grid, NT, 0, st>>>(va, (uint32_t)tile_begin, (uint32_t)tile_end, counter,
                                       order, keys, recs, ranges, nb2, beta3, depth, alpha, stats,
@@ -564,8 +566,8 @@ void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_
                   const GaussRec* recs, const uint2* ranges, float nb2, float beta3, float* depth,
                   float* alpha, float* stats, int64_t stats_stride, float4* part, Control* ctrl,
                   cudaStream_t st) {
-  constexpr int PX = kSplitPx, CH = TW * TH / PX == 32 ? 16 : 32, NT = BlendShape<TW, TH, PX, CH>::NT;
-  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, false, true>;
+  constexpr int PX = kSplitPx, CH = TW * TH / PX == 32 ? 16 : 32, NT = BlendShape<TW, TH, PX, CH, false>::NT;
+  constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, false, true, false>;
   const int64_t items = n_tiles * pieces;
   const int64_t grid = std::min<int64_t>(items, resident_ctas<kern>(NT));
   kern<<<(unsigned)grid, NT, 0, st>>>(va, 0u, (uint32_t)items, &ctrl->next_tile, nullptr, keys, recs,
@@ -574,6 +576,13 @@ void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_
   blend_merge_kernel<TW, TH><<<(unsigned)n_tiles, TW * TH, 0, st>>>(
       va, (uint32_t)n_tiles, pieces, ranges, part, depth, alpha, stats, stats_stride);
 }
+
+// Tiles from which 22 warps per SM finish sooner than 20 faster ones: 8 per CTA. Forward, 20 / 22
+// warps: 1089 uneven views (122 K tiles) 649 / 633 us, 60 scenes (28 K) 214.3 / 212.5, 16 views of
+// 640x480 (19200) 179.2 / 178.7, of 200 Gaussians 77.5 / 76.0, 32 of 20 Gaussians 84.1 / 80.0; one of
+// 1280x720 (3600) 260 / 275. Launches that store straight into host memory wait for the link and
+// lose 0.5%: they ask for the chunk size they would get.
+constexpr int64_t kManyTiles = 8 * 152 * 11;
 
 template <int TW, int TH, int PX>
 void launch_chunk(int chunk, const ViewsArg& va, int64_t tile_begin, int64_t tile_end,
@@ -587,6 +596,10 @@ void launch_chunk(int chunk, const ViewsArg& va, int64_t tile_begin, int64_t til
   else if (chunk == 16 || (chunk != 32 && TW * TH / PX == 32))
     launch_tiles<TW, TH, PX, 16>(va, tile_begin, tile_end, counter, order, keys, recs, ranges,
                                  nb2, beta3, depth, alpha, stats, stats_stride, ctrl, st);
+  else if (PX == 4 && chunk == 0 && tile_end - tile_begin >= kManyTiles)
+    launch_tiles<TW, TH, PX, 32, false, PX == 4>(va, tile_begin, tile_end, counter, order, keys,
+                                                 recs, ranges, nb2, beta3, depth, alpha, stats,
+                                                 stats_stride, ctrl, st);
   else
     launch_tiles<TW, TH, PX, 32>(va, tile_begin, tile_end, counter, order, keys, recs, ranges,
                                  nb2, beta3, depth, alpha, stats, stats_stride, ctrl, st);

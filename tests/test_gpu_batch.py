@@ -327,3 +327,23 @@ def test_tile_order_the_plan_chooses_renders_identically(cuda_device, n, h, w, v
             out.append(b.forward(ms, ps, ws))
             assert b.status()["device_error"] == 0
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("views,h,w,tile", [(24, 400, 401, (16, 16)), (8, 900, 900, (32, 8))])
+def test_many_tiles_equal_their_chunk_size_asked_for(cuda_device, views, h, w, tile):
+    """Launches of many tiles per CTA run at another number of CTAs per SM: the same bits."""
+    rng = np.random.default_rng(views)
+    sc = S.random_gaussians(700, 0.15, rng)
+    ms, ps, ws = scene_to_dev(sc, cuda_device)
+    vs = []
+    for d in S.random_unit_vectors(views, rng):
+        q, t = S.look_at(0.6 * d)
+        vs.append(dict(scene=0, height=h, width=w, fx=float(w), fy=float(w), cx=w / 2, cy=h / 2,
+                       quat=q, trans=t))
+    assert views * -(-h // tile[1]) * -(-w // tile[0]) >= 14592
+    out = []
+    for chunk in (0, 32):
+        b = fe.Batch([(0, 700)], vs, tile=tile, chunk=chunk)
+        out.append(b.forward(ms, ps, ws))
+        assert b.status()["device_error"] == 0
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
