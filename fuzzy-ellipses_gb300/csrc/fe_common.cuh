@@ -225,6 +225,33 @@ __device__ __forceinline__ int find_view(const ViewsArg& va, int64_t key) {
   return lo;
 }
 
+// View of record i, for a warp whose lanes hold consecutive records (all lanes take part): the view
+// of lane 0's by a 32-way search, a load per step where a binary search would wait for 11 (a thousand
+// views); the other lanes' from the next 32 views' first records, held by the lanes.
+__device__ __forceinline__ int warp_view_of_record(const ViewsArg& va, int64_t i) {
+  if (va.table == nullptr) return 0;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t i0 = __shfl_sync(full, i, 0);
+  int lo = 0, cnt = va.count;
+  while (cnt > 1) {
+    const int step = (cnt + 31) / 32, v = lo + lane * step;
+    const bool le = lane * step < cnt && va.table[v].rec_base <= i0;
+    const int k = 31 - __clz(__ballot_sync(full, le || lane == 0));  // (the bases are sorted)
+    cnt = min(step, cnt - k * step);
+    lo += k * step;
+  }
+  const int64_t base = lo + lane < va.count ? va.table[lo + lane].rec_base : INT64_MAX;
+  int mine = lo, k = 1;
+  for (; k < 32; ++k) {
+    const int64_t b = __shfl_sync(full, base, k);
+    if (!__any_sync(full, b <= i)) break;
+    if (b <= i) mine = lo + k;
+  }
+  // (views without records between these can leave the 32 short)
+  return k < 32 ? mine : find_view<&ViewDev::rec_base>(va, i);
+}
+
 // View of a global tile id.
 __device__ __forceinline__ int view_of_tile(const ViewsArg& va, int64_t tile) {
   if (va.table && va.tile_ent) return (int)va.tile_ent[tile].w;

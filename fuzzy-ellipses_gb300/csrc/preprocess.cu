@@ -114,17 +114,39 @@ __device__ __forceinline__ void footprint_and_record(
   }
 }
 
-__global__ void __launch_bounds__(64) preprocess_kernel(
+// A record's share of the row pass: what a lane needs to form its tiles in one of its tile rows.
+struct __align__(16) RowJob {
+  FootRows f;
+  TileRect tr;
+  int32_t n;         // distance between the rows' spans
+  int32_t keys;      // tiles over all its rows
+  int64_t span;      // its span in row 0
+  int64_t row_tot;   // its view's row totals
+};
+static_assert(sizeof(RowJob) == 64, "RowJob layout");
+
+constexpr int kPrepThreads = 64;
+
+// Bound by the latency of its ~2000 dependent instructions per warp (16 views of 1000 records: one
+// warp per scheduler), a third of them the rows of the tallest footprint of 32 when each lane forms
+// its own record's. The rows of a warp's records are dealt to its lanes instead.
+__global__ void __launch_bounds__(kPrepThreads) preprocess_kernel(
     ViewsArg va, int64_t n_rec, const float* __restrict__ means, const float* __restrict__ prec,
     const float* __restrict__ logw, const float* __restrict__ quat,
     const float* __restrict__ trans, int cull_mode, float cull_param, int tile_w, int tile_h,
     GaussRec* __restrict__ recs, TileRect* __restrict__ rects, FootRows* __restrict__ foot,
     uint32_t* __restrict__ spans, uint32_t* __restrict__ touched,
     unsigned long long* __restrict__ row_tot, int max_gy, Control* __restrict__ ctrl) {
+  __shared__ RowJob jobs[kPrepThreads];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  RowJob* job = jobs + (threadIdx.x & ~31u);  // the warp's
   unsigned long long keys = 0;  // this thread's keys (row_tot != NULL)
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rec;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int vi = find_view<&ViewDev::rec_base>(va, i);
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); i0 < n_rec;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const bool on = i0 + lane < n_rec;
+    const int64_t i = on ? i0 + lane : n_rec - 1;
+    const int vi = warp_view_of_record(va, i);
     const ViewDev& V = view_at(va, vi);
     const int64_t gi = V.gauss_base + (i - V.rec_base);
     float R[9], q[4], t[3], m[3], pr[9];
@@ -139,41 +161,67 @@ __global__ void __launch_bounds__(64) preprocess_kernel(
     int tx0, ty0, tx1, ty1;
     footprint_and_record(m, pr, logw[gi], R, t, V, cull_mode, cull_param, tile_w, tile_h, rec, tx0,
                          ty0, tx1, ty1, foot ? &f : nullptr);
-    recs[i] = rec;
     const TileRect tr{(uint16_t)tx0, (uint16_t)ty0, (uint16_t)tx1, (uint16_t)ty1};
-    rects[i] = tr;
+    if (on) {
+      recs[i] = rec;
+      rects[i] = tr;
+    }
     uint32_t n_keys;
     if (foot) {
-      if (!spans) foot[i] = f;  // (the spans are all that is read of it)
-      // Keys of every tile row the footprint reaches (its rows' spans differ).
-      unsigned long long* rc = row_tot ? row_tot + (int64_t)vi * (max_gy + 1) : nullptr;
-      n_keys = 0;
-      for (int y = ty0; y < ty1; ++y) {
-        int x0, x1;
-        foot_row_tiles(f, tr, y, tile_w, tile_h, x0, x1);
-        const uint32_t w = (uint32_t)(x1 - x0);
-        if (spans)
-          spans[V.span_base + (int64_t)y * V.n + (i - V.rec_base)] =
-              (uint32_t)x0 | (uint32_t)x1 << 16;
-        if (rc && w) atomicAdd(&rc[y], (unsigned long long)w);
-        n_keys += w;
+      if (on && !spans) foot[i] = f;  // (the spans are all that is read of it)
+      // Keys of every tile row the footprint reaches (its rows' spans differ). Row job p of the
+      // warp is row p - before[L] of the last lane L with before[L] <= p.
+      const int rows = on ? ty1 - ty0 : 0;
+      int incl = rows;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += x;
       }
+      const int before = incl - rows, total = __shfl_sync(full, incl, 31);
+      job[lane] = RowJob{f, tr, V.n, 0, V.span_base + (i - V.rec_base),
+                         (int64_t)vi * (max_gy + 1)};
+      __syncwarp();
+      for (int p0 = 0; p0 < total; p0 += 32) {
+        const int p = p0 + lane;
+        int L = 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          if (__shfl_sync(full, before, L + o) <= p) L += o;
+        const int row0 = __shfl_sync(full, before, L);
+        if (p < total) {
+          RowJob& j = job[L];
+          const TileRect jr = j.tr;
+          const int y = jr.y0 + (p - row0);
+          int x0, x1;
+          foot_row_tiles(j.f, jr, y, tile_w, tile_h, x0, x1);
+          const uint32_t w = (uint32_t)(x1 - x0);
+          if (spans) spans[j.span + (int64_t)y * j.n] = (uint32_t)x0 | (uint32_t)x1 << 16;
+          if (w) {
+            if (row_tot) atomicAdd(&row_tot[j.row_tot + y], (unsigned long long)w);
+            atomicAdd(&j.keys, (int)w);
+          }
+        }
+      }
+      __syncwarp();
+      n_keys = on ? (uint32_t)job[lane].keys : 0u;
+      __syncwarp();  // (the jobs are rewritten next round)
     } else {
       // Every row of the rectangle spans its full width.
-      const uint32_t w = (uint32_t)(tx1 - tx0);
+      const uint32_t w = on ? (uint32_t)(tx1 - tx0) : 0u;
       n_keys = w * (uint32_t)(ty1 - ty0);
       if (row_tot && w) {
         unsigned long long* rc = row_tot + (int64_t)vi * (max_gy + 1);
         for (int y = ty0; y < ty1; ++y) atomicAdd(&rc[y], (unsigned long long)w);
       }
     }
-    touched[i] = n_keys;
+    if (on) touched[i] = n_keys;
     keys += n_keys;
   }
   if (row_tot != nullptr) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) keys += __shfl_xor_sync(0xffffffffu, keys, o);
-    if ((threadIdx.x & 31) == 0 && keys) atomicAdd(&ctrl->want_keys, keys);
+    for (int o = 16; o > 0; o >>= 1) keys += __shfl_xor_sync(full, keys, o);
+    if (lane == 0 && keys) atomicAdd(&ctrl->want_keys, keys);
   }
 }
 
@@ -496,7 +544,7 @@ void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, co
                        uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
                        Control* ctrl, cudaStream_t st) {
   if (n_rec <= 0) return;
-  const int threads = 64;
+  const int threads = kPrepThreads;
   const int64_t want = (n_rec + threads - 1) / threads;
   const int blocks = (int)(want < 65535 ? want : 65535);
   preprocess_kernel<<<blocks, threads, 0, st>>>(va, n_rec, means, prec, logw, quat, trans,

@@ -347,3 +347,34 @@ def test_many_tiles_equal_their_chunk_size_asked_for(cuda_device, views, h, w, t
         out.append(b.forward(ms, ps, ws))
         assert b.status()["device_error"] == 0
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("empty", [0, 1, 30, 31, 32, 45, 1100])
+def test_records_find_their_view_across_empty_ones(cuda_device, empty):
+    """Records of neighbouring views in one warp, with views of no Gaussians between them: each
+    view's image is its scene's alone."""
+    rng = np.random.default_rng(empty)
+    sizes = [3, 1, 40, 0, 7]
+    scenes, parts, off = [], [], 0
+    for n in sizes:
+        sc = S.random_gaussians(max(n, 1), 0.05, rng)
+        parts.append((sc.means[:n], sc.prec[:n], sc.logw[:n]))
+        scenes.append((off, n))
+        off += n
+    arrays = [torch.from_numpy(np.concatenate(x)).to(cuda_device) for x in zip(*parts)]
+    h, w, order = 20, 24, [0, 1] + [3] * empty + [2, 4]
+    views = []
+    for si in order:
+        q, t = S.look_at(0.4 * S.random_unit_vectors(1, rng)[0])
+        views.append(dict(scene=si, height=h, width=w, fx=24.0, fy=24.0, cx=w / 2, cy=h / 2, quat=q,
+                          trans=t))
+    b = fe.Batch(scenes, views)
+    depth, alpha = b.forward(*arrays)
+    assert b.status()["device_error"] == 0
+    for i in [0, 1, len(order) // 2, len(order) - 2, len(order) - 1]:
+        o, n = scenes[order[i]]
+        v = views[i]
+        d, a = fe.render_forward(*[x[o:o + n].contiguous() for x in arrays], v["fx"], v["fy"],
+                                 v["cx"], v["cy"], v["quat"], v["trans"], h, w)
+        torch.testing.assert_close(b.view_image(depth, i), d, rtol=1e-6, atol=1e-7)
+        torch.testing.assert_close(b.view_image(alpha, i), a, rtol=0, atol=1e-6)
