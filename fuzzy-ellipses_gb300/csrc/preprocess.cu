@@ -129,7 +129,8 @@ constexpr int kPrepThreads = 64;
 
 // Bound by the latency of its ~2000 dependent instructions per warp (16 views of 1000 records: one
 // warp per scheduler), a third of them the rows of the tallest footprint of 32 when each lane forms
-// its own record's. The rows of a warp's records are dealt to its lanes instead.
+// its own record's. The rows of a warp's records are dealt to its lanes instead:
+// forward of those views 178.3 -> 176.7 us, in 8x8 tiles 247 -> 243.
 __global__ void __launch_bounds__(kPrepThreads) preprocess_kernel(
     ViewsArg va, int64_t n_rec, const float* __restrict__ means, const float* __restrict__ prec,
     const float* __restrict__ logw, const float* __restrict__ quat,
@@ -539,8 +540,8 @@ __global__ void __launch_bounds__(64) legacy_preprocess_kernel(
 // ------------------------------------------------------------------------------------------
 
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
-                       const float* logw, const float* quat, const float* trans, int cull_mode, float cull_param, int tile_w,
-                       int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
+                       const float* logw, const float* quat, const float* trans, int cull_mode,
+                       float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
                        uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
                        Control* ctrl, cudaStream_t st) {
   if (n_rec <= 0) return;
