@@ -477,6 +477,9 @@ Pipeline single_view_pipeline(const fe_render_desc* d, const float* means, const
   p.beta2 = d->beta2;
   p.beta3 = d->beta3;
   p.means = means; p.prec = prec; p.logw = logw; p.quat = quat; p.trans = trans;
+  // A chained launch costs the host about a microsecond, which a call of fewer Gaussians, as long
+  // on the host as on the device, would only lose (40 Gaussians at 200x200 40.5 -> 42 us).
+  p.va.chain = p.n_rec > kSegMinN;
   if (d->flags & FE_FLAG_HOST_POSE) {
     std::memcpy(p.va.pose, quat, 4 * sizeof(float));
     std::memcpy(p.va.pose + 4, trans, 3 * sizeof(float));
@@ -512,6 +515,7 @@ int render_features(const fe_render_desc* d, const float* means, const float* pr
   rc = arena_for(st, &a);
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
+  p.va.chain = 1;
   if (!depth) p.pieces = 1;  // (nothing is blended forward)
   RecSpace rs;
   KeySpace ks;
@@ -1369,6 +1373,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   Pipeline p{};
   p.va.table = b->views_d;
   p.va.count = b->n_views;
+  p.va.chain = 1;
   // (written by the tile-major emission, read from the blend on)
   p.va.tile_ent = (b->rows.tiled() && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_ent
                                                                              : nullptr;

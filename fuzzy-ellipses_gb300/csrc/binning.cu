@@ -495,6 +495,8 @@ __device__ __forceinline__ uint32_t filter_row(const RowView& rv, int n, int s0,
 __global__ void __launch_bounds__(kRowThreads) row_offsets_kernel(ViewsArg va, int n_views,
                                                                    int max_gy,
                                                                    unsigned long long* row_tot) {
+  chain_next();
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const int v = (int)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
   if (v >= n_views) return;  // (uniform over the warp)
@@ -521,6 +523,8 @@ __global__ void __launch_bounds__(kRowThreads) row_offsets_kernel(ViewsArg va, i
 // Thread t takes the consecutive views [t vpt, t vpt + vpt).
 __global__ void __launch_bounds__(kRowThreads) view_bases_kernel(int n_views, int max_gy,
                                                                   unsigned long long* row_tot) {
+  chain_next();
+  chain_wait();
   __shared__ unsigned long long ws[kRowWarps];
   const int stride = max_gy + 1;
   const int vpt = (n_views + kRowThreads - 1) / kRowThreads;
@@ -680,6 +684,7 @@ __device__ __forceinline__ void tile_emit_body(
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
     uint4* __restrict__ tile_ent,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ order, int64_t n_tiles, int nseg) {
+  chain_wait();
   __shared__ RowRect list[kRowSeg];
   __shared__ int diff[kMaxRowTiles + 1];         // +1 at x0, -1 at x1 of every covering rectangle
   __shared__ uint32_t pos[kMaxRowTiles];  // per tile: next key slot within the row
@@ -780,6 +785,8 @@ __global__ void __launch_bounds__(kRowThreads) seg_count_kernel(
     const uint32_t* __restrict__ spans, int tile_w, int tile_h, int stride,
     uint32_t* __restrict__ counts, unsigned long long* __restrict__ row_tot,
     Control* __restrict__ ctrl) {
+  chain_next();
+  chain_wait();
   __shared__ int diff[kMaxRowTiles + 1];  // +1 at x0, -1 at x1 of every covering span
   __shared__ unsigned long long wsu[kRowWarps];
   __shared__ uint32_t ws[kRowWarps];
@@ -832,6 +839,8 @@ __global__ void __launch_bounds__(kRowThreads) seg_bases_kernel(
     int64_t capacity, uint32_t* __restrict__ counts, Control* __restrict__ ctrl,
     uint2* __restrict__ ranges, uint4* __restrict__ tile_ent, uint32_t* __restrict__ order,
     int64_t n_tiles) {
+  chain_next();
+  chain_wait();
   __shared__ uint32_t pos[kMaxRowTiles];
   __shared__ unsigned long long wsu[kRowWarps];
   const int tid = threadIdx.x;
@@ -884,6 +893,7 @@ __global__ void __launch_bounds__(kRowThreads) seg_emit_kernel(
     const unsigned long long* __restrict__ row_tot,
     const uint32_t* __restrict__ counts, const Control* __restrict__ ctrl,
     const uint2* __restrict__ ranges, uint64_t* __restrict__ keys) {
+  chain_wait();
   __shared__ RowRect list[kRowSeg];
   __shared__ uint32_t pos[kMaxRowTiles];
   __shared__ unsigned long long wsu[kRowWarps];
@@ -985,6 +995,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     int64_t capacity, Control* __restrict__ ctrl, uint2* __restrict__ ranges,
     uint4* __restrict__ tile_ent, uint64_t* __restrict__ keys, uint32_t* __restrict__ order,
     int64_t n_tiles) {
+  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned full = 0xffffffffu;
   const uint32_t lt_mask = (1u << lane) - 1u;
@@ -1141,15 +1152,15 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
   // launches that form all row bases.
   const bool bases = n_views > kRowBaseViews;
   if (bases) {
-    row_offsets_kernel<<<(unsigned)((n_views + kRowWarps - 1) / kRowWarps), kRowThreads, 0, st>>>(
-        va, n_views, max_gy, row_tot);
-    view_bases_kernel<<<1, kRowThreads, 0, st>>>(n_views, max_gy, row_tot);
+    launch_chained(va.chain, row_offsets_kernel, (unsigned)((n_views + kRowWarps - 1) / kRowWarps),
+                   kRowThreads, st, va, n_views, max_gy, row_tot);
+    launch_chained(va.chain, view_bases_kernel, 1, kRowThreads, st, n_views, max_gy, row_tot);
     if (max_gx <= kWarpRowTiles) {
       // Narrow views: a warp per tile row instead of a block sized for 1024-tile rows.
       const dim3 grid((unsigned)((max_gy + kWarpRowWarps - 1) / kWarpRowWarps), (unsigned)n_views);
-      tile_emit_warp_kernel<<<grid, kWarpRowWarps * 32, 0, st>>>(
-          va, rects, foot, spans, tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges,
-          tile_ent, keys, order, n_tiles);
+      launch_chained(va.chain, tile_emit_warp_kernel, grid, kWarpRowWarps * 32, st, va, rects, foot, spans,
+                     tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges, tile_ent, keys,
+                     order, n_tiles);
       return;
     }
   }
@@ -1163,13 +1174,12 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
   // (16 views of 640x480: 480 blocks) goes faster with the 48 registers it needs (22.5 us
   // against 26.5).
   if ((int64_t)grid.x * grid.y > 2 * 5 * 152)
-    tile_emit_kernel_waves<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h,
-                                                         row_tot, bases, capacity, ctrl, ranges, tile_ent,
-                                                         keys, order, n_tiles, nseg);
+    launch_chained(va.chain, tile_emit_kernel_waves, grid, kRowThreads, st, va, rects, foot, spans,
+                   tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges, tile_ent, keys, order, n_tiles,
+                   nseg);
   else
-    tile_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h, row_tot,
-                                                   bases, capacity, ctrl, ranges, tile_ent, keys, order,
-                                                   n_tiles, nseg);
+    launch_chained(va.chain, tile_emit_kernel, grid, kRowThreads, st, va, rects, foot, spans, tile_w,
+                   tile_h, row_tot, bases, capacity, ctrl, ranges, tile_ent, keys, order, n_tiles, nseg);
 }
 
 int64_t seg_count_words(int64_t n_tiles, int segs) { return n_tiles * segs; }
@@ -1182,12 +1192,12 @@ void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, c
                         cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0 || segs <= 0) return;
   const dim3 grid((unsigned)max_gy, (unsigned)n_views, (unsigned)segs);
-  seg_count_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h, max_gy + 1,
-                                                 counts, row_tot, ctrl);
-  seg_bases_kernel<<<dim3(grid.x, grid.y), kRowThreads, 0, st>>>(
-      va, segs, max_gy + 1, row_tot, capacity, counts, ctrl, ranges, tile_ent, order, n_tiles);
-  seg_emit_kernel<<<grid, kRowThreads, 0, st>>>(va, rects, foot, spans, tile_w, tile_h, max_gy + 1,
-                                                row_tot, counts, ctrl, ranges, keys);
+  launch_chained(va.chain, seg_count_kernel, grid, kRowThreads, st, va, rects, foot, spans, tile_w,
+                 tile_h, max_gy + 1, counts, row_tot, ctrl);
+  launch_chained(va.chain, seg_bases_kernel, dim3(grid.x, grid.y), kRowThreads, st, va, segs,
+                 max_gy + 1, row_tot, capacity, counts, ctrl, ranges, tile_ent, order, n_tiles);
+  launch_chained(va.chain, seg_emit_kernel, grid, kRowThreads, st, va, rects, foot, spans, tile_w,
+                 tile_h, max_gy + 1, row_tot, counts, ctrl, ranges, keys);
 }
 
 void launch_ranges(const uint64_t* keys, const Control* ctrl, int64_t capacity, uint2* ranges,

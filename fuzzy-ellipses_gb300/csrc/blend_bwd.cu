@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(256) bwd_zero_kernel(float* __restrict__ gmean
                                                        float* __restrict__ glogw, int64_t n_gauss,
                                                        RecGrad* __restrict__ rgrad, int64_t n_rec,
                                                        Control* __restrict__ ctrl) {
+  chain_next();
   const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   if (first == 0) ctrl->next_tile = 0u;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
     float beta2, RecGrad* __restrict__ rgrad, Control* ctrl) {
   using Slice = BwdSlice<TW, TH>;
   __shared__ Slice slices[kBwdWarps];
+  chain_wait();
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   Slice& sl = slices[threadIdx.x >> 5];
@@ -389,6 +391,7 @@ __global__ void record_vjp_kernel(ViewsArg va, int64_t n_rec, const float* __res
                                   const float* __restrict__ trans, const GaussRec* __restrict__ recs,
                                   const RecGrad* __restrict__ rgrad, float* __restrict__ gmeans,
                                   float* __restrict__ gprec, float* __restrict__ glogw) {
+  chain_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_rec;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int vi = find_view<&ViewDev::rec_base>(va, i);
@@ -501,9 +504,9 @@ void launch_bwd_tiles(const ViewsArg& va, int64_t n_tiles, const uint32_t* order
   const int64_t items = n_tiles << bits;
   const int64_t grid =
       std::max<int64_t>(1, std::min<int64_t>((items + kBwdWarps - 1) / kBwdWarps, resident));
-  kern<<<(unsigned)grid, 32 * kBwdWarps, 0, st>>>(va, (uint32_t)n_tiles, bits, order, keys, ranges,
-                                                  recs, depth, stats, stride, gdepth, galpha,
-                                                  -beta2 * kLog2e, beta3, beta2, rgrad, ctrl);
+  launch_chained(va.chain, kern, (unsigned)grid, 32 * kBwdWarps, st, va, (uint32_t)n_tiles, bits,
+                 order, keys, ranges, recs, depth, stats, stride, gdepth, galpha, -beta2 * kLog2e, beta3, beta2,
+                 rgrad, ctrl);
 }
 
 }  // namespace
@@ -541,8 +544,8 @@ void launch_record_vjp(const ViewsArg& va, int64_t n_rec, const float* means, co
                        cudaStream_t st) {
   if (n_rec <= 0) return;
   const int64_t want = (n_rec + 127) / 128;
-  record_vjp_kernel<float><<<(int)(want < 65535 ? want : 65535), 128, 0, st>>>(
-      va, n_rec, means, prec, quat, trans, recs, rgrad, gmeans, gprec, glogw);
+  launch_chained(va.chain, record_vjp_kernel<float>, (unsigned)(want < 65535 ? want : 65535), 128, st, va,
+                 n_rec, means, prec, quat, trans, recs, rgrad, gmeans, gprec, glogw);
 }
 
 }  // namespace fe

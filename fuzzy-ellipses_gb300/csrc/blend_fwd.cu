@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
   // kernel's tail, are the lightest, and a tile's range and view come with its id. The lists are
   // used only when they hold every tile exactly once (their counts sum to tile_end); else tiles
   // go in index order.
+  chain_wait();
   if (tid == 0) {
     mbar_init(&sm.bar, 1);
     fence_mbar_init();
@@ -519,6 +520,7 @@ __global__ void __launch_bounds__(TW * TH) blend_merge_kernel(
     ViewsArg va, uint32_t n_tiles, int most, const uint2* __restrict__ ranges,
     const float4* __restrict__ part, float* __restrict__ depth, float* __restrict__ alpha,
     float* __restrict__ stats, int64_t stats_stride) {
+  chain_wait();
   const uint32_t tile = blockIdx.x;
   const uint2 rg = ranges[tile];
   int per;
@@ -556,9 +558,10 @@ void launch_tiles(const ViewsArg& va, int64_t tile_begin, int64_t tile_end, uint
   constexpr int NT = BlendShape<TW, TH, PX, CH, MANY>::NT;
   constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, CLEAN, false, MANY>;
   const int64_t grid = std::min<int64_t>(tile_end - tile_begin, resident_ctas<kern>(NT));
-  kern<<<(unsigned)grid, NT, 0, st>>>(va, (uint32_t)tile_begin, (uint32_t)tile_end, counter,
-                                      order, keys, recs, ranges, nb2, beta3, depth, alpha, stats,
-                                      stats_stride, 0u, nullptr, ctrl);
+  // (a host call's bands, with counters of their own, follow an event or one another)
+  launch_chained(va.chain && counter == &ctrl->next_tile, kern, (unsigned)grid, NT, st, va,
+                 (uint32_t)tile_begin, (uint32_t)tile_end, counter, order, keys, recs, ranges, nb2,
+                 beta3, depth, alpha, stats, stats_stride, 0u, nullptr, ctrl);
 }
 
 template <int TW, int TH>
@@ -570,11 +573,11 @@ void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_
   constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, false, true, false>;
   const int64_t items = n_tiles * pieces;
   const int64_t grid = std::min<int64_t>(items, resident_ctas<kern>(NT));
-  kern<<<(unsigned)grid, NT, 0, st>>>(va, 0u, (uint32_t)items, &ctrl->next_tile, nullptr, keys, recs,
-                                      ranges, nb2, beta3, depth, alpha, stats, stats_stride,
-                                      (uint32_t)n_tiles, part, ctrl);
-  blend_merge_kernel<TW, TH><<<(unsigned)n_tiles, TW * TH, 0, st>>>(
-      va, (uint32_t)n_tiles, pieces, ranges, part, depth, alpha, stats, stats_stride);
+  launch_chained(va.chain, kern, (unsigned)grid, NT, st, va, 0u, (uint32_t)items,
+                 &ctrl->next_tile, nullptr, keys, recs, ranges, nb2, beta3, depth, alpha, stats, stats_stride,
+                 (uint32_t)n_tiles, part, ctrl);
+  launch_chained(va.chain, blend_merge_kernel<TW, TH>, (unsigned)n_tiles, TW * TH, st, va,
+                 (uint32_t)n_tiles, pieces, ranges, part, depth, alpha, stats, stats_stride);
 }
 
 // Tiles from which 22 warps per SM finish sooner than 20 faster ones: 8 per CTA. Forward, 20 / 22

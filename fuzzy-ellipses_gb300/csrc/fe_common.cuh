@@ -190,6 +190,7 @@ struct ViewsArg {
   // has_pose is set.
   float pose[7];
   int32_t has_pose;
+  int32_t chain;  // the pass's kernels are launched chained (see chain_wait)
 };
 
 // Pose `i`'s quaternion and translation: the one passed by value, or from the arrays.
@@ -261,6 +262,18 @@ __device__ __forceinline__ int view_of_tile(const ViewsArg& va, int64_t tile) {
 // ------------------------------------------------------------------------------------------
 // Inline PTX
 // ------------------------------------------------------------------------------------------
+
+// Chained launches: a kernel that the next one of a pass follows lets it launch early (chain_next),
+// and the next one waits for its completion and its writes (chain_wait) before it touches memory, so
+// that the launch and the start of its blocks are hidden behind the end of the one before. The last
+// kernel of the binning does not let the blend launch early: the blend's blocks would fill the SMs
+// as they come free, the heaviest tiles' blocks side by side on one SM (one 1280x720 view of 24000
+// Gaussians 258 -> 300 us). 20 views of 128x128 88.9 -> 80.0 us per step, features of 16 values
+// 70.7 -> 64.1, that large view 260.4 -> 252.4, 16 views of 640x480 174.2 -> 169.6.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;

@@ -5,6 +5,28 @@
 
 namespace fe {
 
+// Launches a kernel that begins with chain_wait(); with `chain` so that it may start before the
+// kernel launched just before it on `st` has ended (not for the first one after a copy, a memset or
+// an event).
+template <class... P, class... A>
+inline void launch_chained(bool chain, void (*kern)(P...), dim3 grid, unsigned threads,
+                           cudaStream_t st, A... args) {
+  if (!chain) {
+    kern<<<grid, threads, 0, st>>>(static_cast<P>(args)...);
+    return;
+  }
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);  // (errors: cudaGetLastError)
+}
+
 // preprocess.cu. spans (may be NULL; with `foot`, which is then not written): each record's tiles
 // x0 | x1 << 16 in every tile row of its rectangle, at ViewDev::span_base, for the tile-major
 // binning. One thread per record forms them where each of the binning's passes did for each row:

@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(TW * TH / PX) features_kernel(
     float beta3, const float* __restrict__ feats, int nf, int per_pass, float* __restrict__ out) {
   constexpr int NT = TW * TH / PX, CW = TW / PX;
   __shared__ __align__(16) FeatSmem<FC> sm;
+  chain_wait();
   const int tid = threadIdx.x;
   const uint32_t tile = blockIdx.x;
   const int vi = view_of_tile(va, tile);
@@ -197,9 +198,9 @@ void launch_tiles(const ViewsArg& va, int64_t n_tiles, const uint64_t* keys, con
   // against 347 us for 1280x720).
   constexpr int PX = 2;
   const int passes = (nf + FC - 1) / FC;
-  features_kernel<TW, TH, PX, FC><<<(unsigned)n_tiles, TW * TH / PX, 0, st>>>(
-      va, keys, ranges, recs, stats, stride, -beta2 * kLog2e, beta3, feats, nf,
-      (nf + passes - 1) / passes, out);
+  launch_chained(va.chain, features_kernel<TW, TH, PX, FC>, (unsigned)n_tiles, TW * TH / PX, st, va, keys,
+                 ranges, recs, stats, stride, -beta2 * kLog2e, beta3, feats, nf,
+                 (nf + passes - 1) / passes, out);
 }
 
 template <int TW, int TH>

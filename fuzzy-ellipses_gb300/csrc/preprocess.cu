@@ -10,6 +10,8 @@
 //    computeCov3D :65-122, computeCov2D :21-60 and auxiliary.h:46-61,144-169), restated with
 //    explicitly rounded float operations so the compiler cannot contract them, which makes its
 //    tile rectangles bit-reproducible (the reference built with -fmad=false computes the same).
+#include <algorithm>
+
 #include "fe_footprint.cuh"
 #include "fe_kernels.cuh"
 
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kPrepThreads) preprocess_kernel(
     uint32_t* __restrict__ spans, uint32_t* __restrict__ touched,
     unsigned long long* __restrict__ row_tot, int max_gy, Control* __restrict__ ctrl) {
   __shared__ RowJob jobs[kPrepThreads];
+  chain_next();
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   RowJob* job = jobs + (threadIdx.x & ~31u);  // the warp's
@@ -544,9 +547,9 @@ void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, co
                        float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
                        uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
                        Control* ctrl, cudaStream_t st) {
-  if (n_rec <= 0) return;
   const int threads = kPrepThreads;
-  const int64_t want = (n_rec + threads - 1) / threads;
+  // (launched without records too: the binning's first kernel is chained to it)
+  const int64_t want = std::max<int64_t>(1, (n_rec + threads - 1) / threads);
   const int blocks = (int)(want < 65535 ? want : 65535);
   preprocess_kernel<<<blocks, threads, 0, st>>>(va, n_rec, means, prec, logw, quat, trans,
                                                 cull_mode, cull_param, tile_w, tile_h, recs,

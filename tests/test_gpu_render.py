@@ -310,3 +310,38 @@ def test_few_tiles_of_many_gaussians(cuda_device, tile, n, H, W):
     for x, y in zip(got, want):
         assert float((x - y).abs().max()) <= 1e-4 * float(y.abs().max())
     b.close()
+
+
+@pytest.mark.parametrize("n,H,W", [(2500, 64, 80), (2501, 64, 80), (2501, 500, 700), (5000, 730, 1090)])
+def test_chained_launches_replay_from_a_graph(cuda_device, n, H, W):
+    """Calls of more than 2500 Gaussians launch their kernels chained (each may start before the one
+    before has ended): captured and replayed, on other data, they render as the eager call does."""
+    rng = np.random.default_rng(n + H)
+    q, t = S.look_at(0.7 * S.random_unit_vectors(1, rng)[0])
+    q, t = [torch.tensor(np.asarray(x), dtype=torch.float32, device=cuda_device) for x in (q, t)]
+    a, b = [scene_to_dev(S.random_gaussians(n, 0.2, rng), cuda_device) for _ in range(2)]
+    data = [x.clone() for x in a]
+    out = [torch.empty((H, W), device=cuda_device) for _ in range(2)]
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+
+    def go():
+        fe.render_forward(*data, float(W), float(W), W / 2, H / 2, q, t, H, W, out=out)
+
+    with torch.cuda.stream(s):
+        go()
+        go()
+    s.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        go()
+    for x, y in zip(data, b):
+        x.copy_(y)
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    got = [x.clone() for x in out]
+    want = fe.render_forward(*b, float(W), float(W), W / 2, H / 2, q, t, H, W)
+    assert fe.device_status() == 0
+    assert got[1].max() > 0.1
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
