@@ -421,6 +421,11 @@ int default_px(int px, int tw, int th, int64_t n_tiles) {
   return px;
 }
 
+// Whether a pass's kernels are launched chained. Each such launch costs the host up to a
+// microsecond, which a pass of few records and tiles, as long on the host as on the device, would
+// only lose (40 Gaussians at 200x200 40.5 -> 42 us, 1000 at 640x480 45 -> 46.5).
+bool chain_pays(int64_t n_rec, int64_t n_tiles) { return n_rec > kSegMinN || n_tiles >= kPx2Tiles; }
+
 // Whether the blend takes the heaviest tiles first without being asked to: when a CTA gets a second
 // tile at least half the time, so that their order matters, and the launch has enough keys for the lists to pay (they cost
 // 1 to 2 us; at least a Gaussian per five tiles of 256 pixels). Per forward, index order / heaviest
@@ -477,9 +482,7 @@ Pipeline single_view_pipeline(const fe_render_desc* d, const float* means, const
   p.beta2 = d->beta2;
   p.beta3 = d->beta3;
   p.means = means; p.prec = prec; p.logw = logw; p.quat = quat; p.trans = trans;
-  // A chained launch costs the host about a microsecond, which a call of fewer Gaussians, as long
-  // on the host as on the device, would only lose (40 Gaussians at 200x200 40.5 -> 42 us).
-  p.va.chain = p.n_rec > kSegMinN;
+  p.va.chain = chain_pays(p.n_rec, p.n_tiles);
   if (d->flags & FE_FLAG_HOST_POSE) {
     std::memcpy(p.va.pose, quat, 4 * sizeof(float));
     std::memcpy(p.va.pose + 4, trans, 3 * sizeof(float));
@@ -515,7 +518,7 @@ int render_features(const fe_render_desc* d, const float* means, const float* pr
   rc = arena_for(st, &a);
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
-  p.va.chain = 1;
+  p.va.chain |= p.n_rec >= 256;  // (the feature pass makes it a longer call on the device)
   if (!depth) p.pieces = 1;  // (nothing is blended forward)
   RecSpace rs;
   KeySpace ks;
@@ -1373,7 +1376,6 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   Pipeline p{};
   p.va.table = b->views_d;
   p.va.count = b->n_views;
-  p.va.chain = 1;
   // (written by the tile-major emission, read from the blend on)
   p.va.tile_ent = (b->rows.tiled() && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_ent
                                                                              : nullptr;
@@ -1395,6 +1397,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   p.cull_param = b->desc.cull_param;
   p.beta2 = b->desc.beta2;
   p.beta3 = b->desc.beta3;
+  p.va.chain = chain_pays(p.n_rec, p.n_tiles);
   p.means = means; p.prec = prec; p.logw = logw; p.quat = b->quat_d; p.trans = b->trans_d;
   return p;
 }

@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(64) legacy_preprocess_kernel(
 
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
                        const float* logw, const float* quat, const float* trans, int cull_mode,
-                       float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
-                       uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
+                       float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects,
+                       FootRows* foot, uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
                        Control* ctrl, cudaStream_t st) {
   const int threads = kPrepThreads;
   // (launched without records too: the binning's first kernel is chained to it)
