@@ -66,8 +66,9 @@ struct BlendShape {
   // registers), which the 8 KB of a 16-pair chunk allow and the 16 KB of a 32-pair one (13 CTAs)
   // do not. 8x8 tiles, 13 / 24 CTAs per SM: 16 views of 1000 Gaussians at 640x480 287 / 247 us per
   // forward, of 200 147 / 119, 1089 uneven views 1068 / 812.
-  // MANY: 22 warps (88 registers, 12 bytes spilled). Each is a little slower, the SM faster, so it is
-  // for launches whose last tiles matter little (see kManyTiles).
+  // MANY: 11 CTAs asked for (22 warps); 80 registers with 12 bytes spilled then let 12 run. Each is a
+  // little slower, the SM faster, so it is for launches whose last tiles matter little (see
+  // kManyTiles).
   static constexpr int MIN_CTAS = NT == 32 ? (CH <= 16 ? 24 : 13) : (MANY ? 704 : 640) / NT;
   static constexpr int CW = TW / PX;
   static constexpr int GP = PX >= 4 || NT == 32 ? 2 : 4;
@@ -580,7 +581,7 @@ void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_
                  (uint32_t)n_tiles, pieces, ranges, part, depth, alpha, stats, stats_stride);
 }
 
-// Tiles from which 22 warps per SM finish sooner than 20 faster ones: 8 per CTA. Forward, 20 / 22
+// Tiles from which 24 warps per SM finish sooner than 20 faster ones: 7 per CTA. Forward, 20 / 24
 // warps: 1089 uneven views (122 K tiles) 649 / 633 us, 60 scenes (28 K) 214.3 / 212.5, 16 views of
 // 640x480 (19200) 179.2 / 178.7, of 200 Gaussians 77.5 / 76.0, 32 of 20 Gaussians 84.1 / 80.0; one of
 // 1280x720 (3600) 260 / 275. Launches that store straight into host memory wait for the link and
