@@ -246,10 +246,11 @@ struct Pipeline {
 };
 
 // Tile-major binning filters every view's footprint rectangles once per tile row, in one block
-// per row. It is used when every view is at most kMaxRowTiles tiles wide and that filtering is
+// per row. It applies when every view is at most kMaxRowTiles tiles wide and that filtering is
 // cheap: at most 4096 Gaussians per view, or at most 16384 when there are enough row blocks to
 // fill the GPU (measured on GB300: faster than emit + sort for 1-64 views of 20-8000 Gaussians,
-// slower for one 1280x720 view of 24000); the emit + radix sort path is used otherwise.
+// slower for one 1280x720 view of 24000). Where segments of the records (below) are faster still
+// and their counts have room, they are the plan; where neither applies, emit + radix sort.
 constexpr int kRowPlanSmallN = 4096;
 constexpr int kRowPlanLargeN = 16384;
 constexpr int kRowPlanBlocks = 152;  // row blocks that fill a GB300 (its SM count)
@@ -301,10 +302,14 @@ RowPlan row_plan(const ViewDev* views, int n_views) {
   return r;
 }
 
-// The segment counts of a segmented plan live in the sort's second key buffer (`cap` keys), which
-// the tile-major binning does not use; a plan they do not fit gives way to emit + sort.
+// The segment counts of a segmented plan live in the sort's second key buffer (`cap` keys, 0 where
+// its size follows the keys), which the tile-major binning does not use; a plan they do not fit
+// gives way to a block per row where that applies, and to emit + sort elsewhere.
 inline void fit_segments(RowPlan& r, int64_t n_tiles, int64_t cap) {
-  if (r.segs > 0 && seg_count_words(n_tiles, r.segs) > 2 * cap) r.segs = 0;
+  if (r.segs > 0 && seg_count_words(n_tiles, r.segs) > 2 * cap) {
+    r.segs = 0;
+    r.ok = r.plain;
+  }
 }
 
 // Footprint rows of the records, or NULL when each footprint's whole rectangle is binned.
