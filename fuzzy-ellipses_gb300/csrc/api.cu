@@ -135,30 +135,42 @@ inline cudaError_t zero_ctrl_rows(const RecSpace& rs, int64_t rows, cudaStream_t
   return cudaMemsetAsync(rs.ctrl, 0, bytes, st);
 }
 
-template <class F>
-size_t carve_rec(char* base, int64_t n_rec, int64_t n_tiles, int64_t part_px, int64_t n_spans,
-                 bool bwd, F&& out, bool batch = false) {
+// What a RecSpace is laid out for. The optional parts are left out unless a pass uses them.
+struct RecSizes {
+  int64_t n_rec, n_tiles;
+  int64_t row_slots;        // tile rows' key counts, over all views
+  bool lists = false;       // work-class lists
+  bool tile_ent = false;
+  bool bwd = false;         // record gradients
+  int64_t part_px = 0;      // pixels of the blend's piece sums
+  int64_t n_spans = 0;      // row spans of the records
+  RecSizes(int64_t rec, int64_t tiles) : n_rec(rec), n_tiles(tiles), row_slots(tiles + 1) {}
+};
+
+// Lays `z` out from `base` (NULL to measure); returns its bytes.
+size_t carve_rec(char* base, const RecSizes& z, RecSpace& s) {
   Carver c{base};
-  RecSpace s;
   s.ctrl = c.take<Control>(1);
   // (directly after the control block: one memset clears both; see zero_ctrl_rows)
-  s.row_tot = c.take<unsigned long long>(n_tiles + 1);
-  s.recs = c.take<GaussRec>(n_rec);
-  s.rects = c.take<TileRect>(n_rec);
-  s.foot = c.take<FootRows>(n_rec);
-  s.touched = c.take<uint32_t>(n_rec);
-  s.incl = c.take<uint32_t>(n_rec);
-  s.scan_tmp = c.take<unsigned long long>(scan_grid(std::max(n_rec, n_tiles)));
-  s.ranges = c.take<uint2>(n_tiles);
-  s.tile_ent = nullptr;
-  if (batch) s.tile_ent = c.take<uint4>(n_tiles);
-  else c.take<uint32_t>(n_tiles);  // (keeps the single-view layout's size)
-  s.order = c.take<uint32_t>((int64_t)kTileClasses * n_tiles * 4);  // uint4 entries
-  s.rgrad = bwd ? c.take<RecGrad>(n_rec) : nullptr;
-  s.part = part_px > 0 ? c.take<float4>(part_px) : nullptr;
-  s.spans = n_spans > 0 ? c.take<uint32_t>(n_spans) : nullptr;
-  out(s);
+  s.row_tot = c.take<unsigned long long>(z.row_slots);
+  s.recs = c.take<GaussRec>(z.n_rec);
+  s.rects = c.take<TileRect>(z.n_rec);
+  s.foot = c.take<FootRows>(z.n_rec);
+  s.touched = c.take<uint32_t>(z.n_rec);
+  s.incl = c.take<uint32_t>(z.n_rec);
+  s.scan_tmp = c.take<unsigned long long>(scan_grid(std::max(z.n_rec, z.n_tiles)));
+  s.ranges = c.take<uint2>(z.n_tiles);
+  s.tile_ent = z.tile_ent ? c.take<uint4>(z.n_tiles) : nullptr;
+  // (uint4 entries)
+  s.order = z.lists ? c.take<uint32_t>((int64_t)kTileClasses * z.n_tiles * 4) : nullptr;
+  s.rgrad = z.bwd ? c.take<RecGrad>(z.n_rec) : nullptr;
+  s.part = z.part_px > 0 ? c.take<float4>(z.part_px) : nullptr;
+  s.spans = z.n_spans > 0 ? c.take<uint32_t>(z.n_spans) : nullptr;
   return c.off;
+}
+size_t rec_bytes(const RecSizes& z) {
+  RecSpace s;
+  return carve_rec(nullptr, z, s);
 }
 
 template <class F>
@@ -349,20 +361,22 @@ bool can_grow(const DevBuf& buf, size_t bytes, cudaStream_t st) {
 int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
                 unsigned long long* h_pinned, bool bwd, cudaStream_t st, RecSpace& rs,
                 KeySpace& ks, int64_t& cap, uint64_t*& sorted) {
-  int64_t n_spans = span_words(p.va.one, 1, p.rect_binning || p.radix);
-  auto rec_bytes = [&] {
-    return carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), n_spans, bwd,
-                     [](const RecSpace&) {});
-  };
+  RecSizes z(p.n_rec, p.n_tiles);
+  z.lists = true;
+  z.bwd = bwd;
+  z.part_px = part_pixels(p);
+  z.n_spans = span_words(p.va.one, 1, p.rect_binning || p.radix);
   // (under capture an arena stays as large as it was warmed up, without the optional parts)
-  if (!can_grow(recbuf, rec_bytes(), st)) {
-    n_spans = 0;
-    if (!can_grow(recbuf, rec_bytes(), st)) p.pieces = 1;
+  if (!can_grow(recbuf, rec_bytes(z), st)) {
+    z.n_spans = 0;
+    if (!can_grow(recbuf, rec_bytes(z), st)) {
+      p.pieces = 1;
+      z.part_px = 0;
+    }
   }
-  int rc = recbuf.reserve(rec_bytes(), st);
+  int rc = recbuf.reserve(rec_bytes(z), st);
   if (rc) return rc;
-  carve_rec(recbuf.ptr, p.n_rec, p.n_tiles, part_pixels(p), n_spans, bwd,
-            [&](const RecSpace& s) { rs = s; });
+  carve_rec(recbuf.ptr, z, rs);
 
   // `worst`: every record touching every tile of its view.
   const bool exact = worst > 0 && (size_t)worst * kBytesPerKey <= key_budget_bytes();
@@ -948,10 +962,10 @@ int fe_reference_binning(int32_t P, int32_t height, int32_t width, float n_std,
   int rc = arena_for(st, &a);
   if (rc) return rc;
   RecSpace rs;
-  const size_t rb = carve_rec(nullptr, P, T, 0, 0, false, [](const RecSpace&) {});
-  rc = a->rec.reserve(rb, st);
+  const RecSizes sizes(P, T);
+  rc = a->rec.reserve(rec_bytes(sizes), st);
   if (rc) return rc;
-  carve_rec(a->rec.ptr, P, T, 0, 0, false, [&](const RecSpace& s_) { rs = s_; });
+  carve_rec(a->rec.ptr, sizes, rs);
   FE_CUDA(cudaMemsetAsync(rs.ctrl, 0, sizeof(Control), st));
   launch_preprocess_reference(P, n_std, means, scales, rots, LegacyMatrices{view, proj, {}, {}},
                               width, height, tan_fovx, tan_fovy, gx, gy, radii, means2d, rs.rects,
@@ -1014,9 +1028,10 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   int rc = arena_for(st, &a);
   if (rc) return rc;
   RecSpace rs;
-  rc = a->rec.reserve(carve_rec(nullptr, P, T, 0, 0, false, [](const RecSpace&) {}), st);
+  const RecSizes sizes(P, T);
+  rc = a->rec.reserve(rec_bytes(sizes), st);
   if (rc) return rc;
-  carve_rec(a->rec.ptr, P, T, 0, 0, false, [&](const RecSpace& s_) { rs = s_; });
+  carve_rec(a->rec.ptr, sizes, rs);
 
   ViewsArg va{};
   va.count = 1;
@@ -1269,16 +1284,13 @@ int commit_batch(fe_batch* b, cudaStream_t st) {
   // (ranges and row totals: sized for the tiles and for the tile-major binning's row slots)
   const int64_t tile_slots =
       std::max<int64_t>(b->n_tiles, (int64_t)b->rows.n_views * (b->rows.max_gy + 1));
-  const int64_t part_px =
-      b->pieces > 1 ? (int64_t)b->pieces * b->n_tiles * b->tile_w * b->tile_h : 0;
-  auto carve = [&](char* base, RecSpace& out) {
-    return carve_rec(base, b->n_rec, tile_slots, part_px, b->n_spans, true,
-                     [&](const RecSpace& s_) { out = s_; }, true);
-  };
-  RecSpace sizes;
-  rc = b->rec.reserve(carve(nullptr, sizes), st);
+  RecSizes z(b->n_rec, tile_slots);
+  z.lists = z.tile_ent = z.bwd = true;
+  z.part_px = b->pieces > 1 ? (int64_t)b->pieces * b->n_tiles * b->tile_w * b->tile_h : 0;
+  z.n_spans = b->n_spans;
+  rc = b->rec.reserve(rec_bytes(z), st);
   if (rc) return rc;
-  carve(b->rec.ptr, b->rs);
+  carve_rec(b->rec.ptr, z, b->rs);
   if (!b->exact) {
     const int64_t budget_keys = (int64_t)(key_budget_bytes() / kBytesPerKey);
     b->cap = std::max<int64_t>(1, std::min<int64_t>({b->worst, budget_keys, INT64_C(0xffffffff)}));
@@ -1827,6 +1839,10 @@ namespace {
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[FE_NOALLOC_SCRATCH_BYTES];
 
+// The limit counts this much of work-class lists per tile (and a word for its view) for every call,
+// whatever it lays out, so that which sizes are accepted does not depend on how tiles are ordered.
+constexpr size_t kNoallocListBytes = 160;
+
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 char* g_noalloc_base[kMaxDevices] = {};
@@ -1873,35 +1889,42 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
 
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
   const int64_t worst = p.n_rec * p.n_tiles;
-  size_t rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, part_pixels(p), 0, false,
-                               [](const RecSpace&) {});
+  RowPlan rp = p.radix ? RowPlan{} : row_plan(&p.va.one, 1);
+  fit_segments(rp, p.n_tiles, worst);
+  RecSizes z(p.n_rec, p.n_tiles);
   const size_t key_bytes = carve_keys(nullptr, worst, [](const KeySpace&) {});
-  if (p.pieces > 1 && rec_bytes + key_bytes > (size_t)FE_NOALLOC_SCRATCH_BYTES) {
-    p.pieces = 1;  // (what fits with whole tiles is accepted)
-    rec_bytes = carve_rec(nullptr, p.n_rec, p.n_tiles, 0, 0, false, [](const RecSpace&) {});
-  }
-  if (worst > INT64_C(0xffffffff) || rec_bytes + key_bytes > (size_t)FE_NOALLOC_SCRATCH_BYTES)
+  const size_t limit = FE_NOALLOC_SCRATCH_BYTES;
+  const size_t counted = align_up(kNoallocListBytes * (size_t)p.n_tiles) +
+                         align_up(sizeof(uint32_t) * (size_t)p.n_tiles);
+  const size_t need = rec_bytes(z) + counted + key_bytes;
+  if (worst > INT64_C(0xffffffff) || need > limit)
     return fail(FE_ERR_SCRATCH_LIMIT,
                 "fe_render_fwd_noalloc: " + std::to_string(p.n_rec) + " Gaussians x " +
                     std::to_string(p.n_tiles) + " tiles need " +
-                    std::to_string(rec_bytes + key_bytes) +
+                    std::to_string(need) +
                     " bytes of worst-case scratch; the fixed scratch holds " +
-                    std::to_string((size_t)FE_NOALLOC_SCRATCH_BYTES) + " bytes");
+                    std::to_string(limit) + " bytes");
 
   char* base = nullptr;
   rc = noalloc_scratch(&base);
   if (rc) return rc;
+  // The optional parts, as far as there is room (the images are the same without them).
+  z.lists = p.heavy_first && rp.tiled();
+  if (rec_bytes(z) + key_bytes > limit) z.lists = p.heavy_first = false;
+  z.part_px = part_pixels(p);
+  if (rec_bytes(z) + key_bytes > limit) {
+    p.pieces = 1;
+    z.part_px = 0;
+  }
   RecSpace rs;
   KeySpace ks;
-  carve_rec(base, p.n_rec, p.n_tiles, part_pixels(p), 0, false, [&](const RecSpace& s) { rs = s; });
-  carve_keys(base + rec_bytes, worst, [&](const KeySpace& s) { ks = s; });
+  const size_t at_keys = carve_rec(base, z, rs);
+  carve_keys(base + at_keys, worst, [&](const KeySpace& s_) { ks = s_; });
 
   // Must start at zero on every call: the control block (key counters, device error word, the
   // blend's tile counter and work-class counts), the row totals of the tile-major binning, and on
   // the emit + sort path the tile ranges (tiles without keys keep an empty range; the tile-major
   // emission writes every tile's range itself).
-  RowPlan rp = p.radix ? RowPlan{} : row_plan(&p.va.one, 1);
-  fit_segments(rp, p.n_tiles, worst);
   FE_CUDA(zero_ctrl_rows(rs, rp.tiled() ? rp.max_gy + 1 : 0, st));
   if (!rp.tiled()) FE_CUDA(cudaMemsetAsync(rs.ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   launch_preprocess(p.va, p.n_rec, p.means, p.prec, p.logw, p.quat, p.trans, p.cull_mode,
@@ -1909,7 +1932,6 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
                     rp.tiled() ? rs.spans : nullptr, rs.touched, rp.ok ? rs.row_tot : nullptr,
                     rp.max_gy, rs.ctrl, st);
   uint64_t* sorted = ks.keys_a;
-  if (!rp.tiled() || !p.heavy_first) rs.order = nullptr;
   if (rp.segs) {
     launch_seg_binning(p.va, 1, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), rs.spans, p.tile_w,
                        p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), worst, rs.ctrl,

@@ -132,3 +132,26 @@ def test_noalloc_rejects_requests_beyond_the_fixed_scratch(cuda_device):
     assert torch.isnan(outs[1]).all()  # nothing was launched
     # The same request through the arena entry still works.
     assert _call("fe_render_fwd", sd, cam, _desc(scene, cam), outs) == 0
+
+
+@pytest.mark.parametrize("n,tile,flags,fits", [
+    (240, (16, 16), 0, True), (240, (16, 16), N.FE_FLAG_HEAVY_TILES_FIRST, True),
+    (250, (16, 16), 0, False), (250, (16, 16), N.FE_FLAG_HEAVY_TILES_FIRST, False),
+    (40, (8, 8), 0, True), (60, (8, 8), 0, False)])
+def test_noalloc_limit_on_large_images(cuda_device, n, tile, flags, fits):
+    """What fits the fixed scratch on a 3840x2160 image, where the per-tile terms weigh: 32400 tiles
+    x (16 B x 240 keys + 164 B of lists and views counted for every call + ranges and row totals)
+    is inside 128 MiB and 250 are not, whether or not the call lists its tiles."""
+    scene = S.random_gaussians(n, 0.2, np.random.default_rng(14))
+    cam = S.Camera(2160, 3840, 3000.0, 3000.0, 1920.0, 1080.0, *S.look_at([0.9, 0.3, 0.2]))
+    sd = scene_to_dev(scene, cuda_device)
+    desc = _desc(scene, cam, tile, flags=flags)
+    got = _outputs(cam.height, cam.width, cuda_device)
+    rc = _call("fe_render_fwd_noalloc", sd, cam, desc, got)
+    if not fits:
+        assert rc == FE_ERR_SCRATCH_LIMIT and torch.isnan(got[1]).all()
+        return
+    assert rc == 0, N.load().fe_last_error_message()
+    ref = _outputs(cam.height, cam.width, cuda_device)
+    assert _call("fe_render_fwd", sd, cam, desc, ref) == 0
+    _assert_close(ref, got)
