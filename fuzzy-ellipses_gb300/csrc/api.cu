@@ -114,8 +114,8 @@ struct RecSpace {
   uint2* ranges;
   uint4* tile_ent;  // tile-major binning of a batch: every tile's place, keys and view
   unsigned long long* row_tot;  // tile-major binning: key counts of the tile rows, per view
-  uint32_t* order;  // tile-major binning: per work class (kTileClasses lists of n_tiles) the
-                    // tiles as uint4 entries (x | y << 16 in the view, first key, end key, view)
+  uint32_t* order;  // tile-major binning: the tiles by work class (list_entry) as uint4 entries
+                    // (x | y << 16 in the view, first key, end key, view)
   RecGrad* rgrad;  // backward only
   float4* part;    // blend in pieces: the pieces' sums
 };
@@ -162,7 +162,7 @@ size_t carve_rec(char* base, const RecSizes& z, RecSpace& s) {
   s.ranges = c.take<uint2>(z.n_tiles);
   s.tile_ent = z.tile_ent ? c.take<uint4>(z.n_tiles) : nullptr;
   // (uint4 entries)
-  s.order = z.lists ? c.take<uint32_t>((int64_t)kTileClasses * z.n_tiles * 4) : nullptr;
+  s.order = z.lists ? c.take<uint32_t>((int64_t)kTileLists * z.n_tiles * 4) : nullptr;
   s.rgrad = z.bwd ? c.take<RecGrad>(z.n_rec) : nullptr;
   s.part = z.part_px > 0 ? c.take<float4>(z.part_px) : nullptr;
   s.spans = z.n_spans > 0 ? c.take<uint32_t>(z.n_spans) : nullptr;
@@ -361,15 +361,22 @@ bool can_grow(const DevBuf& buf, size_t bytes, cudaStream_t st) {
 int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
                 unsigned long long* h_pinned, bool bwd, cudaStream_t st, RecSpace& rs,
                 KeySpace& ks, int64_t& cap, uint64_t*& sorted) {
+  // `worst`: every record touching every tile of its view.
+  const bool exact = worst > 0 && (size_t)worst * kBytesPerKey <= key_budget_bytes();
+  // The single-view pipelines describe their view on the host (va.one).
+  RowPlan rp = (p.va.table || p.radix) ? RowPlan{} : row_plan(&p.va.one, 1);
+  fit_segments(rp, p.n_tiles, exact ? worst : 0);
+
   RecSizes z(p.n_rec, p.n_tiles);
-  z.lists = true;
+  z.lists = p.heavy_first && rp.tiled();
   z.bwd = bwd;
   z.part_px = part_pixels(p);
-  z.n_spans = span_words(p.va.one, 1, p.rect_binning || p.radix);
+  z.n_spans = span_words(p.va.one, 1, p.rect_binning || !rp.tiled());
   // (under capture an arena stays as large as it was warmed up, without the optional parts)
   if (!can_grow(recbuf, rec_bytes(z), st)) {
     z.n_spans = 0;
     if (!can_grow(recbuf, rec_bytes(z), st)) {
+      z.lists = p.heavy_first = false;
       p.pieces = 1;
       z.part_px = 0;
     }
@@ -378,12 +385,6 @@ int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
   if (rc) return rc;
   carve_rec(recbuf.ptr, z, rs);
 
-  // `worst`: every record touching every tile of its view.
-  const bool exact = worst > 0 && (size_t)worst * kBytesPerKey <= key_budget_bytes();
-
-  // The single-view pipelines describe their view on the host (va.one).
-  RowPlan rp = (p.va.table || p.radix) ? RowPlan{} : row_plan(&p.va.one, 1);
-  fit_segments(rp, p.n_tiles, exact ? worst : 0);
   // The tile-major emission writes every tile's range; the emit + sort path writes only the
   // non-empty ones.
   FE_CUDA(zero_ctrl_rows(rs, rp.tiled() ? rp.max_gy + 1 : 0, st));
@@ -410,7 +411,6 @@ int run_binning(Pipeline& p, int64_t worst, DevBuf& recbuf, DevBuf& keybuf,
   carve_keys(keybuf.ptr, cap, [&](const KeySpace& s) { ks = s; });
   if (exact && !rp.tiled())
     launch_scan(rs.touched, rs.incl, p.n_rec, cap, rs.scan_tmp, rs.ctrl, st);
-  if (!rp.tiled() || !p.heavy_first) rs.order = nullptr;  // the blend takes tiles in index order
   if (rp.ok) {
     launch_tile_binning_emit(p.va, rp.n_views, rp.max_gy, rp.max_gx, rs.rects, foot_of(p, rs),
                              rs.spans, p.tile_w, p.tile_h, rs.row_tot, cap, rs.ctrl, rs.ranges,
@@ -1201,6 +1201,7 @@ struct fe_batch {
   RowPlan rows;  // tile-major binning plan (rows.ok) or the emit + sort path
   int pieces = 1;  // most pieces of a tile's keys in the blend
   int64_t n_spans = 0;
+  bool tiled() const { return rows.tiled() && !(desc.flags & FE_FLAG_RADIX_BINNING); }
 };
 
 namespace {
@@ -1256,10 +1257,10 @@ int plan_batch(fe_batch* b, const fe_scene* scenes, int32_t n_scenes, const fe_v
   for (const ViewDev& d : b->views_h) max_n = std::max(max_n, (int)d.n);
   const int px = default_px((int)b->desc.px_per_thread, b->tile_w, b->tile_h, tiles);
   b->pieces = blend_pieces(b->tile_w, b->tile_h, px, (int)(b->desc.flags >> 8) & 0xff, tiles, max_n);
-  b->n_spans = span_words(b->views_h[0], n_views,
-                          (b->desc.flags & (FE_FLAG_RECT_BINNING | FE_FLAG_RADIX_BINNING)) != 0);
   fit_segments(b->rows, tiles,
                b->exact ? 0 : std::min(worst, (int64_t)(key_budget_bytes() / kBytesPerKey)));
+  b->n_spans = span_words(b->views_h[0], n_views,
+                          !b->tiled() || (b->desc.flags & FE_FLAG_RECT_BINNING) != 0);
   return FE_OK;
 }
 
@@ -1281,11 +1282,10 @@ int commit_batch(fe_batch* b, cudaStream_t st) {
                           cudaMemcpyHostToDevice, st));
   FE_CUDA(cudaMemcpyAsync(b->trans_d, b->trans_h.data(), sizeof(float) * b->trans_h.size(),
                           cudaMemcpyHostToDevice, st));
-  // (ranges and row totals: sized for the tiles and for the tile-major binning's row slots)
-  const int64_t tile_slots =
-      std::max<int64_t>(b->n_tiles, (int64_t)b->rows.n_views * (b->rows.max_gy + 1));
-  RecSizes z(b->n_rec, tile_slots);
-  z.lists = z.tile_ent = z.bwd = true;
+  RecSizes z(b->n_rec, b->n_tiles);
+  z.row_slots = b->tiled() ? (int64_t)b->rows.n_views * (b->rows.max_gy + 1) : 1;
+  z.lists = z.tile_ent = b->tiled();  // (the lists also serve a backward)
+  z.bwd = true;
   z.part_px = b->pieces > 1 ? (int64_t)b->pieces * b->n_tiles * b->tile_w * b->tile_h : 0;
   z.n_spans = b->n_spans;
   rc = b->rec.reserve(rec_bytes(z), st);
@@ -1394,8 +1394,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
   p.va.table = b->views_d;
   p.va.count = b->n_views;
   // (written by the tile-major emission, read from the blend on)
-  p.va.tile_ent = (b->rows.tiled() && !(b->desc.flags & FE_FLAG_RADIX_BINNING)) ? b->rs.tile_ent
-                                                                             : nullptr;
+  p.va.tile_ent = b->rs.tile_ent;
   p.n_rec = b->n_rec;
   p.n_tiles = b->n_tiles;
   p.n_pix = b->n_pix;
@@ -1421,14 +1420,7 @@ static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* pre
 
 // The work-class tile lists of the last binning, when it was tile-major (else NULL).
 static const uint32_t* batch_order(const fe_batch* b, const Pipeline& p) {
-  return (p.heavy_first && !p.radix && b->rows.tiled()) ? b->rs.order : nullptr;
-}
-
-// The same for the backward, which always takes the heaviest tiles first where the binning lists
-// them: its warps are each on a tile for 30 us at the median of the 16-view workload and 100 us at
-// the heaviest, so index order leaves a long tail (16-view step 503 -> 477 us, lists included).
-static const uint32_t* bwd_order(const fe_batch* b, const Pipeline& p) {
-  return (!p.radix && b->rows.tiled()) ? b->rs.order : nullptr;
+  return p.heavy_first ? b->rs.order : nullptr;
 }
 
 // Binning of a batch. With exact key sizing the key count is read back after the scan (one
@@ -1733,8 +1725,11 @@ int fe_batch_bwd(fe_batch* b, const float* means, const float* prec, const float
     note_binning(b, means, prec, logw);
   }
   launch_bwd_zero(gmeans, gprec, glogw, b->n_gauss, b->rs.rgrad, p.n_rec, b->rs.ctrl, st);
-  launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, bwd_order(b, p), b->sorted, b->rs.ranges, b->rs.recs,
-                   depth, stats, p.n_pix, gdepth, galpha, p.beta2, p.beta3, b->rs.rgrad,
+  // The backward takes the heaviest tiles first wherever the binning lists them: its warps are each
+  // on a tile for 30 us at the median of the 16-view workload and 100 us at the heaviest, so index
+  // order leaves a long tail (16-view step 503 -> 477 us, lists included).
+  launch_blend_bwd(p.va, p.tile_w, p.tile_h, p.n_tiles, b->rs.order, b->sorted, b->rs.ranges,
+                   b->rs.recs, depth, stats, p.n_pix, gdepth, galpha, p.beta2, p.beta3, b->rs.rgrad,
                    b->rs.ctrl, st);
   launch_record_vjp(p.va, p.n_rec, means, prec, p.quat, p.trans, b->rs.recs, b->rs.rgrad, gmeans,
                     gprec, glogw, st);

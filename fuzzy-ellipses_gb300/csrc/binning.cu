@@ -603,7 +603,7 @@ __device__ __forceinline__ void row_tiles(const int (&cnt)[kTilesPer], unsigned 
     cex += (unsigned)cnt[q];
   }
   if (order) {
-    // Work classes: every tile of the row joins its class's list (order + c n_tiles), a shared
+    // Work classes: every tile of the row joins its class's list (list_entry), a shared
     // count per class and one global atomic per class and row giving the slots.
     __shared__ uint32_t cls_n[kTileClasses], cls_base[kTileClasses];
     if (tid < kTileClasses) cls_n[tid] = 0u;
@@ -624,7 +624,7 @@ __device__ __forceinline__ void row_tiles(const int (&cnt)[kTilesPer], unsigned 
     for (int q = 0; q < kTilesPer; ++q) {
       const int x = kTilesPer * tid + q;
       if (x >= x_lo && x < x_hi)
-        reinterpret_cast<uint4*>(order)[(int64_t)cl[q] * n_tiles + cls_base[cl[q]] + rank[q]] =
+        reinterpret_cast<uint4*>(order)[list_entry(cl[q], cls_base[cl[q]] + rank[q], n_tiles)] =
             make_uint4((uint32_t)x | (uint32_t)row << 16, rgq[q].x, rgq[q].y, blockIdx.y);
     }
   }
@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(kWarpRowWarps * 32) tile_emit_warp_kernel(
     base = __shfl_sync(full, base, leader);
     if (lane < gx) {
       const uint32_t rank = (uint32_t)__popc(same & lt_mask);
-      reinterpret_cast<uint4*>(order)[(int64_t)cl * n_tiles + base + rank] =
+      reinterpret_cast<uint4*>(order)[list_entry(cl, base + rank, n_tiles)] =
           make_uint4((uint32_t)lane | (uint32_t)row << 16, rg.x, rg.y, (uint32_t)v);
     }
   }

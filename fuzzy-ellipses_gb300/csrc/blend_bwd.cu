@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
     int vi, tx, ty;
     if (listed) {
       const int c = 31 - __clz(__ballot_sync(full, lane < kTileClasses && cls_first <= tile));
-      const uint4 e = reinterpret_cast<const uint4*>(order)[(int64_t)c * n_tiles + tile -
-                                                            __shfl_sync(full, cls_first, c)];
+      const uint4 e = reinterpret_cast<const uint4*>(
+          order)[list_entry(c, tile - __shfl_sync(full, cls_first, c), n_tiles)];
       tx = (int)(e.x & 0xffffu);
       ty = (int)(e.x >> 16);
       range = make_uint2(e.y, e.z);

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
   const float hw = 0.5f * (TW - 1), hh = 0.5f * (TH - 1);
   // Heaviest tiles first: with `order` (the tile-major binning's per-class tile lists over all
   // tiles [0, tile_end), uint4 entries: place in the view, first key, end key, view) work index w of class
-  // c maps to entry c tile_end + w - cls_base[c], so the tiles taken last, which set the
+  // c maps to entry w - cls_base[c] of its list, so the tiles taken last, which set the
   // kernel's tail, are the lightest, and a tile's range and view come with its id. The lists are
   // used only when they hold every tile exactly once (their counts sum to tile_end); else tiles
   // go in index order.
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
         const uint32_t b = tid < kTileClasses ? sm.cls_base[tid] : 0u;
         const int c = 31 - __clz(__ballot_sync(0xffffffffu, tid < kTileClasses && b <= w));
         if (tid == c && w < tile_end)
-          sm.entry = reinterpret_cast<const uint4*>(order)[(int64_t)c * tile_end + (w - b)];
+          sm.entry = reinterpret_cast<const uint4*>(order)[list_entry(c, w - b, tile_end)];
       }
       if (tid == 0) sm.tile = w;
     }

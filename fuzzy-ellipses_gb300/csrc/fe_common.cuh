@@ -165,6 +165,14 @@ __device__ __forceinline__ int tile_class(uint32_t keys) {
   return b > 12 ? 0 : 52 - 4 * b - (int)((keys >> (b - 2)) & 3u);
 }
 
+// Entry `slot` of class c's list among n_tiles tiles: the lists of classes 2 k and 2 k + 1 fill one
+// run of n_tiles entries from its two ends (a tile is in one list only, so they do not meet), which
+// keeps the lists at 256 bytes a tile.
+constexpr int kTileLists = (kTileClasses + 1) / 2;  // runs of n_tiles entries
+__device__ __forceinline__ int64_t list_entry(int c, uint32_t slot, int64_t n_tiles) {
+  return (c >> 1) * n_tiles + ((c & 1) ? n_tiles - 1 - slot : slot);
+}
+
 // Small device-side control block at the start of every arena.
 struct Control {
   unsigned long long num_keys;  // keys produced by the last run (clamped to capacity)

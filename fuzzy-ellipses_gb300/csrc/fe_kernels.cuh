@@ -81,7 +81,7 @@ uint64_t* launch_sort(uint64_t* a, uint64_t* b, int key_bits, const Control* ctr
 // empty tile, so the ranges need no zeroing). Same keys and ranges as emit + stable sort +
 // ranges, with the same `foot` (see launch_emit_keys). For many views the row counts are first
 // turned into row offsets and view bases in place (row_tot is consumed). With `order`
-// (kTileClasses lists of n_tiles uint4 entries, 16-byte aligned; ctrl's class counts zeroed)
+// (kTileLists runs of n_tiles uint4 entries, 16-byte aligned; ctrl's class counts zeroed)
 // every tile is also appended to the list of its work class (tile_class of its key count) as
 // (x | y << 16 in its view, first key, end key, view), which launch_blend_fwd then serves heaviest class first
 // without reading the tile's range or view again. With `tile_ent` (n_tiles entries) every tile's

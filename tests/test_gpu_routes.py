@@ -127,3 +127,27 @@ def test_legacy_routes(cuda_device, n, routes, h, w):
     assert float(images[0][1].max()) > 0.1
     for z, a in images[1:]:
         assert torch.equal(z, images[0][0]) and torch.equal(a, images[0][1])
+
+
+def _view(scene, h, w):
+    return dict(scene=scene, height=h, width=w, fx=float(w), fy=float(w), cx=w / 2, cy=h / 2,
+                quat=[1.0, 0.0, 0.0, 0.0], trans=[0.0, 0.0, -1.0])
+
+
+@pytest.mark.parametrize("views,tile,limit", [
+    # one view of 512 tile rows among 1000 of one tile: 1001 x 513 row totals of 8 bytes, and
+    # everything else by the 1512 tiles and 1001 records there are
+    ([_view(0, 8192, 16)] + [_view(0, 16, 16)] * 1000, (16, 16), 16 << 20),
+    # 262144 tiles: lists, entry, range, key and its twin at 256 + 16 + 8 + 16 bytes a tile, grown
+    # buffers a quarter larger
+    ([_view(0, 4096, 4096)], (8, 8), 296 * 262144 * 5 // 4 + (8 << 20)),
+    # the same through the sort: no lists, entries or spans
+    ([_view(0, 4096, 16384)], (8, 8), 32 * 2 * 524288 * 5 // 4 + (8 << 20))])
+def test_batch_scratch_follows_what_the_plan_uses(cuda_device, views, tile, limit):
+    fe.Batch([(0, 1)], [_view(0, 64, 64)]).close()  # (the library's kernels are loaded)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    b = fe.Batch([(0, 1)], views, tile=tile)
+    used = free - torch.cuda.mem_get_info()[0]
+    b.close()
+    assert used <= limit
