@@ -10,11 +10,13 @@
 // float32 with the clamp applied to 1 - a rather than to a: 1 - a is exact for a >= 0.5
 // (Sterbenz), so max(1 - a, 3e-8) equals 1 - min(a, 1 - 3e-8) evaluated exactly, whereas
 // 1 - 3e-8 itself rounds to 1.0 in float32 (which would leave saturated pixels at log(0)).
-// The per-render sums accumulate in float-float (two float32, about 48 bits) within a warp's run of
-// pixels, and in float64 across warps: GB300 computes and converts float64 at a sixty-fourth of
-// the float32 rate. With a float64 sum and product per pixel the kernel took 79 us on 16 renders of
-// 640x480 (59 MB, 0.75 TB/s); it takes 18 us (3.3 TB/s), bound by instruction issue: a logarithm
-// and a division per pixel, about 70 instructions in all.
+// The per-render sums accumulate in float64 and the derivatives are the float64 quotients, rounded.
+// GB300 computes and converts float64 at a sixty-fourth of the float32 rate: with a sum, a product
+// and four conversions per pixel a call on 16 renders of 640x480 (59 MB) took 82 us. One addition is
+// left of them; the conversion before it moves bits, and the quotient comes from float32 products
+// wherever those determine its rounding: 25.5 us. (Sums and quotients in two float32 took 23, with
+// 48 bits.) Bound by instruction issue: a logarithm and a division per pixel, about 80
+// instructions in all.
 #include <algorithm>
 
 #include "fe_kernels.cuh"
@@ -35,52 +37,64 @@ __device__ __forceinline__ int segment_of(const int64_t* __restrict__ seg_end, i
   return lo;
 }
 
-// A float32 pair hi + lo (lo within half an ulp of hi): about 48 bits.
-struct Pair {
+// Pixels of render s.
+__device__ __forceinline__ int64_t pixels_of(const int64_t* __restrict__ seg_end, int s) {
+  return seg_end[s] - (s > 0 ? seg_end[s - 1] : 0);
+}
+
+// 1 / n as two float32 (n below 2^48): hi rounded, lo the rest to within 2^-46 of hi.
+struct Inverse {
   float hi, lo;
+  int64_t n;
 };
-
-// x + y with the rounding of the float32 sum kept. A sum that is not finite has no error term.
-__device__ __forceinline__ Pair add_pairs(Pair x, Pair y) {
-  const float s = x.hi + y.hi, b = s - x.hi;
-  const float e = (x.hi - (s - b)) + (y.hi - b) + (x.lo + y.lo);
-  const float t = s + e;
-  return fabsf(t) < INFINITY ? Pair{t, e - (t - s)} : Pair{s, 0.f};
-}
-
-// x times y.hi + y.lo.
-__device__ __forceinline__ Pair scale(Pair x, Pair y) {
-  const float p = x.hi * y.hi;
-  const float e = fmaf(x.hi, y.hi, -p) + fmaf(x.hi, y.lo, x.lo * y.hi);
-  return fabsf(p) < INFINITY ? Pair{p, e} : Pair{p, 0.f};
-}
-
-// 1 / pixels of render s (fewer than 2^48).
-__device__ __forceinline__ Pair inv_count(const int64_t* __restrict__ seg_end, int s) {
-  const int64_t n = seg_end[s] - (s > 0 ? seg_end[s - 1] : 0);
+__device__ __forceinline__ Inverse inverse_of(int64_t n) {
   const float nh = (float)n, nl = (float)(n - (int64_t)nh);
   const float r = 1.f / nh;
-  return Pair{r, r * (fmaf(-r, nh, 1.f) - r * nl)};
+  return Inverse{r, r * (fmaf(-r, nh, 1.f) - r * nl), n};
 }
 
-// Loss of one pixel, and its derivative times `inv` to within one rounding. Targets of exactly 0
-// or 1 (a silhouette) need one logarithm and one division: the other term's factor is 0 and its
-// logarithm finite.
-__device__ __forceinline__ float bce_pixel(float a, float t, Pair inv, float* g) {
+// (The float64 instructions stay out of line: inlined, the compiler issues them for every pixel and
+// picks a result afterwards, 64 us for 26.)
+__device__ __noinline__ float scaled_f64(float d, int64_t n) {
+  return (float)((double)d * (1.0 / (double)n));
+}
+
+// d / n as float64 arithmetic rounds it to float32. The two float32 products are within 2^-45 of
+// the exact quotient; where that leaves its rounding open (one pixel in 2^19, and anything that is
+// not finite) the float64 product is formed.
+__device__ __forceinline__ float scaled(float d, const Inverse& inv) {
+  const float p = d * inv.hi;
+  const float e = fmaf(d, inv.lo, fmaf(d, inv.hi, -p));
+  const float m = fabsf(p) * 0x1p-44f;
+  const float g = p + (e + m);
+  if (g == p + (e - m)) return g;
+  return scaled_f64(d, inv.n);
+}
+
+// Loss of one pixel, and its derivative over the render's pixels. Targets of exactly 0 or 1 (a
+// silhouette) need one logarithm and one division: the other term's factor is 0 and its logarithm
+// finite.
+__device__ __forceinline__ float bce_pixel(float a, float t, const Inverse& inv, float* g) {
   const float om = 1.f - a;
   const float ac = fmaxf(a, kClipAlpha);
   const float omc = fmaxf(om, kClipAlpha);
   const bool inside = (a > kClipAlpha) && (om > kClipAlpha);
   if ((t == 0.f || t == 1.f) && fabsf(a) < INFINITY) {
     const float x = t == 1.f ? ac : omc;
-    const float d = inside ? (t == 1.f ? -1.f : 1.f) / x : 0.f;
-    const float p = d * inv.hi;
-    *g = p + fmaf(d, inv.lo, fmaf(d, inv.hi, -p));
+    *g = scaled(inside ? (t == 1.f ? -1.f : 1.f) / x : 0.f, inv);
     return -logf(x);
   }
-  const Pair p = scale(Pair{inside ? (-t / ac + (1.f - t) / omc) : 0.f, 0.f}, inv);
-  *g = p.hi + p.lo;
+  *g = scaled(inside ? (-t / ac + (1.f - t) / omc) : 0.f, inv);
   return -(t * logf(ac) + (1.f - t) * logf(omc));
+}
+
+__device__ __noinline__ double widen_slow(float x) { return (double)x; }
+// x as float64. By moving bits for what is neither zero, subnormal nor not finite: the conversion
+// instruction runs at the float64 rate.
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  if (mag - 0x00800000u >= 0x7f000000u) return mag == 0u ? 0.0 : widen_slow(x);
+  return __hiloint2double((int)((b & 0x80000000u) | ((mag >> 3) + 0x38000000u)), (int)(b << 29));
 }
 
 // A warp takes a contiguous run of pixels and goes through it render by render, four pixels per
@@ -96,13 +110,9 @@ __global__ void __launch_bounds__(kThreads) silhouette_bce_kernel(
   for (int64_t at = warp * run; at < end;) {
     const int s = segment_of(seg_end, n_seg, at);
     const int64_t stop = s + 1 < n_seg ? min(seg_end[s], end) : end;
-    const Pair inv = inv_count(seg_end, s);
-    Pair sum{0.f, 0.f};
-    auto add = [&](float x) {  // (the error terms' own sum needs no correction)
-      const float t = sum.hi + x, b = t - sum.hi;
-      sum.lo += (sum.hi - (t - b)) + (x - b);
-      sum.hi = t;
-    };
+    const Inverse inv = inverse_of(pixels_of(seg_end, s));
+    double sum = 0.0;
+    auto add = [&](float x) { sum += widen(x); };
 #pragma unroll 2
     for (int64_t u = (at >> 2) + lane; u < (stop + 3) >> 2; u += 32) {
       const int64_t i = 4 * u;
@@ -123,15 +133,9 @@ __global__ void __launch_bounds__(kThreads) silhouette_bce_kernel(
         }
       }
     }
-    if (!(fabsf(sum.hi) < INFINITY)) sum.lo = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      sum = add_pairs(sum, Pair{__shfl_xor_sync(0xffffffffu, sum.hi, o),
-                                __shfl_xor_sync(0xffffffffu, sum.lo, o)});
-    if (lane == 0) {
-      const Pair mean = scale(sum, inv);
-      atomicAdd(&loss[s], (double)mean.hi + (double)mean.lo);
-    }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) atomicAdd(&loss[s], sum * (1.0 / (double)inv.n));
     at = stop;
   }
 }

@@ -2,6 +2,8 @@
 in a mix of concurrent requests, admission respects the HBM budget; the autotuner picks a valid
 configuration."""
 
+from fractions import Fraction
+
 import numpy as np
 import pytest
 import torch
@@ -233,3 +235,42 @@ def test_silhouette_bce_ragged_renders(cuda_device, offset, soft):
         ref = terms[start:start + k].mean()
         assert abs(loss[s] - ref) <= 2.4e-7 + 2.4e-7 * ref
         start += k
+
+
+@pytest.mark.parametrize("n", [33, 100, 127, 333, 640])
+def test_silhouette_bce_sums_in_float64(cuda_device, n):
+    """A saturated pixel with target t costs (1 - t) L with L = -log(3e-8), so targets 1 - 2^k give
+    terms exact in float32 over any range of exponents. Their mean has the rounding of float64
+    arithmetic: 4 additions per lane, 5 across the warp, 1 / n, a product and at most 5 warps."""
+    def mean_loss(t):
+        t = torch.tensor(t, dtype=torch.float32, device=cuda_device)
+        ends = torch.tensor([t.numel()], device=cuda_device)
+        return float(fe.silhouette_bce(torch.ones_like(t), t, ends)[0])
+    big = Fraction(mean_loss([0.0]))
+    rng = np.random.default_rng(n)
+    for _ in range(8):
+        k = rng.integers(-24, 1, n)
+        k[rng.random(n) < 0.3] = rng.integers(24, 60)
+        t = [1.0 - 2.0 ** int(j) if j <= 0 else -(2.0 ** int(j)) for j in k]
+        exact = sum(Fraction(2) ** int(j) for j in k) * big / n
+        assert abs(Fraction(mean_loss(t)) - exact) <= 16 * exact / 2 ** 53
+
+
+@pytest.mark.parametrize("soft", [False, True])
+@pytest.mark.parametrize("n", [7, 1000, 76799, 307200])
+def test_silhouette_bce_derivatives_round_once(cuda_device, n, soft):
+    """dL/dalpha is the float32 derivative of the pixel's term over the pixel count as float64
+    arithmetic rounds it, bit for bit (saturated and clamped pixels included)."""
+    rng = np.random.default_rng(n)
+    a = rng.random(n).astype(np.float32)
+    a[::5], a[1::7], a[2::11] = 0.0, 1.0, 2e-8
+    t = rng.random(n).astype(np.float32) if soft else (rng.random(n) < 0.5).astype(np.float32)
+    one, clip = np.float32(1), np.float32(3e-8)
+    om = one - a
+    d = -t / np.maximum(a, clip) + (one - t) / np.maximum(om, clip)
+    d = np.where((a > clip) & (om > clip), d, np.float32(0))
+    want = (d.astype(np.float64) * (1.0 / n)).astype(np.float32)
+    ends = torch.tensor([n], device=cuda_device)
+    got = fe.silhouette_bce(torch.from_numpy(a).to(cuda_device), torch.from_numpy(t).to(cuda_device),
+                            ends)[1].cpu().numpy()
+    assert np.array_equal(got, want)
