@@ -130,3 +130,41 @@ def test_long_lists_match_their_pieces(cuda_device, n, n_rays, n_poses):
     seen = ref_a > DEPTH_MASK_ALPHA
     assert np.max(np.abs(a - ref_a)) <= TOL_ALPHA
     assert np.max(np.abs(d - ref_d)[seen] / ref_d[seen]) <= TOL_DEPTH_REL
+
+
+@pytest.mark.parametrize("n,n_poses,step", [(60, 2, 2), (700, 3, 1), (1000, 1, 9)])
+def test_culled_lists_equal_the_thread_per_ray_kernel(cuda_device, n, n_poses, step):
+    """With dense weights every ray tests every Gaussian by itself, with IEEE divisions; without
+    them warps cull for their rays and evaluate in pairs. Depth and alpha are the same bits: the
+    same operations in the same order."""
+    rng = np.random.default_rng(n)
+    scene = S.random_gaussians(n, 0.3, rng)
+    cams = [S.Camera(120, 160, 150.0, 150.0, 80.0, 60.0, *S.look_at(1.0 * d))
+            for d in S.random_unit_vectors(n_poses, rng)]
+    rays = np.concatenate([grid_rays(120, 160, k, step) for k in range(n_poses)]).astype(np.float32)
+    args = scene_to_dev(scene, cuda_device) + (torch.from_numpy(rays).to(cuda_device), 1.0 / 150.0,
+                                               torch.from_numpy(pose_list(cams)).to(cuda_device))
+    d0, a0 = fe.render_pixels(*args, weights=True)[:2]
+    d1, a1 = fe.render_pixels(*args)[:2]
+    assert torch.equal(d0, d1) and torch.equal(a0, a1)
+
+
+@pytest.mark.parametrize("thickness", [8e-20, 1e19])
+def test_discs_at_the_ends_of_the_float_range(cuda_device, thickness):
+    """Discs facing the camera whose precision along the view is the reciprocal of 8e-20 or 1e19:
+    the squared ray term is then within a factor of 4 of the largest or smallest normal float32,
+    and its reciprocal is not normal. Depths as with the division (which has 22 bits there)."""
+    n, rng = 60, np.random.default_rng(1)
+    means = np.concatenate([rng.uniform(-0.2, 0.2, (n, 2)), rng.uniform(0.8, 1.2, (n, 1))], 1)
+    prec = np.tile(np.diag([1.0, 1.0, 1.0 / thickness]), (n, 1, 1))
+    if thickness > 1:
+        prec[:, 0, 0] = prec[:, 1, 1] = 0.02 / thickness
+    arrays = [torch.from_numpy(x.astype(np.float32)).to(cuda_device)
+              for x in (means, prec, rng.normal(0, 0.5, n))]
+    rays = torch.from_numpy(grid_rays(100, 100, 0, 2).astype(np.float32)).to(cuda_device)
+    pose = torch.tensor([[1.0, 0, 0, 0, 0, 0, 0]], device=cuda_device)
+    d0, a0 = fe.render_pixels(*arrays, rays, 0.01, pose, weights=True)[:2]
+    d1, a1 = fe.render_pixels(*arrays, rays, 0.01, pose)[:2]
+    assert float(d0.max()) > 0.5 and bool(torch.isfinite(d0).all())
+    assert bool(((d1 - d0).abs() <= 2e-5 * d0.abs()).all())
+    assert bool(((a1 - a0).abs() <= 2e-5).all())
