@@ -33,8 +33,9 @@ struct FeatSmem {
   uint32_t gid[kFeatChunk];
 };
 
-// Weights (times W) of a record pair at the thread's pixels: 2^(l - m), 0 behind the camera.
-// The arithmetic of blend_group (blend_fwd.cu).
+// Weights (times W) of a record pair at the thread's pixels: 2^(l - m), with MASK 0 behind the camera
+// and at pixels that take no weights (m infinite), whatever the logits are. The arithmetic of
+// blend_group (blend_fwd.cu).
 template <int PX, bool MASK>
 __device__ __forceinline__ void pair_weights(const TilePair& p, const f2_t (&DU)[PX], f2_t DV,
                                              f2_t DVSQ, f2_t B3, f2_t NB2, const float (&m)[PX],
@@ -66,8 +67,8 @@ __device__ __forceinline__ void pair_weights(const TilePair& p, const f2_t (&DU)
     if (MASK) {
       float z0, z1;
       f2_unpack(z, z0, z1);
-      e0[k] = z0 > 0.f ? e0[k] : 0.f;
-      e1[k] = z1 > 0.f ? e1[k] : 0.f;
+      e0[k] = z0 > 0.f && m[k] < INFINITY ? e0[k] : 0.f;
+      e1[k] = z1 > 0.f && m[k] < INFINITY ? e1[k] : 0.f;
     }
   }
 }
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(TW * TH / PX) features_kernel(
   float m[PX], iw[PX];
   int64_t pix[PX];
   bool ok[PX];
+  bool weights = true;  // every pixel of the warp takes some
 #pragma unroll
   for (int k = 0; k < PX; ++k) {
     const float du = (cx * PX + k) - hw;
@@ -105,10 +107,13 @@ __global__ void __launch_bounds__(TW * TH / PX) features_kernel(
     ok[k] = v < V.H && u0 + k < V.W;
     pix[k] = V.pix_base + (int64_t)v * V.W + u0 + k;
     const float W = ok[k] ? stats[stride + pix[k]] : 0.f;
-    // A pixel without front Gaussians has W = 0 and m at the forward's sentinel: no weight.
+    // A pixel without front Gaussians has W = 0 and m at the forward's sentinel, one that an
+    // infinite logit reaches W = NaN: no weights.
     iw[k] = W > 0.f ? 1.f / W : 0.f;
     m[k] = W > 0.f ? stats[pix[k]] : INFINITY;
+    weights &= m[k] < INFINITY || !ok[k];
   }
+  weights = __all_sync(0xffffffffu, weights);
   for (int c0 = 0; c0 < nf; c0 += per_pass) {
     const int cn = min(per_pass, nf - c0);  // at most FC
     f2_t acc[PX][FC / 2];
@@ -145,7 +150,7 @@ __global__ void __launch_bounds__(TW * TH / PX) features_kernel(
       for (int p = 0; p < pairs; ++p) {
         const float2 front = sm.pair[p].f[18];
         float e0[PX], e1[PX];
-        if (front.x != 0.f && front.y != 0.f)
+        if (front.x != 0.f && front.y != 0.f && weights)
           pair_weights<PX, false>(sm.pair[p], DU, DV, DVSQ, B3, NB2, m, e0, e1);
         else
           pair_weights<PX, true>(sm.pair[p], DU, DV, DVSQ, B3, NB2, m, e0, e1);
