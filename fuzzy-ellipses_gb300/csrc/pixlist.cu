@@ -545,7 +545,7 @@ __device__ __forceinline__ void evaluate_pairs(const PixSmem& sm, int cnt, float
 #pragma unroll
         for (int q = 0; q < LR; ++q) {
           const float e = q ? e1 : e0;
-          if (e != 0.f) {  // (a weight of zero adds nothing, whatever the feature)
+          if (z[h][q] > 0.f) {  // (in front and within its bound)
 #pragma unroll
             for (int f = 0; f < (FEAT ? kMaxF : 1); ++f)
               if (f < nf) t.F[q][f] = fmaf(e, row[f], t.F[q][f]);

@@ -168,3 +168,27 @@ def test_discs_at_the_ends_of_the_float_range(cuda_device, thickness):
     assert float(d0.max()) > 0.5 and bool(torch.isfinite(d0).all())
     assert bool(((d1 - d0).abs() <= 2e-5 * d0.abs()).all())
     assert bool(((a1 - a0).abs() <= 2e-5).all())
+
+
+@pytest.mark.parametrize("step", [1, 2])
+def test_list_features_do_not_depend_on_the_kernel(cuda_device, step):
+    """Features of the culled kernel and of the thread-per-ray one (taken with dense weights) are the
+    same bits. A Gaussian whose weight underflows still multiplies its feature, so an infinite one
+    gives NaN along its rays in both."""
+    n, rng = 600, np.random.default_rng(2)
+    scene = S.random_gaussians(n, 0.2, rng)
+    means = scene.means.copy()
+    prec = scene.prec.copy()
+    means[-1], prec[-1] = [0.0, 0.0, 9.0], np.eye(3)  # 10 m away: e^-200 of the others' weight
+    m, p, w = (torch.from_numpy(x).to(cuda_device) for x in (means, prec, scene.logw))
+    feats = rng.normal(size=(n, 5)).astype(np.float32)
+    feats[-1, 2] = np.inf
+    pose = torch.tensor([[1.0, 0, 0, 0, 0, 0, -1.0]], device=cuda_device)
+    rays = torch.from_numpy(grid_rays(120, 120, 0, step).astype(np.float32)).to(cuda_device)
+    args = (m, p, w, rays, 1.0 / 120.0, pose)
+    feats = torch.from_numpy(feats).to(cuda_device)
+    f0 = fe.render_pixels(*args, weights=True, features=feats)[4]
+    f1 = fe.render_pixels(*args, features=feats)[4]
+    assert bool(torch.isnan(f0[:, 2]).any()) and not bool(torch.isnan(f0[:, :2]).any())
+    assert torch.equal(torch.isnan(f0), torch.isnan(f1))
+    assert torch.equal(torch.nan_to_num(f0), torch.nan_to_num(f1))
