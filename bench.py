@@ -476,7 +476,7 @@ def main():
     # ranges with them: its scan, sort and ranges stages are empty (event gaps only). The emit +
     # radix sort path moves 16 B per key per sort pass and reads the sorted keys once more for the
     # ranges (8 B per key, 8 B per tile written).
-    radix_path = batch.launches_per_forward > 3
+    radix_path = batch.plan["binning"] == "sort"
     n_tiles_b = batch_tiles(cams, *cfg["tile"])
     hbm = {
         "preprocess": (52 * scene.n + len(cams) * scene.n * (96 + 8 + 4)) / (stages["preprocess"] * 1e-3) / 1e9,
@@ -665,7 +665,7 @@ def main():
         "data": "synthetic",
         "config": {"workload": WORKLOAD, "step": "batched forward of all 16 cameras",
                    "tile": f"{cfg['tile'][0]}x{cfg['tile'][1]}", "px_per_thread": cfg["px"],
-                   "chunk_pairs": cfg["chunk"], "heavy_tiles_first": cfg["heavy_first"],
+                   "chunk_pairs": cfg["chunk"], "heavy_tiles_first": batch.plan["heavy_first"],
                    "autotuned": tuned is not None,
                    "binning": "tile-major (keys emitted in sorted order)" if args.binning == "tiles"
                    else "key emission + radix sort",
@@ -735,7 +735,7 @@ def main():
                                "candidates_ms": {f"{c['tile'][0]}x{c['tile'][1]}/px{c['px']}/ch{c['chunk']}{'/heavy' if c['heavy_first'] else ''}": round(c["ms"], 4)
                                                  for c in tuned["candidates"]}},
         "clocks": clocks,
-        "gpu_launches": batch.launches_per_forward * args.steps,
+        "gpu_launches": batch.plan["kernels"] * args.steps,
         "wall_s_timed_region": wall,
     }
     print(json.dumps(out), flush=True)
@@ -1038,7 +1038,7 @@ def config3_bench(fe, dev, steps, fma_ops, ex2_ops):
            "views": len(views), "ms_per_step": ms, "renders_per_s": len(views) / (ms * 1e-3),
            "evals_per_step": e_total, "mevals_per_s": e_total / (ms * 1e-3) / 1e6,
            "num_keys": st["num_keys"], "stages_ms": stages,
-           "gpu_launches_per_step": b.launches_per_forward,
+           "gpu_launches_per_step": b.plan["kernels"],
            "blend_roofline": {"bound": "fma+xu", "achieved": blend_evals_s / 1e9,
                               "peak": peak / 1e9, "unit": "Gevals/s",
                               "frac": blend_evals_s / peak,

@@ -1388,7 +1388,7 @@ static void note_binning(fe_batch* b, const float* means, const float* prec, con
   b->binned_for[2] = logw;
 }
 
-static Pipeline batch_pipeline(fe_batch* b, const float* means, const float* prec,
+static Pipeline batch_pipeline(const fe_batch* b, const float* means, const float* prec,
                                const float* logw) {
   Pipeline p{};
   p.va.table = b->views_d;
@@ -1796,6 +1796,17 @@ int fe_batch_launch_count(const fe_batch* b) {
   const int passes = (bits_for(b->n_tiles) + 7) / 8;
   const int scan = b->n_rec <= 65536 ? 1 : 3;
   return 1 + scan + 1 + 3 * passes + 1 + 1;
+}
+
+int fe_batch_get_plan(const fe_batch* b, fe_batch_plan* plan) {
+  if (!b || !plan) return fail(FE_ERR_INVALID_ARGUMENT, "NULL argument");
+  plan->binning = !b->tiled()  ? FE_BINNING_SORT
+                  : b->rows.ok ? FE_BINNING_ROWS
+                               : FE_BINNING_SEGMENTS;
+  plan->pieces = b->pieces;
+  plan->heavy_first = batch_order(b, batch_pipeline(b, nullptr, nullptr, nullptr)) != nullptr;
+  plan->kernels = fe_batch_launch_count(b) + (b->pieces > 1);
+  return FE_OK;
 }
 
 int fe_bench_peak(int kind, int iters, double* ops_per_second, fe_stream_t stream_) {

@@ -74,6 +74,12 @@ class LegacyDesc(ctypes.Structure):
                 ("P", ctypes.c_int32), ("tan_fovx", ctypes.c_float), ("tan_fovy", ctypes.c_float)]
 
 
+class BatchPlan(ctypes.Structure):
+    """Mirror of ``fe_batch_plan``."""
+    _fields_ = [("binning", ctypes.c_int32), ("pieces", ctypes.c_int32),
+                ("heavy_first", ctypes.c_int32), ("kernels", ctypes.c_int32)]
+
+
 class View(ctypes.Structure):
     """Mirror of ``fe_view``."""
     _fields_ = [("scene", ctypes.c_int32), ("height", ctypes.c_int32), ("width", ctypes.c_int32),
@@ -184,6 +190,7 @@ PROTOTYPES = {
     "fe_check_device_status": (ctypes.c_int, [P, ctypes.POINTER(ctypes.c_uint32)]),
     "fe_batch_fwd_timed": (ctypes.c_int, [P] + [P] * 6 + [ctypes.POINTER(ctypes.c_float), P]),
     "fe_batch_launch_count": (ctypes.c_int, [P]),
+    "fe_batch_get_plan": (ctypes.c_int, [P, ctypes.POINTER(BatchPlan)]),
     "fe_bench_peak": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double), P]),
     "fe_selftest_bounded_wait": (ctypes.c_int, [ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint32),
                                                 ctypes.POINTER(ctypes.c_uint64), P]),

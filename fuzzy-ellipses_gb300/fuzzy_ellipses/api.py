@@ -659,7 +659,18 @@ class Batch:
 
     @property
     def launches_per_forward(self):
+        """Kernels one ``forward`` launches, its blend counted as one (see ``plan``)."""
         return int(N.load().fe_batch_launch_count(self._h))
+
+    @property
+    def plan(self):
+        """How a ``forward`` runs: ``binning`` ("rows", "segments" or "sort"), the most ``pieces``
+        the blend cuts a tile's keys into (1: whole tiles), whether it goes ``heavy_first``, and the
+        ``kernels`` it launches (a blend in pieces is two)."""
+        p = N.BatchPlan()
+        N.check(N.load().fe_batch_get_plan(self._h, ctypes.byref(p)))
+        return {"binning": ("sort", "rows", "segments")[p.binning], "pieces": p.pieces,
+                "heavy_first": bool(p.heavy_first), "kernels": p.kernels}
 
     def status(self):
         lib = N.load()

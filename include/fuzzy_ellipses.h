@@ -318,8 +318,20 @@ int fe_batch_status(fe_batch *b, fe_stream_t stream, int64_t *num_keys, int64_t 
 int fe_batch_fwd_timed(fe_batch *b, const float *d_means, const float *d_prec, const float *d_logw,
                        float *d_depth, float *d_alpha, float *d_stats, float *stage_ms,
                        fe_stream_t stream);
-/* Number of kernels one fe_batch_fwd launches. */
+/* Number of kernels one fe_batch_fwd launches, its blend counted as one (see fe_batch_plan). */
 int fe_batch_launch_count(const fe_batch *b);
+
+/* How the forwards of a batch run. */
+#define FE_BINNING_SORT 0     /* key emission and radix sort */
+#define FE_BINNING_ROWS 1     /* tile-major, a block or warp per tile row */
+#define FE_BINNING_SEGMENTS 2 /* tile-major, the records in segments */
+typedef struct fe_batch_plan {
+  int32_t binning;     /* FE_BINNING_* */
+  int32_t pieces;      /* most pieces a tile's keys are cut into by the blend (1: whole tiles) */
+  int32_t heavy_first; /* the blend takes the tiles with the most keys first */
+  int32_t kernels;     /* launched by one fe_batch_fwd (a blend in pieces is two) */
+} fe_batch_plan;
+int fe_batch_get_plan(const fe_batch *b, fe_batch_plan *plan);
 /* ---------------------------------------------------------------------------------------------
  * Continuous-batching render server. No reference counterpart: the reference renders one camera
  * per call (rasterize_main.cu:29-114) and leaves batching and serving to the caller.

@@ -151,3 +151,27 @@ def test_batch_scratch_follows_what_the_plan_uses(cuda_device, views, tile, limi
     used = free - torch.cuda.mem_get_info()[0]
     b.close()
     assert used <= limit
+
+
+@pytest.mark.parametrize("n,views,h,w,kw,binning,pieces", [
+    (300, 4, 480, 640, {}, "rows", False), (300, 40, 100, 100, {}, "rows", False),
+    (1300, 1, 64, 64, {}, "rows", True), (6000, 4, 480, 640, {}, "segments", False),
+    (3000, 1, 64, 64, {}, "segments", True), (300, 4, 480, 640, {"binning": "radix"}, "sort", False),
+    (1300, 1, 64, 64, {"binning": "radix"}, "sort", True),
+    (3000, 1, 64, 64, {"heavy_first": True}, "segments", True)])
+def test_plan_names_the_kernels(cuda_device, n, views, h, w, kw, binning, pieces):
+    """Batch.plan says which binning a forward takes, whether its blend is cut into pieces and how
+    many kernels it launches."""
+    rng = np.random.default_rng(n)
+    sc = S.random_gaussians(n, 0.3, rng)
+    arrays = [to_dev(x, cuda_device) for x in (sc.means, sc.prec, sc.logw)]
+    b = fe.Batch([(0, n)], [_view(0, h, w)] * views, **kw)
+    plan = b.plan
+    assert plan["binning"] == binning and (plan["pieces"] > 1) == pieces
+    out = [torch.empty(b.n_pixels, device=cuda_device) for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def call(stream):
+        N.check(N.load().fe_batch_fwd(b._h, *[x.data_ptr() for x in arrays + out], None, stream))
+    assert kernels_of(call) == plan["kernels"] == b.launches_per_forward + pieces
+    b.close()
