@@ -445,7 +445,8 @@ int default_px(int px, int tw, int th, int64_t n_tiles) {
 // only lose (40 Gaussians at 200x200 40.5 -> 42 us, 1000 at 640x480 45 -> 46.5).
 bool chain_pays(int64_t n_rec, int64_t n_tiles) { return n_rec > kSegMinN || n_tiles >= kPx2Tiles; }
 
-// Whether the blend takes the heaviest tiles first without being asked to: when a CTA gets a second
+// Whether the blend takes the heaviest tiles first. A blend in pieces does not (its tiles are few and
+// their pieces of a size). Elsewhere when asked to, and by itself when a CTA gets a second
 // tile at least half the time, so that their order matters, and the launch has enough keys for the lists to pay (they cost
 // 1 to 2 us; at least a Gaussian per five tiles of 256 pixels). Per forward, index order / heaviest
 // first: one view, 1000 Gaussians at 640x480 42.7 / 41.7 us, close up 88 / 78; 4000 at 800x600 117 /
@@ -453,8 +454,10 @@ bool chain_pays(int64_t n_rec, int64_t n_tiles) { return n_rec > kSegMinN || n_t
 // of 200x200 233 / 173, 16 of 640x480 188 / 181, 60 uneven scenes 243 / 215, 20 views of 200
 // Gaussians at 128x128 97 / 91 per step. Below the line: 16 views of 200 Gaussians at 640x480
 // 80.0 / 80.5, the same in 8x8 tiles 142 / 148, one of 250 at 900x720 38.0 / 39.7.
-bool heavy_tiles_pay(int tw, int th, int px, int pieces, int64_t n_tiles, int64_t n_rec) {
+bool heavy_tiles_first(uint32_t flags, int tw, int th, int px, int pieces, int64_t n_tiles,
+                       int64_t n_rec) {
   if (pieces > 1) return false;
+  if (flags & FE_FLAG_HEAVY_TILES_FIRST) return true;
   const int threads = tw * th / (px > 0 ? px : tw * th == 64 ? 2 : 4);
   const int64_t ctas = 152 * (threads == 32 ? 24 : 640 / threads);
   return 2 * n_tiles >= 3 * ctas && 256 * n_tiles <= 5 * n_rec * tw * th;
@@ -494,8 +497,7 @@ Pipeline single_view_pipeline(const fe_render_desc* d, const float* means, const
   p.pieces = blend_pieces(tw, th, p.px, p.chunk, p.n_tiles, p.n_rec);
   p.radix = (d->flags & FE_FLAG_RADIX_BINNING) != 0;
   p.rect_binning = (d->flags & FE_FLAG_RECT_BINNING) != 0;
-  p.heavy_first = (d->flags & FE_FLAG_HEAVY_TILES_FIRST) != 0 ||
-                  heavy_tiles_pay(tw, th, p.px, p.pieces, p.n_tiles, p.n_rec);
+  p.heavy_first = heavy_tiles_first(d->flags, tw, th, p.px, p.pieces, p.n_tiles, p.n_rec);
   p.cull_mode = d->cull_mode;
   p.cull_param = d->cull_param;
   p.beta2 = d->beta2;
@@ -538,7 +540,10 @@ int render_features(const fe_render_desc* d, const float* means, const float* pr
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
   p.va.chain |= p.n_rec >= 256;  // (the feature pass makes it a longer call on the device)
-  if (!depth) p.pieces = 1;  // (nothing is blended forward)
+  if (!depth) {  // (nothing is blended)
+    p.pieces = 1;
+    p.heavy_first = false;
+  }
   RecSpace rs;
   KeySpace ks;
   int64_t cap = 0;
@@ -653,7 +658,8 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
   rc = arena_for(st, &a);
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
-  p.pieces = 1;  // (nothing is blended forward)
+  p.pieces = 1;  // (nothing is blended forward; the backward has the lists where they are asked for)
+  p.heavy_first |= (d->flags & FE_FLAG_HEAVY_TILES_FIRST) != 0;
   RecSpace rs;
   KeySpace ks;
   int64_t cap = 0;
@@ -700,6 +706,7 @@ int fe_render_binning(const fe_render_desc* d, const float* means, const float* 
   *h_num_keys = 0;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
   p.pieces = 1;  // (nothing is blended)
+  p.heavy_first = false;
   FE_CUDA(cudaMemsetAsync(ranges, 0, sizeof(uint2) * (size_t)p.n_tiles, st));
   if (p.n_rec == 0) return FE_OK;
   if (!means || !prec || !logw) return fail(FE_ERR_INVALID_ARGUMENT, "NULL Gaussian pointer");
@@ -1405,9 +1412,8 @@ static Pipeline batch_pipeline(const fe_batch* b, const float* means, const floa
   p.pieces = b->pieces;
   p.radix = (b->desc.flags & FE_FLAG_RADIX_BINNING) != 0;
   p.rect_binning = (b->desc.flags & FE_FLAG_RECT_BINNING) != 0;
-  p.heavy_first =
-      (b->desc.flags & FE_FLAG_HEAVY_TILES_FIRST) != 0 ||
-      heavy_tiles_pay(b->tile_w, b->tile_h, p.px, p.pieces, p.n_tiles, p.n_rec);
+  p.heavy_first = heavy_tiles_first(b->desc.flags, b->tile_w, b->tile_h, p.px, p.pieces, p.n_tiles,
+                                    p.n_rec);
   p.tile_lists = p.heavy_first || b->keep_binning;
   p.cull_mode = b->desc.cull_mode;
   p.cull_param = b->desc.cull_param;

@@ -507,8 +507,8 @@ class Batch:
     scratch from the device-side count instead (one 8-byte readback per run).
     ``tile``, ``px`` (pixels per thread) and ``chunk`` (record pairs per shared-memory stage)
     select the blend configuration; ``heavy_first=True`` makes the blend take the tiles with the
-    most keys first even where the plan would not by itself (tile-major binning only; see
-    FE_FLAG_HEAVY_TILES_FIRST; the images are the same).
+    most keys first even where the plan would not by itself (tile-major binning and whole tiles only;
+    see FE_FLAG_HEAVY_TILES_FIRST; the images are the same).
     ``keep_binning=True`` lets ``backward`` reuse the binning of the preceding ``forward`` on the
     same Gaussian tensors (their contents must not change in between) instead of recomputing it.
     ``footprint="rect"`` bins every tile of each footprint's bounding rectangle

@@ -77,7 +77,8 @@ typedef enum fe_cull_mode {
  * steps of a quarter octave where they are many) and the blend takes the heaviest tiles first,
  * which shortens the tail of the persistent schedule (one 1280x720 view of 24000 Gaussians 290 ->
  * 250 us). The renderer does this by itself where a launch has enough tiles and Gaussians for it
- * to pay; the flag asks for it everywhere. Same images. */
+ * to pay; the flag asks for it on every launch that blends whole tiles (launches of few tiles cut
+ * them into pieces of their keys and need no order). Same images. */
 #define FE_FLAG_HEAVY_TILES_FIRST 0x10000u
 /* Bin every Gaussian to all tiles of its footprint's bounding rectangle (the reference
  * rasterizer's rule) instead of, in each tile row, only the tiles its footprint ellipse reaches.

@@ -175,3 +175,22 @@ def test_plan_names_the_kernels(cuda_device, n, views, h, w, kw, binning, pieces
         N.check(N.load().fe_batch_fwd(b._h, *[x.data_ptr() for x in arrays + out], None, stream))
     assert kernels_of(call) == plan["kernels"] == b.launches_per_forward + pieces
     b.close()
+
+
+@pytest.mark.parametrize("n,h,w,whole", [(1300, 64, 64, False), (3000, 64, 64, False),
+                                         (1300, 480, 640, True), (3000, 720, 1280, True)])
+def test_asking_for_the_heaviest_tiles_first(cuda_device, n, h, w, whole):
+    """Blends of whole tiles take the order that is asked for; a blend in pieces has none and lists no
+    tiles for it. The images do not depend on it."""
+    sc = S.random_gaussians(n, 0.3, np.random.default_rng(n))
+    arrays = [to_dev(x, cuda_device) for x in (sc.means, sc.prec, sc.logw)]
+    images = []
+    for heavy in (False, True):
+        b = fe.Batch([(0, n)], [_view(0, h, w)], heavy_first=heavy)
+        plan = b.plan
+        assert (plan["pieces"] == 1) == whole
+        if heavy or not whole:
+            assert plan["heavy_first"] == whole
+        images.append(b.forward(*arrays))
+        b.close()
+    assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
