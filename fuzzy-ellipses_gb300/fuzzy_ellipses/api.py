@@ -50,7 +50,7 @@ def _host_vec(x, n):
     if torch.is_tensor(x):
         if x.device.type != "cpu":
             return None
-        x = x.detach().to(torch.float32).numpy()
+        x = x.detach().to(torch.float32).resolve_neg().numpy()
     x = np.asarray(x, dtype=np.float32)
     return x.reshape(n) if x.size == n else None
 

@@ -154,3 +154,19 @@ def test_running_sums_give_the_column_moments(n):
     assert np.isclose(d0 * s0 + 2 * i1, (h * du).sum(), rtol=1e-12, atol=1e-12)
     assert np.isclose(d0 * d0 * s0 + 4 * d0 * i1 + 4 * i2, (h * du * du).sum(), rtol=1e-12,
                       atol=1e-10)
+
+
+def test_host_poses_are_read_like_uploaded_ones():
+    """A pose in host memory goes to the kernels by value: the values an upload would give, for CPU
+    tensors of any type, order and shape, lazily negated ones included; None for another size."""
+    import torch
+
+    from fuzzy_ellipses.api import _host_vec
+    base = torch.tensor([[0.5, -1.0], [2.0, 0.25]])
+    for x in (base, base.double(), base.half(), base.T, base.clone().requires_grad_(),
+              torch.complex(torch.zeros(2, 2), -base).conj().imag, base.tolist(), base.numpy()):
+        want = torch.as_tensor(x).detach().to(torch.float32).contiguous().reshape(4)
+        got = _host_vec(x, 4)
+        assert got.dtype == np.float32 and got.shape == (4,)
+        assert np.array_equal(got, want.resolve_neg().numpy())
+    assert _host_vec(base, 3) is None and _host_vec([1.0, 2.0], 4) is None
