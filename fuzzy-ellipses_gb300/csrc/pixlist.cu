@@ -619,7 +619,8 @@ __global__ void __launch_bounds__(32 * kPixWarps) pixlist_kernel(
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         const int i = c + 32 * h + lane;
-        b[h] = i < n ? pb[i] : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+        // (NaN reaches no box; an empty bound would reach one that rays with c = 0 make infinite)
+        b[h] = i < n ? pb[i] : make_float4(kNone, kNone, kNone, kNone);
       }
 #pragma unroll
       for (int h = 0; h < 4; ++h) {

@@ -192,3 +192,28 @@ def test_list_features_do_not_depend_on_the_kernel(cuda_device, step):
     assert bool(torch.isnan(f0[:, 2]).any()) and not bool(torch.isnan(f0[:, :2]).any())
     assert torch.equal(torch.isnan(f0), torch.isnan(f1))
     assert torch.equal(torch.nan_to_num(f0), torch.nan_to_num(f1))
+
+
+@pytest.mark.parametrize("n,n_rays,nf", [(41, 3000, 3), (129, 3000, 0), (600, 3000, 7),
+                                         (600, 12000, 7), (1153, 200000, 0)])
+def test_rays_in_the_camera_plane_leave_the_others_alone(cuda_device, n, n_rays, nf):
+    """Rays with c = 0 have infinite pixel offsets, so the box around a warp's rays can be the whole
+    plane. The warp still takes the pose's own Gaussians only (their number is no multiple of the 128
+    it looks at together, and the next pose's follow): every ray has the bits of the kernel that tests
+    each Gaussian for each ray."""
+    rng = np.random.default_rng(n)
+    scene = S.random_gaussians(n, 0.3, rng)
+    cams = [S.Camera(100, 100, 100.0, 100.0, 50.0, 50.0, *S.look_at(0.6 * d))
+            for d in S.random_unit_vectors(4, rng)]
+    rays = np.concatenate([rng.uniform(-50, 50, (n_rays, 2)), np.ones((n_rays, 1)),
+                           rng.integers(0, 4, (n_rays, 1))], 1).astype(np.float32)
+    rays[::3, 2] = 0.0
+    m, p, w = scene_to_dev(scene, cuda_device)
+    rays = torch.from_numpy(rays).to(cuda_device)
+    feats = torch.from_numpy(rng.normal(size=(n, nf)).astype(np.float32)).to(cuda_device) if nf else None
+    args = (m, p, w, rays, 0.01, torch.from_numpy(pose_list(cams)).to(cuda_device))
+    want = fe.render_pixels(*args, weights=True, features=feats)
+    got = fe.render_pixels(*args, features=feats)
+    for i in (0, 1, 4)[:3 if nf else 2]:
+        assert torch.equal(torch.isnan(want[i]), torch.isnan(got[i]))
+        assert torch.equal(torch.nan_to_num(want[i]), torch.nan_to_num(got[i]))
