@@ -72,13 +72,15 @@ constexpr int kInterleaved = sizeof(float4) + sizeof(GaussRec);
 using SplitTable = PixTable<sizeof(float4), sizeof(GaussRec)>;
 using InterleavedTable = PixTable<kInterleaved, kInterleaved>;
 
-// Scales a record's ray terms by the power of two that takes |a0| to about one. z = psv / vsv and
-// the density's |y|^2 / vsv do not change, and vsv = |a|^2 stays clear of the ends of the float32
-// range, where the reciprocal of evaluate_pairs is not the division's.
+// Scales the ray terms of a record whose |a0| is below 2^-50 or above 2^50 by the power of two that
+// takes it to about one. z = psv / vsv and the density's |y|^2 / vsv do not change, and vsv = |a|^2
+// stays clear of the ends of the float32 range, where the reciprocal of evaluate_pairs is not the
+// division's. (Terms whose square or its reciprocal has no float32 are left: they give NaN, as the
+// division does.)
 __device__ __forceinline__ void normalise_record(GaussRec& g) {
   const float top = fmaxf(fmaxf(fabsf(g.a0[0]), fabsf(g.a0[1])), fabsf(g.a0[2]));
-  const int e = min(max((int)(__float_as_uint(top) >> 23), 1), 253);
-  const float s = __uint_as_float((uint32_t)(254 - e) << 23);
+  if (!(top >= 0x1p-64f && top < 0x1p64f) || (top >= 0x1p-50f && top <= 0x1p50f)) return;
+  const float s = __uint_as_float((254u - (__float_as_uint(top) >> 23)) << 23);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     g.a0[c] *= s; g.a1[c] *= s; g.a2[c] *= s; g.b[c] *= s;
