@@ -270,10 +270,10 @@ constexpr int kRowPlanBlocks = 152;  // row blocks that fill a GB300 (its SM cou
 // Above kSegMinN Gaussians (of the largest view) the records are taken in segments, a block per
 // tile row and segment (launch_seg_binning): per call, one view of 640x480, segments against a
 // block per row, 1100 Gaussians 60 / 53 us, 2000 73 / 68, 2600 85 / 86, 4000 102 / 119; against
-// emit + sort 8000 157 / 188, 24000 at 1280x720 323 / 357, 50000 167 / 188. Its two passes test every
-// record against every row, where emit + sort works per key: at 1280x720 the two meet near 150000
-// Gaussians, hence the limit on rows x records. Up to 32 views (beyond, each block's sum over the
-// rows before it would be quadratic).
+// emit + sort 8000 157 / 188, 24000 at 1280x720 323 / 357, 50000 167 / 188. Its two passes test
+// every record against every row, where emit + sort works per key: at 1280x720 the two meet near
+// 150000 Gaussians, hence the limit on rows x records. Up to 32 views (beyond, each block's sum
+// over the rows before it would be quadratic).
 constexpr int64_t kSegTests = INT64_C(1) << 23;
 constexpr int kSegMinN = 2500;
 
@@ -445,15 +445,16 @@ int default_px(int px, int tw, int th, int64_t n_tiles) {
 // only lose (40 Gaussians at 200x200 40.5 -> 42 us, 1000 at 640x480 45 -> 46.5).
 bool chain_pays(int64_t n_rec, int64_t n_tiles) { return n_rec > kSegMinN || n_tiles >= kPx2Tiles; }
 
-// Whether the blend takes the heaviest tiles first. A blend in pieces does not (its tiles are few and
-// their pieces of a size). Elsewhere when asked to, and by itself when a CTA gets a second
-// tile at least half the time, so that their order matters, and the launch has enough keys for the lists to pay (they cost
-// 1 to 2 us; at least a Gaussian per five tiles of 256 pixels). Per forward, index order / heaviest
-// first: one view, 1000 Gaussians at 640x480 42.7 / 41.7 us, close up 88 / 78; 4000 at 800x600 117 /
-// 106, close up 354 / 269; 1000 at 1280x720 63.4 / 62.0 (169 / 141), 24000 290 / 250; 32 close views
-// of 200x200 233 / 173, 16 of 640x480 188 / 181, 60 uneven scenes 243 / 215, 20 views of 200
-// Gaussians at 128x128 97 / 91 per step. Below the line: 16 views of 200 Gaussians at 640x480
-// 80.0 / 80.5, the same in 8x8 tiles 142 / 148, one of 250 at 900x720 38.0 / 39.7.
+// Whether the blend takes the heaviest tiles first. A blend in pieces does not (its tiles are few
+// and their pieces of a size). Elsewhere when asked to, and by itself when a CTA gets a second tile
+// at least half the time, so that their order matters, and the launch has enough keys for the lists
+// to pay (they cost 1 to 2 us; at least a Gaussian per five tiles of 256 pixels). Per forward,
+// index order / heaviest first: one view, 1000 Gaussians at 640x480 42.7 / 41.7 us, close up 88 /
+// 78; 4000 at 800x600 117 / 106, close up 354 / 269; 1000 at 1280x720 63.4 / 62.0 (169 / 141),
+// 24000 290 / 250; 32 close views of 200x200 233 / 173, 16 of 640x480 188 / 181, 60 uneven scenes
+// 243 / 215, 20 views of 200 Gaussians at 128x128 97 / 91 per step. Below the line: 16 views of 200
+// Gaussians at 640x480 80.0 / 80.5, the same in 8x8 tiles 142 / 148, one of 250 at 900x720 38.0 /
+// 39.7.
 bool heavy_tiles_first(uint32_t flags, int tw, int th, int px, int pieces, int64_t n_tiles,
                        int64_t n_rec) {
   if (pieces > 1) return false;
@@ -552,8 +553,9 @@ int render_features(const fe_render_desc* d, const float* means, const float* pr
                    sorted);
   if (rc) return rc;
   if (depth)
-    launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces, rs.part,
-                     sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+    launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces,
+                     rs.part, sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats,
+                     npix, rs.ctrl, st);
   launch_features(p.va, p.tile_w, p.tile_h, p.n_tiles, sorted, rs.ranges, rs.recs, stats, npix,
                   p.beta2, p.beta3, features, n_features, out, st);
   FE_CUDA(cudaGetLastError());
@@ -635,7 +637,8 @@ int fe_render_fwd(const fe_render_desc* d, const float* means, const float* prec
                    sorted);
   if (rc) return rc;
   launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces, rs.part,
-                   sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+                   sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix,
+                   rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }
@@ -658,7 +661,8 @@ int fe_render_bwd(const fe_render_desc* d, const float* means, const float* prec
   rc = arena_for(st, &a);
   if (rc) return rc;
   Pipeline p = single_view_pipeline(d, means, prec, logw, quat, trans);
-  p.pieces = 1;  // (nothing is blended forward; the backward has the lists where they are asked for)
+  // (nothing is blended forward; the backward has the lists where they are asked for)
+  p.pieces = 1;
   p.heavy_first |= (d->flags & FE_FLAG_HEAVY_TILES_FIRST) != 0;
   RecSpace rs;
   KeySpace ks;
@@ -1068,8 +1072,9 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
   carve_keys(a->keys.ptr, cap, [&](const KeySpace& s_) { ks = s_; });
   uint64_t* sorted = ks.keys_a;
   if (rp.ok) {
-    launch_tile_binning_emit(va, 1, rp.max_gy, rp.max_gx, rs.rects, nullptr, nullptr, 8, 8, rs.row_tot,
-                             cap,                              rs.ctrl, rs.ranges, nullptr, ks.keys_a, nullptr, T, st);
+    launch_tile_binning_emit(va, 1, rp.max_gy, rp.max_gx, rs.rects, nullptr, nullptr, 8, 8,
+                             rs.row_tot, cap, rs.ctrl, rs.ranges, nullptr, ks.keys_a, nullptr, T,
+                             st);
   } else if (rp.segs) {
     launch_seg_binning(va, 1, rp.max_gy, rp.segs, rs.rects, nullptr, nullptr, 8, 8, rs.row_tot,
                        reinterpret_cast<uint32_t*>(ks.keys_b), cap, rs.ctrl, rs.ranges, nullptr,
@@ -1084,8 +1089,8 @@ static int rasterize_legacy(const fe_legacy_desc* d, const float* means, const f
     launch_blend_fwd_clean(va, T, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z, out_alpha,
                            rs.ctrl, st);
   else
-    launch_blend_fwd(va, 8, 8, 0, 0, T, nullptr, 1, nullptr, sorted, rs.recs, rs.ranges, 21.4f, 2.66f, out_z,
-                     out_alpha, nullptr, 0, rs.ctrl, st);
+    launch_blend_fwd(va, 8, 8, 0, 0, T, nullptr, 1, nullptr, sorted, rs.recs, rs.ranges, 21.4f,
+                     2.66f, out_z, out_alpha, nullptr, 0, rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }
@@ -1263,7 +1268,8 @@ int plan_batch(fe_batch* b, const fe_scene* scenes, int32_t n_scenes, const fe_v
   int max_n = 0;
   for (const ViewDev& d : b->views_h) max_n = std::max(max_n, (int)d.n);
   const int px = default_px((int)b->desc.px_per_thread, b->tile_w, b->tile_h, tiles);
-  b->pieces = blend_pieces(b->tile_w, b->tile_h, px, (int)(b->desc.flags >> 8) & 0xff, tiles, max_n);
+  b->pieces = blend_pieces(b->tile_w, b->tile_h, px, (int)(b->desc.flags >> 8) & 0xff, tiles,
+                           max_n);
   fit_segments(b->rows, tiles,
                b->exact ? 0 : std::min(worst, (int64_t)(key_budget_bytes() / kBytesPerKey)));
   b->n_spans = span_words(b->views_h[0], n_views,
@@ -1471,9 +1477,9 @@ static int batch_binning(fe_batch* b, const Pipeline& p, cudaStream_t st, cudaEv
     if (ev) FE_CUDA(cudaEventRecord(ev[4], st));
   } else if (rp.segs) {
     launch_seg_binning(p.va, rp.n_views, rp.max_gy, rp.segs, rs.rects, foot_of(p, rs), rs.spans,
-                       p.tile_w, p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b), b->cap,
-                       rs.ctrl, rs.ranges, rs.tile_ent, ks.keys_a, p.tile_lists ? rs.order : nullptr,
-                       p.n_tiles, st);
+                       p.tile_w, p.tile_h, rs.row_tot, reinterpret_cast<uint32_t*>(ks.keys_b),
+                       b->cap, rs.ctrl, rs.ranges, rs.tile_ent, ks.keys_a,
+                       p.tile_lists ? rs.order : nullptr, p.n_tiles, st);
     b->sorted = ks.keys_a;
     if (ev) FE_CUDA(cudaEventRecord(ev[3], st));
     if (ev) FE_CUDA(cudaEventRecord(ev[4], st));
@@ -1586,8 +1592,9 @@ static int batch_forward(fe_batch* b, const float* means, const float* prec, con
   // (see kManyTiles)
   const int chunk = !heavy_order && p.chunk == 0 && p.tile_w * p.tile_h > 64 ? 32 : p.chunk;
   launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, chunk, p.n_tiles,
-                   heavy_order ? batch_order(b, p) : nullptr, p.pieces, b->rs.part, b->sorted, b->rs.recs,
-                   b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats, p.n_pix, b->rs.ctrl, st);
+                   heavy_order ? batch_order(b, p) : nullptr, p.pieces, b->rs.part, b->sorted,
+                   b->rs.recs, b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats, p.n_pix,
+                   b->rs.ctrl, st);
   FE_CUDA(cudaGetLastError());
   return FE_OK;
 }
@@ -1782,8 +1789,8 @@ int fe_batch_fwd_timed(fe_batch* b, const float* means, const float* prec, const
   }
   note_binning(b, means, prec, logw);
   launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, batch_order(b, p), p.pieces,
-                   b->rs.part, b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, depth, alpha, stats,
-                   p.n_pix, b->rs.ctrl, st);
+                   b->rs.part, b->sorted, b->rs.recs, b->rs.ranges, p.beta2, p.beta3, depth,
+                   alpha, stats, p.n_pix, b->rs.ctrl, st);
   FE_CUDA(cudaEventRecord(ev[6], st));
   FE_CUDA(cudaEventSynchronize(ev[6]));
   for (int i = 0; i < 6; ++i) FE_CUDA(cudaEventElapsedTime(&stage_ms[i], ev[i], ev[i + 1]));
@@ -1960,7 +1967,8 @@ int fe_render_fwd_noalloc(const fe_render_desc* d, const float* means, const flo
     launch_ranges(sorted, rs.ctrl, worst, rs.ranges, st);
   }
   launch_blend_fwd(p.va, p.tile_w, p.tile_h, p.px, p.chunk, p.n_tiles, rs.order, p.pieces, rs.part,
-                   sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix, rs.ctrl, st);
+                   sorted, rs.recs, rs.ranges, p.beta2, p.beta3, depth, alpha, stats, npix,
+                   rs.ctrl, st);
   if (device_error)
     FE_CUDA(cudaMemcpyAsync(device_error, &rs.ctrl->error, sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, st));

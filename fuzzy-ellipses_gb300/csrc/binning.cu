@@ -762,8 +762,8 @@ __device__ __forceinline__ void tile_emit_body(
       csum += (unsigned)run;
     }
   }
-  row_tiles(cnt, csum, x_lo, x_hi, row, tile0, row_base, K, lim, ctrl, ranges, tile_ent, order, n_tiles,
-            pos, wsu);
+  row_tiles(cnt, csum, x_lo, x_hi, row, tile0, row_base, K, lim, ctrl, ranges, tile_ent, order,
+            n_tiles, pos, wsu);
   for (int s0 = 0; s0 < n; s0 += kRowSeg) {
     // (with a single segment the list is still in shared memory)
     if (n > kRowSeg) total = filter_row(rv, n, s0, row, list, ws);
@@ -774,9 +774,9 @@ __device__ __forceinline__ void tile_emit_body(
 
 // ---- Tile-major binning of many Gaussians ------------------------------------------------------
 // A row block that filters tens of thousands of records alone is slow, so the records are taken in
-// segments of kRowSeg, a block per (row, segment): one pass counts each tile's keys per segment (and
-// the row's and the run's totals), one turns the counts into slots, one writes the keys. Same keys
-// and ranges as above; one view of 24000 Gaussians at 1280x720: 8 + 9 + 26 us against 73 us
+// segments of kRowSeg, a block per (row, segment): one pass counts each tile's keys per segment
+// (and the row's and the run's totals), one turns the counts into slots, one writes the keys. Same
+// keys and ranges as above; one view of 24000 Gaussians at 1280x720: 8 + 9 + 26 us against 73 us
 // for scan, emission, radix sort and ranges. (The writing pass at 32 registers for a single wave of
 // its 1080 blocks spills and takes 2 us longer.)
 // counts: per tile row of gx tiles, `segs` rows of gx counts (offset: the row's first tile x segs).
@@ -881,8 +881,8 @@ __global__ void __launch_bounds__(kRowThreads) seg_bases_kernel(
     cnt[q] = x < gx ? (int)pos[x] : 0;
     csum += (unsigned)cnt[q];
   }
-  row_tiles(cnt, csum, 0, gx, row, tile0, row_base, K, lim, ctrl, ranges, tile_ent, order, n_tiles, pos,
-            wsu);
+  row_tiles(cnt, csum, 0, gx, row, tile0, row_base, K, lim, ctrl, ranges, tile_ent, order,
+            n_tiles, pos, wsu);
 }
 
 // A block per (row, segment): the segment's records reaching the row, in id order, written behind
@@ -1158,9 +1158,9 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
     if (max_gx <= kWarpRowTiles) {
       // Narrow views: a warp per tile row instead of a block sized for 1024-tile rows.
       const dim3 grid((unsigned)((max_gy + kWarpRowWarps - 1) / kWarpRowWarps), (unsigned)n_views);
-      launch_chained(va.chain, tile_emit_warp_kernel, grid, kWarpRowWarps * 32, st, va, rects, foot, spans,
-                     tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges, tile_ent, keys,
-                     order, n_tiles);
+      launch_chained(va.chain, tile_emit_warp_kernel, grid, kWarpRowWarps * 32, st, va, rects,
+                     foot, spans, tile_w, tile_h, row_tot, max_gy + 1, capacity, ctrl, ranges,
+                     tile_ent, keys, order, n_tiles);
       return;
     }
   }
@@ -1175,21 +1175,22 @@ void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int m
   // against 26.5).
   if ((int64_t)grid.x * grid.y > 2 * 5 * 152)
     launch_chained(va.chain, tile_emit_kernel_waves, grid, kRowThreads, st, va, rects, foot, spans,
-                   tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges, tile_ent, keys, order, n_tiles,
-                   nseg);
+                   tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges, tile_ent, keys, order,
+                   n_tiles, nseg);
   else
-    launch_chained(va.chain, tile_emit_kernel, grid, kRowThreads, st, va, rects, foot, spans, tile_w,
-                   tile_h, row_tot, bases, capacity, ctrl, ranges, tile_ent, keys, order, n_tiles, nseg);
+    launch_chained(va.chain, tile_emit_kernel, grid, kRowThreads, st, va, rects, foot, spans,
+                   tile_w, tile_h, row_tot, bases, capacity, ctrl, ranges, tile_ent, keys, order,
+                   n_tiles, nseg);
 }
 
 int64_t seg_count_words(int64_t n_tiles, int segs) { return n_tiles * segs; }
 int row_segments(int n) { return (n + kRowSeg - 1) / kRowSeg; }
 
-void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, const TileRect* rects,
-                        const FootRows* foot, const uint32_t* spans, int tile_w, int tile_h,
-                        unsigned long long* row_tot, uint32_t* counts, int64_t capacity,
-                        Control* ctrl, uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order, int64_t n_tiles,
-                        cudaStream_t st) {
+void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs,
+                        const TileRect* rects, const FootRows* foot, const uint32_t* spans,
+                        int tile_w, int tile_h, unsigned long long* row_tot, uint32_t* counts,
+                        int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent,
+                        uint64_t* keys, uint32_t* order, int64_t n_tiles, cudaStream_t st) {
   if (n_views <= 0 || max_gy <= 0 || segs <= 0) return;
   const dim3 grid((unsigned)max_gy, (unsigned)n_views, (unsigned)segs);
   launch_chained(va.chain, seg_count_kernel, grid, kRowThreads, st, va, rects, foot, spans, tile_w,

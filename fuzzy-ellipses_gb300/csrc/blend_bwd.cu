@@ -77,9 +77,10 @@ template <int TW, int TH>
 __global__ void __launch_bounds__(32 * kBwdWarps) blend_bwd_kernel(
     ViewsArg va, uint32_t n_tiles, int seg_bits, const uint32_t* __restrict__ order,
     const uint64_t* __restrict__ keys, const uint2* __restrict__ ranges,
-    const GaussRec* __restrict__ recs, const float* __restrict__ depth, const float* __restrict__ stats, int64_t stride,
-    const float* __restrict__ gdepth, const float* __restrict__ galpha, float nb2, float beta3,
-    float beta2, RecGrad* __restrict__ rgrad, Control* ctrl) {
+    const GaussRec* __restrict__ recs, const float* __restrict__ depth,
+    const float* __restrict__ stats, int64_t stride, const float* __restrict__ gdepth,
+    const float* __restrict__ galpha, float nb2, float beta3, float beta2,
+    RecGrad* __restrict__ rgrad, Control* ctrl) {
   using Slice = BwdSlice<TW, TH>;
   __shared__ Slice slices[kBwdWarps];
   chain_wait();
@@ -505,21 +506,21 @@ void launch_bwd_tiles(const ViewsArg& va, int64_t n_tiles, const uint32_t* order
   const int64_t grid =
       std::max<int64_t>(1, std::min<int64_t>((items + kBwdWarps - 1) / kBwdWarps, resident));
   launch_chained(va.chain, kern, (unsigned)grid, 32 * kBwdWarps, st, va, (uint32_t)n_tiles, bits,
-                 order, keys, ranges, recs, depth, stats, stride, gdepth, galpha, -beta2 * kLog2e, beta3, beta2,
-                 rgrad, ctrl);
+                 order, keys, ranges, recs, depth, stats, stride, gdepth, galpha, -beta2 * kLog2e,
+                 beta3, beta2, rgrad, ctrl);
 }
 
 }  // namespace
 
 
 void launch_blend_bwd(const ViewsArg& va, int tile_w, int tile_h, int64_t n_tiles,
-                      const uint32_t* order, const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
-                      const float* depth, const float* stats, int64_t stats_stride,
-                      const float* grad_depth, const float* grad_alpha, float beta2, float beta3,
-                      RecGrad* rgrad, Control* ctrl, cudaStream_t st) {
+                      const uint32_t* order, const uint64_t* keys, const uint2* ranges,
+                      const GaussRec* recs, const float* depth, const float* stats,
+                      int64_t stats_stride, const float* grad_depth, const float* grad_alpha,
+                      float beta2, float beta3, RecGrad* rgrad, Control* ctrl, cudaStream_t st) {
   if (n_tiles <= 0) return;
 #define FE_BWD(TW_, TH_)                                                                       \
-  launch_bwd_tiles<TW_, TH_>(va, n_tiles, order, keys, ranges, recs, depth, stats, stats_stride,     \
+  launch_bwd_tiles<TW_, TH_>(va, n_tiles, order, keys, ranges, recs, depth, stats, stats_stride, \
                              grad_depth, grad_alpha, beta2, beta3, rgrad, ctrl, st)
   if (tile_w == 8 && tile_h == 8)
     FE_BWD(8, 8);
@@ -544,8 +545,8 @@ void launch_record_vjp(const ViewsArg& va, int64_t n_rec, const float* means, co
                        cudaStream_t st) {
   if (n_rec <= 0) return;
   const int64_t want = (n_rec + 127) / 128;
-  launch_chained(va.chain, record_vjp_kernel<float>, (unsigned)(want < 65535 ? want : 65535), 128, st, va,
-                 n_rec, means, prec, quat, trans, recs, rgrad, gmeans, gprec, glogw);
+  launch_chained(va.chain, record_vjp_kernel<float>, (unsigned)(want < 65535 ? want : 65535), 128,
+                 st, va, n_rec, means, prec, quat, trans, recs, rgrad, gmeans, gprec, glogw);
 }
 
 }  // namespace fe

@@ -66,8 +66,8 @@ struct BlendShape {
   // registers), which the 8 KB of a 16-pair chunk allow and the 16 KB of a 32-pair one (13 CTAs)
   // do not. 8x8 tiles, 13 / 24 CTAs per SM: 16 views of 1000 Gaussians at 640x480 287 / 247 us per
   // forward, of 200 147 / 119, 1089 uneven views 1068 / 812.
-  // MANY: 11 CTAs asked for (22 warps); 80 registers with 12 bytes spilled then let 12 run. Each is a
-  // little slower, the SM faster, so it is for launches whose last tiles matter little (see
+  // MANY: 11 CTAs asked for (22 warps); 80 registers with 12 bytes spilled then let 12 run. Each is
+  // a little slower, the SM faster, so it is for launches whose last tiles matter little (see
   // kManyTiles).
   static constexpr int MIN_CTAS = NT == 32 ? (CH <= 16 ? 24 : 13) : (MANY ? 704 : 640) / NT;
   static constexpr int CW = TW / PX;
@@ -245,11 +245,11 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
   constexpr int RPT = (RC + Sh::NT - 1) / Sh::NT;  // records each thread stages and builds
   const float hw = 0.5f * (TW - 1), hh = 0.5f * (TH - 1);
   // Heaviest tiles first: with `order` (the tile-major binning's per-class tile lists over all
-  // tiles [0, tile_end), uint4 entries: place in the view, first key, end key, view) work index w of class
-  // c maps to entry w - cls_base[c] of its list, so the tiles taken last, which set the
+  // tiles [0, tile_end), uint4 entries: place in the view, first key, end key, view) work index w
+  // of class c maps to entry w - cls_base[c] of its list, so the tiles taken last, which set the
   // kernel's tail, are the lightest, and a tile's range and view come with its id. The lists are
-  // used only when they hold every tile exactly once (their counts sum to tile_end); else tiles
-  // go in index order.
+  // used only when they hold every tile exactly once (their counts sum to tile_end); else tiles go
+  // in index order.
   chain_wait();
   if (tid == 0) {
     mbar_init(&sm.bar, 1);
@@ -320,7 +320,8 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
     bool whole = true;
     if (SPLIT) {
       int per;
-      const uint32_t pieces = (uint32_t)tile_pieces((int)(rg.y - rg.x), (int)(tile_end / n_tiles), per);
+      const uint32_t pieces = (uint32_t)tile_pieces((int)(rg.y - rg.x), (int)(tile_end / n_tiles),
+                                                    per);
       if (piece > 0 && piece >= pieces) {
         __syncthreads();  // sm.tile is rewritten next iteration
         continue;
@@ -514,8 +515,8 @@ __global__ void __launch_bounds__(BlendShape<TW, TH, PX, CH, MANY>::NT,
   }
 }
 
-// The pixels of the tiles that were blended in pieces: a thread per pixel merges the pieces' sums in
-// piece order. One block per tile; the tiles of a single piece are already written.
+// The pixels of the tiles that were blended in pieces: a thread per pixel merges the pieces' sums
+// in piece order. One block per tile; the tiles of a single piece are already written.
 template <int TW, int TH>
 __global__ void __launch_bounds__(TW * TH) blend_merge_kernel(
     ViewsArg va, uint32_t n_tiles, int most, const uint2* __restrict__ ranges,
@@ -529,7 +530,8 @@ __global__ void __launch_bounds__(TW * TH) blend_merge_kernel(
   if (pieces <= 1) return;
   const ViewDev& V = view_at(va, view_of_tile(va, tile));
   const int lt = (int)(tile - V.tile_base);
-  const int u = (lt % V.gx) * TW + (int)threadIdx.x % TW, v = (lt / V.gx) * TH + (int)threadIdx.x / TW;
+  const int u = (lt % V.gx) * TW + (int)threadIdx.x % TW;
+  const int v = (lt / V.gx) * TH + (int)threadIdx.x / TW;
   if (u >= V.W || v >= V.H) return;
   float m = kNoLogit, W = 0.f, Z = 0.f, A = 0.f;
 #pragma unroll 4
@@ -570,21 +572,22 @@ void launch_split(const ViewsArg& va, int64_t n_tiles, int pieces, const uint64_
                   const GaussRec* recs, const uint2* ranges, float nb2, float beta3, float* depth,
                   float* alpha, float* stats, int64_t stats_stride, float4* part, Control* ctrl,
                   cudaStream_t st) {
-  constexpr int PX = kSplitPx, CH = TW * TH / PX == 32 ? 16 : 32, NT = BlendShape<TW, TH, PX, CH, false>::NT;
+  constexpr int PX = kSplitPx, CH = TW * TH / PX == 32 ? 16 : 32;
+  constexpr int NT = BlendShape<TW, TH, PX, CH, false>::NT;
   constexpr auto kern = blend_fwd_kernel<TW, TH, PX, CH, false, true, false>;
   const int64_t items = n_tiles * pieces;
   const int64_t grid = std::min<int64_t>(items, resident_ctas<kern>(NT));
   launch_chained(va.chain, kern, (unsigned)grid, NT, st, va, 0u, (uint32_t)items,
-                 &ctrl->next_tile, nullptr, keys, recs, ranges, nb2, beta3, depth, alpha, stats, stats_stride,
-                 (uint32_t)n_tiles, part, ctrl);
+                 &ctrl->next_tile, nullptr, keys, recs, ranges, nb2, beta3, depth, alpha, stats,
+                 stats_stride, (uint32_t)n_tiles, part, ctrl);
   launch_chained(va.chain, blend_merge_kernel<TW, TH>, (unsigned)n_tiles, TW * TH, st, va,
                  (uint32_t)n_tiles, pieces, ranges, part, depth, alpha, stats, stats_stride);
 }
 
 // Tiles from which 24 warps per SM finish sooner than 20 faster ones: 7 per CTA. Forward, 20 / 24
 // warps: 1089 uneven views (122 K tiles) 649 / 633 us, 60 scenes (28 K) 214.3 / 212.5, 16 views of
-// 640x480 (19200) 179.2 / 178.7, of 200 Gaussians 77.5 / 76.0, 32 of 20 Gaussians 84.1 / 80.0; one of
-// 1280x720 (3600) 260 / 275. Launches that store straight into host memory wait for the link and
+// 640x480 (19200) 179.2 / 178.7, of 200 Gaussians 77.5 / 76.0, 32 of 20 Gaussians 84.1 / 80.0; one
+// of 1280x720 (3600) 260 / 275. Launches that store straight into host memory wait for the link and
 // lose 0.5%: they ask for the chunk size they would get.
 constexpr int64_t kManyTiles = 8 * 152 * 11;
 
@@ -650,13 +653,13 @@ int blend_pieces(int tile_w, int tile_h, int px, int chunk, int64_t n_tiles, int
   if ((px != 0 && px != kSplitPx) || (px == 0 && !(tile_w == 8 && tile_h == 8)) ||
       (chunk != 0 && chunk != 32) || n_tiles <= 0)
     return 1;
-  // A launch of few tiles leaves SMs idle and lasts as long as its heaviest tile (the keys of a tile
-  // are blended one after the other). Tiles are cut until the pieces could fill the GPU (CTAs as
-  // BlendShape sizes them) twice over, more often the more keys per tile the view can hold; a piece
-  // has at least 128 keys in the densest tile there can be (64 in fact: tile_pieces). Per call,
-  // whole / cut: 2600 Gaussians at 64x64 158 / 57 us, 4378 at 73x419 202 / 96, 1422 at 293x157 96 /
-  // 64, 931 at 347x170 67 / 52, 20000 at 300x400 260 / 168, 8273 at 621x573 172 / 153; with more
-  // pieces where they hold fewer keys, 1100 at 640x480 53 / 58, 1000 at 637x479 75 / 80.
+  // A launch of few tiles leaves SMs idle and lasts as long as its heaviest tile (the keys of a
+  // tile are blended one after the other). Tiles are cut until the pieces could fill the GPU (CTAs
+  // as BlendShape sizes them) twice over, more often the more keys per tile the view can hold; a
+  // piece has at least 128 keys in the densest tile there can be (64 in fact: tile_pieces). Per
+  // call, whole / cut: 2600 Gaussians at 64x64 158 / 57 us, 4378 at 73x419 202 / 96, 1422 at
+  // 293x157 96 / 64, 931 at 347x170 67 / 52, 20000 at 300x400 260 / 168, 8273 at 621x573 172 / 153;
+  // with more pieces where they hold fewer keys, 1100 at 640x480 53 / 58, 1000 at 637x479 75 / 80.
   const int64_t cta = 152 * std::min(16, 640 / (tile_w * tile_h / kSplitPx));
   const int64_t most = cta * (max_n < 2 * n_tiles || max_n <= 1024 ? 2 : max_n <= 4096 ? 4 : 8);
   int pieces = 1;

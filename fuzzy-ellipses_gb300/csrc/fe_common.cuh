@@ -235,8 +235,8 @@ __device__ __forceinline__ int find_view(const ViewsArg& va, int64_t key) {
 }
 
 // View of record i, for a warp whose lanes hold consecutive records (all lanes take part): the view
-// of lane 0's by a 32-way search, a load per step where a binary search would wait for 11 (a thousand
-// views); the other lanes' from the next 32 views' first records, held by the lanes.
+// of lane 0's by a 32-way search, a load per step where a binary search would wait for 11 (a
+// thousand views); the other lanes' from the next 32 views' first records, held by the lanes.
 __device__ __forceinline__ int warp_view_of_record(const ViewsArg& va, int64_t i) {
   if (va.table == nullptr) return 0;
   const unsigned full = 0xffffffffu;
@@ -272,12 +272,12 @@ __device__ __forceinline__ int view_of_tile(const ViewsArg& va, int64_t tile) {
 // ------------------------------------------------------------------------------------------
 
 // Chained launches: a kernel that the next one of a pass follows lets it launch early (chain_next),
-// and the next one waits for its completion and its writes (chain_wait) before it touches memory, so
-// that the launch and the start of its blocks are hidden behind the end of the one before. The last
-// kernel of the binning does not let the blend launch early: the blend's blocks would fill the SMs
-// as they come free, the heaviest tiles' blocks side by side on one SM (one 1280x720 view of 24000
-// Gaussians 258 -> 300 us). 20 views of 128x128 88.9 -> 80.0 us per step, features of 16 values
-// 70.7 -> 64.1, that large view 260.4 -> 252.4, 16 views of 640x480 174.2 -> 169.6.
+// and the next one waits for its completion and its writes (chain_wait) before it touches memory,
+// so that the launch and the start of its blocks are hidden behind the end of the one before. The
+// last kernel of the binning does not let the blend launch early: the blend's blocks would fill the
+// SMs as they come free, the heaviest tiles' blocks side by side on one SM (one 1280x720 view of
+// 24000 Gaussians 258 -> 300 us). 20 views of 128x128 88.9 -> 80.0 us per step, features of 16
+// values 70.7 -> 64.1, that large view 260.4 -> 252.4, 16 views of 640x480 174.2 -> 169.6.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

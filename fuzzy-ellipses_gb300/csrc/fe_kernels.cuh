@@ -33,9 +33,9 @@ inline void launch_chained(bool chain, void (*kern)(P...), dim3 grid, unsigned t
 // one 1280x720 view of 24000 Gaussians 297 -> 292 us, 16 views of 640x480 180 -> 177.5.
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
                        const float* logw, const float* quat, const float* trans, int cull_mode,
-                       float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects, FootRows* foot,
-                       uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
-                       Control* ctrl, cudaStream_t st);
+                       float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects,
+                       FootRows* foot, uint32_t* spans, uint32_t* touched,
+                       unsigned long long* row_tot, int max_gy, Control* ctrl, cudaStream_t st);
 // The legacy interface's view and projection matrices: device arrays, or NULL and by value.
 struct LegacyMatrices {
   const float *d_view, *d_proj;
@@ -43,8 +43,9 @@ struct LegacyMatrices {
 };
 void launch_preprocess_reference(int P, float n_std, const float* means, const float* scales,
                                  const float* rots, const LegacyMatrices& mats, int W, int H,
-                                 float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
-                                 TileRect* rects, uint32_t* touched, cudaStream_t st);
+                                 float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii,
+                                 float* means2d, TileRect* rects, uint32_t* touched,
+                                 cudaStream_t st);
 // Footprints (the reference's) and records of the legacy interface; with row_tot (gy + 1 zeroed
 // entries) also the key counts launch_tile_binning_emit takes, for rectangles without `foot`.
 void launch_legacy_preprocess(int P, float n_std, const float* means, const float* scales,
@@ -83,34 +84,36 @@ uint64_t* launch_sort(uint64_t* a, uint64_t* b, int key_bits, const Control* ctr
 // turned into row offsets and view bases in place (row_tot is consumed). With `order`
 // (kTileLists runs of n_tiles uint4 entries, 16-byte aligned; ctrl's class counts zeroed)
 // every tile is also appended to the list of its work class (tile_class of its key count) as
-// (x | y << 16 in its view, first key, end key, view), which launch_blend_fwd then serves heaviest class first
-// without reading the tile's range or view again. With `tile_ent` (n_tiles entries) every tile's
-// entry of the same form is written at the tile's index (ViewsArg::tile_ent).
+// (x | y << 16 in its view, first key, end key, view), which launch_blend_fwd then serves heaviest
+// class first without reading the tile's range or view again. With `tile_ent` (n_tiles entries)
+// every tile's entry of the same form is written at the tile's index (ViewsArg::tile_ent).
 constexpr int kMaxRowTiles = 1024;
 constexpr int kRowBaseViews = 32;  // above this many views the row bases are formed first
 void launch_tile_binning_emit(const ViewsArg& va, int n_views, int max_gy, int max_gx,
                               const TileRect* rects, const FootRows* foot, const uint32_t* spans,
                               int tile_w, int tile_h, unsigned long long* row_tot,
-                              int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order,
-                              int64_t n_tiles, cudaStream_t st);
+                              int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent,
+                              uint64_t* keys, uint32_t* order, int64_t n_tiles, cudaStream_t st);
 // The same keys, ranges, views and lists for many Gaussians, the records taken in segments
-// (row_segments of the largest view's count) by a block each. launch_preprocess runs without row_tot;
-// row_tot (n_views * (max_gy + 1)) and ctrl are zeroed beforehand; counts: seg_count_words words.
+// (row_segments of the largest view's count) by a block each. launch_preprocess runs without
+// row_tot; row_tot (n_views * (max_gy + 1)) and ctrl are zeroed beforehand; counts: seg_count_words
+// words.
 int row_segments(int n);
 int64_t seg_count_words(int64_t n_tiles, int segs);
-void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs, const TileRect* rects,
-                        const FootRows* foot, const uint32_t* spans, int tile_w, int tile_h,
-                        unsigned long long* row_tot, uint32_t* counts, int64_t capacity,
-                        Control* ctrl, uint2* ranges, uint4* tile_ent, uint64_t* keys, uint32_t* order, int64_t n_tiles,
-                        cudaStream_t st);
+void launch_seg_binning(const ViewsArg& va, int n_views, int max_gy, int segs,
+                        const TileRect* rects, const FootRows* foot, const uint32_t* spans,
+                        int tile_w, int tile_h, unsigned long long* row_tot, uint32_t* counts,
+                        int64_t capacity, Control* ctrl, uint2* ranges, uint4* tile_ent,
+                        uint64_t* keys, uint32_t* order, int64_t n_tiles, cudaStream_t st);
 // Tile ranges of the sorted keys (ranges zeroed beforehand; empty tiles keep {0,0}).
 void launch_ranges(const uint64_t* keys, const Control* ctrl, int64_t capacity, uint2* ranges,
                    cudaStream_t st);
 
 // blend_fwd.cu
 // px: pixels per thread (1, 2 or 4; 0 = default for the tile shape); chunk: record pairs per
-// shared-memory stage (8, 16 or 32; 0 = 32). The blend builds each key's tile record itself from
-// the sorted keys and the Gaussian records (no gathered record stream). Persistent:
+// shared-memory stage (8, 16 or 32; 0: 16 for one-warp CTAs, else 32, from kManyTiles tiles on with
+// 24 warps per SM; see launch_chunk). The blend builds each key's tile record itself from the
+// sorted keys and the Gaussian records (no gathered record stream). Persistent:
 // ctrl->next_tile must be zero. `order`: the tile-major binning's per-class tile lists (heaviest
 // tiles are then taken first) or NULL (tiles in index order).
 // pieces (blend_pieces; 1: whole tiles): the most pieces a tile's keys are cut into, with `part`
@@ -140,10 +143,10 @@ void launch_blend_fwd_band(const ViewsArg& va, int tile_w, int tile_h, int px, i
 // the cotangents (NULL = zero) when the tile is staged.
 // `order`: as launch_blend_fwd.
 void launch_blend_bwd(const ViewsArg& va, int tile_w, int tile_h, int64_t n_tiles,
-                      const uint32_t* order, const uint64_t* keys, const uint2* ranges, const GaussRec* recs,
-                      const float* depth, const float* stats, int64_t stats_stride,
-                      const float* grad_depth, const float* grad_alpha, float beta2, float beta3,
-                      RecGrad* rgrad, Control* ctrl, cudaStream_t st);
+                      const uint32_t* order, const uint64_t* keys, const uint2* ranges,
+                      const GaussRec* recs, const float* depth, const float* stats,
+                      int64_t stats_stride, const float* grad_depth, const float* grad_alpha,
+                      float beta2, float beta3, RecGrad* rgrad, Control* ctrl, cudaStream_t st);
 // Zeroes the gradients (n_gauss Gaussians), the record gradients and the blend's work counter.
 void launch_bwd_zero(float* gmeans, float* gprec, float* glogw, int64_t n_gauss, RecGrad* rgrad,
                      int64_t n_rec, Control* ctrl, cudaStream_t st);
@@ -190,8 +193,8 @@ void launch_transform_points_bwd(int64_t n, const float* points, const float* po
 // pixlist.cu
 // Pixel-list render (fm_render.py render_func_idx_quattrans[_flow], render_func_quat_cam);
 // scratch: pixlist_scratch_bytes(n, n_poses, ordered_rays); ordered_rays > 0 (at most n_rays, from
-// pixlist_ordered_rays) renders the rays bucketed by pose and cell, 0 in the order given. feats (n x nf, nf <= 16), flows, out_feats and
-// weights (n x n_rays) are optional (NULL).
+// pixlist_ordered_rays) renders the rays bucketed by pose and cell, 0 in the order given. feats (n
+// x nf, nf <= 16), flows, out_feats and weights (n x n_rays) are optional (NULL).
 // Ray model: rows of `stride` floats (x, y, c[, pose]); the camera ray is
 // ((x - shift_x) inv_f, (y - shift_y) aspect inv_f, c) of pose `pose` (stride 4) or pose 0.
 struct PixRayModel {

@@ -33,9 +33,9 @@ struct FeatSmem {
   uint32_t gid[kFeatChunk];
 };
 
-// Weights (times W) of a record pair at the thread's pixels: 2^(l - m), with MASK 0 behind the camera
-// and at pixels that take no weights (m infinite), whatever the logits are. The arithmetic of
-// blend_group (blend_fwd.cu).
+// Weights (times W) of a record pair at the thread's pixels: 2^(l - m), with MASK 0 behind the
+// camera and at pixels that take no weights (m infinite), whatever the logits are. The arithmetic
+// of blend_group (blend_fwd.cu).
 template <int PX, bool MASK>
 __device__ __forceinline__ void pair_weights(const TilePair& p, const f2_t (&DU)[PX], f2_t DV,
                                              f2_t DVSQ, f2_t B3, f2_t NB2, const float (&m)[PX],
@@ -203,8 +203,8 @@ void launch_tiles(const ViewsArg& va, int64_t n_tiles, const uint64_t* keys, con
   // against 347 us for 1280x720).
   constexpr int PX = 2;
   const int passes = (nf + FC - 1) / FC;
-  launch_chained(va.chain, features_kernel<TW, TH, PX, FC>, (unsigned)n_tiles, TW * TH / PX, st, va, keys,
-                 ranges, recs, stats, stride, -beta2 * kLog2e, beta3, feats, nf,
+  launch_chained(va.chain, features_kernel<TW, TH, PX, FC>, (unsigned)n_tiles, TW * TH / PX, st,
+                 va, keys, ranges, recs, stats, stride, -beta2 * kLog2e, beta3, feats, nf,
                  (nf + passes - 1) / passes, out);
 }
 

@@ -12,10 +12,10 @@
 // 1 - 3e-8 itself rounds to 1.0 in float32 (which would leave saturated pixels at log(0)).
 // The per-render sums accumulate in float64 and the derivatives are the float64 quotients, rounded.
 // GB300 computes and converts float64 at a sixty-fourth of the float32 rate: with a sum, a product
-// and four conversions per pixel a call on 16 renders of 640x480 (59 MB) took 82 us. One addition is
-// left of them; the conversion before it moves bits, and the quotient comes from float32 products
-// wherever those determine its rounding: 25.5 us. (Sums and quotients in two float32 took 23, with
-// 48 bits.) Bound by instruction issue: a logarithm and a division per pixel, about 80
+// and four conversions per pixel a call on 16 renders of 640x480 (59 MB) took 82 us. One addition
+// is left of them; the conversion before it moves bits, and the quotient comes from float32
+// products wherever those determine its rounding: 25.5 us. (Sums and quotients in two float32 took
+// 23, with 48 bits.) Bound by instruction issue: a logarithm and a division per pixel, about 80
 // instructions in all.
 #include <algorithm>
 

@@ -398,7 +398,8 @@ __global__ void __launch_bounds__(128) pixlist_direct_kernel(
       float4 b[kBatch];
 #pragma unroll
       for (int t = 0; t < kBatch; ++t)
-        b[t] = i0 + t < n ? pt.bound(i0 + t) : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+        b[t] = i0 + t < n ? pt.bound(i0 + t)
+                          : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
       unsigned hit = 0;
 #pragma unroll
       for (int t = 0; t < kBatch; ++t) hit |= in_bound(b[t], r.u, r.v) ? 1u << t : 0u;
@@ -673,9 +674,9 @@ constexpr int64_t kOrderRays = 4 * kFillWarps;
 
 // Few Gaussians, or a long list with few tests in all: every ray tests every Gaussian, since
 // bucketing costs more than it saves. Per call, with flow, directly / bucketed: 1.2 M rays in image
-// order, 20 Gaussians 56 / 75 us, 48 92 / 87, 100 154 / 106, 1000 782 / 192; 9 poses, in image order
-// (shuffled), 112 K rays of 100 Gaussians 40 / 43 (44 / 43), 42 K of 300 45 / 52 (65 / 55), 112 K of
-// 300 57 / 52 (105 / 57), 10 K of 1000 122 / 106 (164 / 105).
+// order, 20 Gaussians 56 / 75 us, 48 92 / 87, 100 154 / 106, 1000 782 / 192; 9 poses, in image
+// order (shuffled), 112 K rays of 100 Gaussians 40 / 43 (44 / 43), 42 K of 300 45 / 52 (65 / 55),
+// 112 K of 300 57 / 52 (105 / 57), 10 K of 1000 122 / 106 (164 / 105).
 bool direct_list(int n, int64_t n_rays, bool weights) {
   if (n <= 40 || weights) return true;
   return n_rays >= kOrderRays && n <= 450 && n_rays <= INT64_C(16000000) / n;

@@ -517,8 +517,8 @@ __global__ void __launch_bounds__(64) legacy_preprocess_kernel(
   if (threadIdx.x < 32) {
     uint32_t keys = 0;
     if (i < P) {
-      const RefFootprint f = reference_footprint(i, n_std, means, scales, rots, mats, W, H, tan_fovx,
-                                                 tan_fovy, focal_x, focal_y, gx, gy);
+      const RefFootprint f = reference_footprint(i, n_std, means, scales, rots, mats, W, H,
+                                                 tan_fovx, tan_fovy, focal_x, focal_y, gx, gy);
       rects[i] = f.rect;
       touched[i] = keys = f.area;
       if (row_tot && f.area)
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(64) legacy_preprocess_kernel(
 void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, const float* prec,
                        const float* logw, const float* quat, const float* trans, int cull_mode,
                        float cull_param, int tile_w, int tile_h, GaussRec* recs, TileRect* rects,
-                       FootRows* foot, uint32_t* spans, uint32_t* touched, unsigned long long* row_tot, int max_gy,
-                       Control* ctrl, cudaStream_t st) {
+                       FootRows* foot, uint32_t* spans, uint32_t* touched,
+                       unsigned long long* row_tot, int max_gy, Control* ctrl, cudaStream_t st) {
   const int threads = kPrepThreads;
   // (launched without records too: the binning's first kernel is chained to it)
   const int64_t want = std::max<int64_t>(1, (n_rec + threads - 1) / threads);
@@ -558,8 +558,9 @@ void launch_preprocess(const ViewsArg& va, int64_t n_rec, const float* means, co
 
 void launch_preprocess_reference(int P, float n_std, const float* means, const float* scales,
                                  const float* rots, const LegacyMatrices& mats, int W, int H,
-                                 float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii, float* means2d,
-                                 TileRect* rects, uint32_t* touched, cudaStream_t st) {
+                                 float tan_fovx, float tan_fovy, int gx, int gy, int32_t* radii,
+                                 float* means2d, TileRect* rects, uint32_t* touched,
+                                 cudaStream_t st) {
   if (P <= 0) return;
   // rasterizer_impl.cu:205-206 (float arithmetic on the host).
   const float fx = (float)W / (2.0f * tan_fovx);

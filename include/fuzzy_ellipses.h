@@ -60,7 +60,9 @@ typedef enum fe_cull_mode {
 
 /* Flags for fe_render_desc.flags */
 #define FE_FLAG_SAVE_STATS 1u /* write per-pixel softmax statistics needed by the backward */
-/* Bits 8..15 of flags: record pairs per shared-memory stage of the blend (8, 16 or 32; 0 = 32). */
+/* Bits 8..15 of flags: record pairs per shared-memory stage of the blend (8, 16 or 32). 0: as fits
+ * the launch -- 16 for 8x8 tiles of two pixels per thread, 32 elsewhere, with more resident blocks
+ * on launches of many tiles. */
 #define FE_FLAG_CHUNK(pairs) (((uint32_t)(pairs) & 0xffu) << 8)
 /* Batches only: size the key scratch from the device-side key count (one 8-byte readback and a
  * stream synchronisation per run) instead of the worst case (views x Gaussians x tiles). */
@@ -226,7 +228,7 @@ int fe_rasterize_legacy(const fe_legacy_desc *desc, const float *d_means, const 
                         float *d_out_alpha, fe_stream_t stream);
 /* fe_rasterize_legacy with the view and projection matrices in host memory, read during the call
  * and passed to the kernels by value. clean != 0: the outputs as the reference's wrapper returns
- * them (fuzzy_ellipses/__init__.py:233-234): NaN and -inf become 0, +inf depth 10 and +inf alpha 1. */
+ * them (fuzzy_ellipses/__init__.py:233-234): NaN and -inf become 0, +inf depth 10, +inf alpha 1. */
 int fe_rasterize_legacy_host(const fe_legacy_desc *desc, const float *d_means,
                              const float *d_weights, const float *d_scales,
                              const float *d_rotations, const float *d_camera_rays,
